@@ -261,3 +261,31 @@ def tolerance(case):
     if case["kind"] == "train":
         return {"rel": 5e-6, "max": 1e-2} if fp32 else {"rel": 1.5e-3, "max": 0.22}
     return {"rel": 5e-5, "max": 5e-4}
+
+
+# ---- the same numbers in 64 bits, from plain torch --------------------------------------------------------------
+
+def exact(case, seed):
+    """What run() returns, in 64 bits; None for training and sampling, whose weights the library itself draws."""
+    if case["kind"] not in ("gemm", "bgemm", "flash"):
+        return None
+    s = prepare(case, seed)
+    if case["kind"] == "gemm":
+        A, B = s["A"].double(), s["B"].double()
+        return (A.T if case["ta"] else A) @ (B.T if case["tb"] else B) + case["beta"] * s["C"].double()
+    if case["kind"] == "bgemm":
+        scores = s["q"].double() @ s["k"].double().transpose(1, 2) / math.sqrt(case["hs"])
+        return scores, s["p"].double() @ s["v"].double()
+    B, T, NH, hs = case["B"], case["T"], case["NH"], case["hs"]
+    heads = lambda x: x.reshape(B, T, NH, hs).transpose(1, 2)                           # noqa: E731
+    rows = lambda x: x.transpose(1, 2).reshape(B, T, NH * hs)                           # noqa: E731
+    q, k, v = (heads(x) for x in s["qkv"].double().chunk(3, dim=-1))
+    dout = heads(s["dout"].double())
+    scores = q @ k.transpose(2, 3) / math.sqrt(hs)
+    scores.masked_fill_(torch.ones(T, T, dtype=torch.bool, device="cuda").triu(1), -math.inf)
+    lse = torch.logsumexp(scores, dim=-1)
+    p = torch.exp(scores - lse[..., None])
+    out = p @ v
+    dp = dout @ v.transpose(2, 3)
+    ds = p * (dp - (dout * out).sum(-1, keepdim=True)) / math.sqrt(hs)
+    return rows(out), lse, torch.cat([rows(ds @ k), rows(ds.transpose(2, 3) @ q), rows(p.transpose(2, 3) @ dout)], dim=-1)
