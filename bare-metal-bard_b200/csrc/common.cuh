@@ -97,6 +97,10 @@ long long launches_total();
 
 inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 
+// Internal flag of gemm_any_bias: the launches of a captured stream may use the per-device scratch, because the caller
+// has sized it by an eager pass, keeps its products in one line and watches scratch_generation().  Without it, products
+// that need scratch stay out of captures.
+constexpr int GEMM_SCRATCH_IN_CAPTURE = 1 << 20;
 // Internal GEMM dispatch shared by attention and the trainer: math is a
 // BMB_MATH_* value, flags the BMB_GEMM_* bits, strides in elements.
 int gemm_any(int math, int flags, int ta, int tb, int batch, int M, int N, int K, float alpha,

@@ -181,6 +181,7 @@ int collect_profile(bmb_trainer *t) {
 // One matmul of the model, optionally bracketed by events.
 int mm(bmb_trainer *t, int flags, int ta, int tb, int M, int N, int K, const float *A, const float *B,
        float beta, float *C, const float *bias = nullptr, cudaStream_t on = nullptr, float *aux_gelu = nullptr) {
+    flags |= GEMM_SCRATCH_IN_CAPTURE;
     if (on) return gemm_any_bias(t->c.math, flags, ta, tb, 1, M, N, K, 1.0f, A, 0, B, 0, beta, C, 0, bias, on, aux_gelu);
     if (t->prof) {
         if (t->ev_used + 2 > t->ev.size()) {
@@ -555,7 +556,11 @@ int run_piece(bmb_trainer *t, bmb_trainer::Piece &pc, bool eager) {
         pc.launches = launches_total() - before;
         count_launch((int)-pc.launches);        // counted again at every replay, this first one included
     }
+    // the replayed fp32 products use the scratch that they were captured with: in turn with other streams' products
+    const bool uses_scratch = t->c.math == BMB_MATH_FP32;
+    if (uses_scratch) BMB_TRY(scratch_acquire(SCR_GEMM_A, t->st));
     BMB_CUDA(cudaGraphLaunch(pc.exec, t->st));
+    if (uses_scratch) BMB_TRY(scratch_release(SCR_GEMM_A, t->st));
     count_launch((int)pc.launches);
     return BMB_OK;
 }

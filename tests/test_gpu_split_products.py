@@ -1,0 +1,77 @@
+"""fp32 products and attention on the tensor cores, every fp32 operand in pieces (csrc/gemm_x3.cu), at the sizes where
+the split can go wrong: edges of tiles and slices, K shared among CTAs, infinities and NaN, a stream being captured."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+GEMMS = [  # M, N, K, ta, tb, beta
+    (512, 512, 192, 0, 1, 0.0),      # the smallest that the rule takes
+    (515, 511, 193, 0, 0, 0.5),      # nothing aligned, one K past a slice
+    (515, 511, 1025, 1, 1, 0.0),
+    (1000, 514, 2047, 1, 0, 1.0),    # K shared among CTAs, even N off 16 bytes
+    (33, 8191, 999, 0, 1, 0.0),      # one ragged row tile
+    (4100, 68, 1000, 1, 0, 0.0),     # one narrow column tile
+    (3000, 3001, 64, 0, 0, -1.0),
+    (2048, 1536, 512, 0, 1, 0.0),
+]
+
+
+@pytest.mark.parametrize("M,N,K,ta,tb,beta", GEMMS)
+def test_split_product_against_64_bits(bmb, cuda, M, N, K, ta, tb, beta):
+    """The pieces leave out 2^-26 of each product, a slice's sum in tensor memory is cut off twice at full size (2^-24
+    each) and every 32 K one rounding is added: below 4 * 2^-24 = 2.4e-7 of the result in the 2-norm up to K = 2048, and
+    below the SIMT kernel's own error."""
+    g = cuda.Generator(device="cuda").manual_seed(M + N + K)
+    rnd = lambda *s: cuda.rand(s, generator=g, device="cuda") * 2 - 1      # noqa: E731
+    A, B, C0 = rnd(*((K, M) if ta else (M, K))), rnd(*((N, K) if tb else (K, N))), rnd(M, N)
+    a, b = (A.T if ta else A), (B.T if tb else B)
+    want = 0.75 * (a.double() @ b.double()) + beta * C0.double()
+    C = C0.clone() if beta else cuda.full((M, N), float("nan"), device="cuda")
+    bmb.call("bmb_gemm_ex", bmb.MATH_FP32, 0, ta, tb, M, N, K, 0.75, A, B, beta, C, None)
+    simt = C0.clone()
+    bmb.call("bmb_sgemm_simt", M, N, K, 0.75, a.contiguous(), b.contiguous(), beta, simt)
+    cuda.cuda.synchronize()
+    err = lambda x: float((x.double() - want).norm() / want.norm())        # noqa: E731
+    assert not cuda.equal(C, simt)                                         # it was the split product that ran
+    assert err(C) < 2.4e-7 and err(C) < err(simt), (err(C), err(simt))
+    again = C0.clone()
+    bmb.call("bmb_gemm_ex", bmb.MATH_FP32, 0, ta, tb, M, N, K, 0.75, A, B, beta, again, None)
+    cuda.cuda.synchronize()
+    assert cuda.equal(C, again)
+
+
+@pytest.mark.parametrize("M,N,K", [(515, 511, 1025), (2048, 1536, 512)])       # parts of K added by a pass, and whole tiles
+def test_split_product_of_infinities_and_nan(bmb, cuda, M, N, K):
+    """Where an element is not finite in the sequential chain it is the same here, and operands at the end of the range
+    (where the first piece would round to infinity) still give finite results."""
+    g = cuda.Generator(device="cuda").manual_seed(5)
+    A, B = (cuda.rand(s, generator=g, device="cuda") * 2 - 1 for s in ((M, K), (K, N)))
+    A[3, 5], A[7, 0], A[9, 1], A[9, 2], A[M - 1, K - 1] = float("inf"), float("-inf"), float("inf"), float("-inf"), float("nan")
+    B[5, 11], B[K - 1, N - 1], B[5, 12] = float("-inf"), float("inf"), 0.0
+    A[20], B[:, 20] = 0.0, 0.0
+    A[20, 4], B[4, 21] = 3.4028234e38, 0.5
+    C, simt = cuda.empty(M, N, device="cuda"), cuda.empty(M, N, device="cuda")
+    bmb.call("bmb_gemm_ex", bmb.MATH_FP32, 0, 0, 0, M, N, K, 1.0, A, B, 0.0, C, None)
+    bmb.call("bmb_sgemm_simt", M, N, K, 1.0, A, B, 0.0, simt)
+    cuda.cuda.synchronize()
+    c, s = C.cpu().numpy(), simt.cpu().numpy()
+    assert np.isnan(s).any() and np.isinf(s).any()
+    assert np.array_equal(np.isnan(c), np.isnan(s)) and np.array_equal(np.isinf(c), np.isinf(s))
+    assert np.array_equal(c[np.isinf(s)], s[np.isinf(s)])
+    assert abs(c[20, 21] / 1.7014117e38 - 1) < 1e-6
+
+
+def test_split_product_stays_out_of_a_capture(bmb, cuda):
+    """A caller's captured products take no scratch (its address would be kept, and branches of the graph would share it)."""
+    n = 1024
+    A, B = cuda.rand(n, n, device="cuda"), cuda.rand(n, n, device="cuda")
+    C, want = cuda.zeros(n, n, device="cuda"), cuda.zeros(n, n, device="cuda")
+    bmb.call("bmb_sgemm_simt", n, n, n, 1.0, A, B, 0.0, want)
+    cuda.cuda.synchronize()
+    graph = cuda.cuda.CUDAGraph()
+    with cuda.cuda.graph(graph):
+        bmb.call("bmb_gemm_ex", bmb.MATH_FP32, 0, 0, 0, n, n, n, 1.0, A, B, 0.0, C, cuda.cuda.current_stream().cuda_stream)
+    graph.replay()
+    cuda.cuda.synchronize()
+    assert cuda.equal(C, want)
