@@ -8,18 +8,21 @@
 // dK/dV (reduced over queries) each stay in registers and are written with
 // plain stores -- dqkv is overwritten, not accumulated.
 //
-// Thread mapping ("row group"): a query row (or, in the dK/dV kernel, a key
-// row) belongs to G = HS/32 adjacent lanes, each holding a 32-float slice of
-// the head dimension in registers.  Key/value (or query/dO) rows are staged
-// in shared memory and read as warp-wide broadcasts; dot products finish with
-// log2(G) shuffles.  Scores are processed KC keys at a time so that the
-// running max is rescaled once per chunk, not once per key.
+// The kernels in use run on warp-level tensor-core instructions, every fp32 product as three TF32 ones
+// (flash_mma.cuh).  Behind them stand the row-group kernels (configuration 1): a query row (or, for dK/dV, a key
+// row) belongs to G = HS/32 adjacent lanes, each holding a 32-float slice of the head dimension in registers; key /
+// value (or query / dO) rows are staged in shared memory and read as warp-wide broadcasts; dot products finish with
+// log2(G) shuffles.  A block whose result is not finite everywhere is computed again by them: split products of
+// infinite operands give NaN where the fp32 chain gives an infinity, or a probability of zero.
 // q, k and v are read straight out of the fused (B,T,3C) projection.
-#include "common.cuh"
+#include "flash_mma.cuh"
 #include <cfloat>
 #include <cmath>
+#include <map>
+#include <mutex>
 
 namespace bmb {
+int launch_flash_dsum(float *dsum, const float *dout, const float *out, int B, int T, int NH, int HS, cudaStream_t st);
 bool flash_tc_supported(int T, int C, int NH, const float *qkv, const float *out);
 int flash_forward_tc(float *out, float *lse, const float *qkv, int B, int T, int C, int NH, bool qkv_rounded,
                      cudaStream_t st);
@@ -43,11 +46,11 @@ __device__ __forceinline__ float group_sum(float v) {
 
 // Copy TILE rows of HS floats (row r at src + r*ld) into dense smem [TILE][HS];
 // rows at or beyond `valid` are zero filled.
-template <int HS, int TILE>
+template <int HS, int TILE, int NT>
 __device__ __forceinline__ void stage_rows(float *__restrict__ dst, const float *__restrict__ src,
                                            long long ld, int valid, int tid) {
     constexpr int V4 = HS / 4;
-    for (int lin = tid; lin < TILE * V4; lin += FT) {
+    for (int lin = tid; lin < TILE * V4; lin += NT) {
         const int r = lin / V4, c = (lin % V4) * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (r < valid) v = LD4(src + (long long)r * ld + c);
@@ -56,24 +59,22 @@ __device__ __forceinline__ void stage_rows(float *__restrict__ dst, const float 
 }
 
 // ------------------------------------------------------------------ forward
-template <int HS, int KC>
-__global__ void __launch_bounds__(FT)
-flash_fwd_simt_k(float *__restrict__ out, float *__restrict__ lse, const float *__restrict__ qkv,
-                 int T, int NH, float scale) {
-    constexpr int G = HS / 32, R = FT / G, TILE = tile_rows<HS>::value;
-    __shared__ __align__(16) float Ks[TILE * HS];
-    __shared__ __align__(16) float Vs[TILE * HS];
-
+// Rows [i0, min(i0 + nrows, T)) of one head, by NT threads (NT / G rows at a time).  smem: 2 * tile_rows * HS floats.
+template <int HS, int KC, int NT>
+__device__ __forceinline__ void fwd_rows(float *__restrict__ smem, float *__restrict__ out, float *__restrict__ lse,
+                                         const float *__restrict__ qkv, int T, int NH, float scale, int bh, int i0, int nrows) {
+    constexpr int G = HS / 32, TILE = tile_rows<HS>::value;
+    float *Ks = smem, *Vs = smem + TILE * HS;
     const int tid = threadIdx.x, sub = tid % G;
-    const int bh = blockIdx.y, b = bh / NH, h = bh % NH;
+    const int b = bh / NH, h = bh % NH;
     const int C = NH * HS;
-    const int i0 = blockIdx.x * R;
+    const int end = min(i0 + nrows, T);           // rows from here on are not ours
     const int row = i0 + tid / G;                 // this thread's query
     const long long ld = 3LL * C;
     const float *base = qkv + (long long)b * T * ld + h * HS;
 
     float q[32], o[32];
-    if (row < T) {
+    if (row < end) {
 #pragma unroll
         for (int d = 0; d < 32; d += 4) {
             const float4 v = LD4(base + (long long)row * ld + sub * 32 + d);
@@ -88,13 +89,12 @@ flash_fwd_simt_k(float *__restrict__ out, float *__restrict__ lse, const float *
     float m = -INFINITY, l = 0.0f;
 
     // Last query row any lane of this warp owns: chunks past it are skipped.
-    const int warp_last = min(T - 1, i0 + ((tid | 31) / G));
-    const int jmax = min(T, i0 + R);
+    const int warp_last = min(end - 1, i0 + ((tid | 31) / G));
 
-    for (int j0 = 0; j0 < jmax; j0 += TILE) {
+    for (int j0 = 0; j0 < end; j0 += TILE) {
         __syncthreads();
-        stage_rows<HS, TILE>(Ks, base + (long long)j0 * ld + C, ld, T - j0, tid);
-        stage_rows<HS, TILE>(Vs, base + (long long)j0 * ld + 2 * C, ld, T - j0, tid);
+        stage_rows<HS, TILE, NT>(Ks, base + (long long)j0 * ld + C, ld, T - j0, tid);
+        stage_rows<HS, TILE, NT>(Vs, base + (long long)j0 * ld + 2 * C, ld, T - j0, tid);
         __syncthreads();
 
         for (int c0 = 0; c0 < TILE; c0 += KC) {
@@ -143,7 +143,7 @@ flash_fwd_simt_k(float *__restrict__ out, float *__restrict__ lse, const float *
         }
     }
 
-    if (row < T) {
+    if (row < end) {
         const float inv = (l > 0.0f) ? 1.0f / l : 0.0f;
         float *dst = out + ((long long)b * T + row) * C + h * HS + sub * 32;
 #pragma unroll
@@ -153,157 +153,119 @@ flash_fwd_simt_k(float *__restrict__ out, float *__restrict__ lse, const float *
     }
 }
 
-// Forward, register-tiled ("rows4"): a thread owns RQ = 4 consecutive query rows x 16 of the head's columns, a row
-// group is HS/16 adjacent lanes.  Every 16-float slice of a K or V row read from shared memory now feeds 4 rows'
-// products (64 multiply-adds per 4 128-bit loads instead of 16), and the products are issued as two-wide
-// fma.rn.f32x2 (each half an IEEE fma); scores finish with log2(HS/16) shuffles.  Measured at B8 H12 T1024 hs64:
-// 0.90 ms against 0.94 ms for the kernel above -- both sit at a fifth of the multiply-add peak, held there by
-// dependent-issue and shared-memory-load latency at 8 warps per SM (213 registers per thread), not by any pipe.
-// The same tiling of the two backward kernels (2 rows x 16 columns) measured 4 % slower than theirs and was dropped.
-__device__ __forceinline__ unsigned long long f2pack(float lo, float hi) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void f2unpack(unsigned long long v, float &lo, float &hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ void f2fma(unsigned long long &d, unsigned long long a, unsigned long long b) {
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
-}
-
 template <int HS, int KC>
 __global__ void __launch_bounds__(FT)
-flash_fwd_rows4_k(float *__restrict__ out, float *__restrict__ lse, const float *__restrict__ qkv,
-                  int T, int NH, float scale) {
-    constexpr int GL = HS / 16, RQ = 4, ROWS = FT / GL * RQ, TILE = tile_rows<HS>::value;
-    __shared__ __align__(16) float Ks[TILE * HS];
-    __shared__ __align__(16) float Vs[TILE * HS];
+flash_fwd_simt_k(float *__restrict__ out, float *__restrict__ lse, const float *__restrict__ qkv,
+                 int T, int NH, float scale) {
+    __shared__ __align__(16) float smem[2 * tile_rows<HS>::value * HS];
+    constexpr int R = FT / (HS / 32);
+    fwd_rows<HS, KC, FT>(smem, out, lse, qkv, T, NH, scale, blockIdx.y, blockIdx.x * R, R);
+}
 
-    const int tid = threadIdx.x, sub = tid % GL;
-    const int bh = blockIdx.y, b = bh / NH, h = bh % NH;
+// Rows [i0, i0 + nrows) again by the row-group code, inside a kernel that found its own result not finite.
+template <int HS, int NT>
+__device__ __noinline__ void fwd_rows_again(float *smem, float *out, float *lse, const float *qkv, int T, int NH, float scale,
+                                            int bh, int i0, int nrows) {
+    constexpr int R = NT / (HS / 32);
+    for (int r = 0; r < nrows; r += R) fwd_rows<HS, 16, NT>(smem, out, lse, qkv, T, NH, scale, bh, i0 + r, min(R, nrows - r));
+}
+
+// Forward on warp-level tensor-core instructions.  A block owns 64 queries of one head, a warp 16 of them; keys come 32
+// at a time, two buffers, the next 32 copied while these are multiplied.  Scores, probabilities and output stay in
+// registers; the running maximum moves once per 32 keys.  Bound by the tensor pipe: 3 instructions of 8 cycles for 8
+// keys x 8 columns x 16 rows in either product, beside which the splits take about half of the issue slots.
+// (the tensor pipe is about half busy: two to three warps a scheduler do not cover the latency of splits and products.)
+// Measured, the kernel before (4 rows x 16 columns a thread on the FMA pipe) -> this: B8 T1024 12 heads of 64 936 -> 274 us,
+// B4 T2048 8 x 128 3608 -> 702, B2 T777 12 x 32 191 -> 46, B1 T64 2 x 32 18.9 -> 7.3.  2-norm errors against 64 bits there:
+// 2.7e-7 -> 1.8e-7, 3.5e-7 -> 2.1e-7, 2.5e-7 -> 1.9e-7, 1.1e-7 -> 1.3e-7.
+template <int HS>
+__global__ void __launch_bounds__(128, HS == 128 ? 2 : HS == 64 ? 3 : 4)
+flash_fwd_mma_k(float *__restrict__ out, float *__restrict__ lse, const float *__restrict__ qkv, int T, int NH, float scale) {
+    extern __shared__ __align__(16) float smem[];
+    float *Qs = smem, *Ks = Qs + 64 * HS, *Vs = Ks + 2 * 32 * HS;      // Ks, Vs: two buffers each
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int bh = blockIdx.x, b = bh / NH, h = bh % NH;
     const int C = NH * HS;
-    const int i0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * ROWS;      // longest blocks first
-    const int row0 = i0 + (tid / GL) * RQ;        // this thread's first query
+    const int i0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * 64;        // longest blocks first
     const long long ld = 3LL * C;
     const float *base = qkv + (long long)b * T * ld + h * HS;
 
-    // q and o as pairs of neighbouring columns: q2[r][i] = columns 2i, 2i+1 of this thread's slice
-    unsigned long long q2[RQ][8], o2[RQ][8];
-#pragma unroll
-    for (int r = 0; r < RQ; ++r) {
-#pragma unroll
-        for (int i = 0; i < 8; i += 2) {
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (row0 + r < T) v = LD4(base + (long long)(row0 + r) * ld + sub * 16 + 2 * i);
-            q2[r][i] = f2pack(v.x * scale, v.y * scale);
-            q2[r][i + 1] = f2pack(v.z * scale, v.w * scale);
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) o2[r][i] = 0ull;
-    }
-    float m[RQ], l[RQ];
-#pragma unroll
-    for (int r = 0; r < RQ; ++r) { m[r] = -INFINITY; l[r] = 0.0f; }
+    auto copy_keys = [&](int j0, int buf) {
+        fm::tile_copy<HS, 32, 128>(Ks + buf * 32 * HS, base + (long long)j0 * ld + C, ld, T - j0);
+        fm::tile_copy<HS, 32, 128>(Vs + buf * 32 * HS, base + (long long)j0 * ld + 2 * C, ld, T - j0);
+        fm::cp_commit();
+    };
+    fm::tile_copy<HS, 64, 128>(Qs, base + (long long)i0 * ld, ld, T - i0);
+    copy_keys(0, 0);
 
-    // Last query row any lane of this warp owns: chunks past it are skipped.
-    const int warp_last = min(T - 1, i0 + ((tid | 31) / GL) * RQ + RQ - 1);
-    const int jmax = min(T, i0 + ROWS);
+    float o[HS / 8][4];
+#pragma unroll
+    for (int c = 0; c < HS / 8; ++c)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o[c][i] = 0.0f;
+    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f};
+    const int row0 = i0 + warp * 16, jmax = min(T, i0 + 64);
 
-    for (int j0 = 0; j0 < jmax; j0 += TILE) {
-        __syncthreads();
-        stage_rows<HS, TILE>(Ks, base + (long long)j0 * ld + C, ld, T - j0, tid);
-        stage_rows<HS, TILE>(Vs, base + (long long)j0 * ld + 2 * C, ld, T - j0, tid);
-        __syncthreads();
-
-        for (int c0 = 0; c0 < TILE; c0 += KC) {
-            if (j0 + c0 > warp_last) break;       // warp-uniform
-            float s[RQ][KC];
+    int buf = 0;
+    for (int j0 = 0; j0 < jmax; j0 += 32, buf ^= 1) {
+        fm::cp_wait_all();
+        __syncthreads();               // everyone's part of these 32 keys is here, and the other buffer has been read
+        if (j0 + 32 < jmax) copy_keys(j0 + 32, buf ^ 1);
+        if (j0 > row0 + 15) continue;  // (per warp) all of these keys lie after all of its queries
+        float s[4][4];
+        fm::scores<HS, 2>(s, Qs, warp * 16, Ks + buf * 32 * HS, 0);
+        const bool edge = j0 + 31 > row0 || j0 + 32 > T;               // some pair is masked
 #pragma unroll
-            for (int c = 0; c < KC; ++c) {
-                const float *kr = Ks + (c0 + c) * HS + sub * 16;
-                unsigned long long k2[8];
+        for (int j = 0; j < 4; ++j)
 #pragma unroll
-                for (int i = 0; i < 8; i += 2) {
-                    const float4 kv = LD4(kr + 2 * i);
-                    k2[i] = f2pack(kv.x, kv.y);
-                    k2[i + 1] = f2pack(kv.z, kv.w);
-                }
-#pragma unroll
-                for (int r = 0; r < RQ; ++r) {
-                    unsigned long long acc = 0ull;
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) f2fma(acc, q2[r][i], k2[i]);
-                    float lo, hi;
-                    f2unpack(acc, lo, hi);
-                    s[r][c] = lo + hi;
+            for (int i = 0; i < 4; ++i) {
+                s[j][i] *= scale;
+                if (edge) {
+                    const int key = j0 + 8 * j + 2 * t + (i & 1), row = row0 + g + 8 * (i >> 1);
+                    if (key > row || key >= T) s[j][i] = -INFINITY;
                 }
             }
+        float resc[2];
 #pragma unroll
-            for (int r = 0; r < RQ; ++r) {
-                const int row = row0 + r;
-                float cmax = -INFINITY;
+        for (int r = 0; r < 2; ++r) {
+            float cmax = s[0][2 * r];
 #pragma unroll
-                for (int c = 0; c < KC; ++c) {
-                    const float a = group_sum<GL>(s[r][c]);
-                    const int kg = j0 + c0 + c;
-                    s[r][c] = (kg > row || kg >= T) ? -INFINITY : a;
-                    cmax = fmaxf(cmax, s[r][c]);
+            for (int j = 0; j < 4; ++j) cmax = fmaxf(cmax, fmaxf(s[j][2 * r], s[j][2 * r + 1]));
+            cmax = fmaxf(cmax, __shfl_xor_sync(0xffffffffu, cmax, 1));
+            cmax = fmaxf(cmax, __shfl_xor_sync(0xffffffffu, cmax, 2));
+            const float mnew = fmaxf(m[r], cmax);
+            const bool seen = mnew > -INFINITY;
+            resc[r] = seen ? __expf(m[r] - mnew) : 1.0f;
+            float csum = 0.0f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int i = 2 * r; i < 2 * r + 2; ++i) {
+                    s[j][i] = seen ? __expf(s[j][i] - mnew) : 0.0f;
+                    csum += s[j][i];
                 }
-                const float mnew = fmaxf(m[r], cmax);
-                const bool live = mnew > -INFINITY;
-                const float resc = live ? __expf(m[r] - mnew) : 1.0f;
-                float csum = 0.0f;
-#pragma unroll
-                for (int c = 0; c < KC; ++c) {
-                    s[r][c] = live ? __expf(s[r][c] - mnew) : 0.0f;
-                    csum += s[r][c];
-                }
-                m[r] = mnew;
-                l[r] = l[r] * resc + csum;
-                const unsigned long long resc2 = f2pack(resc, resc);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    unsigned long long z = 0ull;
-                    f2fma(z, o2[r][i], resc2);                  // o * resc + 0
-                    o2[r][i] = z;
-                }
-            }
-#pragma unroll
-            for (int c = 0; c < KC; ++c) {
-                const float *vr = Vs + (c0 + c) * HS + sub * 16;
-                unsigned long long v2[8];
-#pragma unroll
-                for (int i = 0; i < 8; i += 2) {
-                    const float4 vv = LD4(vr + 2 * i);
-                    v2[i] = f2pack(vv.x, vv.y);
-                    v2[i + 1] = f2pack(vv.z, vv.w);
-                }
-#pragma unroll
-                for (int r = 0; r < RQ; ++r) {
-                    const unsigned long long p2 = f2pack(s[r][c], s[r][c]);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) f2fma(o2[r][i], p2, v2[i]);
-                }
-            }
+            m[r] = mnew;
+            l[r] = l[r] * resc[r] + csum;             // this thread's keys; the row's four lanes are added at the end
         }
+        fm::contract<HS, 2, true>(o, resc[0], resc[1], s, Vs + buf * 32 * HS, 0);
     }
 
+    bool bad = false;
+    float inv[2];
 #pragma unroll
-    for (int r = 0; r < RQ; ++r) {
-        const int row = row0 + r;
-        if (row >= T) continue;
-        const float inv = (l[r] > 0.0f) ? 1.0f / l[r] : 0.0f;
-        float *dst = out + ((long long)b * T + row) * C + h * HS + sub * 16;
-#pragma unroll
-        for (int i = 0; i < 8; i += 2) {
-            float a0, a1, a2, a3;
-            f2unpack(o2[r][i], a0, a1);
-            f2unpack(o2[r][i + 1], a2, a3);
-            ST4(dst + 2 * i) = make_float4(a0 * inv, a1 * inv, a2 * inv, a3 * inv);
+    for (int r = 0; r < 2; ++r) {
+        l[r] += __shfl_xor_sync(0xffffffffu, l[r], 1);
+        l[r] += __shfl_xor_sync(0xffffffffu, l[r], 2);
+        inv[r] = (l[r] > 0.0f) ? 1.0f / l[r] : 0.0f;
+        const int row = row0 + g + 8 * r;
+        if (row < T) {
+            const float v = m[r] + __logf(l[r]);
+            if (t == 0) lse[(long long)bh * T + row] = v;
+            bad = bad || !(fabsf(v) <= 3.402823466e38f);
         }
-        if (sub == 0) lse[(long long)bh * T + row] = m[r] + __logf(l[r]);
     }
+    bad = fm::store_rows<HS>(out + ((long long)b * T + row0) * C + h * HS, C, g, T - row0, o, inv[0], inv[1]) || bad;
+    if (__syncthreads_or(bad)) fwd_rows_again<HS, 128>(smem, out, lse, qkv, T, NH, scale, bh, i0, 64);
 }
 
 // ----------------------------------------------------------------- backward
@@ -351,27 +313,24 @@ __global__ void __launch_bounds__(256) flash_dsum_vec_k(float *__restrict__ dsum
     }
 }
 
-// dQ: a row group owns a query row; keys stream through shared memory.
-template <int HS, int KC>
-__global__ void __launch_bounds__(FT)
-flash_bwd_q_simt_k(float *__restrict__ dqkv, const float *__restrict__ qkv,
-                   const float *__restrict__ dout, const float *__restrict__ lse,
-                   const float *__restrict__ dsum, int T, int NH, float scale) {
-    constexpr int G = HS / 32, R = FT / G, TILE = tile_rows<HS>::value;
-    __shared__ __align__(16) float Ks[TILE * HS];
-    __shared__ __align__(16) float Vs[TILE * HS];
-
+// dQ: a row group owns a query row; keys stream through shared memory.  Rows and threads as in fwd_rows.
+template <int HS, int KC, int NT>
+__device__ __forceinline__ void bwd_q_rows(float *__restrict__ smem, float *__restrict__ dqkv, const float *__restrict__ qkv,
+                                           const float *__restrict__ dout, const float *__restrict__ lse,
+                                           const float *__restrict__ dsum, int T, int NH, float scale, int bh, int i0, int nrows) {
+    constexpr int G = HS / 32, TILE = tile_rows<HS>::value;
+    float *Ks = smem, *Vs = smem + TILE * HS;
     const int tid = threadIdx.x, sub = tid % G;
-    const int bh = blockIdx.y, b = bh / NH, h = bh % NH;
+    const int b = bh / NH, h = bh % NH;
     const int C = NH * HS;
-    const int i0 = blockIdx.x * R;
+    const int end = min(i0 + nrows, T);
     const int row = i0 + tid / G;
     const long long ld = 3LL * C;
     const float *base = qkv + (long long)b * T * ld + h * HS;
 
     float q[32], go[32], dq[32];
     float lrow = 0.0f, drow = 0.0f;
-    if (row < T) {
+    if (row < end) {
         const float *dor = dout + ((long long)b * T + row) * C + h * HS + sub * 32;
 #pragma unroll
         for (int d = 0; d < 32; d += 4) {
@@ -389,12 +348,11 @@ flash_bwd_q_simt_k(float *__restrict__ dqkv, const float *__restrict__ qkv,
 #pragma unroll
     for (int d = 0; d < 32; ++d) dq[d] = 0.0f;
 
-    const int warp_last = min(T - 1, i0 + ((tid | 31) / G));
-    const int jmax = min(T, i0 + R);
-    for (int j0 = 0; j0 < jmax; j0 += TILE) {
+    const int warp_last = min(end - 1, i0 + ((tid | 31) / G));
+    for (int j0 = 0; j0 < end; j0 += TILE) {
         __syncthreads();
-        stage_rows<HS, TILE>(Ks, base + (long long)j0 * ld + C, ld, T - j0, tid);
-        stage_rows<HS, TILE>(Vs, base + (long long)j0 * ld + 2 * C, ld, T - j0, tid);
+        stage_rows<HS, TILE, NT>(Ks, base + (long long)j0 * ld + C, ld, T - j0, tid);
+        stage_rows<HS, TILE, NT>(Vs, base + (long long)j0 * ld + 2 * C, ld, T - j0, tid);
         __syncthreads();
         for (int c0 = 0; c0 < TILE; c0 += KC) {
             if (j0 + c0 > warp_last) break;
@@ -416,7 +374,7 @@ flash_bwd_q_simt_k(float *__restrict__ dqkv, const float *__restrict__ qkv,
                 s = group_sum<G>(s);
                 dp = group_sum<G>(dp);
                 const int kg = j0 + c0 + c;
-                const bool on = (kg <= row) && (kg < T) && (row < T);
+                const bool on = (kg <= row) && (kg < T) && (row < end);
                 const float p = on ? __expf(s - lrow) : 0.0f;
                 const float ds = p * (dp - drow);
 #pragma unroll
@@ -424,7 +382,7 @@ flash_bwd_q_simt_k(float *__restrict__ dqkv, const float *__restrict__ qkv,
             }
         }
     }
-    if (row < T) {
+    if (row < end) {
         float *dst = dqkv + ((long long)b * T + row) * ld + h * HS + sub * 32;
 #pragma unroll
         for (int d = 0; d < 32; d += 4)
@@ -432,29 +390,35 @@ flash_bwd_q_simt_k(float *__restrict__ dqkv, const float *__restrict__ qkv,
     }
 }
 
-// dK, dV: a row group owns a key row; queries at or after it stream through
-// shared memory together with dO, lse and D.
 template <int HS, int KC>
 __global__ void __launch_bounds__(FT)
-flash_bwd_kv_simt_k(float *__restrict__ dqkv, const float *__restrict__ qkv,
-                    const float *__restrict__ dout, const float *__restrict__ lse,
-                    const float *__restrict__ dsum, int T, int NH, float scale) {
-    constexpr int G = HS / 32, R = FT / G;
-    constexpr int QT = 32;   // queries staged per tile
-    __shared__ __align__(16) float Qs[QT * HS];
-    __shared__ __align__(16) float Os[QT * HS];
-    __shared__ float Ls[QT], Ds[QT];
+flash_bwd_q_simt_k(float *__restrict__ dqkv, const float *__restrict__ qkv,
+                   const float *__restrict__ dout, const float *__restrict__ lse,
+                   const float *__restrict__ dsum, int T, int NH, float scale) {
+    __shared__ __align__(16) float smem[2 * tile_rows<HS>::value * HS];
+    constexpr int R = FT / (HS / 32);
+    bwd_q_rows<HS, KC, FT>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, blockIdx.y, blockIdx.x * R, R);
+}
 
+// dK, dV: a row group owns a key row; queries at or after it stream through
+// shared memory together with dO, lse and D.  smem: 2 * QT * (HS + 1) floats.
+constexpr int QT = 32;   // queries staged per tile
+template <int HS, int KC, int NT>
+__device__ __forceinline__ void bwd_kv_rows(float *__restrict__ smem, float *__restrict__ dqkv, const float *__restrict__ qkv,
+                                            const float *__restrict__ dout, const float *__restrict__ lse,
+                                            const float *__restrict__ dsum, int T, int NH, float scale, int bh, int j0, int nrows) {
+    constexpr int G = HS / 32;
+    float *Qs = smem, *Os = Qs + QT * HS, *Ls = Os + QT * HS, *Ds = Ls + QT;
     const int tid = threadIdx.x, sub = tid % G;
-    const int bh = blockIdx.y, b = bh / NH, h = bh % NH;
+    const int b = bh / NH, h = bh % NH;
     const int C = NH * HS;
-    const int j0 = blockIdx.x * R;
+    const int end = min(j0 + nrows, T);
     const int key = j0 + tid / G;
     const long long ld = 3LL * C;
     const float *base = qkv + (long long)b * T * ld + h * HS;
 
     float k[32], v[32], dk[32], dv[32];
-    if (key < T) {
+    if (key < end) {
 #pragma unroll
         for (int d = 0; d < 32; d += 4) {
             const float4 a = LD4(base + (long long)key * ld + C + sub * 32 + d);
@@ -474,7 +438,7 @@ flash_bwd_kv_simt_k(float *__restrict__ dqkv, const float *__restrict__ qkv,
     constexpr int V4 = HS / 4;
     for (int i0 = (j0 / QT) * QT; i0 < T; i0 += QT) {
         __syncthreads();
-        for (int lin = tid; lin < QT * V4; lin += FT) {
+        for (int lin = tid; lin < QT * V4; lin += NT) {
             const int r = lin / V4, c = (lin % V4) * 4;
             float4 qv = make_float4(0.f, 0.f, 0.f, 0.f), gv = qv;
             if (i0 + r < T) {
@@ -510,7 +474,7 @@ flash_bwd_kv_simt_k(float *__restrict__ dqkv, const float *__restrict__ qkv,
             }
             s = group_sum<G>(s) * scale;
             dp = group_sum<G>(dp);
-            const bool on = (qg >= key) && (qg < T) && (key < T);
+            const bool on = (qg >= key) && (qg < T) && (key < end);
             const float p = on ? __expf(s - Ls[r]) : 0.0f;
             const float ds = p * (dp - Ds[r]);
 #pragma unroll
@@ -520,7 +484,7 @@ flash_bwd_kv_simt_k(float *__restrict__ dqkv, const float *__restrict__ qkv,
             }
         }
     }
-    if (key < T) {
+    if (key < end) {
         float *dkp = dqkv + ((long long)b * T + key) * ld + C + h * HS + sub * 32;
         float *dvp = dkp + C;
 #pragma unroll
@@ -531,14 +495,182 @@ flash_bwd_kv_simt_k(float *__restrict__ dqkv, const float *__restrict__ qkv,
     }
 }
 
+template <int HS, int KC>
+__global__ void __launch_bounds__(FT)
+flash_bwd_kv_simt_k(float *__restrict__ dqkv, const float *__restrict__ qkv,
+                    const float *__restrict__ dout, const float *__restrict__ lse,
+                    const float *__restrict__ dsum, int T, int NH, float scale) {
+    __shared__ __align__(16) float smem[2 * QT * (HS + 1)];
+    constexpr int R = FT / (HS / 32);
+    bwd_kv_rows<HS, KC, FT>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, blockIdx.y, blockIdx.x * R, R);
+}
+
+template <int HS, int NT>
+__device__ __noinline__ void bwd_q_rows_again(float *smem, float *dqkv, const float *qkv, const float *dout, const float *lse,
+                                              const float *dsum, int T, int NH, float scale, int bh, int i0, int nrows) {
+    constexpr int R = NT / (HS / 32);
+    for (int r = 0; r < nrows; r += R) bwd_q_rows<HS, 8, NT>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, bh, i0 + r, min(R, nrows - r));
+}
+template <int HS, int NT>
+__device__ __noinline__ void bwd_kv_rows_again(float *smem, float *dqkv, const float *qkv, const float *dout, const float *lse,
+                                               const float *dsum, int T, int NH, float scale, int bh, int j0, int nrows) {
+    constexpr int R = NT / (HS / 32);
+    for (int r = 0; r < nrows; r += R) bwd_kv_rows<HS, 8, NT>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, bh, j0 + r, min(R, nrows - r));
+}
+
+// Backward on warp-level tensor-core instructions: blocks of 16 rows a warp (4 warps; 8 at head size 128, where two
+// tiles of 64 rows would leave one block of 4 warps to an SM), 32 rows of the other side at a time in two buffers.
+template <int HS> struct bwd_warps { static constexpr int value = HS == 128 ? 8 : 4; };
+template <int HS> constexpr int bwd_smem() { return (2 * bwd_warps<HS>::value * 16 * HS + 4 * 32 * HS + 4 * 32) * 4; }
+
+// dQ = scale * sum over keys of dS K, dS = P (dO V^T - D), P = exp(scale Q K^T - lse).
+template <int HS>
+__device__ __forceinline__ void bwd_q_mma(float *__restrict__ smem, float *__restrict__ dqkv, const float *__restrict__ qkv,
+                                          const float *__restrict__ dout, const float *__restrict__ lse,
+                                          const float *__restrict__ dsum, int T, int NH, float scale, int bh, int i0) {
+    constexpr int NW = bwd_warps<HS>::value, NT = NW * 32, ROWS = NW * 16;
+    float *Qs = smem, *Os = Qs + ROWS * HS, *Ks = Os + ROWS * HS, *Vs = Ks + 2 * 32 * HS;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int b = bh / NH, h = bh % NH;
+    const int C = NH * HS;
+    const long long ld = 3LL * C;
+    const float *base = qkv + (long long)b * T * ld + h * HS;
+    auto copy_keys = [&](int j0, int buf) {
+        fm::tile_copy<HS, 32, NT>(Ks + buf * 32 * HS, base + (long long)j0 * ld + C, ld, T - j0);
+        fm::tile_copy<HS, 32, NT>(Vs + buf * 32 * HS, base + (long long)j0 * ld + 2 * C, ld, T - j0);
+        fm::cp_commit();
+    };
+    fm::tile_copy<HS, ROWS, NT>(Qs, base + (long long)i0 * ld, ld, T - i0);
+    fm::tile_copy<HS, ROWS, NT>(Os, dout + ((long long)b * T + i0) * C + h * HS, C, T - i0);
+    copy_keys(0, 0);
+
+    const int row0 = i0 + warp * 16, jmax = min(T, i0 + ROWS);
+    float lrow[2] = {0.0f, 0.0f}, drow[2] = {0.0f, 0.0f};
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const int row = row0 + g + 8 * r;
+        if (row < T) { lrow[r] = lse[(long long)bh * T + row]; drow[r] = dsum[(long long)bh * T + row]; }
+    }
+    float dq[HS / 8][4];
+#pragma unroll
+    for (int c = 0; c < HS / 8; ++c)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) dq[c][i] = 0.0f;
+
+    int buf = 0;
+    for (int j0 = 0; j0 < jmax; j0 += 32, buf ^= 1) {
+        fm::cp_wait_all();
+        __syncthreads();
+        if (j0 + 32 < jmax) copy_keys(j0 + 32, buf ^ 1);
+        if (j0 > row0 + 15) continue;
+        float s[4][4], dp[4][4];
+        fm::scores<HS, 2>(s, Qs, warp * 16, Ks + buf * 32 * HS, 0);
+        fm::scores<HS, 2>(dp, Os, warp * 16, Vs + buf * 32 * HS, 0);
+        const bool edge = j0 + 31 > row0 || j0 + 32 > T || row0 + 16 > T;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int key = j0 + 8 * j + 2 * t + (i & 1), row = row0 + g + 8 * (i >> 1);
+                const bool on = !edge || (key <= row && key < T && row < T);
+                const float p = on ? __expf(s[j][i] * scale - lrow[i >> 1]) : 0.0f;
+                s[j][i] = p * (dp[j][i] - drow[i >> 1]);
+            }
+        fm::contract<HS, 2, false>(dq, 1.0f, 1.0f, s, Ks + buf * 32 * HS, 0);
+    }
+    const bool bad = fm::store_rows<HS>(dqkv + ((long long)b * T + row0) * ld + h * HS, ld, g, T - row0, dq, scale, scale);
+    if (__syncthreads_or(bad)) bwd_q_rows_again<HS, NT>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, bh, i0, ROWS);
+}
+
+// dV = sum over queries of P^T dO, dK = scale * sum of dS^T Q: the transposed scores, keys as rows.
+template <int HS>
+__device__ __forceinline__ void bwd_kv_mma(float *__restrict__ smem, float *__restrict__ dqkv, const float *__restrict__ qkv,
+                                           const float *__restrict__ dout, const float *__restrict__ lse,
+                                           const float *__restrict__ dsum, int T, int NH, float scale, int bh, int j0) {
+    constexpr int NW = bwd_warps<HS>::value, NT = NW * 32, ROWS = NW * 16;
+    float *Ks = smem, *Vs = Ks + ROWS * HS, *Qs = Vs + ROWS * HS, *Os = Qs + 2 * 32 * HS, *Ls = Os + 2 * 32 * HS, *Ds = Ls + 2 * 32;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int b = bh / NH, h = bh % NH;
+    const int C = NH * HS;
+    const long long ld = 3LL * C;
+    const float *base = qkv + (long long)b * T * ld + h * HS;
+    auto copy_queries = [&](int i0, int buf) {
+        fm::tile_copy<HS, 32, NT>(Qs + buf * 32 * HS, base + (long long)i0 * ld, ld, T - i0);
+        fm::tile_copy<HS, 32, NT>(Os + buf * 32 * HS, dout + ((long long)b * T + i0) * C + h * HS, C, T - i0);
+        if (threadIdx.x < 64) {
+            const int r = threadIdx.x & 31;
+            const bool ok = i0 + r < T;
+            const float *src = (threadIdx.x < 32 ? lse : dsum) + (long long)bh * T + (ok ? i0 + r : 0);
+            fm::cp_async4((threadIdx.x < 32 ? Ls : Ds) + buf * 32 + r, src, ok);
+        }
+        fm::cp_commit();
+    };
+    fm::tile_copy<HS, ROWS, NT>(Ks, base + (long long)j0 * ld + C, ld, T - j0);
+    fm::tile_copy<HS, ROWS, NT>(Vs, base + (long long)j0 * ld + 2 * C, ld, T - j0);
+    copy_queries(j0, 0);                   // j0 is a multiple of 32: queries before it see none of these keys
+
+    const int key0 = j0 + warp * 16;
+    float dk[HS / 8][4], dv[HS / 8][4];
+#pragma unroll
+    for (int c = 0; c < HS / 8; ++c)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) dk[c][i] = dv[c][i] = 0.0f;
+
+    int buf = 0;
+    for (int i0 = j0; i0 < T; i0 += 32, buf ^= 1) {
+        fm::cp_wait_all();
+        __syncthreads();
+        if (i0 + 32 < T) copy_queries(i0 + 32, buf ^ 1);
+        if (i0 + 31 < key0) continue;      // (per warp) all of these queries come before all of its keys
+        const float *q = Qs + buf * 32 * HS, *go = Os + buf * 32 * HS, *Lb = Ls + buf * 32, *Db = Ds + buf * 32;
+        const bool edge = i0 < key0 + 15 || i0 + 32 > T || key0 + 16 > T;
+        float p[4][4], ds[4][4];
+        fm::scores<HS, 2>(p, Ks, warp * 16, q, 0);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int c = 8 * j + 2 * t + (i & 1), key = key0 + g + 8 * (i >> 1);
+                const bool on = !edge || (i0 + c >= key && i0 + c < T && key < T);
+                p[j][i] = on ? __expf(p[j][i] * scale - Lb[c]) : 0.0f;
+            }
+        fm::contract<HS, 2, false>(dv, 1.0f, 1.0f, p, go, 0);
+        fm::scores<HS, 2>(ds, Vs, warp * 16, go, 0);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) ds[j][i] = p[j][i] * (ds[j][i] - Db[8 * j + 2 * t + (i & 1)]);
+        fm::contract<HS, 2, false>(dk, 1.0f, 1.0f, ds, q, 0);
+    }
+    float *dkp = dqkv + ((long long)b * T + key0) * ld + C + h * HS;
+    bool bad = fm::store_rows<HS>(dkp, ld, g, T - key0, dk, scale, scale);
+    bad = fm::store_rows<HS>(dkp + C, ld, g, T - key0, dv, 1.0f, 1.0f) || bad;
+    if (__syncthreads_or(bad)) bwd_kv_rows_again<HS, NT>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, bh, j0, ROWS);
+}
+
+// Both in one grid (one partly filled last wave instead of two), the longest blocks first: the first key block has all
+// queries, the last query block all keys.
+// Measured with D, row-group kernels -> this: B8 T1024 12 heads of 64 2436 -> 1025 us, B4 T2048 8 x 128 18754 -> 2709,
+// B2 T777 12 x 32 445 -> 122.  2-norm errors of dq / dk / dv against 64 bits at 8 x 128: 4.9 / 10.8 / 10.8e-7 -> 3.3 / 4.1 / 3.7e-7.
+template <int HS>
+__global__ void __launch_bounds__(bwd_warps<HS>::value * 32, HS == 128 ? 1 : HS == 64 ? 3 : 4)
+flash_bwd_mma_k(float *__restrict__ dqkv, const float *__restrict__ qkv, const float *__restrict__ dout,
+                const float *__restrict__ lse, const float *__restrict__ dsum, int T, int NH, float scale) {
+    extern __shared__ __align__(16) float smem[];
+    constexpr int ROWS = bwd_warps<HS>::value * 16;
+    const int rank = blockIdx.y >> 1, blocks = gridDim.y >> 1;
+    if (blockIdx.y & 1) bwd_q_mma<HS>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, blockIdx.x, (blocks - 1 - rank) * ROWS);
+    else bwd_kv_mma<HS>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, blockIdx.x, rank * ROWS);
+}
+
 struct FwdCfg { int kc; const char *name; };
 struct BwdCfg { int kc; const char *name; };
 // Forward config 2 is the tensor-core kernel (flash_tc.cu), head size 64 only.
-// Forward config 0 is the register-tiled kernel (4 rows x 16 columns per thread), 1 the row-per-lane-group one.
-const FwdCfg FWD[] = {{8, "simt-fp32 rows4 keys8"}, {16, "simt-fp32 rowgroup keys16"},
+// Config 0 of both tables: warp-level tensor-core instructions, fp32 products in three TF32 ones; 1: the row-group code.
+const FwdCfg FWD[] = {{32, "mma-3xtf32 q64 k32"}, {16, "simt-fp32 rowgroup keys16"},
                       {0, "tcgen05-tf32 q2x128 k64 (head size 64 only)"}};
 // Backward config 2 is the tensor-core kernel pair (flash_tc_bwd.cu), head size 64 only.
-const BwdCfg BWD[] = {{4, "simt-fp32 rowgroup keys4"}, {8, "simt-fp32 rowgroup keys8"},
+const BwdCfg BWD[] = {{32, "mma-3xtf32 rows16 per warp, 32 at a time"}, {8, "simt-fp32 rowgroup keys8"},
                       {0, "tcgen05-tf32 dq128x128 dkv128x128 (head size 64 only)"}};
 constexpr int NFWD = 3, NBWD = 3, FWD_TC = 2, BWD_TC = 2;
 
@@ -546,13 +678,25 @@ bool shape_ok(const float *a, const float *b, int C, int NH) {
     return NH > 0 && C % NH == 0 && (((uintptr_t)a | (uintptr_t)b) & 15) == 0;
 }
 
+// Dynamic shared memory above 48 KB is opted into once per kernel and device.
+int allow_smem(const void *kernel, int bytes) {
+    static std::mutex mu;
+    static std::map<std::pair<const void *, int>, bool> done;
+    std::lock_guard<std::mutex> lk(mu);
+    bool &d = done[{kernel, current_device()}];
+    if (!d) BMB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    d = true;
+    return BMB_OK;
+}
+
 template <int HS>
 int run_fwd(int cfg, float *out, float *lse, const float *qkv, int B, int T, int NH, float scale,
             cudaStream_t st) {
     if (cfg == 0) {
-        constexpr int ROWS = FT / (HS / 16) * 4;
-        dim3 grid(ceil_div(T, ROWS), B * NH);
-        flash_fwd_rows4_k<HS, 8><<<grid, FT, 0, st>>>(out, lse, qkv, T, NH, scale);
+        constexpr int SMEM = (64 + 4 * 32) * HS * 4;
+        if (ceil_div(T, 64) > 65535) return fail(BMB_E_ARG, "flash: T=%d too long", T);
+        BMB_TRY(allow_smem((const void *)flash_fwd_mma_k<HS>, SMEM));
+        flash_fwd_mma_k<HS><<<dim3(B * NH, ceil_div(T, 64)), 128, SMEM, st>>>(out, lse, qkv, T, NH, scale);
     } else {
         constexpr int R = FT / (HS / 32);
         dim3 grid(ceil_div(T, R), B * NH);
@@ -566,17 +710,23 @@ int run_fwd(int cfg, float *out, float *lse, const float *qkv, int B, int T, int
 template <int HS>
 int run_bwd(int cfg, float *dqkv, float *dsum, const float *dout, const float *qkv, const float *out,
             const float *lse, int B, int T, int NH, float scale, cudaStream_t st) {
+    if (cfg == 0) {
+        constexpr int ROWS = bwd_warps<HS>::value * 16;
+        if (ceil_div(T, ROWS) > 32767) return fail(BMB_E_ARG, "flash: T=%d too long", T);
+        BMB_TRY(launch_flash_dsum(dsum, dout, out, B, T, NH, HS, st));
+        BMB_TRY(allow_smem((const void *)flash_bwd_mma_k<HS>, bwd_smem<HS>()));
+        flash_bwd_mma_k<HS><<<dim3(B * NH, 2 * ceil_div(T, ROWS)), bwd_warps<HS>::value * 32, bwd_smem<HS>(), st>>>(dqkv, qkv, dout, lse, dsum,
+                                                                                                    T, NH, scale);
+        count_launch();
+        BMB_LAUNCH_CHECK();
+        return BMB_OK;
+    }
     constexpr int R = FT / (HS / 32);
     const long long rows = (long long)B * NH * T;
     flash_dsum_k<<<ceil_div(rows * 32, 256), 256, 0, st>>>(dsum, dout, out, T, NH, HS, rows);
     dim3 grid(ceil_div(T, R), B * NH);
-    if (BWD[cfg].kc == 4) {
-        flash_bwd_kv_simt_k<HS, 4><<<grid, FT, 0, st>>>(dqkv, qkv, dout, lse, dsum, T, NH, scale);
-        flash_bwd_q_simt_k<HS, 4><<<grid, FT, 0, st>>>(dqkv, qkv, dout, lse, dsum, T, NH, scale);
-    } else {
-        flash_bwd_kv_simt_k<HS, 8><<<grid, FT, 0, st>>>(dqkv, qkv, dout, lse, dsum, T, NH, scale);
-        flash_bwd_q_simt_k<HS, 8><<<grid, FT, 0, st>>>(dqkv, qkv, dout, lse, dsum, T, NH, scale);
-    }
+    flash_bwd_kv_simt_k<HS, 8><<<grid, FT, 0, st>>>(dqkv, qkv, dout, lse, dsum, T, NH, scale);
+    flash_bwd_q_simt_k<HS, 8><<<grid, FT, 0, st>>>(dqkv, qkv, dout, lse, dsum, T, NH, scale);
     count_launch(3);
     BMB_LAUNCH_CHECK();
     return BMB_OK;
@@ -610,7 +760,7 @@ extern "C" {
 
 int bmb_flash_num_configs(void) { return NFWD; }
 const char *bmb_flash_config_name(int cfg) { return (cfg >= 0 && cfg < NFWD) ? FWD[cfg].name : "?"; }
-// fp32 arithmetic: the SIMT kernel; TF32/BF16 math modes: the tensor-core kernel.
+// fp32 arithmetic: split products (config 0); TF32/BF16 math modes: the tensor-core kernel.
 int bmb_flash_default_config(void) { return bmb_get_math_mode() == BMB_MATH_FP32 ? 0 : FWD_TC; }
 
 int bmb_flash_attention_forward_cfg(int cfg, float *out, float *lse, const float *qkv, int B, int T,

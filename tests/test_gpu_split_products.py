@@ -75,3 +75,66 @@ def test_split_product_stays_out_of_a_capture(bmb, cuda):
     graph.replay()
     cuda.cuda.synchronize()
     assert cuda.equal(C, want)
+
+
+def attention(bmb, cuda, cfg, qkv, dout, B, T, C, NH):
+    nan = lambda *s: cuda.full(s, float("nan"), device="cuda")             # noqa: E731
+    out, lse, dsum, dqkv = nan(B, T, C), nan(B, NH, T), nan(B, NH, T), nan(B, T, 3 * C)
+    bmb.call("bmb_flash_attention_forward_cfg", cfg, out, lse, qkv, B, T, C, NH)
+    bmb.call("bmb_flash_attention_backward_cfg", cfg, dqkv, dsum, dout, qkv, out, lse, B, T, C, NH)
+    cuda.cuda.synchronize()
+    return out, lse, dqkv
+
+
+@pytest.mark.parametrize("hs", [32, 64, 128])
+@pytest.mark.parametrize("T", [1, 17, 31, 32, 33, 64, 65, 127, 129, 200, 257])     # blocks of 64 / 128 rows, 32 of the other side
+def test_split_attention_against_64_bits(bmb, cuda, hs, T):
+    """Every output row is a sum of products exact to 2^-23 in chains cut off twice: below 2^-21 = 4.8e-7 in the 2-norm,
+    dq and dk (differences of such sums) below 2^-20."""
+    B, NH = 2, 3
+    C = NH * hs
+    g = cuda.Generator(device="cuda").manual_seed(T * 1000 + hs)
+    qkv, dout = cuda.randn(B, T, 3 * C, generator=g, device="cuda"), cuda.randn(B, T, C, generator=g, device="cuda")
+    got = attention(bmb, cuda, 0, qkv, dout, B, T, C, NH)
+    heads = lambda x: x.double().reshape(B, T, NH, hs).transpose(1, 2)      # noqa: E731
+    rows = lambda x: x.transpose(1, 2).reshape(B, T, C)                     # noqa: E731
+    (q, k, v), do = (heads(x) for x in qkv.chunk(3, dim=-1)), heads(dout)
+    s = (q @ k.transpose(2, 3) / hs ** 0.5).masked_fill(cuda.ones(T, T, dtype=cuda.bool, device="cuda").triu(1), float("-inf"))
+    lse = cuda.logsumexp(s, -1)
+    p = cuda.exp(s - lse[..., None])
+    o = p @ v
+    ds = p * (do @ v.transpose(2, 3) - (do * o).sum(-1, keepdim=True)) / hs ** 0.5
+    want = [rows(o), lse, rows(ds @ k), rows(ds.transpose(2, 3) @ q), rows(p.transpose(2, 3) @ do)]
+    for x, w, bar in zip([got[0], got[1], *got[2].chunk(3, dim=-1)], want, [4.8e-7, 4.8e-7, 9.6e-7, 9.6e-7, 4.8e-7]):
+        # a single key: dq and dk are zero but for the rounding of dP - D, so their scale is that of dout
+        scale = do.norm() if T == 1 else w.norm()
+        assert bool(cuda.isfinite(x).all()) and float((x.double() - w).norm() / scale) < bar
+
+
+@pytest.mark.parametrize("hs", [32, 64, 128])
+def test_split_attention_of_infinities_and_nan(bmb, cuda, hs):
+    """Infinite keys (a caller's own mask: probability zero), infinite values, NaN: finite where the row-group kernels
+    (config 1) are finite, and equal there."""
+    B, T, NH = 1, 200, 2
+    C = NH * hs
+    g = cuda.Generator(device="cuda").manual_seed(hs)
+    qkv, dout = cuda.randn(B, T, 3 * C, generator=g, device="cuda"), cuda.randn(B, T, C, generator=g, device="cuda")
+    qkv[0, :, 0] = qkv[0, :, 0].abs() + 1.0
+    qkv[0, 70, C] = float("-inf")                 # head 0, key 70: every score -inf
+    qkv[0, 150, 2 * C + hs] = float("inf")        # head 1, value 150
+    qkv[0, 190, hs + 1] = float("nan")            # head 1, query 190
+    new, old = (attention(bmb, cuda, cfg, qkv, dout, B, T, C, NH) for cfg in (0, 1))
+    assert bool(cuda.isfinite(old[0][0, :, :hs]).all()) and not bool(cuda.isfinite(old[0]).all())
+    for x, y in zip(new[:2], old[:2]):
+        assert cuda.equal(cuda.isfinite(x), cuda.isfinite(y)) and cuda.equal(cuda.isnan(x), cuda.isnan(y))
+        ok = cuda.isfinite(y)
+        assert float((x[ok] - y[ok]).abs().max()) < 1e-5
+    # the backward on the same forward results
+    res = []
+    for cfg in (0, 1):
+        dqkv, dsum = cuda.zeros(B, T, 3 * C, device="cuda"), cuda.zeros(B, NH, T, device="cuda")
+        bmb.call("bmb_flash_attention_backward_cfg", cfg, dqkv, dsum, dout, qkv, old[0], old[1], B, T, C, NH)
+        cuda.cuda.synchronize()
+        res.append(dqkv)
+    ok = cuda.isfinite(res[1])
+    assert cuda.equal(cuda.isfinite(res[0]), ok) and float((res[0][ok] - res[1][ok]).abs().max()) < 2e-5
