@@ -1,0 +1,28 @@
+"""fp32 SIMT products in tiles of 64 and 32 (csrc/gemm_simt_small.cu): the same sequential chains as the 128-wide
+kernels, bit for bit the CPU oracle's, at edges of tiles and slices, aligned and not."""
+import numpy as np
+import pytest
+from helpers import _np, uniform
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("batch,M,N,K", [
+    (1, 1, 1, 1), (1, 31, 33, 32), (1, 32, 64, 4), (1, 100, 70, 33), (1, 65, 130, 128),      # tiles of 32
+    (12, 256, 256, 96), (3, 500, 400, 100), (2, 513, 385, 129), (1, 960, 64, 97),            # and of 64, K from 96
+    (5, 64, 68, 31), (2, 36, 1000, 64), (1, 3, 2000, 130)])
+def test_small_tiles_follow_the_sequential_chain(bmb, orc, cuda, ta, tb, batch, M, N, K):
+    A, B = uniform(batch * M * K, 1), uniform(batch * K * N, 2)
+    want = np.zeros(batch * M * N, np.float32)
+    orc.orc_batched_gemm(ta, tb, batch, M, N, K, 1.0, _np(A), M * K, _np(B), K * N, 0.0, _np(want), M * N)
+    for offset in (0, 1):                      # 16-byte aligned operands, and operands one float off
+        dA, dB = (cuda.zeros(x.size + 4, device="cuda") for x in (A, B))
+        dA[offset:offset + A.size], dB[offset:offset + B.size] = cuda.from_numpy(A).cuda(), cuda.from_numpy(B).cuda()
+        dC = cuda.full((batch * M * N,), float("nan"), device="cuda")
+        prev = bmb.lib().bmb_get_math_mode()
+        bmb.lib().bmb_set_math_mode(bmb.MATH_FP32)
+        bmb.call("bmb_batched_gemm", ta, tb, batch, M, N, K, 1.0, dA[offset:], M * K, dB[offset:], K * N, 0.0, dC, M * N, None)
+        bmb.lib().bmb_set_math_mode(prev)
+        cuda.cuda.synchronize()
+        assert np.array_equal(dC.cpu().numpy(), want), offset
