@@ -101,6 +101,11 @@ inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 // has sized it by an eager pass, keeps its products in one line and watches scratch_generation().  Without it, products
 // that need scratch stay out of captures.
 constexpr int GEMM_SCRATCH_IN_CAPTURE = 1 << 20;
+// Internal flag: nobody compares this product's elements with the sequential fp32 chain, so a split product may serve
+// small ones too.
+constexpr int GEMM_ANY_ORDER = 1 << 21;
+// Internal flag: an fp32 product must be the sequential chain over k.
+constexpr int GEMM_CHAIN = 1 << 22;
 // Internal GEMM dispatch shared by attention and the trainer: math is a
 // BMB_MATH_* value, flags the BMB_GEMM_* bits, strides in elements.
 int gemm_any(int math, int flags, int ta, int tb, int batch, int M, int N, int K, float alpha,

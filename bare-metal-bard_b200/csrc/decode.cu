@@ -1,0 +1,373 @@
+// Sampling in fp32 (src/train_gpt.cu:46-102): the forward pass of one position with the keys and values of the
+// positions before it already in place, and the attention of one sequence's window.
+//
+// A distribution over tokens is an exponential of sums that every layer before it amplifies: two fp32 implementations
+// of a model of 7 layers can differ by 1e-4 of it, and a text is only the same where every draw is. So everything here
+// follows, operation by operation, the order that the pass over a whole batch has: products are the sequential chain of
+// multiply-adds over k (as in the SIMT kernels), layernorm is the one-warp form, attention takes 8 keys at a time.
+//
+// One position: every product is a matrix times one vector, bound by launches, by one trip to L2 (where the weights of a
+// model that samples in a loop stay) and by the chain, 4 cycles a step. So 32 outputs a block, one lane each, rows of
+// weights copied to shared memory ahead of it, and what stands before or after the product (layernorm, residual, GELU)
+// rides in the same launch: five launches a layer. Measured at 6 layers of 6 heads x 64,
+// 256 positions: a text of 300 tokens, 45 of them past the context, 1075 -> 117 ms (the whole batch of 16 x 256 rows each token before).
+#include "common.cuh"
+#include <cmath>
+#include <mutex>
+
+namespace bmb {
+namespace {
+
+constexpr int GV_OUT = 32, GV_NT = 128, GV_K = 128, GV_PITCH = GV_K + 4, GV_STAGES = 4;    // rows 4 banks apart
+constexpr int GV_MAX_IN = 4096, GV_MAX_LN = 1024;
+constexpr int GV_SMEM = (GV_STAGES * GV_OUT * GV_PITCH + GV_MAX_IN) * 4;
+
+// y[o] = f(W[o] . v + bias[o]) (+ add[o]), v = layernorm(x) when ln_w is given (each block for itself: a few hundred
+// values against 32 rows of them), f = GELU when `gelu`. in % 4 == 0.
+__global__ void __launch_bounds__(GV_NT) decode_gemv_k(float *__restrict__ y, const float *__restrict__ x, const float *__restrict__ W,
+                                                       const float *__restrict__ bias, const float *__restrict__ ln_w,
+                                                       const float *__restrict__ ln_b, const float *__restrict__ add, int in, int out, int gelu) {
+    extern __shared__ __align__(16) float smem[];
+    float *v = smem + GV_STAGES * GV_OUT * GV_PITCH;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, o0 = blockIdx.x * GV_OUT;
+    const int nk = (in + GV_K - 1) / GV_K;
+    auto fetch = [&](int kt) {
+        if (kt < nk) {
+            float *s = smem + (kt % GV_STAGES) * GV_OUT * GV_PITCH;
+#pragma unroll
+            for (int i = 0; i < GV_OUT * GV_K / 4 / GV_NT; ++i) {
+                const int lin = i * GV_NT + (int)threadIdx.x, r = lin / (GV_K / 4), c = lin % (GV_K / 4) * 4, k = kt * GV_K + c;
+                const bool ok = o0 + r < out && k < in;
+                const float *p = W + (ok ? (size_t)(o0 + r) * in + k : 0);
+                const uint32_t d = (uint32_t)__cvta_generic_to_shared(s + r * GV_PITCH + c);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(p), "r"(ok ? 16 : 0) : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int i = 0; i < GV_STAGES - 1; ++i) fetch(i);
+    if (!ln_w) {
+        for (int i = threadIdx.x * 4; i < in; i += GV_NT * 4) *reinterpret_cast<float4 *>(v + i) = *reinterpret_cast<const float4 *>(x + i);
+    } else if (warp == 0) {
+        // the sums of the one-warp layernorm, in its order
+        const int n4 = in >> 2;
+        float4 r[GV_MAX_LN / 128];
+        float sum = 0.0f;
+#pragma unroll
+        for (int i = 0; i < GV_MAX_LN / 128; ++i) {
+            const int c4 = lane + 32 * i;
+            r[i] = c4 < n4 ? *reinterpret_cast<const float4 *>(x + c4 * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+            sum += (r[i].x + r[i].y) + (r[i].z + r[i].w);
+        }
+        const float mu = warp_sum(sum) / in;
+        float sq = 0.0f;
+#pragma unroll
+        for (int i = 0; i < GV_MAX_LN / 128; ++i) {
+            if (lane + 32 * i < n4) {
+                const float a = r[i].x - mu, b = r[i].y - mu, c = r[i].z - mu, d = r[i].w - mu;
+                sq += (a * a + b * b) + (c * c + d * d);
+            }
+        }
+        const float var = warp_sum(sq) / in;
+        const float rs = rsqrtf(var + 1e-5f);
+#pragma unroll
+        for (int i = 0; i < GV_MAX_LN / 128; ++i) {
+            const int c4 = lane + 32 * i;
+            if (c4 < n4) {
+                const float4 w = *reinterpret_cast<const float4 *>(ln_w + c4 * 4), b = *reinterpret_cast<const float4 *>(ln_b + c4 * 4);
+                float4 o;
+                o.x = ((r[i].x - mu) * rs) * w.x + b.x;
+                o.y = ((r[i].y - mu) * rs) * w.y + b.y;
+                o.z = ((r[i].z - mu) * rs) * w.z + b.z;
+                o.w = ((r[i].w - mu) * rs) * w.w + b.w;
+                *reinterpret_cast<float4 *>(v + c4 * 4) = o;
+            }
+        }
+    }
+    float s = 0.0f;
+    for (int kt = 0; kt < nk; ++kt) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(GV_STAGES - 2) : "memory");
+        __syncthreads();
+        fetch(kt + GV_STAGES - 1);
+        if (warp != 0) continue;
+        const float *w = smem + (kt % GV_STAGES) * GV_OUT * GV_PITCH + lane * GV_PITCH, *a = v + kt * GV_K;
+        const int left = min(GV_K, in - kt * GV_K);
+#pragma unroll 8
+        for (int k = 0; k < left; k += 4) {
+            const float4 p = *reinterpret_cast<const float4 *>(a + k), q = *reinterpret_cast<const float4 *>(w + k);
+            s = fmaf(p.x, q.x, s); s = fmaf(p.y, q.y, s); s = fmaf(p.z, q.z, s); s = fmaf(p.w, q.w, s);
+        }
+    }
+    const int o = o0 + lane;
+    if (warp == 0 && o < out) {
+        if (bias) s += bias[o];
+        if (gelu) s = gelu_tanh(s);
+        y[o] = add ? add[o] + s : s;
+    }
+}
+
+// x = wte[token] + wpe[pos]
+__global__ void decode_embed_k(float *__restrict__ x, const float *__restrict__ wte, const float *__restrict__ wpe, int token, int pos, int C) {
+    for (int i = threadIdx.x; i < C; i += blockDim.x) x[i] = wte[(size_t)token * C + i] + wpe[(size_t)pos * C + i];
+}
+
+// ---- attention, 8 keys at a time -------------------------------------------------------------------------------------
+constexpr int KC = 8;
+
+// A score: HS/16 neighbouring lanes with 16 columns each, even and odd columns summed apart.
+__device__ __forceinline__ unsigned long long pack(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void fma2(unsigned long long &d, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ void load_query(unsigned long long (&q2)[8], const float *q, float scale) {
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) {
+        const float4 v = *reinterpret_cast<const float4 *>(q + 2 * i);
+        q2[i] = pack(v.x * scale, v.y * scale);
+        q2[i + 1] = pack(v.z * scale, v.w * scale);
+    }
+}
+template <int GL>
+__device__ __forceinline__ float score(const unsigned long long (&q2)[8], const float *k) {
+    unsigned long long acc = 0ull;
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) {
+        const float4 v = *reinterpret_cast<const float4 *>(k + 2 * i);
+        fma2(acc, q2[i], pack(v.x, v.y));
+        fma2(acc, q2[i + 1], pack(v.z, v.w));
+    }
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc));
+    float s = lo + hi;
+#pragma unroll
+    for (int o = 1; o < GL; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+
+// One head of the newest row against keys 0 .. pos; qkv: rows of 3C, the newest at `pos`. The running maximum before and
+// after each 8 keys is a prefix maximum, so scores and exponentials are computed side by side and only the row sum and
+// the output column of each thread follow the keys one after the other.
+// smem: pos + 1 scores in whole groups of 8, then two values a group.
+constexpr int DA_NT = 256;
+template <int HS>
+__global__ void __launch_bounds__(DA_NT) decode_attention_k(float *__restrict__ y, const float *__restrict__ qkv, int pos, int C, float scale) {
+    extern __shared__ __align__(16) float p[];
+    __shared__ float total;
+    constexpr int GL = HS / 16, KEYS = DA_NT / GL;
+    const int n = pos + 1, groups = (n + KC - 1) / KC, tid = threadIdx.x, lane = tid & 31;
+    float *gmax = p + groups * KC, *gsum = gmax + groups;        // running maximum, then rescaling factor; sum of a group
+    const long long ld = 3LL * C;
+    const float *base = qkv + blockIdx.x * HS;
+    const int sub = tid % GL;
+    unsigned long long q2[8];
+    load_query(q2, base + (long long)pos * ld + sub * 16, scale);
+    for (int j0 = 0; j0 < groups * KC; j0 += KEYS) {             // whole warps stay in the loop for the shuffles
+        const int j = j0 + tid / GL;
+        const float s = score<GL>(q2, base + (long long)min(j, pos) * ld + C + sub * 16);
+        if (sub == 0 && j < groups * KC) p[j] = j < n ? s : -INFINITY;
+    }
+    __syncthreads();
+    if (tid < 32) {
+        float before = -INFINITY;
+        for (int g0 = 0; g0 < groups; g0 += 32) {
+            const int g = g0 + lane;
+            float m = -INFINITY;
+            if (g < groups) {
+#pragma unroll
+                for (int c = 0; c < KC; ++c) m = fmaxf(m, p[g * KC + c]);
+            }
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const float up = __shfl_up_sync(0xffffffffu, m, o);
+                if (lane >= o) m = fmaxf(m, up);
+            }
+            m = fmaxf(m, before);
+            if (g < groups) gmax[g] = m;
+            before = __shfl_sync(0xffffffffu, m, 31);
+        }
+    }
+    __syncthreads();
+    const float m = tid > 0 && tid < groups ? gmax[tid - 1] : -INFINITY, mnew = tid < groups ? gmax[tid] : -INFINITY;
+    __syncthreads();                                             // maxima are read before factors take their place
+    if (tid < groups) {                                          // (at most one group a thread)
+        const bool live = mnew > -INFINITY;
+        float csum = 0.0f;
+#pragma unroll
+        for (int c = 0; c < KC; ++c) {
+            const float e = live ? __expf(p[tid * KC + c] - mnew) : 0.0f;
+            p[tid * KC + c] = e;
+            csum += e;
+        }
+        gmax[tid] = live ? __expf(m - mnew) : 1.0f;
+        gsum[tid] = csum;
+    }
+    __syncthreads();
+    float o = 0.0f;
+    if (tid < HS) {
+        const float *v = base + 2 * C + tid;
+        for (int j0 = 0; j0 < n; j0 += 4 * KC) {                 // 32 values under way at a time
+            float x[4 * KC];
+#pragma unroll
+            for (int c = 0; c < 4 * KC; ++c) x[c] = j0 + c < n ? v[(long long)(j0 + c) * ld] : 0.0f;
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                if (j0 + h * KC >= n) break;
+                o = fmaf(o, gmax[j0 / KC + h], 0.0f);
+#pragma unroll
+                for (int c = 0; c < KC; ++c) o = fmaf(p[j0 + h * KC + c], x[h * KC + c], o);
+            }
+        }
+    } else if (tid == HS) {
+        float l = 0.0f;
+        for (int g = 0; g < groups; ++g) l = l * gmax[g] + gsum[g];
+        total = l;
+    }
+    __syncthreads();
+    if (tid < HS) y[blockIdx.x * HS + tid] = o * ((total > 0.0f) ? 1.0f / total : 0.0f);
+}
+
+// All rows of one sequence's window. A row belongs to HS/16 lanes with 16 columns each; keys and values staged in shared
+// memory, a warp passes over keys that lie after its last row.
+constexpr int WA_NT = 128;
+template <int HS>
+__global__ void __launch_bounds__(WA_NT) window_attention_k(float *__restrict__ out, const float *__restrict__ qkv, int T, int C, float scale) {
+    constexpr int GL = HS / 16, ROWS = WA_NT / GL, TILE = HS >= 128 ? 32 : 64;
+    __shared__ __align__(16) float Ks[TILE * HS];
+    __shared__ __align__(16) float Vs[TILE * HS];
+    const int tid = threadIdx.x, sub = tid % GL;
+    const int i0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * ROWS, row = i0 + tid / GL;       // longest blocks first
+    const long long ld = 3LL * C;
+    const float *base = qkv + blockIdx.y * HS;
+    unsigned long long q2[8], o2[8];
+    load_query(q2, base + (long long)min(row, T - 1) * ld + sub * 16, scale);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) o2[i] = 0ull;
+    float m = -INFINITY, l = 0.0f;
+    const int warp_last = min(T - 1, i0 + (tid | 31) / GL), jmax = min(T, i0 + ROWS);
+    for (int j0 = 0; j0 < jmax; j0 += TILE) {
+        __syncthreads();
+        for (int lin = tid; lin < TILE * HS / 4; lin += WA_NT) {
+            const int r = lin / (HS / 4), c = lin % (HS / 4) * 4;
+            float4 k = make_float4(0.f, 0.f, 0.f, 0.f), v = k;
+            if (j0 + r < T) {
+                k = *reinterpret_cast<const float4 *>(base + (long long)(j0 + r) * ld + C + c);
+                v = *reinterpret_cast<const float4 *>(base + (long long)(j0 + r) * ld + 2 * C + c);
+            }
+            *reinterpret_cast<float4 *>(Ks + r * HS + c) = k;
+            *reinterpret_cast<float4 *>(Vs + r * HS + c) = v;
+        }
+        __syncthreads();
+        for (int c0 = 0; c0 < TILE && j0 + c0 <= warp_last; c0 += KC) {
+            float s[KC], cmax = -INFINITY;
+#pragma unroll
+            for (int c = 0; c < KC; ++c) {
+                const float a = score<GL>(q2, Ks + (c0 + c) * HS + sub * 16);
+                const int key = j0 + c0 + c;
+                s[c] = (key > row || key >= T) ? -INFINITY : a;
+                cmax = fmaxf(cmax, s[c]);
+            }
+            const float mnew = fmaxf(m, cmax);
+            const bool live = mnew > -INFINITY;
+            const float resc = live ? __expf(m - mnew) : 1.0f;
+            float csum = 0.0f;
+#pragma unroll
+            for (int c = 0; c < KC; ++c) {
+                s[c] = live ? __expf(s[c] - mnew) : 0.0f;
+                csum += s[c];
+            }
+            m = mnew;
+            l = l * resc + csum;
+            const unsigned long long resc2 = pack(resc, resc);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                unsigned long long z = 0ull;
+                fma2(z, o2[i], resc2);
+                o2[i] = z;
+            }
+#pragma unroll
+            for (int c = 0; c < KC; ++c) {
+                const unsigned long long p2 = pack(s[c], s[c]);
+#pragma unroll
+                for (int i = 0; i < 8; i += 2) {
+                    const float4 v = *reinterpret_cast<const float4 *>(Vs + (c0 + c) * HS + sub * 16 + 2 * i);
+                    fma2(o2[i], p2, pack(v.x, v.y));
+                    fma2(o2[i + 1], p2, pack(v.z, v.w));
+                }
+            }
+        }
+    }
+    if (row >= T) return;
+    const float inv = (l > 0.0f) ? 1.0f / l : 0.0f;
+    float *dst = out + (long long)row * C + blockIdx.y * HS + sub * 16;
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) {
+        float a0, a1, a2, a3;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(a0), "=f"(a1) : "l"(o2[i]));
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(a2), "=f"(a3) : "l"(o2[i + 1]));
+        *reinterpret_cast<float4 *>(dst + 2 * i) = make_float4(a0 * inv, a1 * inv, a2 * inv, a3 * inv);
+    }
+}
+
+}  // namespace
+
+// Sizes these kernels take: the attention's head sizes, a layernorm of one warp, and a context of at most 256 groups of
+// 8 keys (one a thread in decode_attention_k).
+bool decode_accepts(int T, int C, int NH) {
+    const int hs = (NH > 0 && C % NH == 0) ? C / NH : 0;
+    return (hs == 32 || hs == 64 || hs == 128) && C <= GV_MAX_LN && T <= DA_NT * KC;
+}
+
+int decode_embed(float *x, const float *wte, const float *wpe, int token, int pos, int C, cudaStream_t st) {
+    decode_embed_k<<<1, 256, 0, st>>>(x, wte, wpe, token, pos, C);
+    count_launch();
+    BMB_LAUNCH_CHECK();
+    return BMB_OK;
+}
+
+int decode_gemv(float *y, const float *x, const float *W, const float *bias, const float *ln_w, const float *ln_b, const float *add,
+                int in, int out, bool gelu, cudaStream_t st) {
+    static std::mutex mu;
+    static bool set[64];
+    const int d = current_device();
+    if (d < 0 || d >= 64 || in > GV_MAX_IN || (ln_w && in > GV_MAX_LN) || in % 4) return fail(BMB_E_UNSUPPORTED, "decode_gemv: %d inputs", in);
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        if (!set[d]) BMB_CUDA(cudaFuncSetAttribute(decode_gemv_k, cudaFuncAttributeMaxDynamicSharedMemorySize, GV_SMEM));
+        set[d] = true;
+    }
+    decode_gemv_k<<<ceil_div(out, GV_OUT), GV_NT, GV_SMEM, st>>>(y, x, W, bias, ln_w, ln_b, add, in, out, gelu ? 1 : 0);
+    count_launch();
+    BMB_LAUNCH_CHECK();
+    return BMB_OK;
+}
+
+int decode_attention(float *y, const float *qkv, int pos, int C, int NH, cudaStream_t st) {
+    const int hs = C / NH;
+    const float scale = 1.0f / sqrtf((float)hs);
+    const size_t smem = (size_t)ceil_div(pos + 1, KC) * (KC + 2) * sizeof(float);
+    if (hs == 32) decode_attention_k<32><<<NH, DA_NT, smem, st>>>(y, qkv, pos, C, scale);
+    else if (hs == 64) decode_attention_k<64><<<NH, DA_NT, smem, st>>>(y, qkv, pos, C, scale);
+    else decode_attention_k<128><<<NH, DA_NT, smem, st>>>(y, qkv, pos, C, scale);
+    count_launch();
+    BMB_LAUNCH_CHECK();
+    return BMB_OK;
+}
+
+int window_attention(float *out, const float *qkv, int T, int C, int NH, cudaStream_t st) {
+    const int hs = C / NH;
+    const float scale = 1.0f / sqrtf((float)hs);
+    const dim3 grid(ceil_div(T, WA_NT / (hs / 16)), NH);
+    if (hs == 32) window_attention_k<32><<<grid, WA_NT, 0, st>>>(out, qkv, T, C, scale);
+    else if (hs == 64) window_attention_k<64><<<grid, WA_NT, 0, st>>>(out, qkv, T, C, scale);
+    else window_attention_k<128><<<grid, WA_NT, 0, st>>>(out, qkv, T, C, scale);
+    count_launch();
+    BMB_LAUNCH_CHECK();
+    return BMB_OK;
+}
+
+}  // namespace bmb

@@ -7,9 +7,9 @@ namespace bmb {
 int gemm_simt(int transA, int transB, int batch, int M, int N, int K, float alpha, const float *A,
               long long sA, const float *B, long long sB, float beta, float *C, long long sC,
               cudaStream_t st);
-// fp32 products on the tensor cores in three bf16 pieces (gemm_x3.cu).  BMB_E_UNSUPPORTED: the SIMT kernel's.
+// fp32 products on the tensor cores in three bf16 pieces (gemm_x3.cu), bias included.  BMB_E_UNSUPPORTED: the SIMT kernel's.
 int gemm_x3(int transA, int transB, int M, int N, int K, float alpha, const float *A, const float *B, float beta, float *C,
-            bool scratch_in_capture, cudaStream_t st);
+            const float *bias, int flags, cudaStream_t st);
 // Tensor-core path (gemm_tc.cu).  Returns BMB_E_UNSUPPORTED for shapes it does
 // not take; the caller then falls back to the SIMT kernel (still on the GPU).
 int gemm_tc(int math, int flags, int transA, int transB, int batch, int M, int N, int K,
@@ -37,13 +37,14 @@ int gemm_any_bias(int math, int flags, int ta, int tb, int batch, int M, int N, 
     } else {
         // fp32 products: large single ones in three bf16 pieces, all others on the SIMT kernels.  Batched products stay
         // there too, as does registry entry 1: they are held to the sequential fp32 chain.
-        rc = (batch == 1 && A && B && C) ? gemm_x3(ta, tb, M, N, K, alpha, A, B, beta, C, flags & GEMM_SCRATCH_IN_CAPTURE, st) : BMB_E_UNSUPPORTED;
+        rc = (batch == 1 && A && B && C && !(flags & GEMM_CHAIN)) ? gemm_x3(ta, tb, M, N, K, alpha, A, B, beta, C, bias, flags, st) : BMB_E_UNSUPPORTED;
+        const bool bias_done = rc == BMB_OK;
         if (rc == BMB_E_UNSUPPORTED) rc = gemm_simt(ta, tb, batch, M, N, K, alpha, A, sA, B, sB, beta, C, sC, st);
         if (rc != BMB_OK) return rc;
-        // SIMT route: the bias and the optional rounding are separate passes on the same stream.
+        // the optional rounding is a pass of its own on the same stream, as is the bias behind a SIMT product
         void *prev = bmb_get_stream();
         bmb_set_stream((void *)st);
-        if (bias && batch == 1) rc = bmb_bias_forward(C, bias, M, N);
+        if (bias && batch == 1 && !bias_done) rc = bmb_bias_forward(C, bias, M, N);
         if (rc == BMB_OK && (flags & BMB_GEMM_C_ROUNDED) && batch == 1)
             rc = bmb_round_tf32(C, C, (size_t)M * N, (void *)st);
         bmb_set_stream(prev);

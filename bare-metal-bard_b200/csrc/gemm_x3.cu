@@ -135,6 +135,7 @@ struct Result {
     int ta, tb, M, N, K;
     float alpha, beta;
     float *C;
+    const float *bias;             // added to every row, or null
 };
 
 // One element by the sequential chain, as the SIMT kernels have it.
@@ -154,8 +155,9 @@ __device__ __forceinline__ bool not_finite(float x) { return !(fabsf(x) <= 3.402
 __device__ __forceinline__ void put_element(const Result &p, int m, int n, float s) {
     if (not_finite(s)) s = element_again(p, m, n);
     float *c = p.C + (size_t)m * p.N + n;
-    const float o = p.alpha * s;
-    *c = p.beta != 0.0f ? fmaf(p.beta, *c, o) : o;
+    float o = p.alpha * s;
+    if (p.beta != 0.0f) o = fmaf(p.beta, *c, o);
+    *c = p.bias ? o + p.bias[n] : o;
 }
 
 __device__ __forceinline__ void bulk_copy(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
@@ -340,6 +342,7 @@ gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict
                                 o.x = fmaf(p.beta, old.x, o.x);
                                 o.y = fmaf(p.beta, old.y, o.y);
                             }
+                            if (p.bias) { o.x += __ldg(p.bias + n); o.y += __ldg(p.bias + n + 1); }
                             *cp = o;
                         } else {
                             put_element(p, m, n, x);
@@ -387,6 +390,10 @@ __global__ void __launch_bounds__(256) reduce_x3_k(const Result p, int parts, co
                 const float4 old = *cp;
                 o.x = fmaf(p.beta, old.x, o.x); o.y = fmaf(p.beta, old.y, o.y);
                 o.z = fmaf(p.beta, old.z, o.z); o.w = fmaf(p.beta, old.w, o.w);
+            }
+            if (p.bias) {                           // N is a multiple of 4 here: the four are of one row
+                const float *b = p.bias + (int)(r % p.N);
+                o.x += __ldg(b); o.y += __ldg(b + 1); o.z += __ldg(b + 2); o.w += __ldg(b + 3);
             }
             *cp = o;
         }
@@ -440,20 +447,21 @@ XPlan choose_x3(int units, int M, int N, int kblocks) {
 
 }  // namespace
 
-// Takes: 2^28 multiply-adds and more, or 2^18 results and more with K from 192 (measured, SIMT against this:
-// 1024x384x384 43 / 19 us, 4096x128x384 43 / 21, 4096x384x128 17 / 19, 4096x4096x96 70 / 72; two launches and a pass
-// over the operands cost about 13 us whatever the size).  Fewer results than that are left to the SIMT kernels although
-// a long K would gain (256x256x1024 107 / 18 us): they are the products that callers compare, element by element, with
-// the sequential fp32 chain, which the SIMT kernels follow bit for bit and this one does not.
+// Takes products of 2^18 results and more with K from 192, and of 2^31 multiply-adds and more with K from 128 (measured,
+// SIMT against this: 1024x384x384 43 / 19 us, 4096x128x384 43 / 21, 4096x4096x128 89 / 76, but 2048x2048x128 29 / 33,
+// 4096x384x128 17 / 19, 4096x4096x64 50 / 70; two launches and a pass over the operands cost about 13 us whatever the
+// size).  Fewer results are left to the SIMT kernels although a long K would gain (256x256x1024 about 25 / 18 us): they are
+// the products that callers compare, element by element, with the sequential fp32 chain, which the SIMT kernels follow bit
+// for bit and this one does not.  A caller that says it does not (GEMM_ANY_ORDER: the trainer) has them from 2^14 results on.
 // BMB_E_UNSUPPORTED: nothing launched, the product is the SIMT kernels' (also where there is no memory for the images).
-// scratch_in_capture: see GEMM_SCRATCH_IN_CAPTURE.
 int gemm_x3(int transA, int transB, int M, int N, int K, float alpha, const float *A, const float *B, float beta, float *C,
-            bool scratch_in_capture, cudaStream_t st) {
-    if (M < 32 || N < 32 || K < 32) return BMB_E_UNSUPPORTED;
-    if ((double)M * N * K < 268435456.0 && ((double)M * N < 262144.0 || K < 192)) return BMB_E_UNSUPPORTED;
+            const float *bias, int flags, cudaStream_t st) {
+    if (M < 32 || N < 32) return BMB_E_UNSUPPORTED;
+    if (!(K >= 128 && (double)M * N * K >= 2147483648.0) &&
+        !(K >= 192 && (double)M * N >= ((flags & GEMM_ANY_ORDER) ? 16384.0 : 262144.0))) return BMB_E_UNSUPPORTED;
     // A captured launch would carry the scratch's address, and two captured branches would share it unordered.
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (!scratch_in_capture && (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)) {
+    if (!(flags & GEMM_SCRATCH_IN_CAPTURE) && (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)) {
         cudaGetLastError();
         return BMB_E_UNSUPPORTED;
     }
@@ -480,7 +488,7 @@ int gemm_x3(int transA, int transB, int M, int N, int K, float alpha, const floa
     float *w = (float *)(scr + imgA + imgB);
 
     auto vec_of = [](const float *p, int inner) { return ((uintptr_t)p & 15) == 0 && inner % 4 == 0; };
-    const Result p{A, B, transA, transB, M, N, K, alpha, beta, C};
+    const Result p{A, B, transA, transB, M, N, K, alpha, beta, C, bias};
     const bool even = N % 2 == 0 && (plan.parts > 1 || ((uintptr_t)C & 7) == 0);
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
     BMB_TRY(scratch_acquire(SCR_GEMM_A, st));

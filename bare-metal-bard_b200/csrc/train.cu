@@ -19,6 +19,12 @@ int layernorm_bwd_blocks(int N);
 bool flash_tc_supported(int T, int C, int NH, const float *qkv, const float *out);
 int flash_forward_tc(float *out, float *lse, const float *qkv, int B, int T, int C, int NH, bool qkv_rounded,
                      cudaStream_t st);
+bool decode_accepts(int T, int C, int NH);
+int decode_embed(float *x, const float *wte, const float *wpe, int token, int pos, int C, cudaStream_t st);
+int decode_gemv(float *y, const float *x, const float *W, const float *bias, const float *ln_w, const float *ln_b, const float *add,
+                int in, int out, bool gelu, cudaStream_t st);
+int decode_attention(float *y, const float *qkv, int pos, int C, int NH, cudaStream_t st);
+int window_attention(float *out, const float *qkv, int T, int C, int NH, cudaStream_t st);
 int flash_backward_tc(float *dqkv, float *dsum, const float *dout, const float *qkv, const float *out,
                       const float *lse, int B, int T, int C, int NH, bool rounded, cudaStream_t st, float *dbias_qkv = nullptr);
 namespace tc {
@@ -181,7 +187,7 @@ int collect_profile(bmb_trainer *t) {
 // One matmul of the model, optionally bracketed by events.
 int mm(bmb_trainer *t, int flags, int ta, int tb, int M, int N, int K, const float *A, const float *B,
        float beta, float *C, const float *bias = nullptr, cudaStream_t on = nullptr, float *aux_gelu = nullptr) {
-    flags |= GEMM_SCRATCH_IN_CAPTURE;
+    flags |= GEMM_SCRATCH_IN_CAPTURE | GEMM_ANY_ORDER;          // (GEMM_CHAIN outranks them)
     if (on) return gemm_any_bias(t->c.math, flags, ta, tb, 1, M, N, K, 1.0f, A, 0, B, 0, beta, C, 0, bias, on, aux_gelu);
     if (t->prof) {
         if (t->ev_used + 2 > t->ev.size()) {
@@ -203,9 +209,18 @@ int mm(bmb_trainer *t, int flags, int ta, int tb, int M, int N, int K, const flo
     return BMB_OK;
 }
 
+// X W^T + bias outside the fused mode: in fp32 the product adds the bias as it stores (where it is not a split
+// product, the library does it after it); the other modes keep the pass of its own.
+int mm_bias(bmb_trainer *t, int flags, int M, int N, int K, const float *A, const float *B, float *C, const float *bias) {
+    if (t->c.math == BMB_MATH_FP32) return mm(t, flags, 0, 1, M, N, K, A, B, 0.0f, C, bias);
+    BMB_TRY(mm(t, flags, 0, 1, M, N, K, A, B, 0.0f, C));
+    return bmb_bias_forward(C, bias, M, N);
+}
+
 // Shapes and operand conventions shared by the units of a pass.
 struct Dims {
     int B, T, C, L, NH, Vp, V, N;
+    const int *tokens;
     size_t BTC, BT, BT3C, BT4C, qkvr_sz, att_sz, lse_sz;
     const float *W, *P;      // weights as the GEMMs read them (the pre-rounded shadow copy in the tensor-core modes), and as stored
     float *G;
@@ -213,13 +228,17 @@ struct Dims {
     int wflag;               // products with a weight: A = an activation or gradient (rounded by its producer when fused), B = the weight
     int gflag;               // weight-gradient products: both operands are activations / gradients
 };
+void set_rows(Dims &d, int B, int T) {
+    d.B = B; d.T = T; d.N = B * T;
+    d.BTC = (size_t)d.N * d.C; d.BT = d.N; d.BT3C = 3 * d.BTC; d.BT4C = 4 * d.BTC;
+    d.qkvr_sz = 4 * d.BTC; d.att_sz = (size_t)B * d.NH * T * T; d.lse_sz = (size_t)B * d.NH * T;
+}
 Dims dims_of(bmb_trainer *t) {
     const bmb_train_config &c = t->c;
     Dims d;
+    d.tokens = t->d_tokens;
     d.B = c.B; d.T = c.T; d.C = c.n_embd; d.L = c.n_layer; d.NH = c.n_head; d.Vp = c.padded_vocab; d.V = c.vocab_size;
-    d.N = d.B * d.T;
-    d.BTC = (size_t)d.N * d.C; d.BT = d.N; d.BT3C = 3 * d.BTC; d.BT4C = 4 * d.BTC;
-    d.qkvr_sz = 4 * d.BTC; d.att_sz = (size_t)d.B * d.NH * d.T * d.T; d.lse_sz = (size_t)d.B * d.NH * d.T;
+    set_rows(d, d.B, d.T);
     d.W = (c.math == BMB_MATH_FP32 || !t->shadow) ? t->params : t->shadow;
     d.P = t->params;
     d.G = t->grads;
@@ -230,7 +249,7 @@ Dims dims_of(bmb_trainer *t) {
 }
 
 int fwd_embed(bmb_trainer *t, const Dims &d) {
-    BMB_TRY(bmb_encoder_forward(t->encoded, t->d_tokens, d.P + t->poff[P_WTE], d.P + t->poff[P_WPE], d.B, d.T, d.C));
+    BMB_TRY(bmb_encoder_forward(t->encoded, d.tokens, d.P + t->poff[P_WTE], d.P + t->poff[P_WPE], d.B, d.T, d.C));
     // The first layernorm stands alone; every later one (and the final one) rides with the
     // residual add that produces its input.
     return bmb_layernorm_forward(t->ln1, t->ln1_mean, t->ln1_rstd, t->encoded, d.P + t->poff[P_LN1W], d.P + t->poff[P_LN1B], d.N, d.C);
@@ -252,11 +271,12 @@ int fwd_layer(bmb_trainer *t, const Dims &d, int l) {
         BMB_TRY(mm(t, wflag | BMB_GEMM_C_ROUNDED, 0, 1, N, 3 * C, C, ln1, W + t->poff[P_QKVW] + (size_t)l * 3 * C * C, 0.0f, qkv,
                    P + t->poff[P_QKVB] + (size_t)l * 3 * C));
     } else {
-        BMB_TRY(mm(t, wflag, 0, 1, N, 3 * C, C, ln1, W + t->poff[P_QKVW] + (size_t)l * 3 * C * C, 0.0f, qkv));
-        BMB_TRY(bmb_bias_forward(qkv, P + t->poff[P_QKVB] + (size_t)l * 3 * C, N, 3 * C));
+        BMB_TRY(mm_bias(t, wflag, N, 3 * C, C, ln1, W + t->poff[P_QKVW] + (size_t)l * 3 * C * C, qkv, P + t->poff[P_QKVB] + (size_t)l * 3 * C));
     }
     if (c.use_flash && fz && attn_cfg(c) == 2)
         BMB_TRY(flash_forward_tc(atty, t->lse + l * d.lse_sz, qkv, B, T, C, NH, true, t->st));
+    else if (c.use_flash && (wflag & GEMM_CHAIN))
+        BMB_TRY(window_attention(atty, qkv, T, C, NH, t->st));
     else if (c.use_flash)
         BMB_TRY(bmb_flash_attention_forward_cfg(attn_cfg(c), atty, t->lse + l * d.lse_sz, qkv, B, T, C, NH));
     else
@@ -265,8 +285,7 @@ int fwd_layer(bmb_trainer *t, const Dims &d, int l) {
         BMB_TRY(mm(t, wflag, 0, 1, N, C, C, atty, W + t->poff[P_APW] + (size_t)l * C * C, 0.0f, attproj,
                    P + t->poff[P_APB] + (size_t)l * C));
     } else {
-        BMB_TRY(mm(t, wflag, 0, 1, N, C, C, atty, W + t->poff[P_APW] + (size_t)l * C * C, 0.0f, attproj));
-        BMB_TRY(bmb_bias_forward(attproj, P + t->poff[P_APB] + (size_t)l * C, N, C));
+        BMB_TRY(mm_bias(t, wflag, N, C, C, atty, W + t->poff[P_APW] + (size_t)l * C * C, attproj, P + t->poff[P_APB] + (size_t)l * C));
     }
     BMB_TRY(bmb_residual_layernorm_forward(res2, ln2, t->ln2_mean + l * BT, t->ln2_rstd + l * BT, residual, attproj,
                                            P + t->poff[P_LN2W] + (size_t)l * C, P + t->poff[P_LN2B] + (size_t)l * C, N, C));
@@ -276,16 +295,14 @@ int fwd_layer(bmb_trainer *t, const Dims &d, int l) {
                    P + t->poff[P_FCB] + (size_t)l * 4 * C, nullptr, t->fuse_gelu ? fchg : nullptr));
         if (!t->fuse_gelu) BMB_TRY(bmb_gelu_forward(fchg, fch, (int)d.BT4C));
     } else {
-        BMB_TRY(mm(t, wflag, 0, 1, N, 4 * C, C, ln2, W + t->poff[P_FCW] + (size_t)l * 4 * C * C, 0.0f, fch));
-        BMB_TRY(bmb_bias_forward(fch, P + t->poff[P_FCB] + (size_t)l * 4 * C, N, 4 * C));
+        BMB_TRY(mm_bias(t, wflag, N, 4 * C, C, ln2, W + t->poff[P_FCW] + (size_t)l * 4 * C * C, fch, P + t->poff[P_FCB] + (size_t)l * 4 * C));
         BMB_TRY(bmb_gelu_forward(fchg, fch, (int)d.BT4C));
     }
     if (fz) {
         BMB_TRY(mm(t, wflag, 0, 1, N, C, 4 * C, fchg, W + t->poff[P_FPW] + (size_t)l * C * 4 * C, 0.0f, fcproj,
                    P + t->poff[P_FPB] + (size_t)l * C));
     } else {
-        BMB_TRY(mm(t, wflag, 0, 1, N, C, 4 * C, fchg, W + t->poff[P_FPW] + (size_t)l * C * 4 * C, 0.0f, fcproj));
-        BMB_TRY(bmb_bias_forward(fcproj, P + t->poff[P_FPB] + (size_t)l * C, N, C));
+        BMB_TRY(mm_bias(t, wflag, N, C, 4 * C, fchg, W + t->poff[P_FPW] + (size_t)l * C * 4 * C, fcproj, P + t->poff[P_FPB] + (size_t)l * C));
     }
     if (l + 1 < L)
         return bmb_residual_layernorm_forward(res3, t->ln1 + (l + 1) * BTC, t->ln1_mean + (l + 1) * BT, t->ln1_rstd + (l + 1) * BT,
@@ -1197,20 +1214,74 @@ int bmb_trainer_load(bmb_trainer *t, const char *path, int load_optimizer_state,
 }
 
 // ---- sampling (src/train_gpt.cu:46-102) ------------------------------------------------------------
-int bmb_trainer_next_token_probs(bmb_trainer *t, const int *host_tokens, int pos, float *host_probs) {
-    if (!t || !host_tokens || !host_probs || pos < 0 || pos >= t->c.B * t->c.T) return fail(BMB_E_ARG, "next_token_probs: bad argument");
-    Scope sc(t);
+// The logits of one position in t->logits, from tokens already on the device.  They depend on that position's sequence
+// up to it and on nothing else, so in fp32 only those rows go through the layers (one sequence of `pos % T + 1`
+// positions instead of the whole batch), and only the last of them through the head.  The tensor-core modes run the
+// whole batch, whose shapes their kernels and captured plans are made for.
+static int next_token_logits(bmb_trainer *t, int pos, const float **row) {
+    const int T = t->c.T, C = t->c.n_embd;
+    if (t->c.math != BMB_MATH_FP32 || !decode_accepts(T, C, t->c.n_head)) {
+        BMB_TRY(forward(t, false));
+        set_emit_rounded(false);
+        *row = t->logits + (size_t)pos * t->c.padded_vocab;
+        return BMB_OK;
+    }
+    Dims d = dims_of(t);
+    set_rows(d, 1, pos % T + 1);
+    d.wflag |= GEMM_CHAIN;               // the order of sums that sampling keeps (decode.cu)
+    d.tokens = t->d_tokens + pos / T * T;
+    BMB_TRY(fwd_embed(t, d));
+    for (int l = 0; l < d.L; ++l) BMB_TRY(fwd_layer(t, d, l));
+    *row = t->logits;
+    return decode_gemv(t->logits, t->lnf + (size_t)(d.N - 1) * C, d.P + t->poff[P_WTE], nullptr, nullptr, nullptr, nullptr, C, d.Vp, false, t->st);
+}
+
+// The same for the newest position of a growing text: `token` at `pos`, positions before it computed by earlier calls.
+// Their keys and values are the rows of t->qkv, T rows a layer.
+static int decode_logits(bmb_trainer *t, int token, int pos, const float **row) {
+    const Dims d = dims_of(t);
+    const int C = d.C;
+    const float *P = d.P;
+    float *x = t->encoded, *x2 = t->residual2, *y = t->atty, *h = t->fch;      // one row each
+    BMB_TRY(decode_embed(x, P + t->poff[P_WTE], P + t->poff[P_WPE], token, pos, C, t->st));
+    for (int l = 0; l < d.L; ++l) {
+        const size_t lC = (size_t)l * C;
+        float *qkv = t->qkv + (size_t)l * d.T * 3 * C;
+        BMB_TRY(decode_gemv(qkv + (size_t)pos * 3 * C, x, P + t->poff[P_QKVW] + 3 * lC * C, P + t->poff[P_QKVB] + 3 * lC,
+                            P + t->poff[P_LN1W] + lC, P + t->poff[P_LN1B] + lC, nullptr, C, 3 * C, false, t->st));
+        BMB_TRY(decode_attention(y, qkv, pos, C, d.NH, t->st));
+        BMB_TRY(decode_gemv(x2, y, P + t->poff[P_APW] + lC * C, P + t->poff[P_APB] + lC, nullptr, nullptr, x, C, C, false, t->st));
+        BMB_TRY(decode_gemv(h, x2, P + t->poff[P_FCW] + 4 * lC * C, P + t->poff[P_FCB] + 4 * lC, P + t->poff[P_LN2W] + lC,
+                            P + t->poff[P_LN2B] + lC, nullptr, C, 4 * C, true, t->st));
+        BMB_TRY(decode_gemv(x, h, P + t->poff[P_FPW] + 4 * lC * C, P + t->poff[P_FPB] + lC, nullptr, nullptr, x2, 4 * C, C, false, t->st));
+    }
+    *row = t->logits;
+    return decode_gemv(t->logits, x, P + t->poff[P_WTE], nullptr, P + t->poff[P_LNFW], P + t->poff[P_LNFB], nullptr, C, d.Vp, false, t->st);
+}
+
+// Softmax of one row of logits to the host: that of the reference's loss kernel (src/nn.cu:197-237); its target only
+// picks which loss is written, so the first of the resident targets serves.
+static int probs_to_host(bmb_trainer *t, const float *row, float *host_probs) {
     const int Vp = t->c.padded_vocab, V = t->c.vocab_size;
-    if (!t->gen_probs) BMB_CUDA(cudaMalloc(&t->gen_probs, ((size_t)Vp + 1) * sizeof(float)));
-    BMB_CUDA(cudaMemcpyAsync(t->d_tokens, host_tokens, (size_t)t->c.B * t->c.T * sizeof(int), cudaMemcpyDefault, t->st));
-    BMB_TRY(forward(t, false));
-    set_emit_rounded(false);
-    // the softmax of the reference's loss kernel over that one row (src/nn.cu:197-237); its target only picks which
-    // loss is written, so row `pos` of the resident targets serves
-    BMB_TRY(bmb_softmax_crossentropy_forward(t->gen_probs, t->gen_probs + Vp, t->logits + (size_t)pos * Vp, t->d_targets + pos, 1, V, Vp));
+    BMB_TRY(bmb_softmax_crossentropy_forward(t->gen_probs, t->gen_probs + Vp, row, t->d_targets, 1, V, Vp));
     BMB_CUDA(cudaMemcpyAsync(host_probs, t->gen_probs, (size_t)Vp * sizeof(float), cudaMemcpyDeviceToHost, t->st));
     BMB_CUDA(cudaStreamSynchronize(t->st));
     return check_kernel_status();
+}
+
+static int sampling_buffers(bmb_trainer *t) {
+    if (!t->gen_probs) BMB_CUDA(cudaMalloc(&t->gen_probs, ((size_t)t->c.padded_vocab + 1) * sizeof(float)));
+    return BMB_OK;
+}
+
+int bmb_trainer_next_token_probs(bmb_trainer *t, const int *host_tokens, int pos, float *host_probs) {
+    if (!t || !host_tokens || !host_probs || pos < 0 || pos >= t->c.B * t->c.T) return fail(BMB_E_ARG, "next_token_probs: bad argument");
+    Scope sc(t);
+    BMB_TRY(sampling_buffers(t));
+    BMB_CUDA(cudaMemcpyAsync(t->d_tokens, host_tokens, (size_t)t->c.B * t->c.T * sizeof(int), cudaMemcpyDefault, t->st));
+    const float *row = nullptr;
+    BMB_TRY(next_token_logits(t, pos, &row));
+    return probs_to_host(t, row, host_probs);
 }
 
 int bmb_trainer_generate(bmb_trainer *t, int start_token, int steps, unsigned seed, float temperature, int *host_tokens_out) {
@@ -1221,10 +1292,24 @@ int bmb_trainer_generate(bmb_trainer *t, int start_token, int steps, unsigned se
     std::vector<float> row((size_t)Vp);
     std::mt19937 rng(seed);
     std::uniform_real_distribution<float> uni(0.0f, 1.0f);
-    int cur_len = 1;
+    // While the text grows a step computes its newest position only; once the context is full every position moves by
+    // one each step and the window is computed anew.
+    const bool decode = t->c.math == BMB_MATH_FP32 && t->c.use_flash && decode_accepts(T, t->c.n_embd, t->c.n_head);
+    int cur_len = 1, seen = 0;           // positions of the text, and how many of them have their keys and values
     ctx[0] = start_token;
     for (int s = 0; s < steps; ++s) {
-        BMB_TRY(bmb_trainer_next_token_probs(t, ctx.data(), cur_len - 1, row.data()));
+        if (decode && seen == cur_len - 1) {
+            Scope sc(t);
+            BMB_TRY(sampling_buffers(t));
+            const float *logits = nullptr;
+            BMB_TRY(decode_logits(t, ctx[cur_len - 1], cur_len - 1, &logits));
+            // the resident batch is the context, as after a pass over all of it
+            if (s == steps - 1) BMB_CUDA(cudaMemcpyAsync(t->d_tokens, ctx.data(), ctx.size() * sizeof(int), cudaMemcpyHostToDevice, t->st));
+            BMB_TRY(probs_to_host(t, logits, row.data()));
+            seen = cur_len;
+        } else {
+            BMB_TRY(bmb_trainer_next_token_probs(t, ctx.data(), cur_len - 1, row.data()));
+        }
         if (temperature != 1.0f) {
             float sum = 0.0f;
             for (int i = 0; i < V; ++i) { row[i] = powf(row[i], 1.0f / temperature); sum += row[i]; }

@@ -12,7 +12,7 @@ GEMMS = [  # M, N, K, ta, tb, beta
     (1000, 514, 2047, 1, 0, 1.0),    # K shared among CTAs, even N off 16 bytes
     (33, 8191, 999, 0, 1, 0.0),      # one ragged row tile
     (4100, 68, 1000, 1, 0, 0.0),     # one narrow column tile
-    (3000, 3001, 64, 0, 0, -1.0),
+    (4100, 4101, 130, 0, 0, -1.0),   # short K, nothing aligned
     (2048, 1536, 512, 0, 1, 0.0),
 ]
 
