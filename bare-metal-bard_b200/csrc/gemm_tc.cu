@@ -66,14 +66,16 @@ constexpr int BM = 128, BN_WIDE = 256, BN_NARROW = 64, STAGES = 4, KBYTES = 128;
 constexpr int A_BYTES = BM * KBYTES;
 constexpr int EPI_WARPS = 8;                        // two per TMEM lane quadrant, taking alternate 32-column chunks
 constexpr int NTHREADS = 64 + 32 * EPI_WARPS;
+constexpr int RND_WARPS = 4, RND_THREADS = 32 * RND_WARPS;
 constexpr int EPI_BYTES = EPI_WARPS * 32 * 32 * 4;  // one 32 x 32 staging block per epilogue warp, 16-byte units XOR-swizzled by row
 // A tile is MH (1 or 2) blocks of 128 rows tall.  Two blocks share every B slice: per K slice the SM then
 // writes 64 KB and reads 96 KB of shared memory for 8 instructions, against 48 KB + 48 KB for 4 -- with
 // fp32 operands it is shared-memory bandwidth, not the tensor pipe, that bounds the main loop.  The price:
 // the two accumulators fill tensor memory, so the epilogue no longer overlaps the next tile, and the
 // ring is 3 slices deep.
-__host__ __device__ constexpr int stages_for(int mh) { return mh == 2 ? 3 : STAGES; }
-constexpr int smem_bytes(int bn, int mh = 1) { return stages_for(mh) * (mh * A_BYTES + bn * KBYTES) + 1024 /*align*/ + 256 /*barriers*/ + EPI_BYTES; }
+// Narrow tiles have smaller slices and are bound by how much is on its way from memory: their ring is deeper.
+__host__ __device__ constexpr int stages_for(int bn, int mh) { return mh == 2 ? 3 : bn == 64 ? 8 : bn == 128 ? 6 : STAGES; }
+constexpr int smem_bytes(int bn, int mh = 1) { return stages_for(bn, mh) * (mh * A_BYTES + bn * KBYTES) + 1024 /*align*/ + 512 /*barriers*/ + EPI_BYTES; }
 constexpr int CHUNK_BYTES = 32 * KBYTES;   // one MN-major chunk: 32 K rows x 128 bytes of M/N
 
 #ifdef BMB_GEMM_TRACE
@@ -221,15 +223,17 @@ __device__ __forceinline__ void add_result(float4 o, float *__restrict__ C, int 
 // KIND 0 = tf32 (fp32 operands), 1 = f16 (bf16 operands, always K-major).
 // a_mn / b_mn: the operand's tile is MN-major (TF32 only); 2 = its tensor map is the 3-d one that
 // brings all chunks of a slice in one copy.
-template <int KIND, int BN, int MH, int AUX>
-__global__ void __launch_bounds__(NTHREADS, 1)
+// RND: the operands lie in memory as fp32 and four more warps round each slice where it has landed (TF32 only), instead
+// of a pass that writes rounded copies first.
+template <int KIND, int BN, int MH, int AUX, int RND>
+__global__ void __launch_bounds__(NTHREADS + RND * RND_THREADS, 1)
 gemm_tc_k(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
           const __grid_constant__ CUtensorMap mapC, int c_mode, int batch, int M, int N,
           int kblocks, int kelems_per_block, int a_mn, int b_mn, float alpha, float beta, float *__restrict__ C,
           int vec_ok, int dp_tiles, int g_sk, const float *__restrict__ bias, int round_c, int *__restrict__ status,
           float *__restrict__ aux, int round_aux) {
     static_assert(MH == 1 || (MH == 2 && BN == 256), "two-block tiles are 256 columns wide");
-    constexpr int STAGES = stages_for(MH), BMT = BM * MH;
+    constexpr int STAGES = stages_for(BN, MH), BMT = BM * MH;
     constexpr int B_BYTES = BN * KBYTES, STAGE_BYTES = MH * A_BYTES + B_BYTES;
     constexpr uint32_t ACC_COLS = BN > 128 ? 256 : 128; // TMEM columns set aside per 128-row accumulator
     constexpr int NACC = MH == 2 ? 1 : 2;               // accumulator sets: two blocks of rows fill tensor memory
@@ -240,13 +244,14 @@ gemm_tc_k(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
     // operand ring | epilogue staging (1024-byte aligned: it is a TMA store source) | barriers
     uint64_t *bars = reinterpret_cast<uint64_t *>(gen + STAGES * STAGE_BYTES + EPI_BYTES);
     // bars[0..S) full, [S..2S) empty, [2S..2S+2) tmem_full, [2S+2..2S+4) tmem_empty
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 4);
+    // and, with RND, [2S+4..3S+4) rounded
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + (2 + RND) * STAGES + 4);
     volatile int *giveup = reinterpret_cast<volatile int *>(tmem_slot + 1);
     int *armed = reinterpret_cast<int *>(tmem_slot + 2);   // [STAGES] parity last armed per slice, -1 = never
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * STAGES;
-    const uint32_t tfull0 = empty0 + 8 * STAGES, tempty0 = tfull0 + 16;
+    const uint32_t tfull0 = empty0 + 8 * STAGES, tempty0 = tfull0 + 16, rnd0 = tempty0 + 16;
 
     TileSched sch;
     sch.tiles_m = (M + BMT - 1) / BMT;
@@ -263,6 +268,8 @@ gemm_tc_k(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
         GTR(0);
         for (int s = 0; s < STAGES; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); armed[s] = -1; }
         for (int a = 0; a < 2; ++a) { mbar_init(tfull0 + 8 * a, 1); mbar_init(tempty0 + 8 * a, EPI_WARPS); }
+        if (RND)
+            for (int s = 0; s < STAGES; ++s) mbar_init(rnd0 + 8 * s, RND_WARPS);
         *giveup = 0;
         mbar_init_fence();
     }
@@ -343,7 +350,7 @@ gemm_tc_k(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
                 fence_after();
                 const uint32_t d = tmem_base + (uint32_t)acc * ACC_COLS;
                 for (int kb = kb0; kb < kb1; ++kb) {
-                    { GWAIT_BEGIN(); if (!mbar_wait(full0 + 8 * s, ph, giveup)) { ok = false; break; } GWAIT_END(gw_full); }
+                    { GWAIT_BEGIN(); if (!mbar_wait((RND ? rnd0 : full0) + 8 * s, ph, giveup)) { ok = false; break; } GWAIT_END(gw_full); }
                     fence_after();
 #ifdef BMB_GEMM_TRACE
                     if (first_slice) { GTR(3); first_slice = false; }
@@ -370,6 +377,32 @@ gemm_tc_k(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
             }
             GWAIT_FLUSH(10, gw_full);
             GWAIT_FLUSH(11, gw_tempty);
+        }
+    } else if (RND && warp >= 2 + EPI_WARPS) {
+        // ------------------------------------------------------------ rounding
+        // Half a TF32 ulp added to the magnitude turns the tensor core's cut after 10 bits into rounding to nearest, as
+        // cvt.rna does (NaN, whose payload the sum could carry away, is left as it is).  Whole slices in place: the
+        // swizzle moves words, not bits.
+        const int tid = (int)threadIdx.x - NTHREADS;
+        int s = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        while (ok && wi.next(tile, kb0, kb1)) {
+            for (int kb = kb0; kb < kb1; ++kb) {
+                if (!mbar_wait(full0 + 8 * s, ph, giveup)) { ok = false; break; }
+                uint4 *w = reinterpret_cast<uint4 *>(gen + s * STAGE_BYTES) + tid;
+#pragma unroll 8
+                for (int i = 0; i < STAGE_BYTES / 16 / RND_THREADS; ++i) {
+                    uint4 x = w[i * RND_THREADS];
+                    auto up = [](uint32_t u) { return (u & 0x7fffffffu) > 0x7f800000u ? u : u + 0x1000u; };
+                    x.x = up(x.x); x.y = up(x.y); x.z = up(x.z); x.w = up(x.w);
+                    w[i * RND_THREADS] = x;
+                }
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(rnd0 + 8 * s);
+                if (++s == STAGES) { s = 0; ph ^= 1; }
+            }
         }
     } else {
         // ------------------------------------------------------------ epilogue
@@ -1159,7 +1192,7 @@ int plan_gemm(Plan *p, bool bf16, int flags, int batch, int M, int N, int K, int
     return BMB_OK;
 }
 
-template <int KIND, int BN, int MH, int AUX = 0>
+template <int KIND, int BN, int MH, int AUX = 0, int RND = 0>
 int launch_tc(int grid, cudaStream_t st, const CUtensorMap &mapA, const CUtensorMap &mapB, const CUtensorMap &mapC, int c_mode,
               int batch, int M, int N, int kblocks, int kper,
               int amn, int bmn, float alpha, float beta, float *C, int vec_ok, int dp_tiles, int g_sk, const float *bias,
@@ -1169,11 +1202,11 @@ int launch_tc(int grid, cudaStream_t st, const CUtensorMap &mapA, const CUtensor
         std::lock_guard<std::mutex> lk(g_attr_mu);
         const int d = current_device();
         if (d >= 0 && d < 64 && !attr_set[d]) {
-            BMB_CUDA(cudaFuncSetAttribute(gemm_tc_k<KIND, BN, MH, AUX>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(BN, MH)));
+            BMB_CUDA(cudaFuncSetAttribute(gemm_tc_k<KIND, BN, MH, AUX, RND>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(BN, MH)));
             attr_set[d] = true;
         }
     }
-    gemm_tc_k<KIND, BN, MH, AUX><<<grid, NTHREADS, smem_bytes(BN, MH), st>>>(mapA, mapB, mapC, c_mode, batch, M, N, kblocks, kper, amn, bmn, alpha, beta, C, vec_ok,
+    gemm_tc_k<KIND, BN, MH, AUX, RND><<<grid, NTHREADS + RND * RND_THREADS, smem_bytes(BN, MH), st>>>(mapA, mapB, mapC, c_mode, batch, M, N, kblocks, kper, amn, bmn, alpha, beta, C, vec_ok,
                                                                 dp_tiles, g_sk, bias, round_c, status_dev, aux, round_aux);
     return BMB_OK;
 }
@@ -1222,6 +1255,38 @@ int pair_clusters() {
 
 }  // namespace
 
+// Whether a TF32 product rounds its operands as they arrive in shared memory rather than by a pass before it; *plan then
+// is a plan of 128-row tiles.  The pass costs a launch and two trips through memory per operand, rounding in place doubles
+// what a slice moves through shared memory, by which the main loop is bound (so large square products keep the pass).
+static bool rounds_on_arrival(Plan *plan, int flags, int transA, int transB, int batch, int M, int N, int K, const float *A, const float *B,
+                              bool a_rounded, bool b_rounded, int ctas) {
+    if ((a_rounded && b_rounded) || plan->pair || (flags & (BMB_GEMM_TILE_M256 | BMB_GEMM_PAIR))) return false;
+    // read where they lie: what the tensor maps take
+    if ((((uintptr_t)A | (uintptr_t)B) & 15) || (transA ? M : K) % 4 || (transB ? K : N) % 4) return false;
+    Plan p = *plan;
+    if (p.mh != 1 && plan_gemm(&p, false, flags | BMB_GEMM_TILE_M128, batch, M, N, K, ctas) != BMB_OK) return false;
+    // Cycles of either way.  A slice costs the main loop what it moves through shared memory (measured: 256 columns 800
+    // against 1570 with rounding in place, 128 columns 520 and 1100, 64 columns 400 and 1000); tiles of up to 128 columns
+    // with a short K are bound by their stores instead, about 20 bytes a cycle and SM, beside which rounding is free.  A
+    // pass is a launch of about 4500 cycles and 8 bytes an element at 5000 a cycle.  Sides of the line, pass / in place:
+    // 1024^3 25.8 / 24.6 us, 768x768x4096 37.5 / 33.8, 6144x128x6144 97 / 48, batch 96 of 1024x64x1024 234 / 100,
+    // 8 of 256x256x32 20 / 9; but 2048^3 55 / 67, 4096^3 234 / 376, 2560x2560x640 33 / 43, 6144x6144x64 48 / 50.
+    auto cycles = [&](const Plan &q, bool in_place) {
+        const double slice = q.mh == 2 ? 1.72 * 800.0 : in_place ? (q.bn == 256 ? 1570.0 : q.bn == 192 ? 1250.0 : q.bn == 128 ? 1100.0 : 1000.0)
+                                                                 : (q.bn == 256 ? 800.0 : q.bn == 192 ? 650.0 : q.bn == 128 ? 520.0 : 400.0);
+        const double store = q.bn <= 128 && !q.sk_tiles ? BM * q.bn * 4 / 20.0 : 0.0;
+        const double tile = slice * q.kblocks > store ? slice * q.kblocks : store;
+        const double tiles = q.sk_tiles ? (double)q.tiles / q.grid : (double)((q.tiles + ctas - 1) / ctas);
+        return tile * tiles;
+    };
+    double pass = 0.0;
+    if (!a_rounded) pass += 4500.0 + (double)batch * M * K * 8.0 / 5000.0;
+    if (!b_rounded) pass += 4500.0 + (double)batch * N * K * 8.0 / 5000.0;
+    if (cycles(p, true) >= cycles(*plan, false) + pass) return false;
+    *plan = p;
+    return true;
+}
+
 // aux_gelu (optional): a second output, GELU (tanh form, src/nn.cu:118-127) of the result, rounded to TF32 when the
 // library is emitting rounded operands -- the MLP's activation rides in the epilogue of the product before it.
 // Served where every tile is stored by one CTA straight from registers (beta 0, aligned C, no tile shared
@@ -1245,12 +1310,14 @@ int gemm_tc(int math, int flags, int transA, int transB, int batch, int M, int N
     BMB_TRY(plan_gemm(&plan, bf16, flags, batch, M, N, K, ctas));
     if (wants_pair(bf16, flags, transA, transB, batch, M, N))
         plan_pair(&plan, flags, M, N, (flags & BMB_GEMM_HALF_SMS) ? (pair_clusters() + 1) / 2 : pair_clusters());
+    const bool a_rounded = (flags & BMB_GEMM_A_ROUNDED) != 0, b_rounded = (flags & BMB_GEMM_B_ROUNDED) != 0;
+    const bool rnd = !bf16 && !aux_gelu && rounds_on_arrival(&plan, flags, transA, transB, batch, M, N, K, A, B, a_rounded, b_rounded, ctas);
     const int kblocks = plan.kblocks, bn = plan.bn, dp_tiles = plan.dp_tiles;
     Operand a, b;
     StagingRelease release_on_return{a, b, st};
     // per CTA: the pair kernel loads 128 rows of A and half of the B tile
-    BMB_TRY(stage_operand(&a, A, !transA, M, K, bf16, (flags & BMB_GEMM_A_ROUNDED) != 0, SCR_GEMM_A, plan.pair ? BM : plan.mh * BM, st, batch));
-    BMB_TRY(stage_operand(&b, B, transB != 0, N, K, bf16, (flags & BMB_GEMM_B_ROUNDED) != 0, SCR_GEMM_B, plan.pair ? bn / 2 : bn, st, batch));
+    BMB_TRY(stage_operand(&a, A, !transA, M, K, bf16, a_rounded || rnd, SCR_GEMM_A, plan.pair ? BM : plan.mh * BM, st, batch));
+    BMB_TRY(stage_operand(&b, B, transB != 0, N, K, bf16, b_rounded || rnd, SCR_GEMM_B, plan.pair ? bn / 2 : bn, st, batch));
     CUtensorMap mapA, mapB;
     if (a.map3d) BMB_TRY(make_map_mn3d(&mapA, a.ptr, a.rows, a.cols, a.pitch_bytes, a.tile_chunks));
     else BMB_TRY(make_map_2d(&mapA, a.ptr, esize, a.rows, a.cols, a.pitch_bytes, a.box_rows, a.mn_major));
@@ -1306,6 +1373,11 @@ int gemm_tc(int math, int flags, int transA, int transB, int batch, int M, int N
         else if (bn == 192) BMB_TRY((launch_tc<1, 192, 1>(BMB_TC_ARGS)));
         else if (bn == 128) BMB_TRY((launch_tc<1, 128, 1>(BMB_TC_ARGS)));
         else BMB_TRY((launch_tc<1, 64, 1>(BMB_TC_ARGS)));
+    } else if (rnd) {
+        if (bn == 256) BMB_TRY((launch_tc<0, 256, 1, 0, 1>(BMB_TC_ARGS)));
+        else if (bn == 192) BMB_TRY((launch_tc<0, 192, 1, 0, 1>(BMB_TC_ARGS)));
+        else if (bn == 128) BMB_TRY((launch_tc<0, 128, 1, 0, 1>(BMB_TC_ARGS)));
+        else BMB_TRY((launch_tc<0, 64, 1, 0, 1>(BMB_TC_ARGS)));
     } else {
         if (plan.mh == 2) BMB_TRY((launch_tc<0, 256, 2>(BMB_TC_ARGS)));
         else if (bn == 256) BMB_TRY((launch_tc<0, 256, 1>(BMB_TC_ARGS)));
