@@ -5,7 +5,7 @@
 // x = hi + lo, hi the nearest TF32 value, lo = x - hi (exact; the instruction reads its upper 11 bits).  a b is
 // hi hi + hi lo + lo hi up to 2^-23 of |a b|.  The instruction cuts its running sums off instead of rounding them, so
 // a chain is short (two instructions, 16 columns: with four the error at T = 64 is a third larger, with one the kernels are
-// 10 to 20 % slower), the small terms have a chain of their own, and chains are added in fp32.
+// 10 to 20 % slower) and chains are added in fp32; the small terms have one chain of their own, added at the end.
 //
 // Why these instructions and not tcgen05: the operands stay plain fp32 in shared memory (a split copy of 64 rows of
 // K and V at head size 128 is 128 KB), probabilities go from accumulator to operand without leaving registers, and
@@ -63,12 +63,12 @@ __device__ __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uin
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(FIRST ? 0.0f : d[0]), "f"(FIRST ? 0.0f : d[1]),
                    "f"(FIRST ? 0.0f : d[2]), "f"(FIRST ? 0.0f : d[3]));
 }
-// Four neighbouring groups of 8 columns: big[j] (+)= a_hi b_hi, small[j] (+)= a_hi b_lo + a_lo b_hi; FIRST starts the
-// sums.  Issued so that an instruction never waits for the one before it.
-template <bool FIRST>
+// Four neighbouring groups of 8 columns: big[j] (+)= a_hi b_hi, small[j] (+)= a_hi b_lo + a_lo b_hi; FIRST and FIRST_SMALL
+// start the sums.  Issued so that an instruction never waits for the one before it.
+template <bool FIRST, bool FIRST_SMALL>
 __device__ __forceinline__ void mma3x4(float (&big)[4][4], float (&small)[4][4], const HiLo (&a)[4], const HiLo (&b0)[4], const HiLo (&b1)[4]) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) mma<FIRST>(small[j], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b0[j].lo, b1[j].lo);
+    for (int j = 0; j < 4; ++j) mma<FIRST_SMALL>(small[j], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b0[j].lo, b1[j].lo);
 #pragma unroll
     for (int j = 0; j < 4; ++j) mma<FIRST>(big[j], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b0[j].hi, b1[j].hi);
 #pragma unroll
@@ -83,10 +83,6 @@ __device__ __forceinline__ void mma3x4(float (&big)[4][4], float (&small)[4][4],
 template <int HS, int FOLD>
 __device__ __forceinline__ void scores(float (&s)[4][4], const float *A, int a_row, const float *B, int b_row) {
     const int g = (threadIdx.x >> 2) & 7, t = threadIdx.x & 3;
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) s[j][i] = 0.0f;
     float big[4][4], small[4][4];
 #pragma unroll
     for (int kk = 0; kk < HS / 16; ++kk) {
@@ -100,17 +96,22 @@ __device__ __forceinline__ void scores(float (&s)[4][4], const float *A, int a_r
             HiLo b0[4], b1[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) { b0[j] = split(h ? b[j].z : b[j].x); b1[j] = split(h ? b[j].w : b[j].y); }
-            if ((2 * kk + h) % FOLD == 0) mma3x4<true>(big, small, a, b0, b1);
-            else mma3x4<false>(big, small, a, b0, b1);
+            if (kk == 0 && h == 0) mma3x4<true, true>(big, small, a, b0, b1);
+            else if ((2 * kk + h) % FOLD == 0) mma3x4<true, false>(big, small, a, b0, b1);
+            else mma3x4<false, false>(big, small, a, b0, b1);
             if ((2 * kk + h) % FOLD == FOLD - 1) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) s[j][i] += big[j][i] + small[j][i];
+                    for (int i = 0; i < 4; ++i) s[j][i] = 2 * kk + h < FOLD ? big[j][i] : s[j][i] + big[j][i];
                 }
             }
         }
     }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s[j][i] += small[j][i];
 }
 
 // o = o * (f0 | f1) + p (16 x 32, laid out as scores() leaves it) times 32 rows of B.  Columns of o: accumulator
@@ -119,29 +120,38 @@ __device__ __forceinline__ void scores(float (&s)[4][4], const float *A, int a_r
 template <int HS, int FOLD, bool RESCALE>
 __device__ __forceinline__ void contract(float (&o)[HS / 8][4], float f0, float f1, const float (&p)[4][4], const float *B, int b_row) {
     const int g = (threadIdx.x >> 2) & 7, t = threadIdx.x & 3;
+    HiLo a[4][4];
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[ks][i] = split(p[ks][i == 1 ? 2 : i == 2 ? 1 : i]);
 #pragma unroll
     for (int J = 0; J < HS / 32; ++J) {
+        float small[4][4], sum[4][4];
 #pragma unroll
         for (int k0 = 0; k0 < 4; k0 += FOLD) {
-            float big[4][4], small[4][4];
+            float big[4][4];
 #pragma unroll
             for (int ks = k0; ks < k0 + FOLD; ++ks) {
-                const HiLo a[4] = {split(p[ks][0]), split(p[ks][2]), split(p[ks][1]), split(p[ks][3])};
                 const int r = b_row + 8 * ks + 2 * t;
                 const float4 u = tile_ld<HS>(B, r, 8 * J + g), v = tile_ld<HS>(B, r + 1, 8 * J + g);
                 const HiLo b0[4] = {split(u.x), split(u.y), split(u.z), split(u.w)}, b1[4] = {split(v.x), split(v.y), split(v.z), split(v.w)};
-                if (ks == k0) mma3x4<true>(big, small, a, b0, b1);
-                else mma3x4<false>(big, small, a, b0, b1);
+                if (ks == 0) mma3x4<true, true>(big, small, a[ks], b0, b1);
+                else if (ks == k0) mma3x4<true, false>(big, small, a[ks], b0, b1);
+                else mma3x4<false, false>(big, small, a[ks], b0, b1);
             }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                float (&q)[4] = o[4 * J + j];
-                const bool resc = RESCALE && k0 == 0;
+            for (int j = 0; j < 4; ++j)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float sum = big[j][i] + small[j][i];
-                    q[i] = resc ? fmaf(q[i], i < 2 ? f0 : f1, sum) : q[i] + sum;
-                }
+                for (int i = 0; i < 4; ++i) sum[j][i] = k0 == 0 ? big[j][i] : sum[j][i] + big[j][i];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float (&q)[4] = o[4 * J + j];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float x = sum[j][i] + small[j][i];
+                q[i] = RESCALE ? fmaf(q[i], i < 2 ? f0 : f1, x) : q[i] + x;
             }
         }
     }
