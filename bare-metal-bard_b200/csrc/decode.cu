@@ -10,7 +10,7 @@
 // model that samples in a loop stay) and by the chain, 4 cycles a step. So 32 outputs a block, one lane each, rows of
 // weights copied to shared memory ahead of it, and what stands before or after the product (layernorm, residual, GELU)
 // rides in the same launch: five launches a layer. Measured at 6 layers of 6 heads x 64,
-// 256 positions: a text of 300 tokens, 45 of them past the context, 1075 -> 117 ms (the whole batch of 16 x 256 rows each token before).
+// 256 positions: a text of 300 tokens, 45 of them past the context, 1075 -> 102 ms (the whole batch of 16 x 256 rows each token before).
 #include "common.cuh"
 #include <cmath>
 #include <mutex>
@@ -18,7 +18,8 @@
 namespace bmb {
 namespace {
 
-constexpr int GV_OUT = 32, GV_NT = 128, GV_K = 128, GV_PITCH = GV_K + 4, GV_STAGES = 4;    // rows 4 banks apart
+// a warp that follows the chains and four that copy weights ahead of it; rows 4 banks apart
+constexpr int GV_OUT = 32, GV_NT = 160, GV_CP = 128, GV_K = 128, GV_PITCH = GV_K + 4, GV_STAGES = 8;
 constexpr int GV_MAX_IN = 4096, GV_MAX_LN = 1024;
 constexpr int GV_SMEM = (GV_STAGES * GV_OUT * GV_PITCH + GV_MAX_IN) * 4;
 
@@ -32,11 +33,11 @@ __global__ void __launch_bounds__(GV_NT) decode_gemv_k(float *__restrict__ y, co
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, o0 = blockIdx.x * GV_OUT;
     const int nk = (in + GV_K - 1) / GV_K;
     auto fetch = [&](int kt) {
-        if (kt < nk) {
+        if (kt < nk && warp > 0) {
             float *s = smem + (kt % GV_STAGES) * GV_OUT * GV_PITCH;
 #pragma unroll
-            for (int i = 0; i < GV_OUT * GV_K / 4 / GV_NT; ++i) {
-                const int lin = i * GV_NT + (int)threadIdx.x, r = lin / (GV_K / 4), c = lin % (GV_K / 4) * 4, k = kt * GV_K + c;
+            for (int i = 0; i < GV_OUT * GV_K / 4 / GV_CP; ++i) {
+                const int lin = i * GV_CP + (int)threadIdx.x - 32, r = lin / (GV_K / 4), c = lin % (GV_K / 4) * 4, k = kt * GV_K + c;
                 const bool ok = o0 + r < out && k < in;
                 const float *p = W + (ok ? (size_t)(o0 + r) * in + k : 0);
                 const uint32_t d = (uint32_t)__cvta_generic_to_shared(s + r * GV_PITCH + c);
@@ -93,10 +94,29 @@ __global__ void __launch_bounds__(GV_NT) decode_gemv_k(float *__restrict__ y, co
         if (warp != 0) continue;
         const float *w = smem + (kt % GV_STAGES) * GV_OUT * GV_PITCH + lane * GV_PITCH, *a = v + kt * GV_K;
         const int left = min(GV_K, in - kt * GV_K);
-#pragma unroll 8
-        for (int k = 0; k < left; k += 4) {
-            const float4 p = *reinterpret_cast<const float4 *>(a + k), q = *reinterpret_cast<const float4 *>(w + k);
+        auto step = [&](const float4 &p, const float4 &q) {
             s = fmaf(p.x, q.x, s); s = fmaf(p.y, q.y, s); s = fmaf(p.z, q.z, s); s = fmaf(p.w, q.w, s);
+        };
+        if (left == GV_K) {
+            // the next 16 values are read while these 16 are added (the chain alone is 64 cycles)
+            float4 p[2][4], q[2][4];
+            auto read = [&](int k, int h) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    p[h][i] = *reinterpret_cast<const float4 *>(a + k + 4 * i);
+                    q[h][i] = *reinterpret_cast<const float4 *>(w + k + 4 * i);
+                }
+            };
+            read(0, 0);
+#pragma unroll
+            for (int k = 0; k < GV_K; k += 16) {
+                const int h = (k / 16) & 1;
+                if (k + 16 < GV_K) read(k + 16, h ^ 1);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) step(p[h][i], q[h][i]);
+            }
+        } else {
+            for (int k = 0; k < left; k += 4) step(*reinterpret_cast<const float4 *>(a + k), *reinterpret_cast<const float4 *>(w + k));
         }
     }
     const int o = o0 + lane;
@@ -152,20 +172,31 @@ __device__ __forceinline__ float score(const unsigned long long (&q2)[8], const 
 // One head of the newest row against keys 0 .. pos; qkv: rows of 3C, the newest at `pos`. The running maximum before and
 // after each 8 keys is a prefix maximum, so scores and exponentials are computed side by side and only the row sum and
 // the output column of each thread follow the keys one after the other.
-// smem: pos + 1 scores in whole groups of 8, then two values a group.
-constexpr int DA_NT = 256;
+// smem: pos + 1 scores in whole groups of 8, two values a group, and, where they fit, the values of all keys, on their way
+// while the scores are computed.
+constexpr int DA_NT = 512, DA_MAX_V = 160 * 1024;
 template <int HS>
-__global__ void __launch_bounds__(DA_NT) decode_attention_k(float *__restrict__ y, const float *__restrict__ qkv, int pos, int C, float scale) {
-    extern __shared__ __align__(16) float p[];
+__global__ void __launch_bounds__(DA_NT) decode_attention_k(float *__restrict__ y, const float *__restrict__ qkv, int pos, int C, float scale, int stage_v) {
+    extern __shared__ __align__(16) float smem[];
     __shared__ float total;
     constexpr int GL = HS / 16, KEYS = DA_NT / GL;
     const int n = pos + 1, groups = (n + KC - 1) / KC, tid = threadIdx.x, lane = tid & 31;
+    float *vs = smem, *p = smem + (stage_v ? groups * KC * HS : 0);
     float *gmax = p + groups * KC, *gsum = gmax + groups;        // running maximum, then rescaling factor; sum of a group
     const long long ld = 3LL * C;
     const float *base = qkv + blockIdx.x * HS;
     const int sub = tid % GL;
+    if (stage_v) {
+        for (int i = tid; i < groups * KC * HS / 4; i += DA_NT) {
+            const int j = i / (HS / 4), c = i % (HS / 4) * 4;
+            const uint32_t d = (uint32_t)__cvta_generic_to_shared(vs + j * HS + c);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(base + (long long)min(j, pos) * ld + 2 * C + c),
+                         "r"(j < n ? 16 : 0) : "memory");
+        }
+    }
     unsigned long long q2[8];
     load_query(q2, base + (long long)pos * ld + sub * 16, scale);
+#pragma unroll 2
     for (int j0 = 0; j0 < groups * KC; j0 += KEYS) {             // whole warps stay in the loop for the shuffles
         const int j = j0 + tid / GL;
         const float s = score<GL>(q2, base + (long long)min(j, pos) * ld + C + sub * 16);
@@ -206,9 +237,20 @@ __global__ void __launch_bounds__(DA_NT) decode_attention_k(float *__restrict__ 
         gmax[tid] = live ? __expf(m - mnew) : 1.0f;
         gsum[tid] = csum;
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     float o = 0.0f;
-    if (tid < HS) {
+    if (tid < HS && stage_v) {
+#pragma unroll 2
+        for (int g = 0; g < groups; ++g) {                       // (a masked key's probability is zero, its value too)
+            float x[KC], e[KC];
+#pragma unroll
+            for (int c = 0; c < KC; ++c) { x[c] = vs[(g * KC + c) * HS + tid]; e[c] = p[g * KC + c]; }
+            o = fmaf(o, gmax[g], 0.0f);
+#pragma unroll
+            for (int c = 0; c < KC; ++c) o = fmaf(e[c], x[c], o);
+        }
+    } else if (tid < HS) {
         const float *v = base + 2 * C + tid;
         for (int j0 = 0; j0 < n; j0 += 4 * KC) {                 // 32 values under way at a time
             float x[4 * KC];
@@ -231,91 +273,127 @@ __global__ void __launch_bounds__(DA_NT) decode_attention_k(float *__restrict__ 
     if (tid < HS) y[blockIdx.x * HS + tid] = o * ((total > 0.0f) ? 1.0f / total : 0.0f);
 }
 
-// All rows of one sequence's window. A row belongs to HS/16 lanes with 16 columns each; keys and values staged in shared
-// memory, a warp passes over keys that lie after its last row.
-constexpr int WA_NT = 128;
+// All rows of one sequence's window. HS/16 lanes have 16 columns each of two neighbouring rows (what they read of a key or
+// value serves both); keys and values staged in shared memory, a warp passes over keys that lie after its last row. A block
+// of two warps: the window of one sequence is few rows, and the last ones see all keys.
+constexpr int WA_NT = 64, RQ = 2;
 template <int HS>
 __global__ void __launch_bounds__(WA_NT) window_attention_k(float *__restrict__ out, const float *__restrict__ qkv, int T, int C, float scale) {
-    constexpr int GL = HS / 16, ROWS = WA_NT / GL, TILE = HS >= 128 ? 32 : 64;
+    constexpr int GL = HS / 16, ROWS = WA_NT / GL * RQ, TILE = HS >= 128 ? 32 : 64;
     __shared__ __align__(16) float Ks[TILE * HS];
     __shared__ __align__(16) float Vs[TILE * HS];
     const int tid = threadIdx.x, sub = tid % GL;
-    const int i0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * ROWS, row = i0 + tid / GL;       // longest blocks first
+    const int i0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * ROWS, row0 = i0 + tid / GL * RQ;       // longest blocks first
     const long long ld = 3LL * C;
     const float *base = qkv + blockIdx.y * HS;
-    unsigned long long q2[8], o2[8];
-    load_query(q2, base + (long long)min(row, T - 1) * ld + sub * 16, scale);
+    unsigned long long q2[RQ][8], o2[RQ][8];
+    float m[RQ], l[RQ];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) o2[i] = 0ull;
-    float m = -INFINITY, l = 0.0f;
-    const int warp_last = min(T - 1, i0 + (tid | 31) / GL), jmax = min(T, i0 + ROWS);
+    for (int r = 0; r < RQ; ++r) {
+        load_query(q2[r], base + (long long)min(row0 + r, T - 1) * ld + sub * 16, scale);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) o2[r][i] = 0ull;
+        m[r] = -INFINITY; l[r] = 0.0f;
+    }
+    const int warp_last = min(T - 1, i0 + (tid | 31) / GL * RQ + RQ - 1), jmax = min(T, i0 + ROWS);
     for (int j0 = 0; j0 < jmax; j0 += TILE) {
         __syncthreads();
         for (int lin = tid; lin < TILE * HS / 4; lin += WA_NT) {
             const int r = lin / (HS / 4), c = lin % (HS / 4) * 4;
-            float4 k = make_float4(0.f, 0.f, 0.f, 0.f), v = k;
-            if (j0 + r < T) {
-                k = *reinterpret_cast<const float4 *>(base + (long long)(j0 + r) * ld + C + c);
-                v = *reinterpret_cast<const float4 *>(base + (long long)(j0 + r) * ld + 2 * C + c);
-            }
-            *reinterpret_cast<float4 *>(Ks + r * HS + c) = k;
-            *reinterpret_cast<float4 *>(Vs + r * HS + c) = v;
+            const bool ok = j0 + r < T;
+            const float *src = base + (long long)(ok ? j0 + r : 0) * ld + c;
+            const uint32_t k = (uint32_t)__cvta_generic_to_shared(Ks + r * HS + c), v = (uint32_t)__cvta_generic_to_shared(Vs + r * HS + c);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(k), "l"(src + C), "r"(ok ? 16 : 0) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(v), "l"(src + 2 * C), "r"(ok ? 16 : 0) : "memory");
         }
+        asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
         for (int c0 = 0; c0 < TILE && j0 + c0 <= warp_last; c0 += KC) {
-            float s[KC], cmax = -INFINITY;
+            float s[RQ][KC];
 #pragma unroll
             for (int c = 0; c < KC; ++c) {
-                const float a = score<GL>(q2, Ks + (c0 + c) * HS + sub * 16);
-                const int key = j0 + c0 + c;
-                s[c] = (key > row || key >= T) ? -INFINITY : a;
-                cmax = fmaxf(cmax, s[c]);
+                unsigned long long acc[RQ];
+#pragma unroll
+                for (int r = 0; r < RQ; ++r) acc[r] = 0ull;
+#pragma unroll
+                for (int i = 0; i < 8; i += 2) {
+                    const float4 k = *reinterpret_cast<const float4 *>(Ks + (c0 + c) * HS + sub * 16 + 2 * i);
+                    const unsigned long long k0 = pack(k.x, k.y), k1 = pack(k.z, k.w);
+#pragma unroll
+                    for (int r = 0; r < RQ; ++r) { fma2(acc[r], q2[r][i], k0); fma2(acc[r], q2[r][i + 1], k1); }
+                }
+#pragma unroll
+                for (int r = 0; r < RQ; ++r) {
+                    float lo, hi;
+                    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[r]));
+                    s[r][c] = lo + hi;
+                }
             }
-            const float mnew = fmaxf(m, cmax);
-            const bool live = mnew > -INFINITY;
-            const float resc = live ? __expf(m - mnew) : 1.0f;
-            float csum = 0.0f;
+#pragma unroll
+            for (int r = 0; r < RQ; ++r) {
+                float cmax = -INFINITY;
+#pragma unroll
+                for (int c = 0; c < KC; ++c) {
+                    float a = s[r][c];
+#pragma unroll
+                    for (int o = 1; o < GL; o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+                    const int key = j0 + c0 + c;
+                    s[r][c] = (key > row0 + r || key >= T) ? -INFINITY : a;
+                    cmax = fmaxf(cmax, s[r][c]);
+                }
+                const float mnew = fmaxf(m[r], cmax);
+                const bool live = mnew > -INFINITY;
+                const float resc = live ? __expf(m[r] - mnew) : 1.0f;
+                float csum = 0.0f;
+#pragma unroll
+                for (int c = 0; c < KC; ++c) {
+                    s[r][c] = live ? __expf(s[r][c] - mnew) : 0.0f;
+                    csum += s[r][c];
+                }
+                m[r] = mnew;
+                l[r] = l[r] * resc + csum;
+                const unsigned long long resc2 = pack(resc, resc);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    unsigned long long z = 0ull;
+                    fma2(z, o2[r][i], resc2);
+                    o2[r][i] = z;
+                }
+            }
 #pragma unroll
             for (int c = 0; c < KC; ++c) {
-                s[c] = live ? __expf(s[c] - mnew) : 0.0f;
-                csum += s[c];
-            }
-            m = mnew;
-            l = l * resc + csum;
-            const unsigned long long resc2 = pack(resc, resc);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                unsigned long long z = 0ull;
-                fma2(z, o2[i], resc2);
-                o2[i] = z;
-            }
-#pragma unroll
-            for (int c = 0; c < KC; ++c) {
-                const unsigned long long p2 = pack(s[c], s[c]);
 #pragma unroll
                 for (int i = 0; i < 8; i += 2) {
                     const float4 v = *reinterpret_cast<const float4 *>(Vs + (c0 + c) * HS + sub * 16 + 2 * i);
-                    fma2(o2[i], p2, pack(v.x, v.y));
-                    fma2(o2[i + 1], p2, pack(v.z, v.w));
+                    const unsigned long long v0 = pack(v.x, v.y), v1 = pack(v.z, v.w);
+#pragma unroll
+                    for (int r = 0; r < RQ; ++r) {
+                        const unsigned long long p2 = pack(s[r][c], s[r][c]);
+                        fma2(o2[r][i], p2, v0);
+                        fma2(o2[r][i + 1], p2, v1);
+                    }
                 }
             }
         }
     }
-    if (row >= T) return;
-    const float inv = (l > 0.0f) ? 1.0f / l : 0.0f;
-    float *dst = out + (long long)row * C + blockIdx.y * HS + sub * 16;
 #pragma unroll
-    for (int i = 0; i < 8; i += 2) {
-        float a0, a1, a2, a3;
-        asm("mov.b64 {%0, %1}, %2;" : "=f"(a0), "=f"(a1) : "l"(o2[i]));
-        asm("mov.b64 {%0, %1}, %2;" : "=f"(a2), "=f"(a3) : "l"(o2[i + 1]));
-        *reinterpret_cast<float4 *>(dst + 2 * i) = make_float4(a0 * inv, a1 * inv, a2 * inv, a3 * inv);
+    for (int r = 0; r < RQ; ++r) {
+        if (row0 + r >= T) continue;
+        const float inv = (l[r] > 0.0f) ? 1.0f / l[r] : 0.0f;
+        float *dst = out + (long long)(row0 + r) * C + blockIdx.y * HS + sub * 16;
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) {
+            float a0, a1, a2, a3;
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(a0), "=f"(a1) : "l"(o2[r][i]));
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(a2), "=f"(a3) : "l"(o2[r][i + 1]));
+            *reinterpret_cast<float4 *>(dst + 2 * i) = make_float4(a0 * inv, a1 * inv, a2 * inv, a3 * inv);
+        }
     }
 }
 
 }  // namespace
 
-// Sizes these kernels take: the attention's head sizes, a layernorm of one warp, and a context of at most 256 groups of
+// Sizes these kernels take: the attention's head sizes, a layernorm of one warp, and a context of at most 512 groups of
 // 8 keys (one a thread in decode_attention_k).
 bool decode_accepts(int T, int C, int NH) {
     const int hs = (NH > 0 && C % NH == 0) ? C / NH : 0;
@@ -349,10 +427,26 @@ int decode_gemv(float *y, const float *x, const float *W, const float *bias, con
 int decode_attention(float *y, const float *qkv, int pos, int C, int NH, cudaStream_t st) {
     const int hs = C / NH;
     const float scale = 1.0f / sqrtf((float)hs);
-    const size_t smem = (size_t)ceil_div(pos + 1, KC) * (KC + 2) * sizeof(float);
-    if (hs == 32) decode_attention_k<32><<<NH, DA_NT, smem, st>>>(y, qkv, pos, C, scale);
-    else if (hs == 64) decode_attention_k<64><<<NH, DA_NT, smem, st>>>(y, qkv, pos, C, scale);
-    else decode_attention_k<128><<<NH, DA_NT, smem, st>>>(y, qkv, pos, C, scale);
+    const size_t groups = ceil_div(pos + 1, KC), v_bytes = groups * KC * hs * sizeof(float);
+    const int stage_v = v_bytes <= DA_MAX_V;
+    const size_t smem = (stage_v ? v_bytes : 0) + groups * (KC + 2) * sizeof(float);
+    static std::mutex mu;
+    static bool set[64];
+    const int d = current_device();
+    if (d < 0 || d >= 64) return fail(BMB_E_ARG, "device index %d out of range", d);
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        const int most = DA_MAX_V + DA_NT * (KC + 2) * (int)sizeof(float);
+        if (!set[d]) {
+            BMB_CUDA(cudaFuncSetAttribute(decode_attention_k<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+            BMB_CUDA(cudaFuncSetAttribute(decode_attention_k<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+            BMB_CUDA(cudaFuncSetAttribute(decode_attention_k<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+        }
+        set[d] = true;
+    }
+    if (hs == 32) decode_attention_k<32><<<NH, DA_NT, smem, st>>>(y, qkv, pos, C, scale, stage_v);
+    else if (hs == 64) decode_attention_k<64><<<NH, DA_NT, smem, st>>>(y, qkv, pos, C, scale, stage_v);
+    else decode_attention_k<128><<<NH, DA_NT, smem, st>>>(y, qkv, pos, C, scale, stage_v);
     count_launch();
     BMB_LAUNCH_CHECK();
     return BMB_OK;
@@ -361,7 +455,7 @@ int decode_attention(float *y, const float *qkv, int pos, int C, int NH, cudaStr
 int window_attention(float *out, const float *qkv, int T, int C, int NH, cudaStream_t st) {
     const int hs = C / NH;
     const float scale = 1.0f / sqrtf((float)hs);
-    const dim3 grid(ceil_div(T, WA_NT / (hs / 16)), NH);
+    const dim3 grid(ceil_div(T, WA_NT / (hs / 16) * RQ), NH);
     if (hs == 32) window_attention_k<32><<<grid, WA_NT, 0, st>>>(out, qkv, T, C, scale);
     else if (hs == 64) window_attention_k<64><<<grid, WA_NT, 0, st>>>(out, qkv, T, C, scale);
     else window_attention_k<128><<<grid, WA_NT, 0, st>>>(out, qkv, T, C, scale);
