@@ -5,6 +5,7 @@
 #include <cstdio>
 #include <cstdarg>
 #include <cstdint>
+#include <mutex>
 #include "../../include/bmb.h"
 
 namespace bmb {
@@ -79,7 +80,7 @@ struct DpRangeList {
 // that every rank thread shares regardless of device.  Here each device owns
 // its own block, grown on demand and kept until process exit.
 // Returns nullptr (and records an error) on failure.
-enum ScratchSlot { SCR_REDUCE = 0, SCR_GEMM_A = 1, SCR_GEMM_B = 2, SCR_MISC = 3, SCR_SLOTS = 4 };
+enum ScratchSlot { SCR_REDUCE = 0, SCR_GEMM_A = 1, SCR_GEMM_B = 2, SCR_MISC = 3, SCR_SPLIT = 4, SCR_SLOTS = 5 };
 void *device_scratch(ScratchSlot slot, size_t bytes);
 // Order the users of a scratch slot across streams of one device: acquire before the first launch that writes
 // the slot, release after the last launch that reads it (both on the stream those launches go to).
@@ -106,6 +107,10 @@ constexpr int GEMM_SCRATCH_IN_CAPTURE = 1 << 20;
 constexpr int GEMM_ANY_ORDER = 1 << 21;
 // Internal flag: an fp32 product must be the sequential chain over k.
 constexpr int GEMM_CHAIN = 1 << 22;
+// SCR_SPLIT (the images of split fp32 products) is sized, handed over and used under this lock of the current device, held
+// from the scratch's address to the last launch that reads it: products of several threads and streams take turns, and the
+// block is not moved under one of them.
+std::mutex &split_mutex();
 // Internal GEMM dispatch shared by attention and the trainer: math is a
 // BMB_MATH_* value, flags the BMB_GEMM_* bits, strides in elements.
 int gemm_any(int math, int flags, int ta, int tb, int batch, int M, int N, int K, float alpha,

@@ -447,6 +447,12 @@ XPlan choose_x3(int units, int M, int N, int kblocks) {
 
 }  // namespace
 
+std::mutex &split_mutex() {
+    static std::mutex mu[64];
+    const int d = current_device();
+    return mu[d >= 0 && d < 64 ? d : 0];
+}
+
 // Takes products of 2^18 results and more with K from 192, and of 2^31 multiply-adds and more with K from 128 (measured,
 // SIMT against this: 1024x384x384 43 / 19 us, 4096x128x384 43 / 21, 4096x4096x128 89 / 76, but 2048x2048x128 29 / 33,
 // 4096x384x128 17 / 19, 4096x4096x64 50 / 70; two launches and a pass over the operands cost about 13 us whatever the
@@ -481,7 +487,8 @@ int gemm_x3(int transA, int transB, int M, int N, int K, float alpha, const floa
     volatile int *status_host = nullptr;
     BMB_TRY(status_word(&status_dev, &status_host));
     if (*status_host != 0) return fail(BMB_E_TIMEOUT, "an earlier kernel on this device gave up waiting on a barrier");
-    uint8_t *scr = (uint8_t *)device_scratch(SCR_GEMM_A, (size_t)need);
+    std::lock_guard<std::mutex> turn(split_mutex());
+    uint8_t *scr = (uint8_t *)device_scratch(SCR_SPLIT, (size_t)need);
     if (!scr) { cudaGetLastError(); return BMB_E_UNSUPPORTED; }
     oa.img = scr;
     ob.img = scr + imgA;
@@ -491,7 +498,7 @@ int gemm_x3(int transA, int transB, int M, int N, int K, float alpha, const floa
     const Result p{A, B, transA, transB, M, N, K, alpha, beta, C, bias};
     const bool even = N % 2 == 0 && (plan.parts > 1 || ((uintptr_t)C & 7) == 0);
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
-    BMB_TRY(scratch_acquire(SCR_GEMM_A, st));
+    BMB_TRY(scratch_acquire(SCR_SPLIT, st));
     split_x3_k<<<(unsigned)(na + nb), 256, 0, st>>>(oa, ob, na, K, vec_of(A, transA ? M : K), vec_of(B, transB ? K : N));
     int rc = BMB_OK;
     if (plan.bn == 256) rc = launch_x3<256>(grid, oa.img, (int)rowsA, ob.img, (int)rowsB, p, kblocks, plan.parts, w, even, status_dev, st);
@@ -506,7 +513,7 @@ int gemm_x3(int transA, int transB, int M, int N, int K, float alpha, const floa
         count_launch();
     }
     BMB_LAUNCH_CHECK();
-    return scratch_release(SCR_GEMM_A, st);
+    return scratch_release(SCR_SPLIT, st);
 }
 
 }  // namespace bmb

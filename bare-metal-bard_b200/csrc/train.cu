@@ -574,10 +574,18 @@ int run_piece(bmb_trainer *t, bmb_trainer::Piece &pc, bool eager) {
         count_launch((int)-pc.launches);        // counted again at every replay, this first one included
     }
     // the replayed fp32 products use the scratch that they were captured with: in turn with other streams' products
-    const bool uses_scratch = t->c.math == BMB_MATH_FP32;
-    if (uses_scratch) BMB_TRY(scratch_acquire(SCR_GEMM_A, t->st));
-    BMB_CUDA(cudaGraphLaunch(pc.exec, t->st));
-    if (uses_scratch) BMB_TRY(scratch_release(SCR_GEMM_A, t->st));
+    if (t->c.math == BMB_MATH_FP32) {
+        std::unique_lock<std::mutex> turn(split_mutex());
+        if (t->graph_scratch_gen != scratch_generation()) {      // moved since the step looked
+            turn.unlock();
+            return run_units(t, pc.u0, pc.u1);
+        }
+        BMB_TRY(scratch_acquire(SCR_SPLIT, t->st));
+        BMB_CUDA(cudaGraphLaunch(pc.exec, t->st));
+        BMB_TRY(scratch_release(SCR_SPLIT, t->st));
+    } else {
+        BMB_CUDA(cudaGraphLaunch(pc.exec, t->st));
+    }
     count_launch((int)pc.launches);
     return BMB_OK;
 }

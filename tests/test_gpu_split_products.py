@@ -138,3 +138,36 @@ def test_split_attention_of_infinities_and_nan(bmb, cuda, hs):
         res.append(dqkv)
     ok = cuda.isfinite(res[1])
     assert cuda.equal(cuda.isfinite(res[0]), ok) and float((res[0][ok] - res[1][ok]).abs().max()) < 2e-5
+
+
+def test_split_products_of_threads_and_streams_take_turns(bmb, cuda):
+    """Four threads, a stream each, products of different sizes (the scratch grows under way): each result is what the
+    product gives alone."""
+    import threading
+    shapes = [(1024, 1024, 512), (2048, 1024, 768), (600, 3000, 1000), (1536, 2048, 1024)]
+    work, errors = [], []
+    for i, (M, N, K) in enumerate(shapes):
+        g = cuda.Generator(device="cuda").manual_seed(i)
+        A, B = (cuda.rand(s, generator=g, device="cuda") for s in ((M, K), (K, N)))
+        alone = cuda.empty(M, N, device="cuda")
+        bmb.call("bmb_gemm_ex", bmb.MATH_FP32, 0, 0, 0, M, N, K, 1.0, A, B, 0.0, alone, None)
+        work.append((M, N, K, A, B, alone, [cuda.empty(M, N, device="cuda") for _ in range(12)], cuda.cuda.Stream()))
+    cuda.cuda.synchronize()
+
+    def run(w):
+        M, N, K, A, B, _, outs, stream = w
+        try:
+            for C in outs:
+                bmb.call("bmb_gemm_ex", bmb.MATH_FP32, 0, 0, 0, M, N, K, 1.0, A, B, 0.0, C, stream.cuda_stream)
+        except Exception as e:                     # noqa: BLE001
+            errors.append(e)
+
+    threads = [threading.Thread(target=run, args=(w,)) for w in work]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    cuda.cuda.synchronize()
+    assert not errors, errors
+    for w in work:
+        assert all(cuda.equal(C, w[5]) for C in w[6])
