@@ -139,7 +139,7 @@ struct Result {
 };
 
 // One element by the sequential chain, as the SIMT kernels have it.
-__device__ __noinline__ float element_again(const Result &p, int m, int n) {
+__device__ __forceinline__ float element_again(const Result &p, int m, int n) {
     const float *a = p.A, *b = p.B;
     const long long as = p.ta ? p.M : 1, bs = p.tb ? 1 : p.N;
     a += p.ta ? (long long)m : (long long)m * p.K;
@@ -152,7 +152,8 @@ __device__ __noinline__ float element_again(const Result &p, int m, int n) {
     return s;
 }
 __device__ __forceinline__ bool not_finite(float x) { return !(fabsf(x) <= 3.402823466e38f); }
-__device__ __forceinline__ void put_element(const Result &p, int m, int n, float s) {
+// Out of line: a call in the middle of the 128 sums of an epilogue thread would cost registers that there are not.
+__device__ __noinline__ void put_element(const Result &p, int m, int n, float s) {
     if (not_finite(s)) s = element_again(p, m, n);
     float *c = p.C + (size_t)m * p.N + n;
     float o = p.alpha * s;
@@ -305,12 +306,15 @@ gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict
                 const uint32_t trow = tmem_base + (uint32_t)(acc * BN + half * (BN / 2)) + ((uint32_t)(q * 32) << 16);
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
-                    float lo[16], hi[16];
-                    tmem_ld_16x256b_x4_nowait(trow + (uint32_t)(c * 32), lo);
-                    tmem_ld_16x256b_x4_nowait(trow + (uint32_t)(c * 32) + (16u << 16), hi);
+                    float v[16];
+                    tmem_ld_16x256b_x4_nowait(trow + (uint32_t)(c * 32), v);
                     tmem_wait_ld();
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) { sum[c][i] += lo[i]; sum[c][16 + i] += hi[i]; }
+                    for (int i = 0; i < 16; ++i) sum[c][i] += v[i];
+                    tmem_ld_16x256b_x4_nowait(trow + (uint32_t)(c * 32) + (16u << 16), v);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) sum[c][16 + i] += v[i];
                 }
                 fence_before();
                 __syncwarp();
@@ -319,37 +323,69 @@ gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict
             }
             if (!ok) break;
             const int m0 = tm * XM + q * 32 + (lane >> 2), nb = tn * BN + half * (BN / 2) + 2 * (lane & 3);
-            float *W = parts > 1 ? ws + (long long)part * p.M * p.N : nullptr;
+            float *D = parts > 1 ? ws + (long long)part * p.M * p.N : p.C;
+            const float alpha = parts > 1 ? 1.0f : p.alpha, beta = parts > 1 ? 0.0f : p.beta;
+            const float *bias = parts > 1 ? nullptr : p.bias;
+            // sum[c] of row m0 + 8k and columns nb + 32c + 8j, + 1
+            auto value = [&](int c, int j, int k) { return make_float2(sum[c][(k >> 1) * 16 + 4 * j + 2 * (k & 1)], sum[c][(k >> 1) * 16 + 4 * j + 2 * (k & 1) + 1]); };
+            // Nothing hides this end (the next tile's sums need these registers), so the common case is a multiply and a
+            // store per pair: a whole tile, aligned, all sums finite (0 * x is NaN for those that are not).
+            float probe = 0.0f;
 #pragma unroll
             for (int c = 0; c < NC; ++c)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int n = nb + c * 32 + 8 * j;
+                for (int i = 0; i < 32; ++i) probe = fmaf(sum[c][i], 0.0f, probe);
+            if (vec && (tm + 1) * XM <= p.M && (tn + 1) * BN <= p.N && (probe == 0.0f || parts > 1)) {
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {            // rows m0, +8, +16, +24
-                        const int m = m0 + 8 * k;
-                        const float x = sum[c][(k >> 1) * 16 + 4 * j + 2 * (k & 1)], y = sum[c][(k >> 1) * 16 + 4 * j + 2 * (k & 1) + 1];
-                        if (m >= p.M || n >= p.N) continue;
-                        if (parts > 1) {
-                            float *w = W + (size_t)m * p.N + n;
-                            if (vec) *reinterpret_cast<float2 *>(w) = make_float2(x, y);
-                            else { w[0] = x; if (n + 1 < p.N) w[1] = y; }
-                        } else if (vec && !not_finite(x) && !not_finite(y)) {
-                            float2 *cp = reinterpret_cast<float2 *>(p.C + (size_t)m * p.N + n);
-                            float2 o = make_float2(p.alpha * x, p.alpha * y);
-                            if (p.beta != 0.0f) {
-                                const float2 old = *cp;
-                                o.x = fmaf(p.beta, old.x, o.x);
-                                o.y = fmaf(p.beta, old.y, o.y);
+                for (int k = 0; k < 4; ++k) {
+                    float *row = D + (size_t)(m0 + 8 * k) * p.N + nb;
+                    if (beta == 0.0f && !bias) {
+#pragma unroll
+                        for (int c = 0; c < NC; ++c)
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const float2 x = value(c, j, k);
+                                *reinterpret_cast<float2 *>(row + c * 32 + 8 * j) = make_float2(alpha * x.x, alpha * x.y);
                             }
-                            if (p.bias) { o.x += __ldg(p.bias + n); o.y += __ldg(p.bias + n + 1); }
-                            *cp = o;
-                        } else {
-                            put_element(p, m, n, x);
-                            if (n + 1 < p.N) put_element(p, m, n + 1, y);
-                        }
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < NC; ++c)
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const float2 x = value(c, j, k);
+                                float2 *d = reinterpret_cast<float2 *>(row + c * 32 + 8 * j), o = make_float2(alpha * x.x, alpha * x.y);
+                                if (beta != 0.0f) {
+                                    const float2 old = *d;
+                                    o.x = fmaf(beta, old.x, o.x);
+                                    o.y = fmaf(beta, old.y, o.y);
+                                }
+                                if (bias) { o.x += __ldg(bias + nb + c * 32 + 8 * j); o.y += __ldg(bias + nb + c * 32 + 8 * j + 1); }
+                                *d = o;
+                            }
                     }
                 }
+            } else {
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int n = nb + c * 32 + 8 * j;
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const int m = m0 + 8 * k;
+                            const float2 x = value(c, j, k);
+                            if (m >= p.M || n >= p.N) continue;
+                            if (parts > 1) {
+                                float *w = D + (size_t)m * p.N + n;
+                                w[0] = x.x;
+                                if (n + 1 < p.N) w[1] = x.y;
+                            } else {
+                                put_element(p, m, n, x.x);
+                                if (n + 1 < p.N) put_element(p, m, n + 1, x.y);
+                            }
+                        }
+                    }
+            }
         }
     }
 
