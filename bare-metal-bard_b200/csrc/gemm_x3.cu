@@ -11,8 +11,8 @@
 // Against a 64-bit product this is closer than the sequential multiply-adds of the SIMT kernels at every size it
 // takes (uniform operands, 2-norm: K = 16 4.9e-8 against 7.4e-8, 1024 1.2e-7 against 5.7e-7, 8192 2.2e-7 against 1.6e-6).
 //
-// Measured on B200, split pass included, SIMT kernels -> this: 4096^3 2445 -> 629 us (219 TFLOP/s of fp32 products),
-// 8192x3072x768 (NT) 747 -> 224, 768x768x8192 (TN) 658 -> 78, 8192x50304x768 (NT) 11.5 -> 3.1 ms.
+// Measured on B200, split pass included, SIMT kernels -> this: 4096^3 2445 -> 585 us (235 TFLOP/s of fp32 products),
+// 8192x3072x768 (NT) 747 -> 178, 768x768x8192 (TN) 658 -> 76, 8192x50304x768 (NT) 11.5 -> 2.6 ms.
 //
 // Two or three launches: split_x3_k writes both operands as images of the slices the product reads, gemm_x3_k
 // multiplies, and where K is shared among CTAs reduce_x3_k adds the parts in a fixed order (no atomics: two calls
@@ -40,7 +40,7 @@ constexpr int XM = 128;                     // rows of a tile
 constexpr int XA_BYTES = 3 * XM * ROWB;     // 24 KB per slice
 constexpr int X_THREADS = 320;              // producer warp, issuer warp, 8 epilogue warps
 __host__ __device__ constexpr int x_stage_bytes(int bn) { return XA_BYTES + 3 * bn * ROWB; }
-__host__ __device__ constexpr int x_stages(int bn) { return bn == 256 ? 3 : bn == 128 ? 4 : 5; }
+__host__ __device__ constexpr int x_stages(int bn) { return bn >= 192 ? 3 : bn == 128 ? 4 : 5; }
 __host__ __device__ constexpr int x_smem_bytes(int bn) { return x_stages(bn) * x_stage_bytes(bn) + 1024 + 256; }
 
 __host__ __device__ inline long long round_up(long long a, long long b) { return (a + b - 1) / b * b; }
@@ -202,7 +202,7 @@ template <int BN>
 __global__ void __launch_bounds__(X_THREADS, 1)
 gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict__ imgB, int rowsB, const Result p, int kblocks, int parts, float *__restrict__ ws, int vec, int *__restrict__ status) {
     constexpr int STAGES = x_stages(BN), STAGE = x_stage_bytes(BN), PA = XM * ROWB, PB = BN * ROWB;
-    constexpr uint32_t TCOLS = 2 * BN;
+    constexpr uint32_t ACC = BN == 192 ? 256 : BN, TCOLS = 2 * ACC;      // (allocations are powers of two)
     constexpr int NC = BN / 64;                     // 32-column chunks per epilogue warp (half of the columns)
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -272,7 +272,7 @@ gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict
                 for (int kb = kb0; kb < kb1; ++kb) {
                     if (!mbar_wait(tempty0 + 8 * acc, acc_ph ^ 1, giveup) || !mbar_wait(full0 + 8 * s, ph, giveup)) { ok = false; break; }
                     fence_after();
-                    const uint32_t d = tmem_base + (uint32_t)acc * BN;
+                    const uint32_t d = tmem_base + (uint32_t)acc * ACC;
                     const uint32_t sa = base + s * STAGE, sb = sa + XA_BYTES;
                     // pieces of A and B, smallest terms first
                     constexpr int TA[6] = {2, 0, 1, 1, 0, 0}, TB[6] = {0, 2, 1, 0, 1, 0};
@@ -303,7 +303,7 @@ gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict
             for (int kb = kb0; kb < kb1; ++kb) {
                 if (!mbar_wait(tfull0 + 8 * acc, acc_ph, giveup)) { ok = false; break; }
                 fence_after();
-                const uint32_t trow = tmem_base + (uint32_t)(acc * BN + half * (BN / 2)) + ((uint32_t)(q * 32) << 16);
+                const uint32_t trow = tmem_base + acc * ACC + half * (BN / 2) + ((uint32_t)(q * 32) << 16);
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
                     float v[16];
@@ -375,14 +375,31 @@ gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict
                             const int m = m0 + 8 * k;
                             const float2 x = value(c, j, k);
                             if (m >= p.M || n >= p.N) continue;
+                            const bool second = n + 1 < p.N;
+                            float *d = D + (size_t)m * p.N + n;
                             if (parts > 1) {
-                                float *w = D + (size_t)m * p.N + n;
-                                w[0] = x.x;
-                                if (n + 1 < p.N) w[1] = x.y;
-                            } else {
-                                put_element(p, m, n, x.x);
-                                if (n + 1 < p.N) put_element(p, m, n + 1, x.y);
+                                d[0] = x.x;
+                                if (second) d[1] = x.y;
+                                continue;
                             }
+                            // (256 columns: one sum more in registers than there are, so edges take the call, which is slow
+                            // and which the choice of a plan counts)
+                            if (BN == 256 || probe != 0.0f) {
+                                put_element(p, m, n, x.x);
+                                if (second) put_element(p, m, n + 1, x.y);
+                                continue;
+                            }
+                            float2 o = make_float2(alpha * x.x, alpha * x.y);
+                            if (beta != 0.0f) {
+                                o.x = fmaf(beta, d[0], o.x);
+                                if (second) o.y = fmaf(beta, d[1], o.y);
+                            }
+                            if (bias) {
+                                o.x += __ldg(bias + n);
+                                if (second) o.y += __ldg(bias + n + 1);
+                            }
+                            if (vec) *reinterpret_cast<float2 *>(d) = o;        // (N is even: there is a second)
+                            else { d[0] = o.x; if (second) d[1] = o.y; }
                         }
                     }
             }
@@ -461,19 +478,23 @@ int launch_x3(int grid, const uint8_t *imgA, int rowsA, const uint8_t *imgB, int
 }
 
 struct XPlan { int bn, parts; };
+// Widths (us, 256 / 192 / 128 / 64 columns): 8192x768x768 70 / 62 / 75 / 118, 8192x2304x768 132 / 151 / 175 / 284,
+// 4096x1536x384 42 / 37 / 44 / 64, 4096x1152x384 60 / 37 / 33 / 48, 512^3 23 / 22 / 21 / 19.
 // Cycles of a plan: rounds of items over the SMs, each its slices plus the end that the next item's products do
 // not hide, and the pass that adds the parts (its traffic stays in L2: about 3 KB a cycle, and a launch).
 XPlan choose_x3(int units, int M, int N, int kblocks) {
-    const int widths[3] = {256, 128, 64};
-    const double slice[3] = {1750, 1180, 880}, tail[3] = {2600, 1600, 1100};
+    const int widths[4] = {256, 192, 128, 64};
+    const double slice[4] = {1750, 1450, 1180, 880}, tail[4] = {1300, 1050, 800, 600};
     XPlan best{128, 1};
     double best_t = 1e300;
-    for (int w = 0; w < 3; ++w) {
+    for (int w = 0; w < 4; ++w) {
         const long long tiles = (long long)ceil_div(M, XM) * ceil_div(N, widths[w]);
+        const bool ragged = M % XM || N % widths[w];
         for (int s = 1; s <= 16; ++s) {
             if (s > 1 && kblocks / s < 4) break;
             const double rounds = (double)ceil_div(tiles * s, units);
             double t = rounds * (ceil_div(kblocks, s) * slice[w] + tail[w]) + 3000;
+            if (s == 1 && ragged && widths[w] == 256) t += 40000;      // (2000 x 2000 x 500: 58 us, 42 with 128 columns)
             if (s > 1) t += 4000 + (double)M * N * 4 * (2 * s + 1) / 3000;
             if (t < best_t) { best_t = t; best = {widths[w], s}; }
         }
@@ -538,6 +559,7 @@ int gemm_x3(int transA, int transB, int M, int N, int K, float alpha, const floa
     split_x3_k<<<(unsigned)(na + nb), 256, 0, st>>>(oa, ob, na, K, vec_of(A, transA ? M : K), vec_of(B, transB ? K : N));
     int rc = BMB_OK;
     if (plan.bn == 256) rc = launch_x3<256>(grid, oa.img, (int)rowsA, ob.img, (int)rowsB, p, kblocks, plan.parts, w, even, status_dev, st);
+    else if (plan.bn == 192) rc = launch_x3<192>(grid, oa.img, (int)rowsA, ob.img, (int)rowsB, p, kblocks, plan.parts, w, even, status_dev, st);
     else if (plan.bn == 128) rc = launch_x3<128>(grid, oa.img, (int)rowsA, ob.img, (int)rowsB, p, kblocks, plan.parts, w, even, status_dev, st);
     else rc = launch_x3<64>(grid, oa.img, (int)rowsA, ob.img, (int)rowsB, p, kblocks, plan.parts, w, even, status_dev, st);
     if (rc != BMB_OK) return rc;
