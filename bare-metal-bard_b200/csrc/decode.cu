@@ -10,13 +10,35 @@
 // model that samples in a loop stay) and by the chain, 4 cycles a step. So 32 outputs a block, one lane each, rows of
 // weights copied to shared memory ahead of it, and what stands before or after the product (layernorm, residual, GELU)
 // rides in the same launch: five launches a layer. Measured at 6 layers of 6 heads x 64,
-// 256 positions: a text of 300 tokens, 45 of them past the context, 1075 -> 102 ms (the whole batch of 16 x 256 rows each token before).
+// 256 positions: a text of 300 tokens, 45 of them past the context, 1075 -> 82 ms (the whole batch of 16 x 256 rows each token before).
 #include "common.cuh"
 #include <cmath>
 #include <mutex>
 
 namespace bmb {
 namespace {
+
+// The launches of one position form a chain in which each kernel may start while the one before it still runs: it lets its
+// successor start at once, copies what does not depend on its predecessor (weights, earlier positions' values), and then
+// waits for the predecessor's end -- so every kernel has waited for all before it when it ends.
+__device__ __forceinline__ void let_successor_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... P, typename... A>
+int launch_in_chain(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    BMB_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+    count_launch();
+    return BMB_OK;
+}
 
 // a warp that follows the chains and four that copy weights ahead of it; rows 4 banks apart
 constexpr int GV_OUT = 32, GV_NT = 160, GV_CP = 128, GV_K = 128, GV_PITCH = GV_K + 4, GV_STAGES = 8;
@@ -46,8 +68,10 @@ __global__ void __launch_bounds__(GV_NT) decode_gemv_k(float *__restrict__ y, co
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    let_successor_start();
 #pragma unroll
     for (int i = 0; i < GV_STAGES - 1; ++i) fetch(i);
+    wait_for_predecessor();
     if (!ln_w) {
         for (int i = threadIdx.x * 4; i < in; i += GV_NT * 4) *reinterpret_cast<float4 *>(v + i) = *reinterpret_cast<const float4 *>(x + i);
     } else if (warp == 0) {
@@ -186,14 +210,18 @@ __global__ void __launch_bounds__(DA_NT) decode_attention_k(float *__restrict__ 
     const long long ld = 3LL * C;
     const float *base = qkv + blockIdx.x * HS;
     const int sub = tid % GL;
+    let_successor_start();
     if (stage_v) {
+        bool waited = false;                                     // the newest position's row comes from the predecessor
         for (int i = tid; i < groups * KC * HS / 4; i += DA_NT) {
             const int j = i / (HS / 4), c = i % (HS / 4) * 4;
+            if (j >= pos && !waited) { wait_for_predecessor(); waited = true; }
             const uint32_t d = (uint32_t)__cvta_generic_to_shared(vs + j * HS + c);
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(base + (long long)min(j, pos) * ld + 2 * C + c),
                          "r"(j < n ? 16 : 0) : "memory");
         }
     }
+    wait_for_predecessor();
     unsigned long long q2[8];
     load_query(q2, base + (long long)pos * ld + sub * 16, scale);
 #pragma unroll 2
@@ -418,10 +446,7 @@ int decode_gemv(float *y, const float *x, const float *W, const float *bias, con
         if (!set[d]) BMB_CUDA(cudaFuncSetAttribute(decode_gemv_k, cudaFuncAttributeMaxDynamicSharedMemorySize, GV_SMEM));
         set[d] = true;
     }
-    decode_gemv_k<<<ceil_div(out, GV_OUT), GV_NT, GV_SMEM, st>>>(y, x, W, bias, ln_w, ln_b, add, in, out, gelu ? 1 : 0);
-    count_launch();
-    BMB_LAUNCH_CHECK();
-    return BMB_OK;
+    return launch_in_chain(decode_gemv_k, ceil_div(out, GV_OUT), GV_NT, GV_SMEM, st, y, x, W, bias, ln_w, ln_b, add, in, out, gelu ? 1 : 0);
 }
 
 int decode_attention(float *y, const float *qkv, int pos, int C, int NH, cudaStream_t st) {
@@ -444,12 +469,9 @@ int decode_attention(float *y, const float *qkv, int pos, int C, int NH, cudaStr
         }
         set[d] = true;
     }
-    if (hs == 32) decode_attention_k<32><<<NH, DA_NT, smem, st>>>(y, qkv, pos, C, scale, stage_v);
-    else if (hs == 64) decode_attention_k<64><<<NH, DA_NT, smem, st>>>(y, qkv, pos, C, scale, stage_v);
-    else decode_attention_k<128><<<NH, DA_NT, smem, st>>>(y, qkv, pos, C, scale, stage_v);
-    count_launch();
-    BMB_LAUNCH_CHECK();
-    return BMB_OK;
+    if (hs == 32) return launch_in_chain(decode_attention_k<32>, NH, DA_NT, smem, st, y, qkv, pos, C, scale, stage_v);
+    if (hs == 64) return launch_in_chain(decode_attention_k<64>, NH, DA_NT, smem, st, y, qkv, pos, C, scale, stage_v);
+    return launch_in_chain(decode_attention_k<128>, NH, DA_NT, smem, st, y, qkv, pos, C, scale, stage_v);
 }
 
 int window_attention(float *out, const float *qkv, int T, int C, int NH, cudaStream_t st) {
