@@ -80,6 +80,7 @@ int bmb_gemm(int transA, int transB, int M, int N, int K, float alpha, const flo
 int bmb_gemm_ex(int math, int flags, int transA, int transB, int M, int N, int K, float alpha,
                 const float *A, const float *B, float beta, float *C, void *stream) {
     if (math < BMB_MATH_FP32 || math > BMB_MATH_BF16) return fail(BMB_E_ARG, "gemm_ex: math %d", math);
+    flags &= GEMM_SCRATCH_IN_CAPTURE - 1;                    // the bits above are the library's own
     return gemm_any(math, flags, transA, transB, 1, M, N, K, alpha, A, 0, B, 0, beta, C, 0,
                     (cudaStream_t)stream);
 }
@@ -88,6 +89,7 @@ int bmb_gemm_bias_gelu(int math, int flags, int M, int N, int K, const float *A,
                        float *C, float *C_gelu, void *stream) {
     if (math < BMB_MATH_FP32 || math > BMB_MATH_BF16) return fail(BMB_E_ARG, "gemm_bias_gelu: math %d", math);
     if (!A || !W || !C || !C_gelu || M < 1 || N < 1 || K < 1) return fail(BMB_E_ARG, "gemm_bias_gelu: bad argument");
+    flags &= GEMM_SCRATCH_IN_CAPTURE - 1;
     const bool was = emit_rounded();
     set_emit_rounded((flags & BMB_GEMM_AUX_ROUNDED) != 0);
     const int rc = gemm_any_bias(math, flags & ~BMB_GEMM_AUX_ROUNDED, 0, 1, 1, M, N, K, 1.0f, A, 0, W, 0, 0.0f, C, 0, bias,

@@ -20,8 +20,8 @@
 //
 // Image of an operand of R rows (whatever its transposition, the split pass turns it): [K/32][3 pieces][Rp rows]
 // of 64-byte rows (32 bf16 of K) in the 64-byte swizzle that the matrix descriptor names, so that one piece of
-// one slice of a tile is one contiguous bulk copy and needs no tensor map.  K is filled up with zeros; rows past R
-// are never written and only reach columns or rows of the tile that are not stored.
+// one slice of a tile is one contiguous bulk copy and needs no tensor map.  K and the rows of the
+// last tile are filled up with zeros.
 //
 // Infinities and NaN: a_i b_j of the pieces of an infinite operand gives NaN where the fp32 product is infinite,
 // and a sum may overflow in another order.  An element whose sum comes out not finite is therefore computed again
@@ -119,13 +119,11 @@ __global__ void __launch_bounds__(256) split_x3_k(const Operand a, const Operand
         uint32_t p1[4], p2[4], p3[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) split3(v[2 * i], v[2 * i + 1], p1[i], p2[i], p3[i]);
-        if (r < o.rows_pad) {
-            const long long piece = (long long)o.rows_pad * ROWB;
-            uint8_t *d = img + (long long)ks * 3 * piece + (long long)r * ROWB + ((unit ^ ((r >> 1) & 3)) << 4);
-            *reinterpret_cast<uint4 *>(d) = make_uint4(p1[0], p1[1], p1[2], p1[3]);
-            *reinterpret_cast<uint4 *>(d + piece) = make_uint4(p2[0], p2[1], p2[2], p2[3]);
-            *reinterpret_cast<uint4 *>(d + 2 * piece) = make_uint4(p3[0], p3[1], p3[2], p3[3]);
-        }
+        const long long piece = (long long)o.rows_pad * ROWB;
+        uint8_t *d = img + (long long)ks * 3 * piece + (long long)r * ROWB + ((unit ^ ((r >> 1) & 3)) << 4);
+        *reinterpret_cast<uint4 *>(d) = make_uint4(p1[0], p1[1], p1[2], p1[3]);
+        *reinterpret_cast<uint4 *>(d + piece) = make_uint4(p2[0], p2[1], p2[2], p2[3]);
+        *reinterpret_cast<uint4 *>(d + 2 * piece) = make_uint4(p3[0], p3[1], p3[2], p3[3]);
     }
 }
 
@@ -536,8 +534,8 @@ int gemm_x3(int transA, int transB, int M, int N, int K, float alpha, const floa
     const long long ws = plan.parts > 1 ? (long long)plan.parts * M * N * 4 : 0;
     const long long tiles = (long long)ceil_div(M, XM) * ceil_div(N, plan.bn) * plan.parts;
     const long long need = imgA + imgB + ws;              // every one a multiple of 256 bytes but the last
-    Operand oa{A, nullptr, M, (int)rowsA, transA ? 0 : 1, ceil_div(M, 64), ceil_div(kblocks, KG)};
-    Operand ob{B, nullptr, N, (int)rowsB, transB ? 1 : 0, ceil_div(N, 64), ceil_div(kblocks, KG)};
+    Operand oa{A, nullptr, M, (int)rowsA, transA ? 0 : 1, (int)(rowsA / 64), ceil_div(kblocks, KG)};
+    Operand ob{B, nullptr, N, (int)rowsB, transB ? 1 : 0, (int)(rowsB / 64), ceil_div(kblocks, KG)};
     const long long na = (long long)oa.panels * oa.kgroups, nb = (long long)ob.panels * ob.kgroups;
     if (tiles >= (1LL << 30) || na + nb >= (1LL << 31) || need > (16LL << 30)) return BMB_E_UNSUPPORTED;
     int *status_dev = nullptr;
