@@ -174,12 +174,13 @@ __device__ __noinline__ void fwd_rows_again(float *smem, float *out, float *lse,
 // at a time, two buffers, the next 32 copied while these are multiplied.  Scores, probabilities and output stay in
 // registers; the running maximum moves once per 32 keys.  Bound by the tensor pipe: 3 instructions of 8 cycles for 8
 // keys x 8 columns x 16 rows in either product, beside which the splits take about half of the issue slots.
-// (the tensor pipe is about half busy: two to three warps a scheduler do not cover the latency of splits and products.)
-// Measured, the kernel before (4 rows x 16 columns a thread on the FMA pipe) -> this: B8 T1024 12 heads of 64 936 -> 262 us,
-// B4 T2048 8 x 128 3608 -> 670, B2 T777 12 x 32 191 -> 45, B1 T64 2 x 32 18.9 -> 7.6.  2-norm errors against 64 bits there:
+// (the tensor pipe is about half busy: two to three warps a scheduler do not cover the latency of splits and products; more
+// registers a thread, for more of them under way, are worth more than a third block: 1 x 2048 x 4 x 64 124 -> 105 us.)
+// Measured, the kernel before (4 rows x 16 columns a thread on the FMA pipe) -> this: B8 T1024 12 heads of 64 936 -> 253 us,
+// B4 T2048 8 x 128 3608 -> 670, B2 T777 12 x 32 191 -> 42, B1 T64 2 x 32 18.9 -> 7.6.  2-norm errors against 64 bits there:
 // 2.7e-7 -> 1.8e-7, 3.5e-7 -> 2.1e-7, 2.5e-7 -> 1.9e-7, 1.1e-7 -> 1.4e-7.
 template <int HS>
-__global__ void __launch_bounds__(128, HS == 128 ? 2 : HS == 64 ? 3 : 4)
+__global__ void __launch_bounds__(128, HS == 32 ? 3 : 2)
 flash_fwd_mma_k(float *__restrict__ out, float *__restrict__ lse, const float *__restrict__ qkv, int T, int NH, float scale) {
     extern __shared__ __align__(16) float smem[];
     float *Qs = smem, *Ks = Qs + 64 * HS, *Vs = Ks + 2 * 32 * HS;      // Ks, Vs: two buffers each
@@ -650,10 +651,10 @@ __device__ __forceinline__ void bwd_kv_mma(float *__restrict__ smem, float *__re
 
 // Both in one grid (one partly filled last wave instead of two), the longest blocks first: the first key block has all
 // queries, the last query block all keys.
-// Measured with D, row-group kernels -> this: B8 T1024 12 heads of 64 2436 -> 960 us, B4 T2048 8 x 128 18754 -> 2504,
-// B2 T777 12 x 32 445 -> 118.  2-norm errors of dq / dk / dv against 64 bits at 8 x 128: 4.9 / 10.8 / 10.8e-7 -> 3.3 / 3.7 / 3.3e-7.
+// Measured with D, row-group kernels -> this: B8 T1024 12 heads of 64 2436 -> 937 us, B4 T2048 8 x 128 18754 -> 2504,
+// B2 T777 12 x 32 445 -> 105.  2-norm errors of dq / dk / dv against 64 bits at 8 x 128: 4.9 / 10.8 / 10.8e-7 -> 3.3 / 3.7 / 3.3e-7.
 template <int HS>
-__global__ void __launch_bounds__(bwd_warps<HS>::value * 32, HS == 128 ? 1 : HS == 64 ? 3 : 4)
+__global__ void __launch_bounds__(bwd_warps<HS>::value * 32, HS == 128 ? 1 : HS == 64 ? 2 : 3)
 flash_bwd_mma_k(float *__restrict__ dqkv, const float *__restrict__ qkv, const float *__restrict__ dout,
                 const float *__restrict__ lse, const float *__restrict__ dsum, int T, int NH, float scale) {
     extern __shared__ __align__(16) float smem[];
