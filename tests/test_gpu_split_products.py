@@ -140,9 +140,11 @@ def test_split_attention_of_infinities_and_nan(bmb, cuda, hs):
     assert cuda.equal(cuda.isfinite(res[0]), ok) and float((res[0][ok] - res[1][ok]).abs().max()) < 2e-5
 
 
-def test_split_products_of_threads_and_streams_take_turns(bmb, cuda):
+@pytest.mark.parametrize("per_thread", [False, True])
+def test_split_products_of_threads_and_streams_take_turns(bmb, cuda, per_thread):
     """Four threads, a stream each, products of different sizes (the scratch grows under way): each result is what the
-    product gives alone."""
+    product gives alone.  Also on cudaStreamPerThread: one handle, a stream of its own in each thread."""
+    handle = lambda s: 2 if per_thread else s.cuda_stream                  # noqa: E731
     import threading
     shapes = [(1024, 1024, 512), (2048, 1024, 768), (600, 3000, 1000), (1536, 2048, 1024)]
     work, errors = [], []
@@ -158,7 +160,7 @@ def test_split_products_of_threads_and_streams_take_turns(bmb, cuda):
         M, N, K, A, B, _, outs, stream = w
         try:
             for C in outs:
-                bmb.call("bmb_gemm_ex", bmb.MATH_FP32, 0, 0, 0, M, N, K, 1.0, A, B, 0.0, C, stream.cuda_stream)
+                bmb.call("bmb_gemm_ex", bmb.MATH_FP32, 0, 0, 0, M, N, K, 1.0, A, B, 0.0, C, handle(stream))
         except Exception as e:                     # noqa: BLE001
             errors.append(e)
 
