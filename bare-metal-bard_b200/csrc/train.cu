@@ -187,7 +187,7 @@ int collect_profile(bmb_trainer *t) {
 // One matmul of the model, optionally bracketed by events.
 int mm(bmb_trainer *t, int flags, int ta, int tb, int M, int N, int K, const float *A, const float *B,
        float beta, float *C, const float *bias = nullptr, cudaStream_t on = nullptr, float *aux_gelu = nullptr) {
-    flags |= GEMM_SCRATCH_IN_CAPTURE | GEMM_ANY_ORDER;          // (GEMM_CHAIN outranks them)
+    if (t->c.math == BMB_MATH_FP32) flags |= GEMM_SCRATCH_IN_CAPTURE | GEMM_ANY_ORDER;          // (GEMM_CHAIN outranks them)
     if (on) return gemm_any_bias(t->c.math, flags, ta, tb, 1, M, N, K, 1.0f, A, 0, B, 0, beta, C, 0, bias, on, aux_gelu);
     if (t->prof) {
         if (t->ev_used + 2 > t->ev.size()) {
