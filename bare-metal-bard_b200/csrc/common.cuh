@@ -86,6 +86,16 @@ void *device_scratch(ScratchSlot slot, size_t bytes);
 // the slot, release after the last launch that reads it (both on the stream those launches go to).
 int scratch_acquire(ScratchSlot slot, cudaStream_t st);
 int scratch_release(ScratchSlot slot, cudaStream_t st);
+// The release of a block that a call has acquired, at the call's end (its last launch reads the block).
+struct ScratchRelease {
+    ScratchSlot slot;
+    cudaStream_t st;
+    bool on;
+    ~ScratchRelease() { if (on) scratch_release(slot, st); }
+};
+// The slots (bit 1 << slot) that this thread's calls have taken blocks of since the last call of this function: what a
+// captured graph holds, so that its replays can take their turn at them.
+unsigned scratch_slots_taken();
 // Counts the times any scratch block of the current device was (re)allocated.  A caller that keeps
 // scratch addresses beyond one call (the trainer's captured graph) compares it before reusing them.
 unsigned long long scratch_generation();

@@ -32,7 +32,7 @@
 
 namespace bmb {
 int launch_flash_dsum(float *dsum, const float *dout, const float *out, int B, int T, int NH, int HS, cudaStream_t st);
-float *column_partial_rows(size_t floats, bool *deferred);
+float *column_partial_rows(size_t floats, bool *deferred, cudaStream_t st);
 int column_sum_finish(bool deferred, float *dst, const float *partial, int G, int ncols, cudaStream_t st);
 
 namespace {
@@ -894,7 +894,7 @@ int flash_backward_tc(float *dqkv, float *dsum, const float *dout, const float *
     bool deferred = false;
     float *colpart = nullptr;
     if (dbias_qkv) {
-        colpart = column_partial_rows((size_t)part_rows * 3 * C, &deferred);
+        colpart = column_partial_rows((size_t)part_rows * 3 * C, &deferred, st);
         if (!colpart) return BMB_E_CUDA;
     }
     flash_bwd_tc_k<<<grid, dkv::THREADS, dkv::SMEM, st>>>(qk64, qn64, gk64, gn64, dmap, lse, dsum, T, NH, scale, emit_rounded() ? 1 : 0, status_dev,

@@ -752,7 +752,8 @@ int launch_column_add_jobs(const ColumnAddJob *jobs_dev, int njobs, int max_cols
 namespace {
 // Partial rows for a two-stage sum: from the installed collector's arena, else from the per-device scratch.
 // *deferred says which; a full arena or job list falls back to the scratch (and an immediate sum) for that call.
-float *partial_rows(size_t floats, bool *deferred) {
+// Scratch rows are acquired for `st`; the caller releases them behind the sum.
+float *partial_rows(size_t floats, bool *deferred, cudaStream_t st) {
     ColumnAddCollector *cc = g_collector;
     *deferred = false;
     if (cc && cc->njobs < cc->max_jobs) {
@@ -764,7 +765,8 @@ float *partial_rows(size_t floats, bool *deferred) {
             return p;
         }
     }
-    return (float *)device_scratch(SCR_REDUCE, floats * sizeof(float));
+    float *p = (float *)device_scratch(SCR_REDUCE, floats * sizeof(float));
+    return p && scratch_acquire(SCR_REDUCE, st) == BMB_OK ? p : nullptr;
 }
 // Finish a two-stage sum now, or note it for the batched launch.
 int finish_column_sum(bool deferred, float *dst, float *dst2, int ncols_first, const float *partial, int G, int ncols,
@@ -795,8 +797,9 @@ int finish_column_sum(bool deferred, float *dst, float *dst2, int ncols_first, c
 // Column sums whose partial rows another kernel's epilogue leaves (the attention backward, for the qkv bias): where
 // those rows go (the deferred-sum arena while a collector is installed, else per-device scratch) and how the sum into
 // dst (+=) is finished (noted for the batched launch, or launched now).
-float *column_partial_rows(size_t floats, bool *deferred) { return partial_rows(floats, deferred); }
+float *column_partial_rows(size_t floats, bool *deferred, cudaStream_t st) { return partial_rows(floats, deferred, st); }
 int column_sum_finish(bool deferred, float *dst, const float *partial, int G, int ncols, cudaStream_t st) {
+    const ScratchRelease release{SCR_REDUCE, st, !deferred};
     return finish_column_sum(deferred, dst, nullptr, ncols, partial, G, ncols, st);
 }
 
@@ -924,8 +927,9 @@ int bmb_layernorm_backward_colsum(float *dinp, float *dweight, float *dbias, flo
     }
     const int G = layernorm_bwd_blocks(N);
     bool deferred = false;
-    float *partial = partial_rows((size_t)G * 3 * C, &deferred);
+    float *partial = partial_rows((size_t)G * 3 * C, &deferred, st);
     if (!partial) return BMB_E_CUDA;
+    const ScratchRelease release{SCR_REDUCE, st, !deferred};
     return layernorm_backward_with_scratch(dinp, dweight, dbias, dout, inp, weight, mean, rstd, N, C, partial, G, st, dcolsum, deferred);
 }
 
@@ -939,14 +943,17 @@ int bmb_layernorm_backward(float *dinp, float *dweight, float *dbias, const floa
     if (fast) {
         const int G = layernorm_bwd_blocks(N);
         bool deferred = false;
-        float *partial = partial_rows((size_t)G * 2 * C, &deferred);
+        float *partial = partial_rows((size_t)G * 2 * C, &deferred, st);
         if (!partial) return BMB_E_CUDA;
+        const ScratchRelease release{SCR_REDUCE, st, !deferred};
         return layernorm_backward_with_scratch(dinp, dweight, dbias, dout, inp, weight, mean, rstd, N,
                                                C, partial, G, st, nullptr, deferred);
     }
     const int parts = 32;
     float *partial = (float *)device_scratch(SCR_REDUCE, (size_t)parts * 2 * C * sizeof(float));
     if (!partial) return BMB_E_CUDA;
+    BMB_TRY(scratch_acquire(SCR_REDUCE, st));
+    const ScratchRelease release{SCR_REDUCE, st, true};
     BMB_CUDA(cudaMemsetAsync(partial, 0, (size_t)parts * 2 * C * sizeof(float), st));
     layernorm_bwd_block_k<<<N, 128, 0, st>>>(dinp, partial, parts, dout, inp, weight, mean, rstd, C, emit_rounded() ? 1 : 0);
     count_launch();
@@ -1034,8 +1041,9 @@ int bmb_gelu_backward_colsum(float *dinp, float *dcolsum, const float *inp, cons
     if (gy < 1) gy = 1;
     if (gy > N) gy = N;
     bool deferred = false;
-    float *partial = partial_rows((size_t)gy * C, &deferred);
+    float *partial = partial_rows((size_t)gy * C, &deferred, st);
     if (!partial) return BMB_E_CUDA;
+    const ScratchRelease release{SCR_REDUCE, st, !deferred};
     gelu_bwd_colsum_k<<<dim3(strips, gy), 256, 0, st>>>(partial, dinp, inp, dout, N, C, emit_rounded() ? 1 : 0);
     count_launch();
     BMB_LAUNCH_CHECK();
@@ -1072,8 +1080,9 @@ int bmb_bias_backward(float *dbias, const float *dout, int N, int C) {
         if (gy < 1) gy = 1;
         if (gy > N) gy = N;
         bool deferred = false;
-        float *partial = partial_rows((size_t)gy * C, &deferred);
+        float *partial = partial_rows((size_t)gy * C, &deferred, st);
         if (!partial) return BMB_E_CUDA;
+        const ScratchRelease release{SCR_REDUCE, st, !deferred};
         bias_bwd_partial_k<<<dim3(strips, gy), 256, 0, st>>>(partial, dout, N, C);
         count_launch();
         BMB_LAUNCH_CHECK();
@@ -1160,6 +1169,8 @@ int bmb_grad_sumsq_device(const float *grads, size_t n, double *sumsq_out) {
     const int nparts = 2 * sm_count();
     float *partial = (float *)device_scratch(SCR_MISC, 4096 * sizeof(float));
     if (!partial) return BMB_E_CUDA;
+    BMB_TRY(scratch_acquire(SCR_MISC, st));
+    const ScratchRelease release{SCR_MISC, st, true};
     sumsq_partial_k<<<nparts, 256, 0, st>>>(grads, partial, n);
     sumsq_finish_k<<<1, 256, 0, st>>>(partial, nparts, sumsq_out);
     count_launch(2);

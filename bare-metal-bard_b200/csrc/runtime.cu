@@ -61,9 +61,17 @@ unsigned long long scratch_generation() {
     return (d < 0 || d >= 64) ? 0ULL : g_scratch_gen[d].load(std::memory_order_relaxed);
 }
 
+static thread_local unsigned g_slots_taken = 0;
+unsigned scratch_slots_taken() {
+    const unsigned was = g_slots_taken;
+    g_slots_taken = 0;
+    return was;
+}
+
 void *device_scratch(ScratchSlot slot, size_t bytes) {
     const int d = current_device();
     if (d < 0 || d >= 64) { fail(BMB_E_ARG, "device index %d out of range", d); return nullptr; }
+    g_slots_taken |= 1u << slot;
     std::lock_guard<std::mutex> lk(g_scratch_mu);
     Scratch &s = g_scratch[d][slot];
     if (s.cap >= bytes && s.p) return s.p;

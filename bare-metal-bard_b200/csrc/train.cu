@@ -81,6 +81,7 @@ struct bmb_trainer {
         int reduces = -1;                 // chunk whose gradients are final when the piece ends
         cudaGraphExec_t exec = nullptr;
         long long launches = 0;
+        unsigned slots = 0;               // scratch slots that the captured launches use
     };
     std::vector<Piece> pieces;
     unsigned long long graph_scratch_gen = 0;   // the device's scratch generation the graphs were captured under
@@ -557,7 +558,9 @@ int run_piece(bmb_trainer *t, bmb_trainer::Piece &pc, bool eager) {
             t->graph_failed = true;
             return run_units(t, pc.u0, pc.u1);
         }
+        (void)scratch_slots_taken();
         const int rc = run_units(t, pc.u0, pc.u1);
+        pc.slots = scratch_slots_taken();
         const cudaError_t e = cudaStreamEndCapture(t->st, &graph);
         if (rc != BMB_OK || e != cudaSuccess || !graph || gen_before != scratch_generation() ||
             cudaGraphInstantiate(&pc.exec, graph, 0) != cudaSuccess) {
@@ -573,19 +576,20 @@ int run_piece(bmb_trainer *t, bmb_trainer::Piece &pc, bool eager) {
         pc.launches = launches_total() - before;
         count_launch((int)-pc.launches);        // counted again at every replay, this first one included
     }
-    // the replayed fp32 products use the scratch that they were captured with: in turn with other streams' products
-    if (t->c.math == BMB_MATH_FP32) {
-        std::unique_lock<std::mutex> turn(split_mutex());
+    // The replayed launches use the scratch that they were captured with: in turn with what else uses it on this device.
+    std::unique_lock<std::mutex> turn(split_mutex(), std::defer_lock);
+    if (pc.slots >> SCR_SPLIT & 1) {
+        turn.lock();
         if (t->graph_scratch_gen != scratch_generation()) {      // moved since the step looked
             turn.unlock();
             return run_units(t, pc.u0, pc.u1);
         }
-        BMB_TRY(scratch_acquire(SCR_SPLIT, t->st));
-        BMB_CUDA(cudaGraphLaunch(pc.exec, t->st));
-        BMB_TRY(scratch_release(SCR_SPLIT, t->st));
-    } else {
-        BMB_CUDA(cudaGraphLaunch(pc.exec, t->st));
     }
+    for (int s = 0; s < SCR_SLOTS; ++s)
+        if (pc.slots >> s & 1) BMB_TRY(scratch_acquire((ScratchSlot)s, t->st));
+    BMB_CUDA(cudaGraphLaunch(pc.exec, t->st));
+    for (int s = 0; s < SCR_SLOTS; ++s)
+        if (pc.slots >> s & 1) BMB_TRY(scratch_release((ScratchSlot)s, t->st));
     count_launch((int)pc.launches);
     return BMB_OK;
 }

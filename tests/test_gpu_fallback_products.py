@@ -18,11 +18,12 @@ def test_small_products_of_the_tensor_core_modes_follow_the_chain(bmb, cuda, mat
     assert cuda.equal(C, want)
 
 
-@pytest.mark.parametrize("math,fused", [("MATH_TF32", 1), ("MATH_FP32", 0)])
+@pytest.mark.parametrize("math,fused", [("MATH_TF32", 0), ("MATH_TF32", 1), ("MATH_BF16", 0), ("MATH_FP32", 0)])
 def test_trainers_of_one_device_do_not_disturb_each_other(bmb, cuda, math, fused):
     """Two trainers of C = 64 (weight gradients of 64 rows), their captured steps in flight together: the gradients are
     those of each alone.  Learning rate 0, so every step has the same ones; atomic sums of shared tiles may come in
-    another order, which leaves 1e-5 of the norm as the bar."""
+    another order, which leaves 1e-5 of the norm as the bar (BF16: a rounding of an operand that such an order turns over,
+    2^-9 of it, so 1e-2)."""
     B, T, V = 4, 128, 65
     cfg = dict(max_seq_len=T, vocab_size=V, padded_vocab=128, n_layer=2, n_head=1, n_embd=64, B=B, T=T, use_flash=1,
                math=getattr(bmb, math), fused=fused)
@@ -44,5 +45,5 @@ def test_trainers_of_one_device_do_not_disturb_each_other(bmb, cuda, math, fused
     for t, want in zip(trainers, alone):
         g = cuda.empty(t.num_params)
         t.get_grads(g)
-        assert float(want.norm()) > 0 and float((g.double() - want).norm() / want.norm()) < 1e-5
+        assert float(want.norm()) > 0 and float((g.double() - want).norm() / want.norm()) < (1e-2 if math == "MATH_BF16" else 1e-5)
         t.close()
