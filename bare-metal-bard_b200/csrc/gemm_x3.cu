@@ -24,8 +24,10 @@
 // last tile are filled up with zeros.
 //
 // Infinities and NaN: a_i b_j of the pieces of an infinite operand gives NaN where the fp32 product is infinite,
-// and a sum may overflow in another order.  An element whose sum comes out not finite is therefore computed again
-// by the sequential fp32 chain from the original operands (stopping at the first NaN, which nothing can undo).
+// and a sum may overflow in another order.  Where a sum comes out not finite it is therefore not stored but computed again
+// by the sequential fp32 chain from the original operands, in blocks by all threads of a CTA:
+// behind the last product of a CTA, when no barrier is waited for any more, or in the pass that adds the parts.
+// 4096^3: 573 us; with one infinity in A 1.8 ms, with one in every row 5.5 (SIMT kernels 2.4).
 #include "tc_common.cuh"
 #include <cuda_bf16.h>
 #include <mutex>
@@ -136,27 +138,125 @@ struct Result {
     const float *bias;             // added to every row, or null
 };
 
-// One element by the sequential chain, as the SIMT kernels have it.
-__device__ __forceinline__ float element_again(const Result &p, int m, int n) {
-    const float *a = p.A, *b = p.B;
-    const long long as = p.ta ? p.M : 1, bs = p.tb ? 1 : p.N;
-    a += p.ta ? (long long)m : (long long)m * p.K;
-    b += p.tb ? (long long)n * p.K : (long long)n;
-    float s = 0.0f;
-    for (int k = 0; k < p.K; ++k) {
-        s = fmaf(a[k * as], b[k * bs], s);
-        if (s != s) break;
-    }
-    return s;
-}
 __device__ __forceinline__ bool not_finite(float x) { return !(fabsf(x) <= 3.402823466e38f); }
-// Out of line: a call in the middle of the 128 sums of an epilogue thread would cost registers that there are not.
-__device__ __noinline__ void put_element(const Result &p, int m, int n, float s) {
-    if (not_finite(s)) s = element_again(p, m, n);
+__device__ __forceinline__ void store_element(const Result &p, int m, int n, float s) {
     float *c = p.C + (size_t)m * p.N + n;
     float o = p.alpha * s;
     if (p.beta != 0.0f) o = fmaf(p.beta, *c, o);
     *c = p.bias ? o + p.bias[n] : o;
+}
+// Out of line: a call in the middle of the 128 sums of an epilogue thread would cost registers that there are not.
+__device__ __noinline__ void put_element(const Result &p, int m, int n, float s) { store_element(p, m, n, s); }
+
+// 16 TM x 64 elements by the sequential chain over k, as the SIMT kernels have it.  Thread 16 y + x of the first 256 has rows
+// m0 + TM y .. and columns n0 + 4 x ..; every thread of the block calls it.
+constexpr int CN = 64, CK = 32, C_THREADS = 256;
+template <int TM> struct ChainTile { float a[CK][16 * TM + 4], b[CK][CN + 4]; };
+// X rows (or columns) x 32 k of an operand, on the way from global to shared memory: 8 neighbours in memory a thread and trip.
+template <int X>
+struct ChainSlice {
+    float v[X / 64][8];
+    static __device__ __forceinline__ void place(int trip, bool kc, int &x, int &k) {
+        const int lin = trip * C_THREADS + (int)threadIdx.x;
+        x = kc ? lin % X : lin % (X / 8) * 8;
+        k = kc ? lin / X * 8 : lin / (X / 8);
+    }
+    __device__ __forceinline__ void read(const float *src, bool kc, bool vec, int x0, int xe, int k0, int ke) {
+#pragma unroll
+        for (int r = 0; r < X / 64; ++r) {
+            int x, k;
+            place(r, kc, x, k);
+            x += x0; k += k0;
+            const float *s = src + (kc ? (long long)x * ke + k : (long long)k * xe + x);
+            if (vec && x + (kc ? 1 : 8) <= xe && k + (kc ? 8 : 1) <= ke) {
+                const float4 lo = __ldg(reinterpret_cast<const float4 *>(s)), hi = __ldg(reinterpret_cast<const float4 *>(s) + 1);
+                v[r][0] = lo.x; v[r][1] = lo.y; v[r][2] = lo.z; v[r][3] = lo.w;
+                v[r][4] = hi.x; v[r][5] = hi.y; v[r][6] = hi.z; v[r][7] = hi.w;
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[r][i] = x + (kc ? 0 : i) < xe && k + (kc ? i : 0) < ke ? __ldg(s + i) : 0.0f;
+            }
+        }
+    }
+    __device__ __forceinline__ void put(float (*d)[X + 4], bool kc) const {
+#pragma unroll
+        for (int r = 0; r < X / 64; ++r) {
+            int x, k;
+            place(r, kc, x, k);
+            if (kc) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) d[k + i][x] = v[r][i];
+            } else {
+                *reinterpret_cast<float4 *>(&d[k][x]) = make_float4(v[r][0], v[r][1], v[r][2], v[r][3]);
+                *reinterpret_cast<float4 *>(&d[k][x + 4]) = make_float4(v[r][4], v[r][5], v[r][6], v[r][7]);
+            }
+        }
+    }
+};
+template <int TM>
+__device__ __forceinline__ void chain_block(float (&acc)[TM][4], const Result &from, int m0, int n0, ChainTile<TM> &t) {
+    const Result p = from;                          // in registers (behind the reference it is read again after each barrier)
+    const int tid = threadIdx.x;
+    const bool works = tid < C_THREADS, kca = !p.ta, kcb = p.tb != 0;
+    const bool veca = ((uintptr_t)p.A & 15) == 0 && (kca ? p.K : p.M) % 4 == 0, vecb = ((uintptr_t)p.B & 15) == 0 && (kcb ? p.K : p.N) % 4 == 0;
+    ChainSlice<16 * TM> a;
+    ChainSlice<CN> b;
+    unsigned long long sum[TM][2];                  // two columns each: an instruction follows two chains
+#pragma unroll
+    for (int i = 0; i < TM; ++i) sum[i][0] = sum[i][1] = 0ull;
+    if (works) { a.read(p.A, kca, veca, m0, p.M, 0, p.K); b.read(p.B, kcb, vecb, n0, p.N, 0, p.K); }
+    for (int k0 = 0; k0 < p.K; k0 += CK) {
+        __syncthreads();                            // the slice before has been read
+        if (works) { a.put(t.a, kca); b.put(t.b, kcb); }
+        __syncthreads();
+        if (!works) continue;
+        if (k0 + CK < p.K) { a.read(p.A, kca, veca, m0, p.M, k0 + CK, p.K); b.read(p.B, kcb, vecb, n0, p.N, k0 + CK, p.K); }
+#pragma unroll 8
+        for (int k = 0; k < CK; ++k) {
+            float x[TM];
+#pragma unroll
+            for (int i = 0; i < TM; i += 4) {
+                const float4 q = *reinterpret_cast<const float4 *>(&t.a[k][tid / 16 * TM + i]);
+                x[i] = q.x; x[i + 1] = q.y; x[i + 2] = q.z; x[i + 3] = q.w;
+            }
+            const ulonglong2 y = *reinterpret_cast<const ulonglong2 *>(&t.b[k][tid % 16 * 4]);
+#pragma unroll
+            for (int i = 0; i < TM; ++i) {
+                unsigned long long xx;
+                asm("mov.b64 %0, {%1, %1};" : "=l"(xx) : "f"(x[i]));
+                asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(sum[i][0]) : "l"(xx), "l"(y.x));
+                asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(sum[i][1]) : "l"(xx), "l"(y.y));
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; j += 2) asm("mov.b64 {%0, %1}, %2;" : "=f"(acc[i][j]), "=f"(acc[i][j + 1]) : "l"(sum[i][j / 2]));
+}
+// The parts of a tile (128 rows, two halves of half_cols columns) that its epilogue warps left out: byte 4 * half + quarter
+// of `left` stands for 32 rows of one half.  (The tile lies in dynamic shared memory, 16 bytes aligned at `at`; named here
+// and not handed over, so that it is read as such.)
+__device__ __noinline__ void tile_again(const Result &p, int m0, int n0, int half_cols, unsigned long long left, int at) {
+    extern __shared__ uint8_t smem_raw[];
+    ChainTile<8> &t = *reinterpret_cast<ChainTile<8> *>(smem_raw + at);
+    auto missing = [&](int row, int col) { return (left >> (8 * (4 * (col / half_cols) + row / 32)) & 1) != 0; };
+    for (int c = 0; c < 2 * half_cols; c += CN) {
+        const int last = c + CN - 1;
+        bool any = false;
+        for (int r = 0; r < XM; r += 32) any = any || missing(r, c) || missing(r, last);
+        if (!any) continue;
+        float acc[8][4];
+        chain_block<8>(acc, p, m0, n0 + c, t);
+        if (threadIdx.x >= C_THREADS) continue;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int row = (int)threadIdx.x / 16 * 8 + i, col = c + (int)threadIdx.x % 16 * 4 + j;
+                if (m0 + row < p.M && n0 + col < p.N && missing(row, col)) store_element(p, m0 + row, n0 + col, acc[i][j]);
+            }
+    }
 }
 
 __device__ __forceinline__ void bulk_copy(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
@@ -186,6 +286,7 @@ struct XIter {
         i += grid;
         return true;
     }
+    __device__ __forceinline__ int item() const { return i - grid; }     // the last one that next() gave
 };
 
 // One persistent CTA per SM.  Bound by shared memory and the tensor pipe together: a slice of a 128 x 256 tile
@@ -198,7 +299,7 @@ struct XIter {
 //              the registers go to global memory in whole sectors.
 template <int BN>
 __global__ void __launch_bounds__(X_THREADS, 1)
-gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict__ imgB, int rowsB, const Result p, int kblocks, int parts, float *__restrict__ ws, int vec, int *__restrict__ status) {
+gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict__ imgB, int rowsB, const Result p, int kblocks, int parts, float *__restrict__ ws, int vec, uint8_t *left, int *__restrict__ status) {
     constexpr int STAGES = x_stages(BN), STAGE = x_stage_bytes(BN), PA = XM * ROWB, PB = BN * ROWB;
     constexpr uint32_t ACC = BN == 192 ? 256 : BN, TCOLS = 2 * ACC;      // (allocations are powers of two)
     constexpr int NC = BN / 64;                     // 32-column chunks per epilogue warp (half of the columns)
@@ -207,7 +308,7 @@ gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict
     uint8_t *gen = smem_raw + (base - smem_u32(smem_raw));
     uint64_t *bars = reinterpret_cast<uint64_t *>(gen + STAGES * STAGE);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 4);
-    volatile int *giveup = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    volatile int *giveup = reinterpret_cast<volatile int *>(tmem_slot + 1), *again = giveup + 1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * STAGES;
     const uint32_t tfull0 = empty0 + 8 * STAGES, tempty0 = tfull0 + 16;
@@ -220,6 +321,7 @@ gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict
         for (int s = 0; s < STAGES; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
         for (int a = 0; a < 2; ++a) { mbar_init(tfull0 + 8 * a, 1); mbar_init(tempty0 + 8 * a, 8); }
         *giveup = 0;
+        *again = 0;
         mbar_init_fence();
     }
     if (warp == 1) tmem_alloc(smem_u32(tmem_slot), TCOLS);
@@ -333,7 +435,15 @@ gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict
             for (int c = 0; c < NC; ++c)
 #pragma unroll
                 for (int i = 0; i < 32; ++i) probe = fmaf(sum[c][i], 0.0f, probe);
-            if (vec && (tm + 1) * XM <= p.M && (tn + 1) * BN <= p.N && (probe == 0.0f || parts > 1)) {
+            if (parts == 1) {
+                const bool leave = __any_sync(0xffffffffu, probe != 0.0f);
+                if (lane == 0) {
+                    left[(size_t)it.item() * 8 + 4 * half + q] = leave;
+                    if (leave) *again = 1;
+                }
+                if (leave) continue;
+            }
+            if (vec && (tm + 1) * XM <= p.M && (tn + 1) * BN <= p.N) {
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     float *row = D + (size_t)(m0 + 8 * k) * p.N + nb;
@@ -382,7 +492,7 @@ gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict
                             }
                             // (256 columns: one sum more in registers than there are, so edges take the call, which is slow
                             // and which the choice of a plan counts)
-                            if (BN == 256 || probe != 0.0f) {
+                            if (BN == 256) {
                                 put_element(p, m, n, x.x);
                                 if (second) put_element(p, m, n + 1, x.y);
                                 continue;
@@ -415,50 +525,83 @@ gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict
         *reinterpret_cast<volatile int *>(status) = 1;
         __threadfence_system();
     }
-}
-
-// The parts of a K shared among CTAs, added in order.
-__global__ void __launch_bounds__(256) reduce_x3_k(const Result p, int parts, const float *__restrict__ ws, int vec4) {
-    const long long n = (long long)p.M * p.N;
-    const long long step = (long long)gridDim.x * blockDim.x;
-    if (vec4) {
-        for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n / 4; e += step) {
-            float4 s = __ldg(reinterpret_cast<const float4 *>(ws) + e);
-            for (int q = 1; q < parts; ++q) {
-                const float4 x = __ldg(reinterpret_cast<const float4 *>(ws + q * n) + e);
-                s.x += x.x; s.y += x.y; s.z += x.z; s.w += x.w;
-            }
-            const long long r = 4 * e;
-            if (not_finite(s.x) || not_finite(s.y) || not_finite(s.z) || not_finite(s.w)) {
-                const float v[4] = {s.x, s.y, s.z, s.w};
-#pragma unroll
-                for (int i = 0; i < 4; ++i) put_element(p, (int)((r + i) / p.N), (int)((r + i) % p.N), v[i]);
-                continue;
-            }
-            float4 o = make_float4(p.alpha * s.x, p.alpha * s.y, p.alpha * s.z, p.alpha * s.w);
-            float4 *cp = reinterpret_cast<float4 *>(p.C + r);
-            if (p.beta != 0.0f) {
-                const float4 old = *cp;
-                o.x = fmaf(p.beta, old.x, o.x); o.y = fmaf(p.beta, old.y, o.y);
-                o.z = fmaf(p.beta, old.z, o.z); o.w = fmaf(p.beta, old.w, o.w);
-            }
-            if (p.bias) {                           // N is a multiple of 4 here: the four are of one row
-                const float *b = p.bias + (int)(r % p.N);
-                o.x += __ldg(b); o.y += __ldg(b + 1); o.z += __ldg(b + 2); o.w += __ldg(b + 3);
-            }
-            *cp = o;
-        }
-    } else {
-        for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += step) {
-            float s = ws[e];
-            for (int q = 1; q < parts; ++q) s += ws[q * n + e];
-            put_element(p, (int)(e / p.N), (int)(e % p.N), s);
+    // (all products and copies are done: the ring is free)
+    if (*again && !*giveup) {
+        it.init((p.M + XM - 1) / XM, (p.N + BN - 1) / BN, parts, kblocks);
+        while (it.next(tm, tn, part, kb0, kb1)) {
+            const unsigned long long l = *reinterpret_cast<const volatile unsigned long long *>(left + (size_t)it.item() * 8);
+            if (l) tile_again(p, tm * XM, tn * BN, BN / 2, l, (int)(gen - smem_raw));
         }
     }
 }
 
+// Those of a thread's elements of a 64 x 64 block that `again` names (bit 4 i + j).
+__device__ __noinline__ void block_again(const Result &p, int m0, int n0, unsigned again) {
+    __shared__ __align__(16) ChainTile<4> t;
+    float acc[4][4];
+    chain_block<4>(acc, p, m0, n0, t);
+    const int m = m0 + (int)threadIdx.x / 16 * 4, n = n0 + (int)threadIdx.x % 16 * 4;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if ((again >> (4 * i + j) & 1) && m + i < p.M && n + j < p.N) store_element(p, m + i, n + j, acc[i][j]);
+}
+// The parts of a K shared among CTAs, added in order: 64 x 64 elements a block, as chain_block has them.
+__global__ void __launch_bounds__(C_THREADS) reduce_x3_k(const Result p, int parts, const float *__restrict__ ws, int vec4) {
+    const int tiles_n = (p.N + CN - 1) / CN, m0 = (int)(blockIdx.x / tiles_n) * 64, n0 = (int)(blockIdx.x % tiles_n) * CN;
+    const int m = m0 + (int)threadIdx.x / 16 * 4, n = n0 + (int)threadIdx.x % 16 * 4;
+    const long long part = (long long)p.M * p.N;
+    float s[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s[i][j] = 0.0f;
+    for (int q = 0; q < parts; ++q) {
+        const float *w = ws + q * part + (long long)m * p.N + n;
+#pragma unroll
+        for (int i = 0; i < 4; ++i, w += p.N) {
+            if (m + i >= p.M) continue;
+            if (vec4) {
+                if (n >= p.N) continue;
+                const float4 x = __ldg(reinterpret_cast<const float4 *>(w));
+                s[i][0] += x.x; s[i][1] += x.y; s[i][2] += x.z; s[i][3] += x.w;
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (n + j < p.N) s[i][j] += __ldg(w + j);
+            }
+        }
+    }
+    unsigned again = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) again |= (not_finite(s[i][j]) ? 1u : 0u) << (4 * i + j);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (m + i >= p.M || n >= p.N) continue;
+        if (!vec4 || again) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (n + j < p.N && !(again >> (4 * i + j) & 1)) store_element(p, m + i, n + j, s[i][j]);
+            continue;
+        }
+        float4 *c = reinterpret_cast<float4 *>(p.C + (size_t)(m + i) * p.N + n);
+        float4 o = make_float4(p.alpha * s[i][0], p.alpha * s[i][1], p.alpha * s[i][2], p.alpha * s[i][3]);
+        if (p.beta != 0.0f) {
+            const float4 old = *c;
+            o.x = fmaf(p.beta, old.x, o.x); o.y = fmaf(p.beta, old.y, o.y);
+            o.z = fmaf(p.beta, old.z, o.z); o.w = fmaf(p.beta, old.w, o.w);
+        }
+        if (p.bias) { o.x += __ldg(p.bias + n); o.y += __ldg(p.bias + n + 1); o.z += __ldg(p.bias + n + 2); o.w += __ldg(p.bias + n + 3); }
+        *c = o;
+    }
+    if (__syncthreads_or(again != 0)) block_again(p, m0, n0, again);
+}
+
 template <int BN>
-int launch_x3(int grid, const uint8_t *imgA, int rowsA, const uint8_t *imgB, int rowsB, const Result &p, int kblocks, int parts, float *ws, int vec, int *status, cudaStream_t st) {
+int launch_x3(int grid, const uint8_t *imgA, int rowsA, const uint8_t *imgB, int rowsB, const Result &p, int kblocks, int parts, float *ws, int vec, uint8_t *left, int *status, cudaStream_t st) {
     static std::mutex mu;
     static bool set[64];
     const int d = current_device();
@@ -471,7 +614,7 @@ int launch_x3(int grid, const uint8_t *imgA, int rowsA, const uint8_t *imgB, int
         }
     }
     gemm_x3_k<BN><<<grid, X_THREADS, x_smem_bytes(BN), st>>>(imgA, rowsA, imgB, rowsB, p, kblocks, parts, ws,
-                                                             vec, status);
+                                                             vec, left, status);
     return BMB_OK;
 }
 
@@ -533,7 +676,8 @@ int gemm_x3(int transA, int transB, int M, int N, int K, float alpha, const floa
     const long long imgA = (long long)kblocks * 3 * rowsA * ROWB, imgB = (long long)kblocks * 3 * rowsB * ROWB;
     const long long ws = plan.parts > 1 ? (long long)plan.parts * M * N * 4 : 0;
     const long long tiles = (long long)ceil_div(M, XM) * ceil_div(N, plan.bn) * plan.parts;
-    const long long need = imgA + imgB + ws;              // every one a multiple of 256 bytes but the last
+    const long long marks = plan.parts > 1 ? 0 : 8 * tiles;
+    const long long need = imgA + imgB + ws + marks;      // the images: multiples of 256 bytes (without parts there is no ws)
     Operand oa{A, nullptr, M, (int)rowsA, transA ? 0 : 1, (int)(rowsA / 64), ceil_div(kblocks, KG)};
     Operand ob{B, nullptr, N, (int)rowsB, transB ? 1 : 0, (int)(rowsB / 64), ceil_div(kblocks, KG)};
     const long long na = (long long)oa.panels * oa.kgroups, nb = (long long)ob.panels * ob.kgroups;
@@ -548,6 +692,7 @@ int gemm_x3(int transA, int transB, int M, int N, int K, float alpha, const floa
     oa.img = scr;
     ob.img = scr + imgA;
     float *w = (float *)(scr + imgA + imgB);
+    uint8_t *left = scr + imgA + imgB;                    // 8 bytes a tile, where there are no parts
 
     auto vec_of = [](const float *p, int inner) { return ((uintptr_t)p & 15) == 0 && inner % 4 == 0; };
     const Result p{A, B, transA, transB, M, N, K, alpha, beta, C, bias};
@@ -556,16 +701,15 @@ int gemm_x3(int transA, int transB, int M, int N, int K, float alpha, const floa
     BMB_TRY(scratch_acquire(SCR_SPLIT, st));
     split_x3_k<<<(unsigned)(na + nb), 256, 0, st>>>(oa, ob, na, K, vec_of(A, transA ? M : K), vec_of(B, transB ? K : N));
     int rc = BMB_OK;
-    if (plan.bn == 256) rc = launch_x3<256>(grid, oa.img, (int)rowsA, ob.img, (int)rowsB, p, kblocks, plan.parts, w, even, status_dev, st);
-    else if (plan.bn == 192) rc = launch_x3<192>(grid, oa.img, (int)rowsA, ob.img, (int)rowsB, p, kblocks, plan.parts, w, even, status_dev, st);
-    else if (plan.bn == 128) rc = launch_x3<128>(grid, oa.img, (int)rowsA, ob.img, (int)rowsB, p, kblocks, plan.parts, w, even, status_dev, st);
-    else rc = launch_x3<64>(grid, oa.img, (int)rowsA, ob.img, (int)rowsB, p, kblocks, plan.parts, w, even, status_dev, st);
+    if (plan.bn == 256) rc = launch_x3<256>(grid, oa.img, (int)rowsA, ob.img, (int)rowsB, p, kblocks, plan.parts, w, even, left, status_dev, st);
+    else if (plan.bn == 192) rc = launch_x3<192>(grid, oa.img, (int)rowsA, ob.img, (int)rowsB, p, kblocks, plan.parts, w, even, left, status_dev, st);
+    else if (plan.bn == 128) rc = launch_x3<128>(grid, oa.img, (int)rowsA, ob.img, (int)rowsB, p, kblocks, plan.parts, w, even, left, status_dev, st);
+    else rc = launch_x3<64>(grid, oa.img, (int)rowsA, ob.img, (int)rowsB, p, kblocks, plan.parts, w, even, left, status_dev, st);
     if (rc != BMB_OK) return rc;
     count_launch(2);
     if (plan.parts > 1) {
         const int vec4 = N % 4 == 0 && ((uintptr_t)C & 15) == 0;
-        const long long blocks = ceil_div((long long)M * N, vec4 ? 1024 : 256);
-        reduce_x3_k<<<(unsigned)(blocks < 8 * sm_count() ? blocks : 8 * sm_count()), 256, 0, st>>>(p, plan.parts, w, vec4);
+        reduce_x3_k<<<(unsigned)((long long)ceil_div(M, 64) * ceil_div(N, CN)), C_THREADS, 0, st>>>(p, plan.parts, w, vec4);
         count_launch();
     }
     BMB_LAUNCH_CHECK();

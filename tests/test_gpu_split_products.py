@@ -62,6 +62,45 @@ def test_split_product_of_infinities_and_nan(bmb, cuda, M, N, K):
     assert abs(c[20, 21] / 1.7014117e38 - 1) < 1e-6
 
 
+@pytest.mark.parametrize("M,N,K,ta,tb,beta", [
+    (515, 511, 1025, 0, 1, 0.5),     # the parts of K added by a pass, nothing aligned
+    (512, 516, 2048, 1, 0, 1.0),     # and in words
+    (2048, 1536, 512, 0, 0, 0.5),    # whole tiles, with an old value that must be read once
+    (1300, 4100, 200, 1, 1, -1.0),   # ragged tiles
+    (4100, 68, 1000, 0, 0, 0.0),     # narrow ones
+])
+def test_infinities_all_over_follow_the_chain(bmb, cuda, M, N, K, ta, tb, beta):
+    """Every third row of A holds an infinity and every 50th column of B a NaN: what is not finite in the sequential chain is
+    the same here, and the rest is within what a split product differs from the chain (both are below 1e-6 in the 2-norm)."""
+    g = cuda.Generator(device="cuda").manual_seed(M + N)
+    A, B, C0 = (cuda.rand(s, generator=g, device="cuda") + 0.5 for s in ((M, K), (K, N), (M, N)))
+    A[::3, K // 2], B[K - 1, ::50] = float("inf"), float("nan")
+    B[K // 2, 7] = -1.0
+    C, want = C0.clone(), C0.clone()
+    bmb.call("bmb_gemm_ex", bmb.MATH_FP32, 0, ta, tb, M, N, K, 0.5, A.T.contiguous() if ta else A, B.T.contiguous() if tb else B, beta, C, None)
+    bmb.call("bmb_sgemm_simt", M, N, K, 0.5, A, B, beta, want)
+    cuda.cuda.synchronize()
+    assert bool(cuda.isinf(want[0, 1:50]).all()) and float(want[0, 7]) == float("-inf") and bool(cuda.isnan(want[:, 0]).all())
+    assert cuda.equal(cuda.isnan(C), cuda.isnan(want)) and cuda.equal(cuda.isinf(C), cuda.isinf(want))
+    ok, inf = cuda.isfinite(want), cuda.isinf(want)
+    assert cuda.equal(C[inf], want[inf]) and bool(ok.any())
+    assert float((C[ok] - want[ok]).norm() / want[ok].norm()) < 2e-6
+
+
+def test_a_long_product_of_infinities_ends(bmb, cuda):
+    """A tile's sums are all computed again at K = 65536: no wait of the kernel's may depend on that."""
+    M, N, K = 1536, 3072, 65536
+    A, B, C = cuda.ones(M, K, device="cuda"), cuda.ones(K, N, device="cuda"), cuda.zeros(M, N, device="cuda")
+    B[0] = float("inf")
+    for _ in range(2):
+        bmb.call("bmb_gemm_ex", bmb.MATH_FP32, 0, 0, 0, M, N, K, 1.0, A, B, 0.0, C, None)
+    cuda.cuda.synchronize()
+    bmb.call("bmb_kernel_status", None)
+    assert bool((C == float("inf")).all())
+    bmb.call("bmb_gemm_ex", bmb.MATH_TF32, 0, 0, 0, 256, 256, 256, 1.0, A, A, 0.0, C, None)      # (fails if a wait had run out)
+    cuda.cuda.synchronize()
+
+
 def test_split_product_stays_out_of_a_capture(bmb, cuda):
     """A caller's captured products take no scratch (its address would be kept, and branches of the graph would share it)."""
     n = 1024
