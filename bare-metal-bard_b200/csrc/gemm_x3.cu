@@ -23,11 +23,17 @@
 // one slice of a tile is one contiguous bulk copy and needs no tensor map.  K and the rows of the
 // last tile are filled up with zeros.
 //
-// Infinities and NaN: a_i b_j of the pieces of an infinite operand gives NaN where the fp32 product is infinite,
-// and a sum may overflow in another order.  Where a sum comes out not finite it is therefore not stored but computed again
-// by the sequential fp32 chain from the original operands, in blocks by all threads of a CTA:
-// behind the last product of a CTA, when no barrier is waited for any more, or in the pass that adds the parts.
-// 4096^3: 573 us; with one infinity in A 1.8 ms, with one in every row 5.5 (SIMT kernels 2.4).
+// What the pieces cannot serve is not stored but computed again by the sequential fp32 chain from the original operands,
+// in blocks by all threads of a CTA: behind the last product of a CTA, when no barrier is waited for any more, or in the
+// pass that adds the parts.
+//   Sums that are not finite: a_i b_j of the pieces of an infinite operand gives NaN where the fp32 product is infinite,
+//   and a sum may overflow in another order.
+//   Panels of 64 rows (or columns) with an element that has bits below 2^-133, the smallest bf16 number (elements below
+//   about 2^-109): the split pass notes where three pieces do not add up to the element.
+//   Sums below 2^-100.
+// 4096^3: 575 us; with one infinity in A 1.8 ms, with one in every row 5.5 (SIMT kernels 2.4).
+// 2-norm errors at K = 512, this against the SIMT kernels: 0.95e-7 and 4.1e-7 with A and B of ordinary size and with A 2^-108
+// and B 2^108 times that; the same bits from 2^-110 on.
 #include "tc_common.cuh"
 #include <cuda_bf16.h>
 #include <mutex>
@@ -53,15 +59,19 @@ struct Operand {
     int rows, rows_pad;           // R and the image's rows
     int k_contig;                 // 1: element (r, k) at r * K + k; 0: at k * R + r
     int panels, kgroups;          // work split: panels of 64 rows, groups of KG slices
+    uint8_t *lost;                // [panels][kgroups, filled up to words]: an element of the block has bits that its pieces do not hold
 };
 constexpr int KG = 4;             // slices a block of the split pass takes one after the other
 
-__device__ __forceinline__ void split3(float x, float y, uint32_t &p1, uint32_t &p2, uint32_t &p3) {
+// `lost` gets bits where the pieces do not add up: a bit of x or y lies below bf16's smallest number (or it is not finite).
+__device__ __forceinline__ void split3(float x, float y, uint32_t &p1, uint32_t &p2, uint32_t &p3, uint32_t &lost) {
     constexpr float BMAX = 3.3895313892515355e38f;      // largest bf16: above it the first piece must not become infinite
     const __nv_bfloat162 a = __floats2bfloat162_rn(fminf(fmaxf(x, -BMAX), BMAX), fminf(fmaxf(y, -BMAX), BMAX));
     const float rx = x - __low2float(a), ry = y - __high2float(a);
     const __nv_bfloat162 b = __floats2bfloat162_rn(rx, ry);
-    const __nv_bfloat162 c = __floats2bfloat162_rn(rx - __low2float(b), ry - __high2float(b));
+    const float sx = rx - __low2float(b), sy = ry - __high2float(b);
+    const __nv_bfloat162 c = __floats2bfloat162_rn(sx, sy);
+    lost |= __float_as_uint(sx - __low2float(c)) | __float_as_uint(sy - __high2float(c));
     p1 = *reinterpret_cast<const uint32_t *>(&a);
     p2 = *reinterpret_cast<const uint32_t *>(&b);
     p3 = *reinterpret_cast<const uint32_t *>(&c);
@@ -82,6 +92,7 @@ __global__ void __launch_bounds__(256) split_x3_k(const Operand a, const Operand
     const int row_in = threadIdx.x >> 2, unit = threadIdx.x & 3;
     const int r = panel * 64 + row_in;
     const int nslices = (K + XK - 1) / XK;
+    uint32_t lost = 0;
     for (int ks = kgroup * KG; ks < nslices && ks < (kgroup + 1) * KG; ++ks) {
         float v[8];
         const int k0 = ks * XK + unit * 8;
@@ -120,13 +131,16 @@ __global__ void __launch_bounds__(256) split_x3_k(const Operand a, const Operand
         }
         uint32_t p1[4], p2[4], p3[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) split3(v[2 * i], v[2 * i + 1], p1[i], p2[i], p3[i]);
+        for (int i = 0; i < 4; ++i) split3(v[2 * i], v[2 * i + 1], p1[i], p2[i], p3[i], lost);
         const long long piece = (long long)o.rows_pad * ROWB;
         uint8_t *d = img + (long long)ks * 3 * piece + (long long)r * ROWB + ((unit ^ ((r >> 1) & 3)) << 4);
         *reinterpret_cast<uint4 *>(d) = make_uint4(p1[0], p1[1], p1[2], p1[3]);
         *reinterpret_cast<uint4 *>(d + piece) = make_uint4(p2[0], p2[1], p2[2], p2[3]);
         *reinterpret_cast<uint4 *>(d + 2 * piece) = make_uint4(p3[0], p3[1], p3[2], p3[3]);
     }
+    lost = __syncthreads_or(lost != 0);
+    const int words = (o.kgroups + 3) / 4, i = kgroup + (int)threadIdx.x;     // the last block clears the rest of its word
+    if (threadIdx.x == 0 || (kgroup == o.kgroups - 1 && i < 4 * words)) o.lost[(long long)panel * words * 4 + i] = threadIdx.x == 0 && lost;
 }
 
 // What a product needs besides the images: where the operands lie (for elements computed again) and the result.
@@ -136,9 +150,18 @@ struct Result {
     float alpha, beta;
     float *C;
     const float *bias;             // added to every row, or null
+    const uint32_t *lostA, *lostB; // Operand::lost, `words` a panel
+    int words;
 };
-
+// Word i of what says whether panel a of A, and panels b, b + 1, .. of B, lost bits.
+__device__ __forceinline__ const uint32_t *lost_word(const Result &p, int a, int b, int i) {
+    return i < p.words ? p.lostA + (long long)a * p.words + i : p.lostB + (long long)b * p.words + (i - p.words);
+}
 __device__ __forceinline__ bool not_finite(float x) { return !(fabsf(x) <= 3.402823466e38f); }
+// A sum that is not taken: not finite, or so small that what the tensor core cuts off below the smallest fp32 number,
+// up to 2^-149 an instruction, is more than a rounding of it.
+constexpr float TOO_SMALL = 7.8886090522101181e-31f;     // 2^-100
+__device__ __forceinline__ bool doubtful(float x) { return not_finite(x) || (fabsf(x) < TOO_SMALL && x != 0.0f); }
 __device__ __forceinline__ void store_element(const Result &p, int m, int n, float s) {
     float *c = p.C + (size_t)m * p.N + n;
     float o = p.alpha * s;
@@ -155,7 +178,8 @@ template <int TM> struct ChainTile { float a[CK][16 * TM + 4], b[CK][CN + 4]; };
 // X rows (or columns) x 32 k of an operand, on the way from global to shared memory: 8 neighbours in memory a thread and trip.
 template <int X>
 struct ChainSlice {
-    float v[X / 64][8];
+    static constexpr int UNITS = X * CK / 8, TRIPS = (UNITS + C_THREADS - 1) / C_THREADS;
+    float v[TRIPS][8];
     static __device__ __forceinline__ void place(int trip, bool kc, int &x, int &k) {
         const int lin = trip * C_THREADS + (int)threadIdx.x;
         x = kc ? lin % X : lin % (X / 8) * 8;
@@ -163,7 +187,8 @@ struct ChainSlice {
     }
     __device__ __forceinline__ void read(const float *src, bool kc, bool vec, int x0, int xe, int k0, int ke) {
 #pragma unroll
-        for (int r = 0; r < X / 64; ++r) {
+        for (int r = 0; r < TRIPS; ++r) {
+            if (UNITS % C_THREADS && r * C_THREADS + (int)threadIdx.x >= UNITS) break;
             int x, k;
             place(r, kc, x, k);
             x += x0; k += k0;
@@ -180,7 +205,8 @@ struct ChainSlice {
     }
     __device__ __forceinline__ void put(float (*d)[X + 4], bool kc) const {
 #pragma unroll
-        for (int r = 0; r < X / 64; ++r) {
+        for (int r = 0; r < TRIPS; ++r) {
+            if (UNITS % C_THREADS && r * C_THREADS + (int)threadIdx.x >= UNITS) break;
             int x, k;
             place(r, kc, x, k);
             if (kc) {
@@ -214,10 +240,12 @@ __device__ __forceinline__ void chain_block(float (&acc)[TM][4], const Result &f
 #pragma unroll 8
         for (int k = 0; k < CK; ++k) {
             float x[TM];
+            if (TM % 4 == 0) {
 #pragma unroll
-            for (int i = 0; i < TM; i += 4) {
-                const float4 q = *reinterpret_cast<const float4 *>(&t.a[k][tid / 16 * TM + i]);
-                x[i] = q.x; x[i + 1] = q.y; x[i + 2] = q.z; x[i + 3] = q.w;
+                for (int i = 0; i < TM; i += 4) *reinterpret_cast<float4 *>(x + i) = *reinterpret_cast<const float4 *>(&t.a[k][tid / 16 * TM + i]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < TM; ++i) x[i] = t.a[k][tid / 16 * TM + i];
             }
             const ulonglong2 y = *reinterpret_cast<const ulonglong2 *>(&t.b[k][tid % 16 * 4]);
 #pragma unroll
@@ -395,6 +423,14 @@ gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict
         uint32_t acc_ph = 0;
         bool ok = true;
         while (ok && it.next(tm, tn, part, kb0, kb1)) {
+            // this lane's share of the words on whether this warp's panels lost bits; asked for here (volatile), beside the first
+            // products, and wanted at the end: at K up to 5000 a word a lane
+            uint32_t lost = 0;
+            if (parts == 1) {
+                const int pa = (tm * XM + q * 32) / 64, pb = (tn * BN + half * (BN / 2)) / 64, nb = (tn * BN + half * (BN / 2) + BN / 2 - 1) / 64 - pb + 1;
+                if (lane < (1 + nb) * p.words) asm volatile("ld.global.b32 %0, [%1];" : "=r"(lost) : "l"(lost_word(p, pa, pb, lane)));
+                for (int i = lane + 32; i < (1 + nb) * p.words; i += 32) lost |= __ldg(lost_word(p, pa, pb, i));
+            }
             float sum[NC][32];
 #pragma unroll
             for (int c = 0; c < NC; ++c)
@@ -429,14 +465,24 @@ gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict
             // sum[c] of row m0 + 8k and columns nb + 32c + 8j, + 1
             auto value = [&](int c, int j, int k) { return make_float2(sum[c][(k >> 1) * 16 + 4 * j + 2 * (k & 1)], sum[c][(k >> 1) * 16 + 4 * j + 2 * (k & 1) + 1]); };
             // Nothing hides this end (the next tile's sums need these registers), so the common case is a multiply and a
-            // store per pair: a whole tile, aligned, all sums finite (0 * x is NaN for those that are not).
-            float probe = 0.0f;
-#pragma unroll
-            for (int c = 0; c < NC; ++c)
-#pragma unroll
-                for (int i = 0; i < 32; ++i) probe = fmaf(sum[c][i], 0.0f, probe);
+            // store per pair: a whole tile, aligned, of whole operands, all sums finite and none too small.
             if (parts == 1) {
-                const bool leave = __any_sync(0xffffffffu, probe != 0.0f);
+                float least = 1.0f, most = 0.0f;
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+#pragma unroll
+                    for (int i = 0; i < 32; i += 2) {
+                        asm("min.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(least) : "f"(sum[c][i]), "f"(sum[c][i + 1]));
+                        asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(most) : "f"(sum[c][i]), "f"(sum[c][i + 1]));
+                    }
+                bool leave = lost != 0 || not_finite(most);
+                if (least < TOO_SMALL) {                // (or there are zeros)
+#pragma unroll
+                    for (int c = 0; c < NC; ++c)
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) leave = leave || doubtful(sum[c][i]);
+                }
+                leave = __any_sync(0xffffffffu, leave);
                 if (lane == 0) {
                     left[(size_t)it.item() * 8 + 4 * half + q] = leave;
                     if (leave) *again = 1;
@@ -535,60 +581,48 @@ gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict
     }
 }
 
-// Those of a thread's elements of a 64 x 64 block that `again` names (bit 4 i + j).
-__device__ __noinline__ void block_again(const Result &p, int m0, int n0, unsigned again) {
-    __shared__ __align__(16) ChainTile<4> t;
-    float acc[4][4];
-    chain_block<4>(acc, p, m0, n0, t);
-    const int m = m0 + (int)threadIdx.x / 16 * 4, n = n0 + (int)threadIdx.x % 16 * 4;
+// Those of a thread's four elements that `mine` names, of a 16 x 64 block.
+__device__ __noinline__ void block_again(const Result &p, int m0, int n0, uint32_t mine) {
+    __shared__ __align__(16) ChainTile<1> t;
+    float acc[1][4];
+    chain_block<1>(acc, p, m0, n0, t);
+    const int m = m0 + (int)threadIdx.x / 16, n = n0 + (int)threadIdx.x % 16 * 4;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if ((again >> (4 * i + j) & 1) && m + i < p.M && n + j < p.N) store_element(p, m + i, n + j, acc[i][j]);
+    for (int j = 0; j < 4; ++j)
+        if ((mine >> j & 1) && m < p.M && n + j < p.N) store_element(p, m, n + j, acc[0][j]);
 }
-// The parts of a K shared among CTAs, added in order: 64 x 64 elements a block, as chain_block has them.
-__global__ void __launch_bounds__(C_THREADS) reduce_x3_k(const Result p, int parts, const float *__restrict__ ws, int vec4) {
-    const int tiles_n = (p.N + CN - 1) / CN, m0 = (int)(blockIdx.x / tiles_n) * 64, n0 = (int)(blockIdx.x % tiles_n) * CN;
-    const int m = m0 + (int)threadIdx.x / 16 * 4, n = n0 + (int)threadIdx.x % 16 * 4;
+// The parts of a K shared among CTAs, added in order: 16 x 64 elements a block, four of a row a thread (as chain_block).
+__global__ void __launch_bounds__(C_THREADS, 6) reduce_x3_k(const Result p, int parts, const float *__restrict__ ws, int vec4) {
+    const int tiles_n = (p.N + CN - 1) / CN, m0 = (int)(blockIdx.x / tiles_n) * 16, n0 = (int)(blockIdx.x % tiles_n) * CN;
+    const int m = m0 + (int)threadIdx.x / 16, n = n0 + (int)threadIdx.x % 16 * 4;
     const long long part = (long long)p.M * p.N;
-    float s[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) s[i][j] = 0.0f;
-    for (int q = 0; q < parts; ++q) {
-        const float *w = ws + q * part + (long long)m * p.N + n;
-#pragma unroll
-        for (int i = 0; i < 4; ++i, w += p.N) {
-            if (m + i >= p.M) continue;
-            if (vec4) {
-                if (n >= p.N) continue;
-                const float4 x = __ldg(reinterpret_cast<const float4 *>(w));
-                s[i][0] += x.x; s[i][1] += x.y; s[i][2] += x.z; s[i][3] += x.w;
-            } else {
+    uint32_t lost = 0;
+    for (int i = threadIdx.x; i < 2 * p.words; i += C_THREADS) lost |= __ldg(lost_word(p, m0 / 64, n0 / 64, i));
+    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    const bool inside = m < p.M && n < p.N;
+    if (inside) {
+        const float *w = ws + (long long)m * p.N + n;
+        if (vec4) {
+#pragma unroll 4
+            for (int q = 0; q < parts; ++q) {
+                const float4 x = __ldg(reinterpret_cast<const float4 *>(w + q * part));
+                s[0] += x.x; s[1] += x.y; s[2] += x.z; s[3] += x.w;
+            }
+        } else {
+            for (int q = 0; q < parts; ++q)
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    if (n + j < p.N) s[i][j] += __ldg(w + j);
-            }
+                    if (n + j < p.N) s[j] += __ldg(w + q * part + j);
         }
     }
-    unsigned again = 0;
+    uint32_t mine = 0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) again |= (not_finite(s[i][j]) ? 1u : 0u) << (4 * i + j);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        if (m + i >= p.M || n >= p.N) continue;
-        if (!vec4 || again) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (n + j < p.N && !(again >> (4 * i + j) & 1)) store_element(p, m + i, n + j, s[i][j]);
-            continue;
-        }
-        float4 *c = reinterpret_cast<float4 *>(p.C + (size_t)(m + i) * p.N + n);
-        float4 o = make_float4(p.alpha * s[i][0], p.alpha * s[i][1], p.alpha * s[i][2], p.alpha * s[i][3]);
+    for (int j = 0; j < 4; ++j) mine |= (doubtful(s[j]) ? 1u : 0u) << j;
+    const bool again = __syncthreads_or(lost != 0 || mine != 0);
+    if (again && __syncthreads_or(lost != 0)) mine = 15;
+    if (inside && vec4 && !mine) {
+        float4 *c = reinterpret_cast<float4 *>(p.C + (size_t)m * p.N + n);
+        float4 o = make_float4(p.alpha * s[0], p.alpha * s[1], p.alpha * s[2], p.alpha * s[3]);
         if (p.beta != 0.0f) {
             const float4 old = *c;
             o.x = fmaf(p.beta, old.x, o.x); o.y = fmaf(p.beta, old.y, o.y);
@@ -596,8 +630,12 @@ __global__ void __launch_bounds__(C_THREADS) reduce_x3_k(const Result p, int par
         }
         if (p.bias) { o.x += __ldg(p.bias + n); o.y += __ldg(p.bias + n + 1); o.z += __ldg(p.bias + n + 2); o.w += __ldg(p.bias + n + 3); }
         *c = o;
+    } else if (inside) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (n + j < p.N && !(mine >> j & 1)) store_element(p, m, n + j, s[j]);
     }
-    if (__syncthreads_or(again != 0)) block_again(p, m0, n0, again);
+    if (again) block_again(p, m0, n0, mine);
 }
 
 template <int BN>
@@ -676,11 +714,13 @@ int gemm_x3(int transA, int transB, int M, int N, int K, float alpha, const floa
     const long long imgA = (long long)kblocks * 3 * rowsA * ROWB, imgB = (long long)kblocks * 3 * rowsB * ROWB;
     const long long ws = plan.parts > 1 ? (long long)plan.parts * M * N * 4 : 0;
     const long long tiles = (long long)ceil_div(M, XM) * ceil_div(N, plan.bn) * plan.parts;
-    const long long marks = plan.parts > 1 ? 0 : 8 * tiles;
-    const long long need = imgA + imgB + ws + marks;      // the images: multiples of 256 bytes (without parts there is no ws)
-    Operand oa{A, nullptr, M, (int)rowsA, transA ? 0 : 1, (int)(rowsA / 64), ceil_div(kblocks, KG)};
-    Operand ob{B, nullptr, N, (int)rowsB, transB ? 1 : 0, (int)(rowsB / 64), ceil_div(kblocks, KG)};
+    Operand oa{A, nullptr, M, (int)rowsA, transA ? 0 : 1, (int)(rowsA / 64), ceil_div(kblocks, KG), nullptr};
+    Operand ob{B, nullptr, N, (int)rowsB, transB ? 1 : 0, (int)(rowsB / 64), ceil_div(kblocks, KG), nullptr};
     const long long na = (long long)oa.panels * oa.kgroups, nb = (long long)ob.panels * ob.kgroups;
+    const int words = ceil_div(oa.kgroups, 4);
+    const long long flagsA = 4LL * words * oa.panels, flagsB = 4LL * words * ob.panels;
+    const long long marks = plan.parts > 1 ? 0 : 8 * tiles;
+    const long long need = imgA + imgB + ws + marks + flagsA + flagsB;      // the images: multiples of 256 bytes (without parts there is no ws)
     if (tiles >= (1LL << 30) || na + nb >= (1LL << 31) || need > (16LL << 30)) return BMB_E_UNSUPPORTED;
     int *status_dev = nullptr;
     volatile int *status_host = nullptr;
@@ -693,9 +733,11 @@ int gemm_x3(int transA, int transB, int M, int N, int K, float alpha, const floa
     ob.img = scr + imgA;
     float *w = (float *)(scr + imgA + imgB);
     uint8_t *left = scr + imgA + imgB;                    // 8 bytes a tile, where there are no parts
+    oa.lost = scr + imgA + imgB + ws + marks;
+    ob.lost = oa.lost + flagsA;
 
     auto vec_of = [](const float *p, int inner) { return ((uintptr_t)p & 15) == 0 && inner % 4 == 0; };
-    const Result p{A, B, transA, transB, M, N, K, alpha, beta, C, bias};
+    const Result p{A, B, transA, transB, M, N, K, alpha, beta, C, bias, (const uint32_t *)oa.lost, (const uint32_t *)ob.lost, words};
     const bool even = N % 2 == 0 && (plan.parts > 1 || ((uintptr_t)C & 7) == 0);
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
     BMB_TRY(scratch_acquire(SCR_SPLIT, st));
@@ -709,7 +751,7 @@ int gemm_x3(int transA, int transB, int M, int N, int K, float alpha, const floa
     count_launch(2);
     if (plan.parts > 1) {
         const int vec4 = N % 4 == 0 && ((uintptr_t)C & 15) == 0;
-        reduce_x3_k<<<(unsigned)((long long)ceil_div(M, 64) * ceil_div(N, CN)), C_THREADS, 0, st>>>(p, plan.parts, w, vec4);
+        reduce_x3_k<<<(unsigned)((long long)ceil_div(M, 16) * ceil_div(N, CN)), C_THREADS, 0, st>>>(p, plan.parts, w, vec4);
         count_launch();
     }
     BMB_LAUNCH_CHECK();

@@ -87,6 +87,42 @@ def test_infinities_all_over_follow_the_chain(bmb, cuda, M, N, K, ta, tb, beta):
     assert float((C[ok] - want[ok]).norm() / want[ok].norm()) < 2e-6
 
 
+@pytest.mark.parametrize("M,N,K", [(512, 512, 192), (515, 1030, 193), (512, 516, 2048)])       # whole tiles, ragged ones, parts of K
+@pytest.mark.parametrize("a,b", [(-104, 104), (-108, 108), (-112, 112), (120, -120), (-126, 126), (-62, -62), (-64, -64), (-70, -62)])
+def test_small_operands_keep_their_bits(bmb, cuda, M, N, K, a, b):
+    """Operands scaled by 2^a and 2^b: pieces end at 2^-133, and sums of the tensor core at 2^-149.  The error against 64 bits is
+    no larger than the sequential chain's."""
+    g = cuda.Generator(device="cuda").manual_seed(K)
+    A, B = ((cuda.rand(s, generator=g, device="cuda") * 2 - 1) * 2.0 ** e for s, e in (((M, K), a), ((K, N), b)))
+    want = A.double() @ B.double()
+    C, simt = cuda.empty(M, N, device="cuda"), cuda.empty(M, N, device="cuda")
+    bmb.call("bmb_gemm_ex", bmb.MATH_FP32, 0, 0, 0, M, N, K, 1.0, A, B, 0.0, C, None)
+    bmb.call("bmb_sgemm_simt", M, N, K, 1.0, A, B, 0.0, simt)
+    cuda.cuda.synchronize()
+    scale = float(want.norm())
+    err = lambda x: float((x.double() - want).norm()) / scale               # noqa: E731
+    assert 0 < err(simt) and err(C) <= err(simt), (err(C), err(simt))
+
+
+def test_one_small_row_and_column(bmb, cuda):
+    """A row and a column of small numbers among ordinary ones, old values read once: the rest stays a split product."""
+    M, N, K = 512, 768, 256
+    g = cuda.Generator(device="cuda").manual_seed(1)
+    A, B, C0 = (cuda.rand(s, generator=g, device="cuda") * 2 - 1 for s in ((M, K), (K, N), (M, N)))
+    A[70] *= 2.0 ** -118
+    B[:, 500] *= 2.0 ** -118
+    want = A.double() @ B.double() + 0.5 * C0.double()
+    C, simt, plain = C0.clone(), C0.clone(), cuda.empty(M, N, device="cuda")
+    bmb.call("bmb_gemm_ex", bmb.MATH_FP32, 0, 0, 0, M, N, K, 1.0, A, B, 0.5, C, None)
+    bmb.call("bmb_sgemm_simt", M, N, K, 1.0, A, B, 0.5, simt)
+    bmb.call("bmb_gemm_ex", bmb.MATH_FP32, 0, 0, 0, M, N, K, 1.0, A, B, 0.0, plain, None)
+    cuda.cuda.synchronize()
+    assert float((C.double() - want).norm() / want.norm()) < 2.4e-7
+    assert cuda.equal(C[64:96], simt[64:96]) and cuda.equal(C[:, 500], simt[:, 500]) and not cuda.equal(C[200:], simt[200:])
+    exact = A[70].double() @ B.double()
+    assert float((plain[70].double() - exact).norm() / exact.norm()) < 1e-6
+
+
 def test_a_long_product_of_infinities_ends(bmb, cuda):
     """A tile's sums are all computed again at K = 65536: no wait of the kernel's may depend on that."""
     M, N, K = 1536, 3072, 65536
