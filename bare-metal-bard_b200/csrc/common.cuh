@@ -96,7 +96,7 @@ struct ScratchRelease {
 // The slots (bit 1 << slot) that this thread's calls have taken blocks of since the last call of this function: what a
 // captured graph holds, so that its replays can take their turn at them.
 unsigned scratch_slots_taken();
-// Counts the times any scratch block of the current device was (re)allocated.  A caller that keeps
+// Counts the times any scratch block of the current device but SCR_SPLIT was (re)allocated.  A caller that keeps
 // scratch addresses beyond one call (the trainer's captured graph) compares it before reusing them.
 unsigned long long scratch_generation();
 int current_device();
@@ -119,8 +119,16 @@ constexpr int GEMM_ANY_ORDER = 1 << 21;
 constexpr int GEMM_CHAIN = 1 << 22;
 // SCR_SPLIT (the images of split fp32 products) is sized, handed over and used under this lock of the current device, held
 // from the scratch's address to the last launch that reads it: products of several threads and streams take turns, and the
-// block is not moved under one of them.
+// block is not moved under one of them.  These functions are called with the lock held.
 std::mutex &split_mutex();
+// The block, at least `bytes` long, to be acquired for `st`; nullptr where there is no memory, or `st` is being captured and
+// the block would have to grow.  Growing waits for the block's last use.
+void *split_scratch(size_t bytes, cudaStream_t st);
+// Waits for the block's last use and frees it if it is larger than `above` bytes and nobody keeps it (trainers do, one count
+// each: their captured steps hold its address).
+void split_scratch_give_back(size_t above);
+void split_scratch_keep(int change);
+unsigned long long split_scratch_generation();      // counts the block's moves, as scratch_generation() those of the others
 // Internal GEMM dispatch shared by attention and the trainer: math is a
 // BMB_MATH_* value, flags the BMB_GEMM_* bits, strides in elements.
 int gemm_any(int math, int flags, int ta, int tb, int batch, int M, int N, int K, float alpha,

@@ -656,6 +656,10 @@ int launch_x3(int grid, const uint8_t *imgA, int rowsA, const uint8_t *imgB, int
     return BMB_OK;
 }
 
+// A larger block is given back by the product that took it (unless a trainer keeps it): (M + N) K above 1.8e8, products of
+// milliseconds.
+constexpr size_t SPLIT_KEPT = 1ull << 30;
+
 struct XPlan { int bn, parts; };
 // Widths (us, 256 / 192 / 128 / 64 columns): 8192x768x768 70 / 62 / 75 / 118, 8192x2304x768 132 / 151 / 175 / 284,
 // 4096x1536x384 42 / 37 / 44 / 64, 4096x1152x384 60 / 37 / 33 / 48, 512^3 23 / 22 / 21 / 19.
@@ -727,8 +731,8 @@ int gemm_x3(int transA, int transB, int M, int N, int K, float alpha, const floa
     BMB_TRY(status_word(&status_dev, &status_host));
     if (*status_host != 0) return fail(BMB_E_TIMEOUT, "an earlier kernel on this device gave up waiting on a barrier");
     std::lock_guard<std::mutex> turn(split_mutex());
-    uint8_t *scr = (uint8_t *)device_scratch(SCR_SPLIT, (size_t)need);
-    if (!scr) { cudaGetLastError(); return BMB_E_UNSUPPORTED; }
+    uint8_t *scr = (uint8_t *)split_scratch((size_t)need, st);
+    if (!scr) return BMB_E_UNSUPPORTED;
     oa.img = scr;
     ob.img = scr + imgA;
     float *w = (float *)(scr + imgA + imgB);
@@ -755,7 +759,9 @@ int gemm_x3(int transA, int transB, int M, int N, int K, float alpha, const floa
         count_launch();
     }
     BMB_LAUNCH_CHECK();
-    return scratch_release(SCR_SPLIT, st);
+    BMB_TRY(scratch_release(SCR_SPLIT, st));
+    if (cs == cudaStreamCaptureStatusNone && !(flags & GEMM_SCRATCH_IN_CAPTURE)) split_scratch_give_back(SPLIT_KEPT);
+    return BMB_OK;
 }
 
 }  // namespace bmb

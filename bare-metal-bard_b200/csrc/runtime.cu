@@ -122,6 +122,60 @@ int scratch_release(ScratchSlot slot, cudaStream_t st) {
     return BMB_OK;
 }
 
+// ---- the block of split fp32 products ----
+static int g_split_keepers[64];
+static unsigned long long g_split_gen[64];
+
+// While another stream is being captured in the global mode, this thread's allocations would be refused and end that capture.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+static bool split_scratch_drop(int d) {
+    Scratch &s = g_scratch[d][SCR_SPLIT];
+    if (!s.p) return true;
+    RelaxedCapture relaxed;
+    const SlotUse &u = g_slot_use[d][SCR_SPLIT];             // (written under split_mutex(), as everything here)
+    if ((u.valid && cudaEventSynchronize(u.done) != cudaSuccess) || cudaFree(s.p) != cudaSuccess) { cudaGetLastError(); return false; }
+    s = Scratch();
+    ++g_split_gen[d];
+    return true;
+}
+
+void *split_scratch(size_t bytes, cudaStream_t st) {
+    const int d = current_device();
+    if (d < 0 || d >= 64) return nullptr;
+    g_slots_taken |= 1u << SCR_SPLIT;
+    Scratch &s = g_scratch[d][SCR_SPLIT];
+    if (s.p && s.cap >= bytes) return s.p;
+    if (capturing(st) || !split_scratch_drop(d)) return nullptr;
+    RelaxedCapture relaxed;
+    const size_t want = bytes < (1u << 20) ? (1u << 20) : bytes;
+    void *p = nullptr;
+    if (cudaMalloc(&p, want) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    s.p = p; s.cap = want;
+    ++g_split_gen[d];
+    return p;
+}
+
+void split_scratch_give_back(size_t above) {
+    const int d = current_device();
+    if (d < 0 || d >= 64 || g_split_keepers[d] > 0 || g_scratch[d][SCR_SPLIT].cap <= above) return;
+    (void)split_scratch_drop(d);
+}
+
+unsigned long long split_scratch_generation() {
+    const int d = current_device();
+    return (d < 0 || d >= 64) ? 0ULL : g_split_gen[d];
+}
+
+void split_scratch_keep(int change) {
+    const int d = current_device();
+    if (d >= 0 && d < 64) g_split_keepers[d] += change;
+}
+
 }  // namespace bmb
 
 extern "C" {

@@ -84,7 +84,8 @@ struct bmb_trainer {
         unsigned slots = 0;               // scratch slots that the captured launches use
     };
     std::vector<Piece> pieces;
-    unsigned long long graph_scratch_gen = 0;   // the device's scratch generation the graphs were captured under
+    unsigned long long graph_scratch_gen = 0;   // the device's scratch generation the graphs were captured under,
+    unsigned long long graph_split_gen = 0;     // and that of the split products' block
     // Fused exchange, overlapped forms: the parameter space is cut into three chunks -- A: embeddings + layer 0,
     // B: layers 1 .. c2-1, C: layers c2 .. L-1 + final layernorm.  Backward finishes C, then B, then A, and each
     // chunk's reduce runs on the exchange stream while backward goes on; the next forward needs A, then B, then
@@ -106,6 +107,7 @@ struct bmb_trainer {
     // phases in that step and the next, printed to stderr once both have drained.
     int tl_step = 0;
     std::vector<std::pair<std::string, cudaEvent_t>> tl;
+    bool keeps_split = false;     // counted among those whose captured steps hold the split products' block
     float *gen_probs = nullptr;   // one row of next-token probabilities, allocated by the first sampling call
     // The two products of a linear layer's backward (dX = dY W and dW = dY^T X: the same FLOP count, both waiting only
     // for dY) run side by side, each on half of the SMs: dX on the main stream, dW on this one, forked and joined
@@ -545,13 +547,18 @@ void plan_pieces(bmb_trainer *t) {
     }
 }
 
+unsigned long long split_generation() {
+    std::lock_guard<std::mutex> turn(split_mutex());
+    return split_scratch_generation();
+}
+
 // One piece on t->st: replay of its captured graph, or eager launches (`eager`: first pass, GEMM event
 // profiling on, graphs switched off, or a capture failed).
 int run_piece(bmb_trainer *t, bmb_trainer::Piece &pc, bool eager) {
     if (eager || t->graph_failed) return run_units(t, pc.u0, pc.u1);
     if (!pc.exec) {
         const long long before = launches_total();
-        const unsigned long long gen_before = scratch_generation();
+        const unsigned long long gen_before = scratch_generation(), split_before = split_generation();
         cudaGraph_t graph = nullptr;
         if (cudaStreamBeginCapture(t->st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
             cudaGetLastError();
@@ -563,6 +570,7 @@ int run_piece(bmb_trainer *t, bmb_trainer::Piece &pc, bool eager) {
         pc.slots = scratch_slots_taken();
         const cudaError_t e = cudaStreamEndCapture(t->st, &graph);
         if (rc != BMB_OK || e != cudaSuccess || !graph || gen_before != scratch_generation() ||
+            ((pc.slots >> SCR_SPLIT & 1) && split_before != split_generation()) ||
             cudaGraphInstantiate(&pc.exec, graph, 0) != cudaSuccess) {
             // nothing ran during the capture: fall back to eager launches for good and run this piece now
             cudaGetLastError();
@@ -573,6 +581,7 @@ int run_piece(bmb_trainer *t, bmb_trainer::Piece &pc, bool eager) {
         }
         cudaGraphDestroy(graph);
         t->graph_scratch_gen = gen_before;
+        t->graph_split_gen = split_before;
         pc.launches = launches_total() - before;
         count_launch((int)-pc.launches);        // counted again at every replay, this first one included
     }
@@ -580,7 +589,7 @@ int run_piece(bmb_trainer *t, bmb_trainer::Piece &pc, bool eager) {
     std::unique_lock<std::mutex> turn(split_mutex(), std::defer_lock);
     if (pc.slots >> SCR_SPLIT & 1) {
         turn.lock();
-        if (t->graph_scratch_gen != scratch_generation()) {      // moved since the step looked
+        if (t->graph_split_gen != split_scratch_generation()) {  // moved since the step looked
             turn.unlock();
             return run_units(t, pc.u0, pc.u1);
         }
@@ -600,8 +609,12 @@ int run_piece(bmb_trainer *t, bmb_trainer::Piece &pc, bool eager) {
 bool step_is_eager(bmb_trainer *t) {
     if (!t->use_graph || t->graph_failed || t->prof) return true;
     bool any = false;
-    for (auto &pc : t->pieces) any = any || pc.exec;
-    if (any && t->graph_scratch_gen != scratch_generation()) {
+    bool split = false;
+    for (auto &pc : t->pieces) {
+        any = any || pc.exec;
+        split = split || (pc.exec && (pc.slots >> SCR_SPLIT & 1));
+    }
+    if (any && (t->graph_scratch_gen != scratch_generation() || (split && t->graph_split_gen != split_generation()))) {
         drop_graphs(t);
         t->eager_passes = 0;
         any = false;
@@ -686,6 +699,11 @@ int trainer_build(bmb_trainer *t, const bmb_train_config &c, unsigned seed) {
     for (int c = 0; c < bmb_trainer::NCHUNK; ++c) {
         BMB_CUDA(cudaEventCreateWithFlags(&t->ev_seg[c], cudaEventDisableTiming));
         BMB_CUDA(cudaEventCreateWithFlags(&t->ev_upd[c], cudaEventDisableTiming));
+    }
+    if (c.math == BMB_MATH_FP32) {
+        std::lock_guard<std::mutex> turn(split_mutex());
+        split_scratch_keep(1);
+        t->keeps_split = true;
     }
     param_sizes(t->psize, c);
     t->num_params = 0;
@@ -817,6 +835,11 @@ int bmb_trainer_destroy(bmb_trainer *t) {
     if (t->ev_fork) cudaEventDestroy(t->ev_fork);
     if (t->ev_join) cudaEventDestroy(t->ev_join);
     if (t->st_dw) cudaStreamDestroy(t->st_dw);
+    if (t->keeps_split) {                 // the last one gives the block back
+        std::lock_guard<std::mutex> turn(split_mutex());
+        split_scratch_keep(-1);
+        split_scratch_give_back(0);
+    }
     if (t->st) cudaStreamDestroy(t->st);
     delete t;
     return BMB_OK;

@@ -370,7 +370,8 @@ int bmb_trainer_loss_async(bmb_trainer *t, float *pinned_host_loss);
 int bmb_trainer_sync(bmb_trainer *t);
 /* Floats held by one replica: parameters (x4 with gradients and the two AdamW moments), forward
  * activations, backward scratch -- the figures the reference prints before training and under
- * --alloc-only (src/train_gpt.cu:339-355). */
+ * --alloc-only (src/train_gpt.cu:339-355).  The per-device scratch that all callers share is not counted; in fp32
+ * mode it holds 6 bytes per operand element of the largest product, until the last fp32 trainer is destroyed. */
 int bmb_trainer_memory(const bmb_trainer *t, size_t *param_floats, size_t *activation_floats,
                        size_t *scratch_floats);
 /* Blocks: the gradient norm the last bmb_trainer_step clipped against, ||sum over ranks of g|| / ranks

@@ -248,3 +248,51 @@ def test_split_products_of_threads_and_streams_take_turns(bmb, cuda, per_thread)
     assert not errors, errors
     for w in work:
         assert all(cuda.equal(C, w[5]) for C in w[6])
+
+
+def test_growing_the_scratch_leaves_a_capture_alone(bmb, cuda):
+    """A product whose images need a larger block than any before, on one stream, while another stream is being captured in
+    the global mode: the capture goes on, and both results are right."""
+    n = 256
+    small, large = cuda.rand(n, n, device="cuda"), [cuda.rand(s, device="cuda") for s in ((3000, 9000), (9000, 3001))]
+    C, D, E = cuda.empty(n, n, device="cuda"), cuda.empty(3000, 3001, device="cuda"), cuda.empty(3000, 3001, device="cuda")
+    bmb.call("bmb_gemm_ex", bmb.MATH_FP32, 0, 0, 0, 600, 600, 600, 1.0, large[0], large[1], 0.0, D, None)      # (a first, small one)
+    bmb.call("bmb_sgemm_simt", 3000, 3001, 9000, 1.0, large[0], large[1], 0.0, E)
+    side, graph = cuda.cuda.Stream(), cuda.cuda.CUDAGraph()
+    cuda.cuda.synchronize()
+    with cuda.cuda.graph(graph, capture_error_mode="global"):
+        bmb.call("bmb_gemm_ex", bmb.MATH_FP32, 0, 0, 0, n, n, n, 1.0, small, small, 0.0, C, cuda.cuda.current_stream().cuda_stream)
+        bmb.call("bmb_gemm_ex", bmb.MATH_FP32, 0, 0, 0, 3000, 3001, 9000, 1.0, large[0], large[1], 0.0, D, side.cuda_stream)
+    graph.replay()
+    cuda.cuda.synchronize()
+    assert float((D - E).norm() / E.norm()) < 4e-6 and not cuda.equal(D, E)
+    want = cuda.empty_like(C)
+    bmb.call("bmb_sgemm_simt", n, n, n, 1.0, small, small, 0.0, want)
+    cuda.cuda.synchronize()
+    assert cuda.equal(C, want)
+
+
+def test_large_scratch_is_given_back(bmb, cuda):
+    """1.6 GB of images are free again behind the product that took them, and so is a trainer's block behind the trainer."""
+    M, K = 2048, 65536
+    A, B, C = cuda.rand(M, K, device="cuda"), cuda.rand(K, M, device="cuda"), cuda.empty(M, M, device="cuda")
+    free = lambda: (cuda.cuda.synchronize(), cuda.cuda.mem_get_info()[0])[1]      # noqa: E731
+    bmb.call("bmb_gemm_ex", bmb.MATH_FP32, 0, 0, 0, 512, 512, 512, 1.0, A, B, 0.0, C, None)
+    before = free()
+    bmb.call("bmb_gemm_ex", bmb.MATH_FP32, 0, 0, 0, M, M, K, 1.0, A, B, 0.0, C, None)
+    assert free() > before - (64 << 20)
+    want = A[5].double() @ B.double()
+    assert float((C[5].double() - want).norm() / want.norm()) < 1e-6
+    del A, B, C
+    cuda.cuda.empty_cache()
+    cfg = dict(max_seq_len=512, vocab_size=20000, padded_vocab=20096, n_layer=1, n_head=4, n_embd=256, B=8, T=512, use_flash=1, math=bmb.MATH_FP32, fused=0)
+    tok = np.zeros((8, 512), np.int32)
+    before = free()
+    for _ in range(2):
+        t = bmb.Trainer(seed=1, **cfg)
+        for step in (1, 2, 3):
+            t.upload(tok, tok)
+            t.step(0.0, step)
+        t.sync()
+        t.close()
+        assert free() > before - (8 << 20)
