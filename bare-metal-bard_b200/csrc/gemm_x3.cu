@@ -23,9 +23,9 @@
 // one slice of a tile is one contiguous bulk copy and needs no tensor map.  K and the rows of the
 // last tile are filled up with zeros.
 //
-// What the pieces cannot serve is not stored but computed again by the sequential fp32 chain from the original operands,
-// in blocks by all threads of a CTA: behind the last product of a CTA, when no barrier is waited for any more, or in the
-// pass that adds the parts.
+// What the pieces cannot serve is not stored but computed again by the sequential fp32 chain from the original operands:
+// behind the last product of a CTA, when no barrier is waited for any more, in blocks by all its threads, or in the pass that
+// adds the parts.
 //   Sums that are not finite: a_i b_j of the pieces of an infinite operand gives NaN where the fp32 product is infinite,
 //   and a sum may overflow in another order.
 //   Panels of 64 rows (or columns) with an element that has bits below 2^-133, the smallest bf16 number (elements below
@@ -37,6 +37,7 @@
 #include "tc_common.cuh"
 #include <cuda_bf16.h>
 #include <mutex>
+#include <type_traits>
 
 namespace bmb {
 using namespace tc;
@@ -152,6 +153,8 @@ struct Result {
     const float *bias;             // added to every row, or null
     const uint32_t *lostA, *lostB; // Operand::lost, `words` a panel
     int words;
+    uint8_t *lost;                 // the same a panel (of A, then of B), for the pass that adds the parts
+    int panels_a, panels;
 };
 // Word i of what says whether panel a of A, and panels b, b + 1, .. of B, lost bits.
 __device__ __forceinline__ const uint32_t *lost_word(const Result &p, int a, int b, int i) {
@@ -171,14 +174,14 @@ __device__ __forceinline__ void store_element(const Result &p, int m, int n, flo
 // Out of line: a call in the middle of the 128 sums of an epilogue thread would cost registers that there are not.
 __device__ __noinline__ void put_element(const Result &p, int m, int n, float s) { store_element(p, m, n, s); }
 
-// 16 TM x 64 elements by the sequential chain over k, as the SIMT kernels have it.  Thread 16 y + x of the first 256 has rows
-// m0 + TM y .. and columns n0 + 4 x ..; every thread of the block calls it.
-constexpr int CN = 64, CK = 32, C_THREADS = 256;
-template <int TM> struct ChainTile { float a[CK][16 * TM + 4], b[CK][CN + 4]; };
+// 128 x 64 elements by the sequential chain over k, as the SIMT kernels have it.  Thread 16 y + x of the first 256 has rows
+// m0 + 8 y .. and columns n0 + 4 x ..; every thread of the block calls it.
+constexpr int TM = 8, CN = 64, CK = 32, C_THREADS = 256;
+struct ChainTile { float a[CK][16 * TM + 4], b[CK][CN + 4]; };
 // X rows (or columns) x 32 k of an operand, on the way from global to shared memory: 8 neighbours in memory a thread and trip.
 template <int X>
 struct ChainSlice {
-    static constexpr int UNITS = X * CK / 8, TRIPS = (UNITS + C_THREADS - 1) / C_THREADS;
+    static constexpr int TRIPS = X * CK / 8 / C_THREADS;
     float v[TRIPS][8];
     static __device__ __forceinline__ void place(int trip, bool kc, int &x, int &k) {
         const int lin = trip * C_THREADS + (int)threadIdx.x;
@@ -188,7 +191,6 @@ struct ChainSlice {
     __device__ __forceinline__ void read(const float *src, bool kc, bool vec, int x0, int xe, int k0, int ke) {
 #pragma unroll
         for (int r = 0; r < TRIPS; ++r) {
-            if (UNITS % C_THREADS && r * C_THREADS + (int)threadIdx.x >= UNITS) break;
             int x, k;
             place(r, kc, x, k);
             x += x0; k += k0;
@@ -206,7 +208,6 @@ struct ChainSlice {
     __device__ __forceinline__ void put(float (*d)[X + 4], bool kc) const {
 #pragma unroll
         for (int r = 0; r < TRIPS; ++r) {
-            if (UNITS % C_THREADS && r * C_THREADS + (int)threadIdx.x >= UNITS) break;
             int x, k;
             place(r, kc, x, k);
             if (kc) {
@@ -219,8 +220,7 @@ struct ChainSlice {
         }
     }
 };
-template <int TM>
-__device__ __forceinline__ void chain_block(float (&acc)[TM][4], const Result &from, int m0, int n0, ChainTile<TM> &t) {
+__device__ __forceinline__ void chain_block(float (&acc)[TM][4], const Result &from, int m0, int n0, ChainTile &t) {
     const Result p = from;                          // in registers (behind the reference it is read again after each barrier)
     const int tid = threadIdx.x;
     const bool works = tid < C_THREADS, kca = !p.ta, kcb = p.tb != 0;
@@ -240,13 +240,8 @@ __device__ __forceinline__ void chain_block(float (&acc)[TM][4], const Result &f
 #pragma unroll 8
         for (int k = 0; k < CK; ++k) {
             float x[TM];
-            if (TM % 4 == 0) {
 #pragma unroll
-                for (int i = 0; i < TM; i += 4) *reinterpret_cast<float4 *>(x + i) = *reinterpret_cast<const float4 *>(&t.a[k][tid / 16 * TM + i]);
-            } else {
-#pragma unroll
-                for (int i = 0; i < TM; ++i) x[i] = t.a[k][tid / 16 * TM + i];
-            }
+            for (int i = 0; i < TM; i += 4) *reinterpret_cast<float4 *>(x + i) = *reinterpret_cast<const float4 *>(&t.a[k][tid / 16 * TM + i]);
             const ulonglong2 y = *reinterpret_cast<const ulonglong2 *>(&t.b[k][tid % 16 * 4]);
 #pragma unroll
             for (int i = 0; i < TM; ++i) {
@@ -267,21 +262,21 @@ __device__ __forceinline__ void chain_block(float (&acc)[TM][4], const Result &f
 // and not handed over, so that it is read as such.)
 __device__ __noinline__ void tile_again(const Result &p, int m0, int n0, int half_cols, unsigned long long left, int at) {
     extern __shared__ uint8_t smem_raw[];
-    ChainTile<8> &t = *reinterpret_cast<ChainTile<8> *>(smem_raw + at);
+    ChainTile &t = *reinterpret_cast<ChainTile *>(smem_raw + at);
     auto missing = [&](int row, int col) { return (left >> (8 * (4 * (col / half_cols) + row / 32)) & 1) != 0; };
     for (int c = 0; c < 2 * half_cols; c += CN) {
         const int last = c + CN - 1;
         bool any = false;
         for (int r = 0; r < XM; r += 32) any = any || missing(r, c) || missing(r, last);
         if (!any) continue;
-        float acc[8][4];
-        chain_block<8>(acc, p, m0, n0 + c, t);
+        float acc[TM][4];
+        chain_block(acc, p, m0, n0 + c, t);
         if (threadIdx.x >= C_THREADS) continue;
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < TM; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const int row = (int)threadIdx.x / 16 * 8 + i, col = c + (int)threadIdx.x % 16 * 4 + j;
+                const int row = (int)threadIdx.x / 16 * TM + i, col = c + (int)threadIdx.x % 16 * 4 + j;
                 if (m0 + row < p.M && n0 + col < p.N && missing(row, col)) store_element(p, m0 + row, n0 + col, acc[i][j]);
             }
     }
@@ -419,6 +414,14 @@ gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict
         }
     } else {
         const int q = warp & 3, half = (warp - 2) >> 2;
+        if (parts > 1 && warp == 2) {
+            for (int i = blockIdx.x; i < p.panels; i += gridDim.x) {
+                uint32_t l = 0;
+                for (int w = lane; w < p.words; w += 32) l |= __ldg((i < p.panels_a ? p.lostA + (long long)i * p.words : p.lostB + (long long)(i - p.panels_a) * p.words) + w);
+                l = __any_sync(0xffffffffu, l != 0);
+                if (lane == 0) p.lost[i] = l;
+            }
+        }
         int acc = 0;
         uint32_t acc_ph = 0;
         bool ok = true;
@@ -581,61 +584,80 @@ gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict
     }
 }
 
-// Those of a thread's four elements that `mine` names, of a 16 x 64 block.
-__device__ __noinline__ void block_again(const Result &p, int m0, int n0, uint32_t mine) {
-    __shared__ __align__(16) ChainTile<1> t;
-    float acc[1][4];
-    chain_block<1>(acc, p, m0, n0, t);
-    const int m = m0 + (int)threadIdx.x / 16, n = n0 + (int)threadIdx.x % 16 * 4;
+// Those of four neighbouring elements of a row that `again` names, by the sequential chain.  16 neighbouring threads read the
+// same values of A and neighbouring ones of B, four steps of k at a time.
+__device__ __noinline__ void four_again(const Result &from, int m, int n, uint32_t again) {
+    const Result p = from;
+    const long long as = p.ta ? p.M : 1, bk = p.tb ? 1 : p.N, bn = p.tb ? p.K : 1;
+    const float *a = p.A + (p.ta ? (long long)m : (long long)m * p.K), *b = p.B + n * bn;
+    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    auto steps = [&](int k, auto count) {
+        constexpr int N = decltype(count)::value;
+        float x[N], y[N][4];
+#pragma unroll
+        for (int q = 0; q < N; ++q) {
+            x[q] = __ldg(a + (k + q) * as);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) y[q][j] = n + j < p.N ? __ldg(b + (k + q) * bk + j * bn) : 0.0f;
+        }
+#pragma unroll
+        for (int q = 0; q < N; ++q)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s[j] = fmaf(x[q], y[q][j], s[j]);
+    };
+    int k = 0;
+    for (; k + 4 <= p.K; k += 4) steps(k, std::integral_constant<int, 4>());
+    for (; k < p.K; ++k) steps(k, std::integral_constant<int, 1>());
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-        if ((mine >> j & 1) && m < p.M && n + j < p.N) store_element(p, m, n + j, acc[0][j]);
+        if ((again >> j & 1) && n + j < p.N) store_element(p, m, n + j, s[j]);
 }
-// The parts of a K shared among CTAs, added in order: 16 x 64 elements a block, four of a row a thread (as chain_block).
-__global__ void __launch_bounds__(C_THREADS, 6) reduce_x3_k(const Result p, int parts, const float *__restrict__ ws, int vec4) {
-    const int tiles_n = (p.N + CN - 1) / CN, m0 = (int)(blockIdx.x / tiles_n) * 16, n0 = (int)(blockIdx.x % tiles_n) * CN;
-    const int m = m0 + (int)threadIdx.x / 16, n = n0 + (int)threadIdx.x % 16 * 4;
-    const long long part = (long long)p.M * p.N;
-    uint32_t lost = 0;
-    for (int i = threadIdx.x; i < 2 * p.words; i += C_THREADS) lost |= __ldg(lost_word(p, m0 / 64, n0 / 64, i));
-    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    const bool inside = m < p.M && n < p.N;
-    if (inside) {
-        const float *w = ws + (long long)m * p.N + n;
-        if (vec4) {
-#pragma unroll 4
-            for (int q = 0; q < parts; ++q) {
-                const float4 x = __ldg(reinterpret_cast<const float4 *>(w + q * part));
-                s[0] += x.x; s[1] += x.y; s[2] += x.z; s[3] += x.w;
+// The parts of a K shared among CTAs, added in order.
+__global__ void __launch_bounds__(256) reduce_x3_k(const Result p, int parts, const float *__restrict__ ws, int vec4) {
+    const long long n = (long long)p.M * p.N, step = (long long)gridDim.x * blockDim.x;
+    auto lost = [&](int row, int col) { return (p.lost[row / 64] | p.lost[p.panels_a + col / 64]) != 0; };
+    if (vec4) {
+        for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n / 4; e += step) {
+            float4 s = __ldg(reinterpret_cast<const float4 *>(ws) + e);
+            const int row = n < (1LL << 31) ? (int)((uint32_t)(4 * e) / (uint32_t)p.N) : (int)(4 * e / p.N), col = (int)(4 * e - (long long)row * p.N);
+            const bool whole = !lost(row, col);
+            for (int q = 1; q < parts; ++q) {
+                const float4 x = __ldg(reinterpret_cast<const float4 *>(ws + q * n) + e);
+                s.x += x.x; s.y += x.y; s.z += x.z; s.w += x.w;
             }
-        } else {
-            for (int q = 0; q < parts; ++q)
+            if (!whole || doubtful(s.x) || doubtful(s.y) || doubtful(s.z) || doubtful(s.w)) {
+                const float v[4] = {s.x, s.y, s.z, s.w};
+                uint32_t again = whole ? 0u : 15u;
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (n + j < p.N) s[j] += __ldg(w + q * part + j);
+                for (int i = 0; i < 4; ++i) {
+                    again |= (doubtful(v[i]) ? 1u : 0u) << i;
+                    if (!(again >> i & 1)) put_element(p, row, col + i, v[i]);
+                }
+                four_again(p, row, col, again);
+                continue;
+            }
+            float4 o = make_float4(p.alpha * s.x, p.alpha * s.y, p.alpha * s.z, p.alpha * s.w);
+            float4 *cp = reinterpret_cast<float4 *>(p.C + 4 * e);
+            if (p.beta != 0.0f) {
+                const float4 old = *cp;
+                o.x = fmaf(p.beta, old.x, o.x); o.y = fmaf(p.beta, old.y, o.y);
+                o.z = fmaf(p.beta, old.z, o.z); o.w = fmaf(p.beta, old.w, o.w);
+            }
+            if (p.bias) {                           // N is a multiple of 4 here: the four are of one row
+                const float *b = p.bias + col;
+                o.x += __ldg(b); o.y += __ldg(b + 1); o.z += __ldg(b + 2); o.w += __ldg(b + 3);
+            }
+            *cp = o;
+        }
+    } else {
+        for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += step) {
+            float s = ws[e];
+            for (int q = 1; q < parts; ++q) s += ws[q * n + e];
+            const int row = (int)(e / p.N), col = (int)(e - (long long)row * p.N);
+            if (doubtful(s) || lost(row, col)) four_again(p, row, col, 1u);
+            else put_element(p, row, col, s);
         }
     }
-    uint32_t mine = 0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) mine |= (doubtful(s[j]) ? 1u : 0u) << j;
-    const bool again = __syncthreads_or(lost != 0 || mine != 0);
-    if (again && __syncthreads_or(lost != 0)) mine = 15;
-    if (inside && vec4 && !mine) {
-        float4 *c = reinterpret_cast<float4 *>(p.C + (size_t)m * p.N + n);
-        float4 o = make_float4(p.alpha * s[0], p.alpha * s[1], p.alpha * s[2], p.alpha * s[3]);
-        if (p.beta != 0.0f) {
-            const float4 old = *c;
-            o.x = fmaf(p.beta, old.x, o.x); o.y = fmaf(p.beta, old.y, o.y);
-            o.z = fmaf(p.beta, old.z, o.z); o.w = fmaf(p.beta, old.w, o.w);
-        }
-        if (p.bias) { o.x += __ldg(p.bias + n); o.y += __ldg(p.bias + n + 1); o.z += __ldg(p.bias + n + 2); o.w += __ldg(p.bias + n + 3); }
-        *c = o;
-    } else if (inside) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (n + j < p.N && !(mine >> j & 1)) store_element(p, m, n + j, s[j]);
-    }
-    if (again) block_again(p, m0, n0, mine);
 }
 
 template <int BN>
@@ -724,7 +746,7 @@ int gemm_x3(int transA, int transB, int M, int N, int K, float alpha, const floa
     const int words = ceil_div(oa.kgroups, 4);
     const long long flagsA = 4LL * words * oa.panels, flagsB = 4LL * words * ob.panels;
     const long long marks = plan.parts > 1 ? 0 : 8 * tiles;
-    const long long need = imgA + imgB + ws + marks + flagsA + flagsB;      // the images: multiples of 256 bytes (without parts there is no ws)
+    const long long need = imgA + imgB + ws + marks + flagsA + flagsB + oa.panels + ob.panels;      // the images: multiples of 256 bytes (without parts there is no ws)
     if (tiles >= (1LL << 30) || na + nb >= (1LL << 31) || need > (16LL << 30)) return BMB_E_UNSUPPORTED;
     int *status_dev = nullptr;
     volatile int *status_host = nullptr;
@@ -741,7 +763,8 @@ int gemm_x3(int transA, int transB, int M, int N, int K, float alpha, const floa
     ob.lost = oa.lost + flagsA;
 
     auto vec_of = [](const float *p, int inner) { return ((uintptr_t)p & 15) == 0 && inner % 4 == 0; };
-    const Result p{A, B, transA, transB, M, N, K, alpha, beta, C, bias, (const uint32_t *)oa.lost, (const uint32_t *)ob.lost, words};
+    const Result p{A, B, transA, transB, M, N, K, alpha, beta, C, bias, (const uint32_t *)oa.lost, (const uint32_t *)ob.lost, words,
+                   ob.lost + flagsB, oa.panels, oa.panels + ob.panels};
     const bool even = N % 2 == 0 && (plan.parts > 1 || ((uintptr_t)C & 7) == 0);
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
     BMB_TRY(scratch_acquire(SCR_SPLIT, st));
@@ -755,7 +778,8 @@ int gemm_x3(int transA, int transB, int M, int N, int K, float alpha, const floa
     count_launch(2);
     if (plan.parts > 1) {
         const int vec4 = N % 4 == 0 && ((uintptr_t)C & 15) == 0;
-        reduce_x3_k<<<(unsigned)((long long)ceil_div(M, 16) * ceil_div(N, CN)), C_THREADS, 0, st>>>(p, plan.parts, w, vec4);
+        const long long blocks = ceil_div((long long)M * N, vec4 ? 1024 : 256);
+        reduce_x3_k<<<(unsigned)(blocks < 8 * sm_count() ? blocks : 8 * sm_count()), 256, 0, st>>>(p, plan.parts, w, vec4);
         count_launch();
     }
     BMB_LAUNCH_CHECK();
