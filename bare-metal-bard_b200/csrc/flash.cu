@@ -170,6 +170,10 @@ __device__ __noinline__ void fwd_rows_again(float *smem, float *out, float *lse,
     for (int r = 0; r < nrows; r += R) fwd_rows<HS, 16, NT>(smem, out, lse, qkv, T, NH, scale, bh, i0 + r, min(R, nrows - r));
 }
 
+// How the products are split (flash_mma.cuh): scores and output, and sums of gradients.
+__host__ __device__ constexpr fm::Form scores_form(bool fine) { return fine ? fm::FINE : fm::COARSE_CUT; }
+__host__ __device__ constexpr fm::Form gradient_form(bool fine) { return fine ? fm::FINE : fm::COARSE; }
+
 // Forward on warp-level tensor-core instructions.  A block owns 64 queries of one head, a warp 16 of them; keys come 32
 // at a time, two buffers, the next 32 copied while these are multiplied.  Scores, probabilities and output stay in
 // registers; the running maximum moves once per 32 keys.  Bound by the tensor pipe: 3 instructions of 8 cycles for 8
@@ -177,9 +181,9 @@ __device__ __noinline__ void fwd_rows_again(float *smem, float *out, float *lse,
 // (the tensor pipe is about half busy: two to three warps a scheduler do not cover the latency of splits and products; more
 // registers a thread, for more of them under way, are worth more than a third block: 1 x 2048 x 4 x 64 124 -> 105 us.)
 // Measured, the kernel before (4 rows x 16 columns a thread on the FMA pipe) -> this: B8 T1024 12 heads of 64 936 -> 253 us,
-// B4 T2048 8 x 128 3608 -> 670, B2 T777 12 x 32 191 -> 42, B1 T64 2 x 32 18.9 -> 7.6.  2-norm errors against 64 bits there:
-// 2.7e-7 -> 1.8e-7, 3.5e-7 -> 2.1e-7, 2.5e-7 -> 1.9e-7, 1.1e-7 -> 1.4e-7.
-template <int HS>
+// B4 T2048 8 x 128 3608 -> 670, B2 T777 12 x 32 191 -> 42, B1 T64 2 x 32 18.9 -> 7.1.  2-norm errors against 64 bits there:
+// 2.7e-7 -> 1.7e-7, 3.5e-7 -> 1.8e-7, 2.5e-7 -> 1.6e-7, 1.2e-7 -> 0.9e-7.
+template <int HS, bool FINE>
 __global__ void __launch_bounds__(128, HS == 32 ? 3 : 2)
 flash_fwd_mma_k(float *__restrict__ out, float *__restrict__ lse, const float *__restrict__ qkv, int T, int NH, float scale) {
     extern __shared__ __align__(16) float smem[];
@@ -214,13 +218,12 @@ flash_fwd_mma_k(float *__restrict__ out, float *__restrict__ lse, const float *_
         if (j0 + 32 < jmax) copy_keys(j0 + 32, buf ^ 1);
         if (j0 > row0 + 15) continue;  // (per warp) all of these keys lie after all of its queries
         float s[4][4];
-        fm::scores<HS, 2>(s, Qs, warp * 16, Ks + buf * 32 * HS, 0);
+        fm::scores<HS, scores_form(FINE)>(s, scale, Qs, warp * 16, Ks + buf * 32 * HS, 0);
         const bool edge = j0 + 31 > row0 || j0 + 32 > T;               // some pair is masked
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                s[j][i] *= scale;
                 if (edge) {
                     const int key = j0 + 8 * j + 2 * t + (i & 1), row = row0 + g + 8 * (i >> 1);
                     if (key > row || key >= T) s[j][i] = -INFINITY;
@@ -248,7 +251,7 @@ flash_fwd_mma_k(float *__restrict__ out, float *__restrict__ lse, const float *_
             m[r] = mnew;
             l[r] = l[r] * resc[r] + csum;             // this thread's keys; the row's four lanes are added at the end
         }
-        fm::contract<HS, 2, true>(o, resc[0], resc[1], s, Vs + buf * 32 * HS, 0);
+        fm::contract<HS, scores_form(FINE), true>(o, resc[0], resc[1], s, Vs + buf * 32 * HS, 0);
     }
 
     bool bad = false;
@@ -525,7 +528,7 @@ template <int HS> struct bwd_warps { static constexpr int value = HS == 128 ? 8 
 template <int HS> constexpr int bwd_smem() { return (2 * bwd_warps<HS>::value * 16 * HS + 4 * 32 * HS + 4 * 32) * 4; }
 
 // dQ = scale * sum over keys of dS K, dS = P (dO V^T - D), P = exp(scale Q K^T - lse).
-template <int HS>
+template <int HS, bool FINE>
 __device__ __forceinline__ void bwd_q_mma(float *__restrict__ smem, float *__restrict__ dqkv, const float *__restrict__ qkv,
                                           const float *__restrict__ dout, const float *__restrict__ lse,
                                           const float *__restrict__ dsum, int T, int NH, float scale, int bh, int i0) {
@@ -565,8 +568,8 @@ __device__ __forceinline__ void bwd_q_mma(float *__restrict__ smem, float *__res
         if (j0 + 32 < jmax) copy_keys(j0 + 32, buf ^ 1);
         if (j0 > row0 + 15) continue;
         float s[4][4], dp[4][4];
-        fm::scores<HS, 2>(s, Qs, warp * 16, Ks + buf * 32 * HS, 0);
-        fm::scores<HS, 2>(dp, Os, warp * 16, Vs + buf * 32 * HS, 0);
+        fm::scores<HS, scores_form(FINE)>(s, scale, Qs, warp * 16, Ks + buf * 32 * HS, 0);
+        fm::scores<HS, scores_form(FINE)>(dp, 1.0f, Os, warp * 16, Vs + buf * 32 * HS, 0);
         const bool edge = j0 + 31 > row0 || j0 + 32 > T || row0 + 16 > T;
 #pragma unroll
         for (int j = 0; j < 4; ++j)
@@ -574,17 +577,17 @@ __device__ __forceinline__ void bwd_q_mma(float *__restrict__ smem, float *__res
             for (int i = 0; i < 4; ++i) {
                 const int key = j0 + 8 * j + 2 * t + (i & 1), row = row0 + g + 8 * (i >> 1);
                 const bool on = !edge || (key <= row && key < T && row < T);
-                const float p = on ? __expf(s[j][i] * scale - lrow[i >> 1]) : 0.0f;
+                const float p = on ? __expf(s[j][i] - lrow[i >> 1]) : 0.0f;
                 s[j][i] = p * (dp[j][i] - drow[i >> 1]);
             }
-        fm::contract<HS, 2, false>(dq, 1.0f, 1.0f, s, Ks + buf * 32 * HS, 0);
+        fm::contract<HS, gradient_form(FINE), false>(dq, 1.0f, 1.0f, s, Ks + buf * 32 * HS, 0);
     }
     const bool bad = fm::store_rows<HS>(dqkv + ((long long)b * T + row0) * ld + h * HS, ld, g, T - row0, dq, scale, scale);
     if (__syncthreads_or(bad)) bwd_q_rows_again<HS, NT>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, bh, i0, ROWS);
 }
 
 // dV = sum over queries of P^T dO, dK = scale * sum of dS^T Q: the transposed scores, keys as rows.
-template <int HS>
+template <int HS, bool FINE>
 __device__ __forceinline__ void bwd_kv_mma(float *__restrict__ smem, float *__restrict__ dqkv, const float *__restrict__ qkv,
                                            const float *__restrict__ dout, const float *__restrict__ lse,
                                            const float *__restrict__ dsum, int T, int NH, float scale, int bh, int j0) {
@@ -626,22 +629,22 @@ __device__ __forceinline__ void bwd_kv_mma(float *__restrict__ smem, float *__re
         const float *q = Qs + buf * 32 * HS, *go = Os + buf * 32 * HS, *Lb = Ls + buf * 32, *Db = Ds + buf * 32;
         const bool edge = i0 < key0 + 15 || i0 + 32 > T || key0 + 16 > T;
         float p[4][4], ds[4][4];
-        fm::scores<HS, 2>(p, Ks, warp * 16, q, 0);
+        fm::scores<HS, scores_form(FINE)>(p, scale, Ks, warp * 16, q, 0);
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int c = 8 * j + 2 * t + (i & 1), key = key0 + g + 8 * (i >> 1);
                 const bool on = !edge || (i0 + c >= key && i0 + c < T && key < T);
-                p[j][i] = on ? __expf(p[j][i] * scale - Lb[c]) : 0.0f;
+                p[j][i] = on ? __expf(p[j][i] - Lb[c]) : 0.0f;
             }
-        fm::contract<HS, 2, false>(dv, 1.0f, 1.0f, p, go, 0);
-        fm::scores<HS, 2>(ds, Vs, warp * 16, go, 0);
+        fm::contract<HS, gradient_form(FINE), false>(dv, 1.0f, 1.0f, p, go, 0);
+        fm::scores<HS, scores_form(FINE)>(ds, 1.0f, Vs, warp * 16, go, 0);
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
             for (int i = 0; i < 4; ++i) ds[j][i] = p[j][i] * (ds[j][i] - Db[8 * j + 2 * t + (i & 1)]);
-        fm::contract<HS, 2, false>(dk, 1.0f, 1.0f, ds, q, 0);
+        fm::contract<HS, gradient_form(FINE), false>(dk, 1.0f, 1.0f, ds, q, 0);
     }
     float *dkp = dqkv + ((long long)b * T + key0) * ld + C + h * HS;
     bool bad = fm::store_rows<HS>(dkp, ld, g, T - key0, dk, scale, scale);
@@ -651,17 +654,17 @@ __device__ __forceinline__ void bwd_kv_mma(float *__restrict__ smem, float *__re
 
 // Both in one grid (one partly filled last wave instead of two), the longest blocks first: the first key block has all
 // queries, the last query block all keys.
-// Measured with D, row-group kernels -> this: B8 T1024 12 heads of 64 2436 -> 937 us, B4 T2048 8 x 128 18754 -> 2504,
-// B2 T777 12 x 32 445 -> 105.  2-norm errors of dq / dk / dv against 64 bits at 8 x 128: 4.9 / 10.8 / 10.8e-7 -> 3.3 / 3.7 / 3.3e-7.
-template <int HS>
+// Measured with D, row-group kernels -> this: B8 T1024 12 heads of 64 2436 -> 960 us, B4 T2048 8 x 128 18754 -> 2501,
+// B2 T777 12 x 32 445 -> 105.  2-norm errors of dq / dk / dv against 64 bits at 8 x 128: 4.9 / 10.8 / 10.8e-7 -> 3.2 / 3.7 / 3.3e-7.
+template <int HS, bool FINE>
 __global__ void __launch_bounds__(bwd_warps<HS>::value * 32, HS == 128 ? 1 : HS == 64 ? 2 : 3)
 flash_bwd_mma_k(float *__restrict__ dqkv, const float *__restrict__ qkv, const float *__restrict__ dout,
                 const float *__restrict__ lse, const float *__restrict__ dsum, int T, int NH, float scale) {
     extern __shared__ __align__(16) float smem[];
     constexpr int ROWS = bwd_warps<HS>::value * 16;
     const int rank = blockIdx.y >> 1, blocks = gridDim.y >> 1;
-    if (blockIdx.y & 1) bwd_q_mma<HS>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, blockIdx.x, (blocks - 1 - rank) * ROWS);
-    else bwd_kv_mma<HS>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, blockIdx.x, rank * ROWS);
+    if (blockIdx.y & 1) bwd_q_mma<HS, FINE>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, blockIdx.x, (blocks - 1 - rank) * ROWS);
+    else bwd_kv_mma<HS, FINE>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, blockIdx.x, rank * ROWS);
 }
 
 struct FwdCfg { int kc; const char *name; };
@@ -674,6 +677,11 @@ const FwdCfg FWD[] = {{32, "mma-3xtf32 q64 k32"}, {16, "simt-fp32 rowgroup keys1
 const BwdCfg BWD[] = {{32, "mma-3xtf32 rows16 per warp, 32 at a time"}, {8, "simt-fp32 rowgroup keys8"},
                       {0, "tcgen05-tf32 dq128x128 dkv128x128 (head size 64 only)"}};
 constexpr int NFWD = 3, NBWD = 3, FWD_TC = 2, BWD_TC = 2;
+
+// Sequences up to here take six products for one instead of three: against kernels on the FMA pipe in chains of 8, the error of
+// the output at T = 128 is 0.69 (three products: 1.00 to 1.04), at T = 8 0.84 (1.5), and from 129 on three are no worse than
+// those.  128 x 128 positions, 4 heads of 64: forward 22 -> 37 us, backward 76 -> 123 (the FMA pipe: 54 and 184).
+constexpr int FINE_T = 128;
 
 bool shape_ok(const float *a, const float *b, int C, int NH) {
     return NH > 0 && C % NH == 0 && (((uintptr_t)a | (uintptr_t)b) & 15) == 0;
@@ -696,8 +704,9 @@ int run_fwd(int cfg, float *out, float *lse, const float *qkv, int B, int T, int
     if (cfg == 0) {
         constexpr int SMEM = (64 + 4 * 32) * HS * 4;
         if (ceil_div(T, 64) > 65535) return fail(BMB_E_ARG, "flash: T=%d too long", T);
-        BMB_TRY(allow_smem((const void *)flash_fwd_mma_k<HS>, SMEM));
-        flash_fwd_mma_k<HS><<<dim3(B * NH, ceil_div(T, 64)), 128, SMEM, st>>>(out, lse, qkv, T, NH, scale);
+        const auto kernel = T <= FINE_T ? flash_fwd_mma_k<HS, true> : flash_fwd_mma_k<HS, false>;
+        BMB_TRY(allow_smem((const void *)kernel, SMEM));
+        kernel<<<dim3(B * NH, ceil_div(T, 64)), 128, SMEM, st>>>(out, lse, qkv, T, NH, scale);
     } else {
         constexpr int R = FT / (HS / 32);
         dim3 grid(ceil_div(T, R), B * NH);
@@ -715,9 +724,9 @@ int run_bwd(int cfg, float *dqkv, float *dsum, const float *dout, const float *q
         constexpr int ROWS = bwd_warps<HS>::value * 16;
         if (ceil_div(T, ROWS) > 32767) return fail(BMB_E_ARG, "flash: T=%d too long", T);
         BMB_TRY(launch_flash_dsum(dsum, dout, out, B, T, NH, HS, st));
-        BMB_TRY(allow_smem((const void *)flash_bwd_mma_k<HS>, bwd_smem<HS>()));
-        flash_bwd_mma_k<HS><<<dim3(B * NH, 2 * ceil_div(T, ROWS)), bwd_warps<HS>::value * 32, bwd_smem<HS>(), st>>>(dqkv, qkv, dout, lse, dsum,
-                                                                                                    T, NH, scale);
+        const auto kernel = T <= FINE_T ? flash_bwd_mma_k<HS, true> : flash_bwd_mma_k<HS, false>;
+        BMB_TRY(allow_smem((const void *)kernel, bwd_smem<HS>()));
+        kernel<<<dim3(B * NH, 2 * ceil_div(T, ROWS)), bwd_warps<HS>::value * 32, bwd_smem<HS>(), st>>>(dqkv, qkv, dout, lse, dsum, T, NH, scale);
         count_launch();
         BMB_LAUNCH_CHECK();
         return BMB_OK;

@@ -66,7 +66,7 @@ void *bmb_get_stream(void);
 /* Arithmetic used by bmb_gemm / bmb_batched_gemm / flash attention when the
  * caller does not say.  fp32 = SIMT FFMA, bit-comparable with the reference's
  * fp32 kernels up to summation order, or, for large single products and for
- * attention, split products on the tensor cores with a smaller error than that; tf32 = tcgen05 kind::tf32 with operands
+ * attention (elements from 2^-108 on), split products on the tensor cores with a smaller error than that; tf32 = tcgen05 kind::tf32 with operands
  * rounded to nearest TF32 first and fp32 accumulation in tensor memory;
  * bf16 = tcgen05 kind::f16 on bf16-rounded operands. */
 #define BMB_MATH_FP32 0
