@@ -561,6 +561,7 @@ __device__ __forceinline__ void bwd_q_mma(float *__restrict__ smem, float *__res
 #pragma unroll
         for (int i = 0; i < 4; ++i) dq[c][i] = 0.0f;
 
+    float most = 0.0f;                 // a score may overflow before it is scaled (the row-group code scales q first)
     int buf = 0;
     for (int j0 = 0; j0 < jmax; j0 += 32, buf ^= 1) {
         fm::cp_wait_all();
@@ -574,6 +575,10 @@ __device__ __forceinline__ void bwd_q_mma(float *__restrict__ smem, float *__res
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
+            for (int i = 0; i < 4; i += 2) asm("max.abs.f32 %0, %0, %1, %2;" : "+f"(most) : "f"(s[j][i]), "f"(s[j][i + 1]));
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int key = j0 + 8 * j + 2 * t + (i & 1), row = row0 + g + 8 * (i >> 1);
                 const bool on = !edge || (key <= row && key < T && row < T);
@@ -582,7 +587,7 @@ __device__ __forceinline__ void bwd_q_mma(float *__restrict__ smem, float *__res
             }
         fm::contract<HS, gradient_form(FINE), false>(dq, 1.0f, 1.0f, s, Ks + buf * 32 * HS, 0);
     }
-    const bool bad = fm::store_rows<HS>(dqkv + ((long long)b * T + row0) * ld + h * HS, ld, g, T - row0, dq, scale, scale);
+    const bool bad = fm::store_rows<HS>(dqkv + ((long long)b * T + row0) * ld + h * HS, ld, g, T - row0, dq, scale, scale) || most > 3.402823466e38f;
     if (__syncthreads_or(bad)) bwd_q_rows_again<HS, NT>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, bh, i0, ROWS);
 }
 

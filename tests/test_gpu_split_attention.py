@@ -1,5 +1,5 @@
 """fp32 attention in split products (csrc/flash.cu, configuration 0): its errors against 64 bits are no larger than those of
-kernels on the FMA pipe in chains of 8, at any length."""
+kernels on the FMA pipe in chains of 8, at any length, and what those kernels took it takes."""
 import numpy as np
 import pytest
 
@@ -64,3 +64,26 @@ def test_small_operands(bmb, cuda, hs, T, scales):
     err = errors(bmb, cuda, hs, T, scales)
     out, lse, dqkv = chains(hs, T)
     assert all(e <= 1.03 * c for e, c in zip(err, (out, lse, 1.3 * dqkv, 1.3 * dqkv, 1.3 * dqkv))), err
+
+
+@pytest.mark.parametrize("hs", [32, 64, 128])
+def test_scores_that_overflow_before_they_are_scaled(bmb, cuda, hs):
+    """q k of -1.8 times the largest number, scaled by hs^-1/2: the one key of a first row has probability 1 there."""
+    B, T, NH = 1, 40, 1
+    C = hs
+    g = cuda.Generator(device="cuda").manual_seed(hs)
+    qkv, dout = cuda.randn(B, T, 3 * C, generator=g, device="cuda"), cuda.randn(B, T, C, generator=g, device="cuda")
+    qkv[0, :, :C], qkv[0, :, C:2 * C] = 0.0, 0.0
+    x = float((1.8 * 3.4e38 / hs) ** 0.5)
+    qkv[0, 0, :C], qkv[0, 0, C:2 * C] = x, -x
+    got = []
+    for cfg in (0, 1):
+        out, lse, dsum, dqkv = (cuda.zeros(s, device="cuda") for s in ((B, T, C), (B, NH, T), (B, NH, T), (B, T, 3 * C)))
+        bmb.call("bmb_flash_attention_forward_cfg", cfg, out, lse, qkv, B, T, C, NH)
+        out[0, 0] += 1e-3                        # so that dP - D is not zero there
+        bmb.call("bmb_flash_attention_backward_cfg", cfg, dqkv, dsum, dout, qkv, out, lse, B, T, C, NH)
+        cuda.cuda.synchronize()
+        got.append((out, lse, dqkv[..., :C]))
+    for a, b in zip(*got):
+        assert bool(cuda.isfinite(b).all()) and float((a - b).abs().max()) <= 1e-5 * float(b.abs().max())
+    assert float(got[1][2][0, 0].abs().max()) > 0
