@@ -706,9 +706,9 @@ int allow_smem(const void *kernel, int bytes) {
 template <int HS>
 int run_fwd(int cfg, float *out, float *lse, const float *qkv, int B, int T, int NH, float scale,
             cudaStream_t st) {
+    if (cfg == 0 && ceil_div(T, 64) > 65535) cfg = 1;              // (blocks of rows on grid y)
     if (cfg == 0) {
         constexpr int SMEM = (64 + 4 * 32) * HS * 4;
-        if (ceil_div(T, 64) > 65535) return fail(BMB_E_ARG, "flash: T=%d too long", T);
         const auto kernel = T <= FINE_T ? flash_fwd_mma_k<HS, true> : flash_fwd_mma_k<HS, false>;
         BMB_TRY(allow_smem((const void *)kernel, SMEM));
         kernel<<<dim3(B * NH, ceil_div(T, 64)), 128, SMEM, st>>>(out, lse, qkv, T, NH, scale);
@@ -725,9 +725,9 @@ int run_fwd(int cfg, float *out, float *lse, const float *qkv, int B, int T, int
 template <int HS>
 int run_bwd(int cfg, float *dqkv, float *dsum, const float *dout, const float *qkv, const float *out,
             const float *lse, int B, int T, int NH, float scale, cudaStream_t st) {
+    constexpr int ROWS = bwd_warps<HS>::value * 16;
+    if (cfg == 0 && ceil_div(T, ROWS) > 32767) cfg = 1;
     if (cfg == 0) {
-        constexpr int ROWS = bwd_warps<HS>::value * 16;
-        if (ceil_div(T, ROWS) > 32767) return fail(BMB_E_ARG, "flash: T=%d too long", T);
         BMB_TRY(launch_flash_dsum(dsum, dout, out, B, T, NH, HS, st));
         const auto kernel = T <= FINE_T ? flash_bwd_mma_k<HS, true> : flash_bwd_mma_k<HS, false>;
         BMB_TRY(allow_smem((const void *)kernel, bwd_smem<HS>()));
