@@ -39,7 +39,9 @@ int gemm_any_bias(int math, int flags, int ta, int tb, int batch, int M, int N, 
         // there too, as does registry entry 1: they are held to the sequential fp32 chain.  So do the products that the
         // tensor-core modes leave to fp32 kernels: in a trainer of those modes they run side by side on two streams and in
         // captures, where the images' scratch, one per device, would be shared unordered.
-        rc = (math == BMB_MATH_FP32 && batch == 1 && A && B && C && !(flags & GEMM_CHAIN)) ? gemm_x3(ta, tb, M, N, K, alpha, A, B, beta, C, bias, flags, st) : BMB_E_UNSUPPORTED;
+        // (A bias that the pass behind a SIMT product refuses is refused at any size.)
+        const bool bias_ok = !bias || (N % 4 == 0 && (((uintptr_t)bias | (uintptr_t)C) & 15) == 0);
+        rc = (math == BMB_MATH_FP32 && batch == 1 && A && B && C && bias_ok && !(flags & GEMM_CHAIN)) ? gemm_x3(ta, tb, M, N, K, alpha, A, B, beta, C, bias, flags, st) : BMB_E_UNSUPPORTED;
         const bool bias_done = rc == BMB_OK;
         if (rc == BMB_E_UNSUPPORTED) rc = gemm_simt(ta, tb, batch, M, N, K, alpha, A, sA, B, sB, beta, C, sC, st);
         if (rc != BMB_OK) return rc;

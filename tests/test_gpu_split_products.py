@@ -250,6 +250,16 @@ def test_split_products_of_threads_and_streams_take_turns(bmb, cuda, per_thread)
         assert all(cuda.equal(C, w[5]) for C in w[6])
 
 
+@pytest.mark.parametrize("N,offset", [(514, 0), (516, 1)])
+def test_a_bias_that_is_refused_is_refused_at_any_size(bmb, cuda, N, offset):
+    """Columns that are no multiple of 4, or a bias off 16 bytes, beside a small product and a split one."""
+    g = cuda.zeros(2 ** 20, device="cuda")
+    for M, K in [(8, 8), (1024, 512)]:
+        with pytest.raises(Exception):
+            bmb.call("bmb_gemm_bias_gelu", bmb.MATH_FP32, 0, M, N, K, g, g, g[offset:], cuda.empty(M * N, device="cuda"), cuda.empty(M * N, device="cuda"), None)
+    cuda.cuda.synchronize()
+
+
 def test_growing_the_scratch_leaves_a_capture_alone(bmb, cuda):
     """A product whose images need a larger block than any before, on one stream, while another stream is being captured in
     the global mode: the capture goes on, and both results are right."""
