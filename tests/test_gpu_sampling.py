@@ -81,3 +81,33 @@ def test_sampling_against_64_bits(bmb, cuda, heads, hs, B, T, V, flash):
     t.step(0.0, 2)
     assert abs(t.loss() - loss) < 1e-6
     t.close()
+
+
+@pytest.mark.parametrize("heads,hs,T,layers", [
+    (2, 32, 300, 2),        # more than 256 positions: the running maximum is carried from one 32 groups of keys to the next
+    (1, 128, 400, 1),       # more than 320 at 128 columns (and 640 at 64): the values no longer fit in shared memory
+    (2, 64, 700, 1),
+    (9, 32, 70, 2),         # 1152 inputs: the ring of weight slices comes round
+])
+def test_long_texts_position_by_position(bmb, cuda, heads, hs, T, layers):
+    """Texts that fill the context, drawn one position at a time. The distributions of the window path, which follows the same
+    order of sums, choose the same tokens by the same coins; they themselves are within 1e-4 of the model in 64 bits."""
+    V, Vp, B = 65, 128, 2
+    t = bmb.Trainer(seed=5, max_seq_len=T, vocab_size=V, padded_vocab=Vp, n_layer=layers, n_head=heads, n_embd=heads * hs, B=B, T=T,
+                    use_flash=1, math=bmb.MATH_FP32, fused=0)
+    m = Model64(cuda, t)
+    seed = 3
+    text = t.generate(0, T - 1, seed, 1.0)
+    coins = np.random.RandomState(seed).randint(0, 2 ** 32, size=T - 1, dtype=np.uint32).astype(np.float32) / np.float32(2 ** 32)
+    tokens = np.zeros((B, T), np.int32)
+    tokens[0, 1:] = text
+    got = cuda.empty(Vp)
+    for s in list(range(0, T - 1, 7)) + list(range(T - 12, T - 1)):
+        bmb.call("bmb_trainer_next_token_probs", t.h, tokens, s, got)
+        p = got.numpy()[:V].astype(np.float64)
+        cdf = np.cumsum(p / p.sum())
+        tok = min(int(np.searchsorted(cdf, coins[s], side="right")), V - 1)
+        assert tok == text[s] or np.abs(cdf - coins[s]).min() < 1e-6, (s, tok, text[s])     # (sums of 65 fp32 numbers)
+        if s % 49 == 0 or s == T - 2:
+            assert np.abs(p / m.probs(tokens[0, :s + 1]) - 1).max() < 1e-4, s
+    t.close()
