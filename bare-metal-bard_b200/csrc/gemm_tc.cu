@@ -1269,8 +1269,9 @@ static bool rounds_on_arrival(Plan *plan, int flags, int transA, int transB, int
     // against 1570 with rounding in place, 128 columns 520 and 1100, 64 columns 400 and 1000); tiles of up to 128 columns
     // with a short K are bound by their stores instead, about 20 bytes a cycle and SM, beside which rounding is free.  A
     // pass is a launch of about 4500 cycles and 8 bytes an element at 5000 a cycle.  Sides of the line, pass / in place:
-    // 1024^3 25.8 / 24.6 us, 768x768x4096 37.5 / 33.8, 6144x128x6144 97 / 48, batch 96 of 1024x64x1024 234 / 100,
-    // 8 of 256x256x32 20 / 9; but 2048^3 55 / 67, 4096^3 234 / 376, 2560x2560x640 33 / 43, 6144x6144x64 48 / 50.
+    // 768x768x4096 37.5 / 33.8 us, 6144x128x6144 97 / 48, batch 96 of 1024x64x1024 234 / 100,
+    // 8 of 256x256x32 20 / 9; but 2048^3 55 / 67, 4096^3 234 / 376, 2560x2560x640 33 / 43, 6144x6144x64 48 / 50
+    // (and 1024^3, 25.8 / 24.6, which the rule leaves to the pass).
     auto cycles = [&](const Plan &q, bool in_place) {
         const double slice = q.mh == 2 ? 1.72 * 800.0 : in_place ? (q.bn == 256 ? 1570.0 : q.bn == 192 ? 1250.0 : q.bn == 128 ? 1100.0 : 1000.0)
                                                                  : (q.bn == 256 ? 800.0 : q.bn == 192 ? 650.0 : q.bn == 128 ? 520.0 : 400.0);

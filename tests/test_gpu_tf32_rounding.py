@@ -48,3 +48,32 @@ def test_rounding_on_arrival_of_batches(bmb, cuda):
     assert cuda.equal(out[0], out[2]) and cuda.equal(out[1], out[3])
     want = rounded(cuda, q).double() @ rounded(cuda, k).double().transpose(1, 2) * 0.125
     assert float((out[0].double() - want).norm() / want.norm()) < 2e-6
+
+
+# One launch (and one that prepares shared tiles) where operands are rounded on arrival, up to two passes more where not.
+@pytest.mark.parametrize("M,N,K,flags,beta,launches", [
+    (128, 64, 32, NO_SPLIT, 0.0, 1),
+    (132, 68, 36, NO_SPLIT, 0.0, 1),
+    (1000, 300, 100, NO_SPLIT, 0.0, 1),
+    (1024, 1024, 256, 0, 0.0, 1),
+    (200, 1000, 2000, 0, 0.0, 2),            # tiles shared along K: their sums start from beta C, written by a launch before
+    (768, 768, 4096, 0, 0.0, 2),
+    (768, 768, 4096, 0, 0.5, 2),
+    (768, 768, 4096, 0, 1.0, 1),
+    (6144, 128, 6144, 0, 0.0, 2),
+    (200, 1000, 2000, NO_SPLIT, 0.0, 3),     # here the passes cost less
+    (2048, 2048, 2048, NO_SPLIT, 0.0, 3),
+    (4096, 4096, 4096, NO_SPLIT, 0.0, 3),
+])
+def test_where_operands_are_rounded_on_arrival(bmb, cuda, M, N, K, flags, beta, launches):
+    """The route, by the launches it takes, and the result against the 64-bit product of rounded operands: the tensor core cuts
+    its sum off at each of K / 8 instructions, at most 2^-23 of a running sum that is no larger than its end is in the mean."""
+    g = cuda.Generator(device="cuda").manual_seed(M + K)
+    A, B, C0 = (cuda.randn(s, generator=g, device="cuda") for s in ((M, K), (K, N), (M, N)))
+    C = C0.clone()
+    before = bmb.lib().bmb_launch_count()
+    bmb.call("bmb_gemm_ex", bmb.MATH_TF32, flags, 0, 0, M, N, K, 1.0, A, B, beta, C, None)
+    assert bmb.lib().bmb_launch_count() - before == launches
+    cuda.cuda.synchronize()
+    want = rounded(cuda, A).double() @ rounded(cuda, B).double() + beta * C0.double()
+    assert float((C.double() - want).norm() / want.norm()) < K / 8 * 2.0 ** -23
