@@ -39,7 +39,7 @@ BMB_ALIAS(sgemm_doublebuffer, sgemm_simt_fp32)
 BMB_ALIAS(sgemm_tensorcore, sgemm_tcgen05_tf32)
 
 extern const KernelEntry KERNELS[] = {
-    {1, "simt_fp32", sgemm_simt_fp32, "sm_100a FFMA, 128x128x16 tile, 8x8 per thread, register-prefetch double buffer", 1e-6},
+    {1, "simt_fp32", sgemm_simt_fp32, "sm_100a FFMA, one sequential fp32 chain per element; tiles of 128, 64 or 32 by the size", 1e-6},
     {2, "tcgen05_tf32", sgemm_tcgen05_tf32, "tcgen05.mma kind::tf32, TMA-fed swizzled ring, TMEM accumulators, rna-rounded operands", 5e-4},
     {3, "tcgen05_bf16", sgemm_tcgen05_bf16, "tcgen05.mma kind::f16 on bf16-rounded operands, fp32 accumulate in TMEM", 8e-3},
 };

@@ -1,4 +1,4 @@
-// Fused causal attention, fp32 SIMT path (src/flash.h:36-62, src/flash.cu).
+// Fused causal attention in fp32 (src/flash.h:36-62, src/flash.cu): split products, and the row-group SIMT code behind them.
 //
 // The score matrix never reaches global memory: the forward walks key tiles
 // with a running row max / row sum and writes out (B,T,C) plus

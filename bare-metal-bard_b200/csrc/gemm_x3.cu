@@ -539,8 +539,7 @@ gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict
                                 if (second) d[1] = x.y;
                                 continue;
                             }
-                            // (256 columns: one sum more in registers than there are, so edges take the call, which is slow
-                            // and which the choice of a plan counts)
+                            // (256 columns: one sum more in registers than there are, so edges take the call, which is slow)
                             if (BN == 256) {
                                 put_element(p, m, n, x.x);
                                 if (second) put_element(p, m, n + 1, x.y);
@@ -699,7 +698,8 @@ XPlan choose_x3(int units, int M, int N, int kblocks) {
             if (s > 1 && kblocks / s < 4) break;
             const double rounds = (double)ceil_div(tiles * s, units);
             double t = rounds * (ceil_div(kblocks, s) * slice[w] + tail[w]) + 3000;
-            if (s == 1 && ragged && widths[w] == 256) t += 40000;      // (2000 x 2000 x 500: 58 us, 42 with 128 columns)
+            // the tile with an edge ends last, whatever their number (one size: 2000 x 2000 x 500 58 us, 42 with 128 columns)
+            if (s == 1 && ragged && widths[w] == 256) t += 40000;
             if (s > 1) t += 4000 + (double)M * N * 4 * (2 * s + 1) / 3000;
             if (t < best_t) { best_t = t; best = {widths[w], s}; }
         }

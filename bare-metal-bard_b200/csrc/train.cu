@@ -170,8 +170,8 @@ struct Scope {
 // and gradients where they lie), and the bias add rides in the GEMM epilogue.
 bool fused_tf32(const bmb_train_config &c) { return c.fused && c.math == BMB_MATH_TF32; }
 
-// Attention kernel configuration for this trainer's arithmetic: the SIMT fp32
-// kernels, or the tensor-core pair (config 2 of both tables) when the GEMMs
+// Attention kernel configuration for this trainer's arithmetic: the fp32 kernels
+// (split products, config 0), or the tensor-core pair (config 2 of both tables) when the GEMMs
 // run on tensor cores and the head size is the one those kernels serve.
 int attn_cfg(const bmb_train_config &c) {
     return (c.math != BMB_MATH_FP32 && c.n_embd / c.n_head == 64) ? 2 : 0;
