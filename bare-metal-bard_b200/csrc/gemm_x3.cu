@@ -153,8 +153,6 @@ struct Result {
     const float *bias;             // added to every row, or null
     const uint32_t *lostA, *lostB; // Operand::lost, `words` a panel
     int words;
-    uint8_t *lost;                 // the same a panel (of A, then of B), for the pass that adds the parts
-    int panels_a, panels;
 };
 // Word i of what says whether panel a of A, and panels b, b + 1, .. of B, lost bits.
 __device__ __forceinline__ const uint32_t *lost_word(const Result &p, int a, int b, int i) {
@@ -414,14 +412,6 @@ gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict
         }
     } else {
         const int q = warp & 3, half = (warp - 2) >> 2;
-        if (parts > 1 && warp == 2) {
-            for (int i = blockIdx.x; i < p.panels; i += gridDim.x) {
-                uint32_t l = 0;
-                for (int w = lane; w < p.words; w += 32) l |= __ldg((i < p.panels_a ? p.lostA + (long long)i * p.words : p.lostB + (long long)(i - p.panels_a) * p.words) + w);
-                l = __any_sync(0xffffffffu, l != 0);
-                if (lane == 0) p.lost[i] = l;
-            }
-        }
         int acc = 0;
         uint32_t acc_ph = 0;
         bool ok = true;
@@ -429,7 +419,7 @@ gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict
             // this lane's share of the words on whether this warp's panels lost bits; asked for here (volatile), beside the first
             // products, and wanted at the end: at K up to 5000 a word a lane
             uint32_t lost = 0;
-            if (parts == 1) {
+            {
                 const int pa = (tm * XM + q * 32) / 64, pb = (tn * BN + half * (BN / 2)) / 64, nb = (tn * BN + half * (BN / 2) + BN / 2 - 1) / 64 - pb + 1;
                 if (lane < (1 + nb) * p.words) asm volatile("ld.global.b32 %0, [%1];" : "=r"(lost) : "l"(lost_word(p, pa, pb, lane)));
                 for (int i = lane + 32; i < (1 + nb) * p.words; i += 32) lost |= __ldg(lost_word(p, pa, pb, i));
@@ -491,6 +481,11 @@ gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict
                     if (leave) *again = 1;
                 }
                 if (leave) continue;
+            } else if (__any_sync(0xffffffffu, lost != 0)) {         // the pass that adds the parts computes these
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) sum[c][i] = __int_as_float(0x7fffffff);
             }
             if (vec && (tm + 1) * XM <= p.M && (tn + 1) * BN <= p.N) {
 #pragma unroll
@@ -614,19 +609,17 @@ __device__ __noinline__ void four_again(const Result &from, int m, int n, uint32
 // The parts of a K shared among CTAs, added in order.
 __global__ void __launch_bounds__(256) reduce_x3_k(const Result p, int parts, const float *__restrict__ ws, int vec4) {
     const long long n = (long long)p.M * p.N, step = (long long)gridDim.x * blockDim.x;
-    auto lost = [&](int row, int col) { return (p.lost[row / 64] | p.lost[p.panels_a + col / 64]) != 0; };
     if (vec4) {
         for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n / 4; e += step) {
             float4 s = __ldg(reinterpret_cast<const float4 *>(ws) + e);
-            const int row = n < (1LL << 31) ? (int)((uint32_t)(4 * e) / (uint32_t)p.N) : (int)(4 * e / p.N), col = (int)(4 * e - (long long)row * p.N);
-            const bool whole = !lost(row, col);
             for (int q = 1; q < parts; ++q) {
                 const float4 x = __ldg(reinterpret_cast<const float4 *>(ws + q * n) + e);
                 s.x += x.x; s.y += x.y; s.z += x.z; s.w += x.w;
             }
-            if (!whole || doubtful(s.x) || doubtful(s.y) || doubtful(s.z) || doubtful(s.w)) {
+            if (doubtful(s.x) || doubtful(s.y) || doubtful(s.z) || doubtful(s.w)) {
+                const int row = (int)(4 * e / p.N), col = (int)(4 * e % p.N);
                 const float v[4] = {s.x, s.y, s.z, s.w};
-                uint32_t again = whole ? 0u : 15u;
+                uint32_t again = 0;
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     again |= (doubtful(v[i]) ? 1u : 0u) << i;
@@ -643,7 +636,7 @@ __global__ void __launch_bounds__(256) reduce_x3_k(const Result p, int parts, co
                 o.z = fmaf(p.beta, old.z, o.z); o.w = fmaf(p.beta, old.w, o.w);
             }
             if (p.bias) {                           // N is a multiple of 4 here: the four are of one row
-                const float *b = p.bias + col;
+                const float *b = p.bias + (int)(4 * e % p.N);
                 o.x += __ldg(b); o.y += __ldg(b + 1); o.z += __ldg(b + 2); o.w += __ldg(b + 3);
             }
             *cp = o;
@@ -652,9 +645,8 @@ __global__ void __launch_bounds__(256) reduce_x3_k(const Result p, int parts, co
         for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += step) {
             float s = ws[e];
             for (int q = 1; q < parts; ++q) s += ws[q * n + e];
-            const int row = (int)(e / p.N), col = (int)(e - (long long)row * p.N);
-            if (doubtful(s) || lost(row, col)) four_again(p, row, col, 1u);
-            else put_element(p, row, col, s);
+            if (doubtful(s)) four_again(p, (int)(e / p.N), (int)(e % p.N), 1u);
+            else put_element(p, (int)(e / p.N), (int)(e % p.N), s);
         }
     }
 }
@@ -746,7 +738,7 @@ int gemm_x3(int transA, int transB, int M, int N, int K, float alpha, const floa
     const int words = ceil_div(oa.kgroups, 4);
     const long long flagsA = 4LL * words * oa.panels, flagsB = 4LL * words * ob.panels;
     const long long marks = plan.parts > 1 ? 0 : 8 * tiles;
-    const long long need = imgA + imgB + ws + marks + flagsA + flagsB + oa.panels + ob.panels;      // the images: multiples of 256 bytes (without parts there is no ws)
+    const long long need = imgA + imgB + ws + marks + flagsA + flagsB;      // the images: multiples of 256 bytes (without parts there is no ws)
     if (tiles >= (1LL << 30) || na + nb >= (1LL << 31) || need > (16LL << 30)) return BMB_E_UNSUPPORTED;
     int *status_dev = nullptr;
     volatile int *status_host = nullptr;
@@ -763,8 +755,7 @@ int gemm_x3(int transA, int transB, int M, int N, int K, float alpha, const floa
     ob.lost = oa.lost + flagsA;
 
     auto vec_of = [](const float *p, int inner) { return ((uintptr_t)p & 15) == 0 && inner % 4 == 0; };
-    const Result p{A, B, transA, transB, M, N, K, alpha, beta, C, bias, (const uint32_t *)oa.lost, (const uint32_t *)ob.lost, words,
-                   ob.lost + flagsB, oa.panels, oa.panels + ob.panels};
+    const Result p{A, B, transA, transB, M, N, K, alpha, beta, C, bias, (const uint32_t *)oa.lost, (const uint32_t *)ob.lost, words};
     const bool even = N % 2 == 0 && (plan.parts > 1 || ((uintptr_t)C & 7) == 0);
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
     BMB_TRY(scratch_acquire(SCR_SPLIT, st));
