@@ -16,14 +16,14 @@ Rank 0 prints ONE JSON line.
             device->host read of the step's loss.
 * `roofline` the GEMMs of the step (the dominant kernels): FLOP of every
             GEMM call / its event-timed duration, against the tensor peak
-            derived from MEASURED_PEAKS.json (TF32 = BF16 / 2) or, in fp32
-            mode, the SIMT peak at the SM clock sampled during that leg.
+            derived from MEASURED_PEAKS.json (TF32 = BF16 / 2, fp32 as split
+            products = BF16 / 6).
 * `gemm`, `attention`, `bgemm`   (N = 1) the square GEMM sweep in fp32 and TF32, fused causal
             attention forward / backward at B=8 H=12 T=1024 hs=64, and the attention-shaped
             batched GEMM (batch 96), each as absolute numbers and as a fraction of the
             roofline that bounds it, with the SM clock sampled during that leg.
-* `fp32_mode`  (N = 1) a short run of the same training step in fp32 SIMT arithmetic, the
-            reference's own precision.
+* `fp32_mode`  (N = 1) a short run of the same training step in fp32 arithmetic, the
+            reference's own precision (split products: the peak is BF16 / 6).
 * `cpu_baseline`, `cpu_matmul`  the CPU oracle's train step and fp32 matmul (oracle/liborc.so)
             on bounded samples, rank 0 at N = 1 only, with the thread count.
 * `losses_head`  the mean loss of each of the first optimiser steps (at most 20), the same
@@ -229,6 +229,11 @@ def simt_peak_tflops(torch, mhz):
     return 2.0 * 128 * nsm * mhz * 1e6 / 1e12
 
 
+def split_peak_tflops(peaks):
+    """fp32 products on the tensor cores: six bf16 instructions' worth, or three TF32 ones, stand for one product."""
+    return peaks["bf16"] / 6.0
+
+
 def gemm_sweep(bmb, torch, peaks, clocks):
     """Square GEMM sweep, fp32 SIMT and TF32: 5 warm-ups, 20 timed calls, best and median.  The fp32
     fraction is taken against the SIMT peak at the SM clock sampled while that size's fp32 calls ran."""
@@ -265,7 +270,7 @@ def gemm_sweep(bmb, torch, peaks, clocks):
 
 
 def attention_leg(bmb, torch, peaks, clocks):
-    """Fused causal attention at B=8 H=12 T=1024 hs=64: tensor-core (TF32) and fp32 SIMT kernels,
+    """Fused causal attention at B=8 H=12 T=1024 hs=64: tensor-core (TF32) and fp32 kernels,
     forward and backward, as time, useful TFLOP/s (4*B*NH*hs*T*(T+1)/2, tools/test_flash.cu:186-187;
     backward 2.5x and the reference's 3.5x count) and fractions of the TF32 tensor peak and of HBM
     bandwidth on the algorithmic bytes (101.1 MB forward, 202.2 MB backward)."""
@@ -305,11 +310,11 @@ def attention_leg(bmb, torch, peaks, clocks):
     fb, fm = timed(torch, lambda: bmb.call("bmb_flash_attention_forward_cfg", 0, out, lse, qkv, B, Tn, Cn, NH), warmup=3, iters=10)
     bb, bm_ = timed(torch, lambda: bmb.call("bmb_flash_attention_backward_cfg", 0, dqkv, dsum, dout, qkv, out, lse, B, Tn, Cn, NH), warmup=3, iters=10)
     ck = clocks.window(t0, time.time())
-    simt = simt_peak_tflops(torch, ck["sm_mhz"] or clocks.max_mhz or 1965.0)
+    split = split_peak_tflops(peaks)
     res["fp32"] = {"fwd_us": round(fb * 1e3, 1), "bwd_us": round(bb * 1e3, 1), "fwd_useful_tflops": round(useful / fb / 1e9, 1),
-                   "fwd_frac_of_simt_peak": round(useful / fb / 1e9 / simt, 3),
-                   "bwd_tflops_2p5x": round(2.5 * useful / bb / 1e9, 1), "bwd_frac_of_simt_peak_2p5x": round(2.5 * useful / bb / 1e9 / simt, 3),
-                   "simt_peak_tflops": round(simt, 1), "sm_mhz": ck["sm_mhz"],
+                   "fwd_frac_of_split_peak": round(useful / fb / 1e9 / split, 3),
+                   "bwd_tflops_2p5x": round(2.5 * useful / bb / 1e9, 1), "bwd_frac_of_split_peak_2p5x": round(2.5 * useful / bb / 1e9 / split, 3),
+                   "split_peak_tflops": round(split, 1), "sm_mhz": ck["sm_mhz"],
                    "tokens_per_s_fwd_bwd": round(B * Tn / ((fb + bb) * 1e-3), 0)}
     return res
 
@@ -409,8 +414,8 @@ def make_trainer(bmb, math, fused):
                        eps=HP["eps"], weight_decay=HP["weight_decay"], grad_clip=HP["grad_clip"], **GPT124M)
 
 
-def fp32_mode_leg(bmb, torch, dist_mod, clocks, steps=5, warmup=3):
-    """The same training step in fp32 SIMT arithmetic (the reference's precision): `warmup` untimed steps,
+def fp32_mode_leg(bmb, torch, dist_mod, peaks, clocks, steps=5, warmup=3):
+    """The same training step in fp32 arithmetic (the reference's precision): `warmup` untimed steps,
     then `steps` device-timed steps on a resident batch and `steps` more end to end."""
     tr = make_trainer(bmb, bmb.MATH_FP32, 0)
     stream = torch.cuda.ExternalStream(tr.stream)
@@ -448,13 +453,13 @@ def fp32_mode_leg(bmb, torch, dist_mod, clocks, steps=5, warmup=3):
         tr.sync()
     ms_e2e = (time.time() - w0) * 1e3 / steps
     tr.close()
-    simt = simt_peak_tflops(torch, ck["sm_mhz"] or clocks.max_mhz or 1965.0)
+    split = split_peak_tflops(peaks)
     flop = flops_per_step_per_gpu(124475904)
     return dict(dtype="fp32", steps=steps, warmup=warmup, ms_per_step=round(ms, 2), value=round(B_PER_GPU * T / (ms * 1e-3), 1),
                 unit="tokens/s", e2e=dict(value=round(B_PER_GPU * T / (ms_e2e * 1e-3), 1), unit="tokens/s",
                                           h2d_bytes_per_step=2 * B_PER_GPU * T * 4, d2h_bytes_per_step=4),
-                model_tflops=round(flop / (ms * 1e-3) / 1e12, 1), frac_of_simt_peak=round(flop / (ms * 1e-3) / 1e12 / simt, 3),
-                simt_peak_tflops=round(simt, 1), sm_mhz=ck["sm_mhz"], losses_head=[round(float(v), 4) for v in losses])
+                model_tflops=round(flop / (ms * 1e-3) / 1e12, 1), frac_of_split_peak=round(flop / (ms * 1e-3) / 1e12 / split, 3),
+                split_peak_tflops=round(split, 1), sm_mhz=ck["sm_mhz"], losses_head=[round(float(v), 4) for v in losses])
 
 
 def dp_selfcheck(bmb, torch, dist_mod, comm, rank, world):
@@ -673,8 +678,8 @@ def run_bmb(args):
         return
     achieved = prof["gemm_flop"] / (prof["gemm_ms"] * 1e-3) / 1e12 if prof["gemm_ms"] > 0 else 0.0
     if math == bmb.MATH_FP32:
-        peak = simt_peak_tflops(torch, (step_clocks or {}).get("sm_mhz") or 1965.0)
-        bound, peak_note = "fp32-simt", "2*128*SMs*SM clock sampled during the timed steps"
+        peak = peaks["bf16_sustained"] / 6.0
+        bound, peak_note = "tensor", "sustained BF16 of MEASURED_PEAKS.json (%s) / 6: fp32 products in six bf16 ones" % peaks["source"]
     else:
         scale = 2.0 if math == bmb.MATH_TF32 else 1.0
         peak = peaks["bf16_sustained"] / scale
@@ -692,7 +697,7 @@ def run_bmb(args):
                                                   os.environ.get("BMB_TRAINER_OVERLAP", "0"), "one chunk after backward"))),
                   "l2": "per-step working set (~10 GB of activations) exceeds the 126 MB L2",
                   "arithmetic": "TF32 tensor-core GEMMs and attention, fp32 everywhere else" if math == bmb.MATH_TF32 else
-                                ("fp32 SIMT" if math == bmb.MATH_FP32 else "BF16 tensor-core GEMMs")},
+                                ("fp32, products split into bf16 pieces" if math == bmb.MATH_FP32 else "BF16 tensor-core GEMMs")},
         "e2e": {"value": round(e2e_value, 1), "unit": "tokens/s", "h2d_bytes_per_step": 2 * B_PER_GPU * T * 4,
                 "d2h_bytes_per_step": 4, "loss_read": "every step, one step late (asynchronous copy to pinned memory)"},
         "gpu_launches": int(prof["launches"]),
@@ -726,7 +731,7 @@ def run_bmb(args):
             line["gemm"] = gemm_sweep(bmb, torch, peaks, clocks)
             time.sleep(0.5)
             if math != bmb.MATH_FP32:
-                line["fp32_mode"] = fp32_mode_leg(bmb, torch, dist_mod, clocks)
+                line["fp32_mode"] = fp32_mode_leg(bmb, torch, dist_mod, peaks, clocks)
         if not args.no_cpu:
             line["cpu_baseline"] = cpu_baseline()
             line["cpu_matmul"] = cpu_matmul()
