@@ -727,6 +727,10 @@ int run_bwd(int cfg, float *dqkv, float *dsum, const float *dout, const float *q
             const float *lse, int B, int T, int NH, float scale, cudaStream_t st) {
     constexpr int ROWS = bwd_warps<HS>::value * 16;
     if (cfg == 0 && ceil_div(T, ROWS) > 32767) cfg = 1;
+    // Short rows of 128 columns and more heads than SMs: a block's 128 rows are padding for the most part (64 x 4 heads, T = 8 92 us
+    // against 60 by row groups, 32 96 / 81, but 64 164 / 294; 2 x 4 heads, T = 8 33 / 38).
+    const long long heads = (long long)B * NH;
+    if (cfg == 0 && HS == 128 && T <= 32 && heads > sm_count() && heads <= 65535) cfg = 1;
     if (cfg == 0) {
         BMB_TRY(launch_flash_dsum(dsum, dout, out, B, T, NH, HS, st));
         const auto kernel = T <= FINE_T ? flash_bwd_mma_k<HS, true> : flash_bwd_mma_k<HS, false>;
