@@ -176,7 +176,7 @@ flash_fwd_tc_k(const __grid_constant__ CUtensorMap mapQK, const __grid_constant_
 
     if (warp == 8) {
         // ------------------------------------------------------------ producer
-        if (lane == 0) {
+        if (elect_one()) {
             bool ok = true;
             int kv = 0;                                   // key / value blocks loaded so far (all items)
             int armed_q = -1, armed_k[K_STAGES], armed_v[V_STAGES];
@@ -228,7 +228,7 @@ flash_fwd_tc_k(const __grid_constant__ CUtensorMap mapQK, const __grid_constant_
         }
     } else if (warp == 9 || warp == 10) {
         // ------------------------------------- issuer of one query tile: S = Q K^T and O += P V
-        if (lane == 0) {
+        if (elect_one()) {
             const int t = warp - 9;
             // Q (K-major) x K (K-major), 64 keys at a time; P (tensor memory) x V (MN-major), accumulated into O
             const uint32_t idesc_s = make_idesc(2, 0, 0, KB, QT), idesc_pv = make_idesc(2, 0, 1, HS, QT);

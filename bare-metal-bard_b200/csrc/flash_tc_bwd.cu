@@ -167,7 +167,7 @@ flash_bwd_dq_body(const CUtensorMap &mapQKV_k, const CUtensorMap &mapQKV_n, cons
 
     if (warp == 8) {
         // ------------------------------------- loads of Q, dO and the K-major K / V blocks
-        if (lane == 0) {
+        if (elect_one()) {
             // in the order of first use: Q and the first K block (the scores), then dO and the first V block (dP)
             mbar_arrive_expect_tx(bar(Q_FULL), 32768);
             for (int half = 0; half < 2; ++half)
@@ -210,7 +210,7 @@ flash_bwd_dq_body(const CUtensorMap &mapQKV_k, const CUtensorMap &mapQKV_n, cons
         }
     } else if (warp == 10) {
         // ------------------------------------------- loads of the MN-major K granules
-        if (lane == 0) {
+        if (elect_one()) {
             bool ok = true;
             int armed_n[2] = {-1, -1};
             for (int j = 0; ok && j < nb; ++j)
@@ -231,7 +231,7 @@ flash_bwd_dq_body(const CUtensorMap &mapQKV_k, const CUtensorMap &mapQKV_n, cons
         // ------------------------------------------------- issuer of S = Q K^T
         // Two threads feed the tensor core, because one cannot issue N = 64 instructions as fast as the
         // pipe retires them; this one runs ahead with the scores of the next block.
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc_kk = make_idesc(2, 0, 0, KB, QT);     // [128 x 128] = A(K-major) x B(K-major)
             bool ok = mbar_wait(bar(Q_FULL), 0, giveup);
             for (int j = 0; ok && j < nb; ++j) {
@@ -252,7 +252,7 @@ flash_bwd_dq_body(const CUtensorMap &mapQKV_k, const CUtensorMap &mapQKV_n, cons
         }
     } else if (warp == 11) {
         // ----------------------------- issuer of dP = dO V^T and dQ += dS K
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc_kk = make_idesc(2, 0, 0, KB, QT);     // [128 x 128] = A(K-major) x B(K-major)
             const uint32_t idesc_kn = make_idesc(2, 0, 1, HS, QT);     // dQ: dS (tensor memory) x K (MN-major)
             auto issue_dp = [&](uint32_t bsm) {
@@ -508,7 +508,7 @@ flash_bwd_dkv_body(const CUtensorMap &mapQKV_k64, const CUtensorMap &mapQKV_n64,
 
     if (warp == 8) {
         // --------------------------- loads of K, V and the K-major Q / dO blocks
-        if (lane == 0) {
+        if (elect_one()) {
             // in the order of first use: K and the first Q block (the scores), then V and the first dO block (dP)
             mbar_arrive_expect_tx(bar(KV_FULL), 32768);
             for (int half = 0; half < 2; ++half)
@@ -549,7 +549,7 @@ flash_bwd_dkv_body(const CUtensorMap &mapQKV_k64, const CUtensorMap &mapQKV_n64,
         }
     } else if (warp == 10) {
         // ------------------------------ loads of the MN-major Q and dO granules
-        if (lane == 0) {
+        if (elect_one()) {
             bool ok = true;
             int armed_n[2] = {-1, -1};
             for (int i = 0; ok && i < nb; ++i)
@@ -574,7 +574,7 @@ flash_bwd_dkv_body(const CUtensorMap &mapQKV_k64, const CUtensorMap &mapQKV_n64,
         // pipe retires them.  Warp 9 owns the S^T / P^T buffers: it issues S^T = K Q^T and dV += P^T dO.
         // Warp 11 owns the dP^T / dS^T buffer: dP^T = V dO^T and dK += dS^T Q.  Each buffer is written and
         // read by the products of one thread only, and the tensor core runs a thread's products in order.
-        if (lane == 0) {
+        if (elect_one()) {
             const bool first = (warp == 9);
             const uint32_t idesc_st = make_idesc(2, 0, 0, QB, KT);     // [128 keys x 128 queries], both operands K-major
             const uint32_t idesc_acc = make_idesc(2, 0, 1, HS, KT);    // [128 keys x 64] = A (tensor memory) x B (MN-major)

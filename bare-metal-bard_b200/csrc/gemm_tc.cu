@@ -282,7 +282,7 @@ gemm_tc_k(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
 
     if (warp == 0) {
         // ------------------------------------------------------------ producer
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0;
             uint32_t ph = 0;
             bool ok = true;
@@ -333,7 +333,7 @@ gemm_tc_k(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
         }
     } else if (warp == 1) {
         // -------------------------------------------------------------- issuer
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = make_idesc(KIND == 0 ? 2u : 1u, a_mn ? 1u : 0u, b_mn ? 1u : 0u, BN, BM);
             // per 32-byte K step: K-major tiles move 32 bytes along the row, MN-major tiles move 8 K rows
             const uint32_t a_step = a_mn ? 1024u : 32u, b_step = b_mn ? 1024u : 32u;
@@ -637,7 +637,7 @@ gemm_tc_pair_k(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
 
     if (warp == 0) {
         // ------------------------------------------------------------ producer (each CTA for its own tiles)
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0;
             uint32_t ph = 0;
             bool ok = true;
@@ -678,7 +678,7 @@ gemm_tc_pair_k(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         }
     } else if (warp == 1) {
         // -------------------------------------------------------------- issuer (leader only)
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && elect_one()) {
             const uint32_t idesc = make_idesc(2u, a_mn ? 1u : 0u, b_mn ? 1u : 0u, BN, BMT);
             const uint32_t a_step = a_mn ? 1024u : 32u, b_step = b_mn ? 1024u : 32u;
             const uint32_t peer_empty0 = map_to_cta(empty0, 1), peer_tfull0 = map_to_cta(tfull0, 1);

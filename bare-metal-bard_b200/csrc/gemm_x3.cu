@@ -352,7 +352,7 @@ gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0;
             uint32_t ph = 0;
             bool ok = true;
@@ -384,7 +384,7 @@ gemm_x3_k(const uint8_t *__restrict__ imgA, int rowsA, const uint8_t *__restrict
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = make_idesc(1u, 0u, 0u, BN, XM);
             int s = 0, acc = 0;
             uint32_t ph = 0, acc_ph = 0;

@@ -13,6 +13,15 @@ constexpr long long WAIT_CYCLES = 4000000000LL;  // about two seconds at 2 GHz
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// One lane of a whole warp, always the same.  Code under this test is known to run in one thread; under `lane == 0` it is not, and
+// then every tcgen05.mma takes the detour that per-lane operands would need: 95 cycles an instruction whatever its shape,
+// against 24 (N = 32), 40 (64) and 72 (128) with A in tensor memory (16-bit operands, M = 128; measured).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
+}
+
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
