@@ -141,11 +141,38 @@ int gemm_any_bias(int math, int flags, int ta, int tb, int batch, int M, int N, 
 // (aux_gelu: a second output of the same shape, GELU of the result -- in the product's epilogue where the
 //  tensor-core kernel can, by a pass of its own otherwise)
 
+// bmb_flash_attention_*_ex; in_trainer: forward and backward both run, and, as with GEMM_SCRATCH_IN_CAPTURE, a captured stream's
+// launches may use SCR_SPLIT, because the caller has sized it and takes care of its moves.
+int flash_forward(int cfg, int flags, float *out, float *lse, const float *qkv, int B, int T, int C, int NH, bool in_trainer);
+int flash_backward(int cfg, int flags, float *dqkv, float *dsum, const float *dout, const float *qkv, const float *out, const float *lse,
+                   int B, int T, int C, int NH, bool in_trainer);
+
 }  // namespace bmb
 
 // ---- device helpers ---------------------------------------------------------
 #ifdef __CUDACC__
 namespace bmb {
+// A launch that may start when the blocks of the one before it in the stream have all said so (let_successor_start) or ended; it
+// waits for that one's end itself (wait_for_predecessor) before it reads what that wrote.  Its set-up and its launch then lie
+// beside the end of the one before.
+__device__ __forceinline__ void let_successor_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... P, typename... A>
+int launch_in_chain(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    BMB_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+    count_launch();
+    return BMB_OK;
+}
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

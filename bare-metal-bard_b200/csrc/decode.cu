@@ -21,25 +21,6 @@ namespace {
 // The launches of one position form a chain in which each kernel may start while the one before it still runs: it lets its
 // successor start at once, copies what does not depend on its predecessor (weights, earlier positions' values), and then
 // waits for the predecessor's end -- so every kernel has waited for all before it when it ends.
-__device__ __forceinline__ void let_successor_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-template <typename... P, typename... A>
-int launch_in_chain(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t st, A... args) {
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    BMB_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
-    count_launch();
-    return BMB_OK;
-}
-
 // a warp that follows the chains and four that copy weights ahead of it; rows 4 banks apart
 constexpr int GV_OUT = 32, GV_NT = 160, GV_CP = 128, GV_K = 128, GV_PITCH = GV_K + 4, GV_STAGES = 8;
 constexpr int GV_MAX_IN = 4096, GV_MAX_LN = 1024;
@@ -446,7 +427,7 @@ int decode_gemv(float *y, const float *x, const float *W, const float *bias, con
         if (!set[d]) BMB_CUDA(cudaFuncSetAttribute(decode_gemv_k, cudaFuncAttributeMaxDynamicSharedMemorySize, GV_SMEM));
         set[d] = true;
     }
-    return launch_in_chain(decode_gemv_k, ceil_div(out, GV_OUT), GV_NT, GV_SMEM, st, y, x, W, bias, ln_w, ln_b, add, in, out, gelu ? 1 : 0);
+    return launch_in_chain(decode_gemv_k, dim3(ceil_div(out, GV_OUT)), GV_NT, GV_SMEM, st, y, x, W, bias, ln_w, ln_b, add, in, out, gelu ? 1 : 0);
 }
 
 int decode_attention(float *y, const float *qkv, int pos, int C, int NH, cudaStream_t st) {
@@ -469,9 +450,9 @@ int decode_attention(float *y, const float *qkv, int pos, int C, int NH, cudaStr
         }
         set[d] = true;
     }
-    if (hs == 32) return launch_in_chain(decode_attention_k<32>, NH, DA_NT, smem, st, y, qkv, pos, C, scale, stage_v);
-    if (hs == 64) return launch_in_chain(decode_attention_k<64>, NH, DA_NT, smem, st, y, qkv, pos, C, scale, stage_v);
-    return launch_in_chain(decode_attention_k<128>, NH, DA_NT, smem, st, y, qkv, pos, C, scale, stage_v);
+    if (hs == 32) return launch_in_chain(decode_attention_k<32>, dim3(NH), DA_NT, smem, st, y, qkv, pos, C, scale, stage_v);
+    if (hs == 64) return launch_in_chain(decode_attention_k<64>, dim3(NH), DA_NT, smem, st, y, qkv, pos, C, scale, stage_v);
+    return launch_in_chain(decode_attention_k<128>, dim3(NH), DA_NT, smem, st, y, qkv, pos, C, scale, stage_v);
 }
 
 int window_attention(float *out, const float *qkv, int T, int C, int NH, cudaStream_t st) {

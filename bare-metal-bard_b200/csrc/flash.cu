@@ -16,6 +16,7 @@
 // infinite operands give NaN where the fp32 chain gives an infinity, or a probability of zero.
 // q, k and v are read straight out of the fused (B,T,3C) projection.
 #include "flash_mma.cuh"
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include <map>
@@ -28,6 +29,9 @@ int flash_forward_tc(float *out, float *lse, const float *qkv, int B, int T, int
                      cudaStream_t st);
 int flash_backward_tc(float *dqkv, float *dsum, const float *dout, const float *qkv, const float *out,
                       const float *lse, int B, int T, int C, int NH, bool rounded, cudaStream_t st, float *dbias_qkv = nullptr);
+int flash_forward_x2(float *out, float *lse, const float *qkv, int B, int T, int NH, int hs, float scale, bool in_trainer, cudaStream_t st);
+int flash_backward_x2(float *dqkv, float *dsum, const float *dout, const float *qkv, const float *out, const float *lse, int B, int T, int NH, int hs,
+                      float scale, bool in_trainer, cudaStream_t st);
 namespace {
 
 #define LD4(p) (*reinterpret_cast<const float4 *>(p))
@@ -170,6 +174,13 @@ __device__ __noinline__ void fwd_rows_again(float *smem, float *out, float *lse,
     for (int r = 0; r < nrows; r += R) fwd_rows<HS, 16, NT>(smem, out, lse, qkv, T, NH, scale, bh, i0 + r, min(R, nrows - r));
 }
 
+// Whether head blockIdx.x has one of its nflags bytes set (flash_x2.cu leaves such heads to these kernels).
+__device__ __forceinline__ bool head_flagged(const uint8_t *flags, int nflags) {
+    bool f = false;
+    for (int i = threadIdx.x; i < nflags; i += blockDim.x) f = f || flags[(long long)blockIdx.x * nflags + i];
+    return __syncthreads_or(f);
+}
+
 // How the products are split (flash_mma.cuh): scores and output, and sums of gradients.
 __host__ __device__ constexpr fm::Form scores_form(bool fine) { return fine ? fm::FINE : fm::COARSE_CUT; }
 __host__ __device__ constexpr fm::Form gradient_form(bool fine) { return fine ? fm::FINE : fm::COARSE; }
@@ -184,14 +195,12 @@ __host__ __device__ constexpr fm::Form gradient_form(bool fine) { return fine ? 
 // B4 T2048 8 x 128 3608 -> 670, B2 T777 12 x 32 191 -> 42, B1 T64 2 x 32 18.9 -> 7.1.  2-norm errors against 64 bits there:
 // 2.7e-7 -> 1.7e-7, 3.5e-7 -> 1.8e-7, 2.5e-7 -> 1.6e-7, 1.2e-7 -> 0.9e-7.
 template <int HS, bool FINE>
-__global__ void __launch_bounds__(128, HS == 32 ? 3 : 2)
-flash_fwd_mma_k(float *__restrict__ out, float *__restrict__ lse, const float *__restrict__ qkv, int T, int NH, float scale) {
-    extern __shared__ __align__(16) float smem[];
+__device__ __forceinline__ void fwd_mma(float *__restrict__ smem, float *__restrict__ out, float *__restrict__ lse, const float *__restrict__ qkv,
+                                        int T, int NH, float scale, int i0) {
     float *Qs = smem, *Ks = Qs + 64 * HS, *Vs = Ks + 2 * 32 * HS;      // Ks, Vs: two buffers each
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int bh = blockIdx.x, b = bh / NH, h = bh % NH;
     const int C = NH * HS;
-    const int i0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * 64;        // longest blocks first
     const long long ld = 3LL * C;
     const float *base = qkv + (long long)b * T * ld + h * HS;
 
@@ -270,6 +279,19 @@ flash_fwd_mma_k(float *__restrict__ out, float *__restrict__ lse, const float *_
     }
     bad = fm::store_rows<HS>(out + ((long long)b * T + row0) * C + h * HS, C, g, T - row0, o, inv[0], inv[1]) || bad;
     if (__syncthreads_or(bad)) fwd_rows_again<HS, 128>(smem, out, lse, qkv, T, NH, scale, bh, i0, 64);
+}
+// `blocks` blocks of rows a head, the longest first; a grid that is lower walks them.
+template <int HS, bool FINE>
+__global__ void __launch_bounds__(128, HS == 32 ? 3 : 2)
+flash_fwd_mma_k(float *__restrict__ out, float *__restrict__ lse, const float *__restrict__ qkv, int T, int NH, float scale,
+                const uint8_t *__restrict__ flags, int nflags, int blocks) {
+    extern __shared__ __align__(16) float smem[];
+    if (flags) wait_for_predecessor();
+    if (flags && !head_flagged(flags, nflags)) return;
+    for (int y = blockIdx.y; y < blocks; y += gridDim.y) {
+        if (y != (int)blockIdx.y) __syncthreads();             // the rows before have been read
+        fwd_mma<HS, FINE>(smem, out, lse, qkv, T, NH, scale, (blocks - 1 - y) * 64);
+    }
 }
 
 // ----------------------------------------------------------------- backward
@@ -664,12 +686,17 @@ __device__ __forceinline__ void bwd_kv_mma(float *__restrict__ smem, float *__re
 template <int HS, bool FINE>
 __global__ void __launch_bounds__(bwd_warps<HS>::value * 32, HS == 128 ? 1 : HS == 64 ? 2 : 3)
 flash_bwd_mma_k(float *__restrict__ dqkv, const float *__restrict__ qkv, const float *__restrict__ dout,
-                const float *__restrict__ lse, const float *__restrict__ dsum, int T, int NH, float scale) {
+                const float *__restrict__ lse, const float *__restrict__ dsum, int T, int NH, float scale,
+                const uint8_t *__restrict__ flags, int nflags, int blocks) {
     extern __shared__ __align__(16) float smem[];
+    if (flags) wait_for_predecessor();
+    if (flags && !head_flagged(flags, nflags)) return;
     constexpr int ROWS = bwd_warps<HS>::value * 16;
-    const int rank = blockIdx.y >> 1, blocks = gridDim.y >> 1;
-    if (blockIdx.y & 1) bwd_q_mma<HS, FINE>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, blockIdx.x, (blocks - 1 - rank) * ROWS);
-    else bwd_kv_mma<HS, FINE>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, blockIdx.x, rank * ROWS);
+    for (int y = blockIdx.y; y < 2 * blocks; y += gridDim.y) {
+        if (y != (int)blockIdx.y) __syncthreads();             // the rows before have been read
+        if (y & 1) bwd_q_mma<HS, FINE>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, blockIdx.x, (blocks - 1 - (y >> 1)) * ROWS);
+        else bwd_kv_mma<HS, FINE>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, blockIdx.x, (y >> 1) * ROWS);
+    }
 }
 
 struct FwdCfg { int kc; const char *name; };
@@ -688,6 +715,18 @@ constexpr int NFWD = 3, NBWD = 3, FWD_TC = 2, BWD_TC = 2;
 // those.  128 x 128 positions, 4 heads of 64: forward 22 -> 37 us, backward 76 -> 123 (the FMA pipe: 54 and 184).
 constexpr int FINE_T = 128;
 
+// Whether flash_x2.cu takes a call: where its three launches and its tiles of 128 rows pay.  The backward goes the way that the
+// forward of its sizes went, although it gains from T = 192 on wherever that is: its scores then err as those that lse was made of
+// (errors of dqkv 4 to 9 % smaller).  A trainer runs both, so there the two together count.  us, these kernels / flash_x2.cu, heads x T,
+// forward | backward.  32 columns: 48 x 400 25 / 25 | 60 / 40, 16 x 400 17 / 21 | 50 / 24, 96 x 256 19 / 22 | 50 / 37, 2 x 512 21 / 21 | 54 / 23;
+// 64: 48 x 256 19 / 19 | 56 / 29, 96 x 256 25 / 27 | 88 / 51, 96 x 400 58 / 43 | 199 / 99, 48 x 200 18 / 19 | 50 / 29;
+// 128: 48 x 200 35 / 31 | 101 / 50, 96 x 256 46 / 57 | 208 / 115, 96 x 400 115 / 93 | 462 / 207, 48 x 136 25 / 27 | 74 / 39.
+bool wants_x2(int hs, long long heads, int T, bool trains) {
+    if (trains && T >= 192) return true;
+    if (hs == 32) return T >= 512 || (T >= 384 && heads >= 40);
+    return T >= 384 || (T >= (hs == 64 ? 240 : 192) && heads <= 64);
+}
+
 bool shape_ok(const float *a, const float *b, int C, int NH) {
     return NH > 0 && C % NH == 0 && (((uintptr_t)a | (uintptr_t)b) & 15) == 0;
 }
@@ -703,15 +742,48 @@ int allow_smem(const void *kernel, int bytes) {
     return BMB_OK;
 }
 
+// With flags hardly a head has work: about two blocks an SM look at them.
+int grid_height(int blocks, int heads, const uint8_t *flags) {
+    return flags ? std::min(blocks, std::max(1, ceil_div(2 * sm_count(), heads))) : blocks;
+}
+template <int HS>
+int launch_fwd_mma(float *out, float *lse, const float *qkv, int B, int T, int NH, float scale, const uint8_t *flags, int nflags, cudaStream_t st) {
+    constexpr int SMEM = (64 + 4 * 32) * HS * 4;
+    const auto kernel = T <= FINE_T ? flash_fwd_mma_k<HS, true> : flash_fwd_mma_k<HS, false>;
+    BMB_TRY(allow_smem((const void *)kernel, SMEM));
+    const int blocks = ceil_div(T, 64);
+    const dim3 grid(B * NH, grid_height(blocks, B * NH, flags));
+    if (flags) return launch_in_chain(kernel, grid, 128, SMEM, st, out, lse, qkv, T, NH, scale, flags, nflags, blocks);
+    kernel<<<grid, 128, SMEM, st>>>(out, lse, qkv, T, NH, scale, flags, nflags, blocks);
+    count_launch();
+    BMB_LAUNCH_CHECK();
+    return BMB_OK;
+}
+template <int HS>
+int launch_bwd_mma(float *dqkv, const float *dsum, const float *dout, const float *qkv, const float *lse, int B, int T, int NH, float scale,
+                   const uint8_t *flags, int nflags, cudaStream_t st) {
+    constexpr int ROWS = bwd_warps<HS>::value * 16;
+    const auto kernel = T <= FINE_T ? flash_bwd_mma_k<HS, true> : flash_bwd_mma_k<HS, false>;
+    BMB_TRY(allow_smem((const void *)kernel, bwd_smem<HS>()));
+    const int blocks = ceil_div(T, ROWS), threads = bwd_warps<HS>::value * 32;
+    const dim3 grid(B * NH, grid_height(2 * blocks, B * NH, flags));
+    if (flags) return launch_in_chain(kernel, grid, threads, bwd_smem<HS>(), st, dqkv, qkv, dout, lse, dsum, T, NH, scale, flags, nflags, blocks);
+    kernel<<<grid, threads, bwd_smem<HS>(), st>>>(dqkv, qkv, dout, lse, dsum, T, NH, scale, flags, nflags, blocks);
+    count_launch();
+    BMB_LAUNCH_CHECK();
+    return BMB_OK;
+}
+
 template <int HS>
 int run_fwd(int cfg, float *out, float *lse, const float *qkv, int B, int T, int NH, float scale,
-            cudaStream_t st) {
+            bool in_trainer, cudaStream_t st) {
     if (cfg == 0 && ceil_div(T, 64) > 65535) cfg = 1;              // (blocks of rows on grid y)
     if (cfg == 0) {
-        constexpr int SMEM = (64 + 4 * 32) * HS * 4;
-        const auto kernel = T <= FINE_T ? flash_fwd_mma_k<HS, true> : flash_fwd_mma_k<HS, false>;
-        BMB_TRY(allow_smem((const void *)kernel, SMEM));
-        kernel<<<dim3(B * NH, ceil_div(T, 64)), 128, SMEM, st>>>(out, lse, qkv, T, NH, scale);
+        if (wants_x2(HS, (long long)B * NH, T, in_trainer)) {
+            const int rc = flash_forward_x2(out, lse, qkv, B, T, NH, HS, scale, in_trainer, st);
+            if (rc != BMB_E_UNSUPPORTED) return rc;
+        }
+        return launch_fwd_mma<HS>(out, lse, qkv, B, T, NH, scale, nullptr, 0, st);
     } else {
         constexpr int R = FT / (HS / 32);
         dim3 grid(ceil_div(T, R), B * NH);
@@ -724,7 +796,7 @@ int run_fwd(int cfg, float *out, float *lse, const float *qkv, int B, int T, int
 
 template <int HS>
 int run_bwd(int cfg, float *dqkv, float *dsum, const float *dout, const float *qkv, const float *out,
-            const float *lse, int B, int T, int NH, float scale, cudaStream_t st) {
+            const float *lse, int B, int T, int NH, float scale, bool in_trainer, cudaStream_t st) {
     constexpr int ROWS = bwd_warps<HS>::value * 16;
     if (cfg == 0 && ceil_div(T, ROWS) > 32767) cfg = 1;
     // Short rows of 128 columns and more heads than SMs: a block's 128 rows are padding for the most part (64 x 4 heads, T = 8 92 us
@@ -732,13 +804,12 @@ int run_bwd(int cfg, float *dqkv, float *dsum, const float *dout, const float *q
     const long long heads = (long long)B * NH;
     if (cfg == 0 && HS == 128 && T <= 32 && heads > sm_count() && heads <= 65535) cfg = 1;
     if (cfg == 0) {
+        if (wants_x2(HS, (long long)B * NH, T, in_trainer)) {
+            const int rc = flash_backward_x2(dqkv, dsum, dout, qkv, out, lse, B, T, NH, HS, scale, in_trainer, st);
+            if (rc != BMB_E_UNSUPPORTED) return rc;
+        }
         BMB_TRY(launch_flash_dsum(dsum, dout, out, B, T, NH, HS, st));
-        const auto kernel = T <= FINE_T ? flash_bwd_mma_k<HS, true> : flash_bwd_mma_k<HS, false>;
-        BMB_TRY(allow_smem((const void *)kernel, bwd_smem<HS>()));
-        kernel<<<dim3(B * NH, 2 * ceil_div(T, ROWS)), bwd_warps<HS>::value * 32, bwd_smem<HS>(), st>>>(dqkv, qkv, dout, lse, dsum, T, NH, scale);
-        count_launch();
-        BMB_LAUNCH_CHECK();
-        return BMB_OK;
+        return launch_bwd_mma<HS>(dqkv, dsum, dout, qkv, lse, B, T, NH, scale, nullptr, 0, st);
     }
     constexpr int R = FT / (HS / 32);
     const long long rows = (long long)B * NH * T;
@@ -752,6 +823,16 @@ int run_bwd(int cfg, float *dqkv, float *dsum, const float *dout, const float *q
 }
 
 }  // namespace
+
+int flash_fwd_mma(int hs, float *out, float *lse, const float *qkv, int B, int T, int NH, float scale, const uint8_t *flags, int nflags, cudaStream_t st) {
+    const auto run = hs == 32 ? launch_fwd_mma<32> : hs == 64 ? launch_fwd_mma<64> : launch_fwd_mma<128>;
+    return run(out, lse, qkv, B, T, NH, scale, flags, nflags, st);
+}
+int flash_bwd_mma(int hs, float *dqkv, const float *dsum, const float *dout, const float *qkv, const float *lse, int B, int T, int NH, float scale,
+                  const uint8_t *flags, int nflags, cudaStream_t st) {
+    const auto run = hs == 32 ? launch_bwd_mma<32> : hs == 64 ? launch_bwd_mma<64> : launch_bwd_mma<128>;
+    return run(dqkv, dsum, dout, qkv, lse, B, T, NH, scale, flags, nflags, st);
+}
 
 int launch_flash_dsum(float *dsum, const float *dout, const float *out, int B, int T, int NH, int HS, cudaStream_t st) {
     const long long rows = (long long)B * NH * T;
@@ -789,6 +870,12 @@ int bmb_flash_attention_forward_cfg(int cfg, float *out, float *lse, const float
 
 int bmb_flash_attention_forward_ex(int cfg, int flags, float *out, float *lse, const float *qkv, int B, int T,
                                    int C, int NH) {
+    return flash_forward(cfg, flags, out, lse, qkv, B, T, C, NH, false);
+}
+
+}  // extern "C"
+namespace bmb {
+int flash_forward(int cfg, int flags, float *out, float *lse, const float *qkv, int B, int T, int C, int NH, bool in_trainer) {
     if (cfg < 0 || cfg >= NFWD) return fail(BMB_E_UNSUPPORTED, "flash: no forward config %d", cfg);
     if (B <= 0 || T <= 0) return BMB_OK;
     if (!shape_ok(out, qkv, C, NH)) return fail(BMB_E_ARG, "flash: bad shape or alignment (C=%d NH=%d)", C, NH);
@@ -801,12 +888,14 @@ int bmb_flash_attention_forward_ex(int cfg, int flags, float *out, float *lse, c
         return flash_forward_tc(out, lse, qkv, B, T, C, NH, (flags & BMB_FLASH_OPERANDS_ROUNDED) != 0, st);
     }
     switch (hs) {
-    case 32:  return run_fwd<32>(cfg, out, lse, qkv, B, T, NH, scale, st);
-    case 64:  return run_fwd<64>(cfg, out, lse, qkv, B, T, NH, scale, st);
-    case 128: return run_fwd<128>(cfg, out, lse, qkv, B, T, NH, scale, st);
+    case 32:  return run_fwd<32>(cfg, out, lse, qkv, B, T, NH, scale, in_trainer, st);
+    case 64:  return run_fwd<64>(cfg, out, lse, qkv, B, T, NH, scale, in_trainer, st);
+    case 128: return run_fwd<128>(cfg, out, lse, qkv, B, T, NH, scale, in_trainer, st);
     default:  return fail(BMB_E_UNSUPPORTED, "flash: no tile config for head size %d", hs);
     }
 }
+}  // namespace bmb
+extern "C" {
 
 int bmb_flash_attention_forward(float *out, float *lse, const float *qkv, int B, int T, int C,
                                 int NH) {
@@ -829,6 +918,13 @@ int bmb_flash_attention_backward_cfg(int cfg, float *dqkv, float *dsum, const fl
 int bmb_flash_attention_backward_ex(int cfg, int flags, float *dqkv, float *dsum, const float *dout,
                                     const float *qkv, const float *out, const float *lse, int B,
                                     int T, int C, int NH) {
+    return flash_backward(cfg, flags, dqkv, dsum, dout, qkv, out, lse, B, T, C, NH, false);
+}
+
+}  // extern "C"
+namespace bmb {
+int flash_backward(int cfg, int flags, float *dqkv, float *dsum, const float *dout, const float *qkv, const float *out, const float *lse,
+                   int B, int T, int C, int NH, bool in_trainer) {
     if (cfg < 0 || cfg >= NBWD) return fail(BMB_E_UNSUPPORTED, "flash: no backward config %d", cfg);
     if (B <= 0 || T <= 0) return BMB_OK;
     if (!shape_ok(dqkv, qkv, C, NH) || !shape_ok(dout, out, C, NH))
@@ -842,12 +938,14 @@ int bmb_flash_attention_backward_ex(int cfg, int flags, float *dqkv, float *dsum
         return flash_backward_tc(dqkv, dsum, dout, qkv, out, lse, B, T, C, NH, (flags & BMB_FLASH_OPERANDS_ROUNDED) != 0, st);
     }
     switch (hs) {
-    case 32:  return run_bwd<32>(cfg, dqkv, dsum, dout, qkv, out, lse, B, T, NH, scale, st);
-    case 64:  return run_bwd<64>(cfg, dqkv, dsum, dout, qkv, out, lse, B, T, NH, scale, st);
-    case 128: return run_bwd<128>(cfg, dqkv, dsum, dout, qkv, out, lse, B, T, NH, scale, st);
+    case 32:  return run_bwd<32>(cfg, dqkv, dsum, dout, qkv, out, lse, B, T, NH, scale, in_trainer, st);
+    case 64:  return run_bwd<64>(cfg, dqkv, dsum, dout, qkv, out, lse, B, T, NH, scale, in_trainer, st);
+    case 128: return run_bwd<128>(cfg, dqkv, dsum, dout, qkv, out, lse, B, T, NH, scale, in_trainer, st);
     default:  return fail(BMB_E_UNSUPPORTED, "flash: no backward tile config for head size %d", hs);
     }
 }
+}  // namespace bmb
+extern "C" {
 
 int bmb_flash_attention_backward(float *dqkv, float *dsum, const float *dout, const float *qkv,
                                  const float *out, const float *lse, int B, int T, int C, int NH) {

@@ -281,7 +281,7 @@ int fwd_layer(bmb_trainer *t, const Dims &d, int l) {
     else if (c.use_flash && (wflag & GEMM_CHAIN))
         BMB_TRY(window_attention(atty, qkv, T, C, NH, t->st));
     else if (c.use_flash)
-        BMB_TRY(bmb_flash_attention_forward_cfg(attn_cfg(c), atty, t->lse + l * d.lse_sz, qkv, B, T, C, NH));
+        BMB_TRY(flash_forward(attn_cfg(c), 0, atty, t->lse + l * d.lse_sz, qkv, B, T, C, NH, true));
     else
         BMB_TRY(bmb_attention_forward(atty, t->qkvr + l * d.qkvr_sz, t->att + l * d.att_sz, qkv, B, T, C, NH));
     if (fz) {
@@ -410,7 +410,7 @@ int bwd_layer(bmb_trainer *t, const Dims &d, int l) {
         BMB_TRY(flash_backward_tc(t->dqkv, t->dsum, t->datty, qkv, atty, t->lse + l * d.lse_sz, B, T, C, NH, true, t->st,
                                   bias_in_attention ? G + t->poff[P_QKVB] + 3 * lC : nullptr));
     else if (c.use_flash)
-        BMB_TRY(bmb_flash_attention_backward_cfg(attn_cfg(c), t->dqkv, t->dsum, t->datty, qkv, atty, t->lse + l * d.lse_sz, B, T, C, NH));
+        BMB_TRY(flash_backward(attn_cfg(c), 0, t->dqkv, t->dsum, t->datty, qkv, atty, t->lse + l * d.lse_sz, B, T, C, NH, true));
     else
         BMB_TRY(bmb_attention_backward(t->dqkv, t->dqkvr, t->datt, t->datt, t->datty, t->qkvr + l * d.qkvr_sz,
                                        t->att + l * d.att_sz, B, T, C, NH));
@@ -700,7 +700,7 @@ int trainer_build(bmb_trainer *t, const bmb_train_config &c, unsigned seed) {
         BMB_CUDA(cudaEventCreateWithFlags(&t->ev_seg[c], cudaEventDisableTiming));
         BMB_CUDA(cudaEventCreateWithFlags(&t->ev_upd[c], cudaEventDisableTiming));
     }
-    if (c.math == BMB_MATH_FP32) {
+    if (c.math == BMB_MATH_FP32 || (c.use_flash && attn_cfg(c) == 0)) {
         std::lock_guard<std::mutex> turn(split_mutex());
         split_scratch_keep(1);
         t->keeps_split = true;

@@ -1,0 +1,99 @@
+"""fp32 attention in fp16 pieces (csrc/flash_x2.cu) at the edges of its tiles, and the heads that it leaves to the kernels behind it,
+against the row-group kernels (configuration 1) and 64 bits."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def inputs(cuda, B, T, NH, hs, seed):
+    C = NH * hs
+    g = cuda.Generator(device="cuda").manual_seed(seed)
+    return cuda.randn(B, T, 3 * C, generator=g, device="cuda"), cuda.randn(B, T, C, generator=g, device="cuda")
+
+
+def attention(bmb, cuda, cfg, qkv, dout, NH, lse_add=0.0):
+    B, T, C = dout.shape
+    out, lse, dsum, dqkv = (cuda.full(s, float("nan"), device="cuda") for s in ((B, T, C), (B, NH, T), (B, NH, T), (B, T, 3 * C)))
+    bmb.call("bmb_flash_attention_forward_cfg", cfg, out, lse, qkv, B, T, C, NH)
+    bmb.call("bmb_flash_attention_backward_cfg", cfg, dqkv, dsum, dout, qkv, out, lse + lse_add, B, T, C, NH)
+    cuda.cuda.synchronize()
+    return out, lse, dsum, dqkv
+
+
+def relative(x, y):
+    return float((x.double() - y.double()).norm() / y.double().norm())
+
+
+# One head of 64-bit errors up to 3e-7 (tests of split attention), so two fp32 implementations are up to 8e-7 apart.
+BOUND = 1e-6
+
+
+@pytest.mark.parametrize("hs", [32, 64, 128])
+@pytest.mark.parametrize("B,T,NH", [(1, 512, 1), (1, 513, 2), (2, 575, 1), (1, 640, 3), (1, 641, 1), (1, 767, 1), (1, 833, 2), (3, 1025, 1),
+                                    (20, 512, 8)])                 # the last: more pairs of tiles than SMs
+def test_edges_of_tiles(bmb, cuda, hs, B, T, NH):
+    qkv, dout = inputs(cuda, B, T, NH, hs, T + hs)
+    for x, y in zip(attention(bmb, cuda, 0, qkv, dout, NH), attention(bmb, cuda, 1, qkv, dout, NH)):
+        assert bool(cuda.isfinite(x).all()) and relative(x, y) <= BOUND
+    again = attention(bmb, cuda, 0, qkv, dout, NH)
+    assert all(cuda.equal(x, y) for x, y in zip(again, attention(bmb, cuda, 0, qkv, dout, NH)))
+
+
+@pytest.mark.parametrize("hs", [32, 64, 128])
+@pytest.mark.parametrize("what", ["tiny", "huge", "a row", "inf", "nan", "zero"])
+@pytest.mark.parametrize("which", [0, 1, 2, 3])
+def test_heads_that_the_pieces_cannot_serve(bmb, cuda, hs, what, which):
+    """One of four heads has a block of 64 positions out of range; it and the others come out as they do from the row groups."""
+    B, T, NH = 2, 520, 2
+    C = NH * hs
+    qkv, dout = inputs(cuda, B, T, NH, hs, 7 * hs + which)
+    block = (dout if which == 3 else qkv[..., which * C:(which + 1) * C])[1, 128:192, hs:2 * hs]
+    if what == "tiny":
+        block *= 2.0 ** -60
+    elif what == "huge":
+        block *= 2.0 ** 40 if which > 1 else 2.0 ** 3
+    elif what == "a row":
+        block[5] *= 2.0 ** -30
+    elif what == "zero":
+        block.zero_()
+    else:
+        block[5, 3] = float(what)
+    if what == "huge" and which < 2:
+        block *= 2.0 ** 28
+        (qkv[..., (1 - which) * C:(2 - which) * C])[1, :, hs:2 * hs] *= 2.0 ** -31
+    got, want = attention(bmb, cuda, 0, qkv, dout, NH), attention(bmb, cuda, 1, qkv, dout, NH)
+    heads = lambda x: x.reshape(B, T, -1, hs).transpose(1, 2).reshape(B, -1, NH, T, hs) if x.shape[1] == T else x    # noqa: E731
+    for x, y in zip(got, want):
+        assert cuda.equal(cuda.isfinite(x), cuda.isfinite(y)) and cuda.equal(cuda.isnan(x), cuda.isnan(y))
+        for a, b in zip(heads(x).unbind(0), heads(y).unbind(0)):
+            fin = cuda.isfinite(b)
+            scale = cuda.where(fin, b, cuda.zeros_like(b)).abs().max()
+            if scale > 0:
+                assert float((cuda.where(fin, a - b, cuda.zeros_like(a)) / scale).norm() / cuda.where(fin, b / scale, cuda.zeros_like(b)).norm()) <= BOUND
+
+
+@pytest.mark.parametrize("hs", [32, 64, 128])
+def test_lse_of_other_scores(bmb, cuda, hs):
+    """Probabilities beyond 1 (an lse that is not these scores') are beyond what the pieces are scaled for."""
+    qkv, dout = inputs(cuda, 1, 512, 2, hs, hs)
+    got, want = attention(bmb, cuda, 0, qkv, dout, 2, -6.0), attention(bmb, cuda, 1, qkv, dout, 2, -6.0)
+    assert relative(got[3], want[3]) <= BOUND
+
+
+def test_captured_calls(bmb, cuda):
+    """A caller's capture holds no address of the library's scratch; the captured call gives what an eager one gives."""
+    B, T, NH, hs = 1, 512, 2, 64
+    C = NH * hs
+    qkv, dout = inputs(cuda, B, T, NH, hs, 3)
+    eager = attention(bmb, cuda, 0, qkv, dout, NH)
+    out, lse = cuda.empty(B, T, C, device="cuda"), cuda.empty(B, NH, T, device="cuda")
+    stream = cuda.cuda.Stream()
+    graph = cuda.cuda.CUDAGraph()
+    with cuda.cuda.stream(stream):
+        with cuda.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+            bmb.lib().bmb_set_stream(cuda.cuda.current_stream().cuda_stream)
+            bmb.call("bmb_flash_attention_forward_cfg", 0, out, lse, qkv, B, T, C, NH)
+    bmb.lib().bmb_set_stream(None)
+    graph.replay()
+    cuda.cuda.synchronize()
+    assert relative(out, eager[0]) <= BOUND and relative(lse, eager[1]) <= BOUND
