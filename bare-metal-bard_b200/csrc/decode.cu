@@ -282,122 +282,116 @@ __global__ void __launch_bounds__(DA_NT) decode_attention_k(float *__restrict__ 
     if (tid < HS) y[blockIdx.x * HS + tid] = o * ((total > 0.0f) ? 1.0f / total : 0.0f);
 }
 
-// All rows of one sequence's window. HS/16 lanes have 16 columns each of two neighbouring rows (what they read of a key or
-// value serves both); keys and values staged in shared memory, a warp passes over keys that lie after its last row. A block
-// of two warps: the window of one sequence is few rows, and the last ones see all keys.
-constexpr int WA_NT = 64, RQ = 2;
+// All rows of one sequence's window: as decode_attention_k, WR neighbouring rows of a head a block, so that what is read of a key
+// or value serves all of them.  Scores and exponentials are computed side by side and only a row's sum and its output follow the
+// keys one after the other, a thread a column: at 256 positions of 6 heads x 64 10 us, against 38 for a walk over the keys in which
+// every 8 of them waited for the 8 before.
+// smem: the rows' queries, their scores in whole groups of 8, a factor and a sum a group, and, where they fit, the values.
+constexpr int WR = 8, WA_NT = 256, WA_MAX_V = 96 * 1024;
 template <int HS>
-__global__ void __launch_bounds__(WA_NT) window_attention_k(float *__restrict__ out, const float *__restrict__ qkv, int T, int C, float scale) {
-    constexpr int GL = HS / 16, ROWS = WA_NT / GL * RQ, TILE = HS >= 128 ? 32 : 64;
-    __shared__ __align__(16) float Ks[TILE * HS];
-    __shared__ __align__(16) float Vs[TILE * HS];
-    const int tid = threadIdx.x, sub = tid % GL;
-    const int i0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * ROWS, row0 = i0 + tid / GL * RQ;       // longest blocks first
+__global__ void __launch_bounds__(WA_NT) window_attention_k(float *__restrict__ out, const float *__restrict__ qkv, int T, int C, float scale, int stage_v) {
+    extern __shared__ __align__(16) float smem[];
+    constexpr int GL = HS / 16, KEYS = WA_NT / GL, SETS = WA_NT / HS, RT = WR / SETS;      // RT rows a thread in the output
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int i0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * WR, n = min(T, i0 + WR);      // longest blocks first
+    const int groups = (n + KC - 1) / KC, keys = groups * KC;
+    float *qs = smem, *p = qs + WR * HS, *factor = p + WR * keys, *gsum = factor + WR * groups, *vs = gsum + WR * groups;
     const long long ld = 3LL * C;
     const float *base = qkv + blockIdx.y * HS;
-    unsigned long long q2[RQ][8], o2[RQ][8];
-    float m[RQ], l[RQ];
-#pragma unroll
-    for (int r = 0; r < RQ; ++r) {
-        load_query(q2[r], base + (long long)min(row0 + r, T - 1) * ld + sub * 16, scale);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) o2[r][i] = 0ull;
-        m[r] = -INFINITY; l[r] = 0.0f;
-    }
-    const int warp_last = min(T - 1, i0 + (tid | 31) / GL * RQ + RQ - 1), jmax = min(T, i0 + ROWS);
-    for (int j0 = 0; j0 < jmax; j0 += TILE) {
-        __syncthreads();
-        for (int lin = tid; lin < TILE * HS / 4; lin += WA_NT) {
-            const int r = lin / (HS / 4), c = lin % (HS / 4) * 4;
-            const bool ok = j0 + r < T;
-            const float *src = base + (long long)(ok ? j0 + r : 0) * ld + c;
-            const uint32_t k = (uint32_t)__cvta_generic_to_shared(Ks + r * HS + c), v = (uint32_t)__cvta_generic_to_shared(Vs + r * HS + c);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(k), "l"(src + C), "r"(ok ? 16 : 0) : "memory");
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(v), "l"(src + 2 * C), "r"(ok ? 16 : 0) : "memory");
+    if (stage_v) {
+        for (int i = tid; i < keys * HS / 4; i += WA_NT) {
+            const int j = i / (HS / 4), c = i % (HS / 4) * 4;
+            const uint32_t d = (uint32_t)__cvta_generic_to_shared(vs + j * HS + c);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(base + (long long)min(j, T - 1) * ld + 2 * C + c),
+                         "r"(j < T ? 16 : 0) : "memory");
         }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncthreads();
-        for (int c0 = 0; c0 < TILE && j0 + c0 <= warp_last; c0 += KC) {
-            float s[RQ][KC];
+    }
+    for (int i = tid; i < WR * HS; i += WA_NT) qs[i] = base[(long long)min(i0 + i / HS, T - 1) * ld + i % HS] * scale;
+    __syncthreads();
+    const int sub = tid % GL;
+    for (int j0 = 0; j0 < keys; j0 += KEYS) {                    // whole warps stay in the loop for the shuffles
+        const int j = j0 + tid / GL;
+        const float *k = base + (long long)min(j, T - 1) * ld + C + sub * 16;
+        unsigned long long k2[8];
 #pragma unroll
-            for (int c = 0; c < KC; ++c) {
-                unsigned long long acc[RQ];
+        for (int i = 0; i < 8; i += 2) {
+            const float4 v = *reinterpret_cast<const float4 *>(k + 2 * i);
+            k2[i] = pack(v.x, v.y);
+            k2[i + 1] = pack(v.z, v.w);
+        }
 #pragma unroll
-                for (int r = 0; r < RQ; ++r) acc[r] = 0ull;
+        for (int r = 0; r < WR; ++r) {
+            unsigned long long acc = 0ull;
 #pragma unroll
-                for (int i = 0; i < 8; i += 2) {
-                    const float4 k = *reinterpret_cast<const float4 *>(Ks + (c0 + c) * HS + sub * 16 + 2 * i);
-                    const unsigned long long k0 = pack(k.x, k.y), k1 = pack(k.z, k.w);
-#pragma unroll
-                    for (int r = 0; r < RQ; ++r) { fma2(acc[r], q2[r][i], k0); fma2(acc[r], q2[r][i + 1], k1); }
-                }
-#pragma unroll
-                for (int r = 0; r < RQ; ++r) {
-                    float lo, hi;
-                    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[r]));
-                    s[r][c] = lo + hi;
-                }
+            for (int i = 0; i < 8; i += 2) {
+                const float4 q = *reinterpret_cast<const float4 *>(qs + r * HS + sub * 16 + 2 * i);
+                fma2(acc, pack(q.x, q.y), k2[i]);
+                fma2(acc, pack(q.z, q.w), k2[i + 1]);
             }
+            float lo, hi;
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc));
+            float s = lo + hi;
 #pragma unroll
-            for (int r = 0; r < RQ; ++r) {
-                float cmax = -INFINITY;
+            for (int o = 1; o < GL; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (sub == 0 && j < keys) p[r * keys + j] = (j > i0 + r || j >= T) ? -INFINITY : s;
+        }
+    }
+    __syncthreads();
+    {
+        // a warp a row: prefix maxima, 8 keys a lane, and with them the exponentials
+        float *pr = p + warp * keys, before = -INFINITY;
+        for (int g0 = 0; g0 < groups; g0 += 32) {
+            const int g = g0 + lane;
+            float x[KC], m = -INFINITY;
 #pragma unroll
-                for (int c = 0; c < KC; ++c) {
-                    float a = s[r][c];
+            for (int c = 0; c < KC; ++c) { x[c] = g < groups ? pr[g * KC + c] : -INFINITY; m = fmaxf(m, x[c]); }
 #pragma unroll
-                    for (int o = 1; o < GL; o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-                    const int key = j0 + c0 + c;
-                    s[r][c] = (key > row0 + r || key >= T) ? -INFINITY : a;
-                    cmax = fmaxf(cmax, s[r][c]);
-                }
-                const float mnew = fmaxf(m[r], cmax);
+            for (int o = 1; o < 32; o <<= 1) {
+                const float up = __shfl_up_sync(0xffffffffu, m, o);
+                if (lane >= o) m = fmaxf(m, up);
+            }
+            const float mnew = fmaxf(m, before), up = __shfl_up_sync(0xffffffffu, mnew, 1), mold = lane ? up : before;
+            before = __shfl_sync(0xffffffffu, mnew, 31);
+            if (g < groups) {
                 const bool live = mnew > -INFINITY;
-                const float resc = live ? __expf(m[r] - mnew) : 1.0f;
                 float csum = 0.0f;
 #pragma unroll
                 for (int c = 0; c < KC; ++c) {
-                    s[r][c] = live ? __expf(s[r][c] - mnew) : 0.0f;
-                    csum += s[r][c];
+                    const float e = live ? __expf(x[c] - mnew) : 0.0f;
+                    pr[g * KC + c] = e;
+                    csum += e;
                 }
-                m[r] = mnew;
-                l[r] = l[r] * resc + csum;
-                const unsigned long long resc2 = pack(resc, resc);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    unsigned long long z = 0ull;
-                    fma2(z, o2[r][i], resc2);
-                    o2[r][i] = z;
-                }
-            }
-#pragma unroll
-            for (int c = 0; c < KC; ++c) {
-#pragma unroll
-                for (int i = 0; i < 8; i += 2) {
-                    const float4 v = *reinterpret_cast<const float4 *>(Vs + (c0 + c) * HS + sub * 16 + 2 * i);
-                    const unsigned long long v0 = pack(v.x, v.y), v1 = pack(v.z, v.w);
-#pragma unroll
-                    for (int r = 0; r < RQ; ++r) {
-                        const unsigned long long p2 = pack(s[r][c], s[r][c]);
-                        fma2(o2[r][i], p2, v0);
-                        fma2(o2[r][i + 1], p2, v1);
-                    }
-                }
+                factor[warp * groups + g] = live ? __expf(mold - mnew) : 1.0f;
+                gsum[warp * groups + g] = csum;
             }
         }
     }
+    if (stage_v) asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    const int d = tid % HS, r0 = tid / HS * RT;
+    float o[RT], l[RT];
 #pragma unroll
-    for (int r = 0; r < RQ; ++r) {
-        if (row0 + r >= T) continue;
-        const float inv = (l[r] > 0.0f) ? 1.0f / l[r] : 0.0f;
-        float *dst = out + (long long)(row0 + r) * C + blockIdx.y * HS + sub * 16;
+    for (int r = 0; r < RT; ++r) o[r] = l[r] = 0.0f;
+#pragma unroll 2
+    for (int g = 0; g < groups; ++g) {
+        float x[KC];
 #pragma unroll
-        for (int i = 0; i < 8; i += 2) {
-            float a0, a1, a2, a3;
-            asm("mov.b64 {%0, %1}, %2;" : "=f"(a0), "=f"(a1) : "l"(o2[r][i]));
-            asm("mov.b64 {%0, %1}, %2;" : "=f"(a2), "=f"(a3) : "l"(o2[r][i + 1]));
-            *reinterpret_cast<float4 *>(dst + 2 * i) = make_float4(a0 * inv, a1 * inv, a2 * inv, a3 * inv);
+        for (int c = 0; c < KC; ++c) {
+            const int j = g * KC + c;
+            x[c] = stage_v ? vs[j * HS + d] : (j < T ? base[(long long)j * ld + 2 * C + d] : 0.0f);
+        }
+#pragma unroll
+        for (int r = 0; r < RT; ++r) {
+            const float *e = p + (r0 + r) * keys + g * KC, f = factor[(r0 + r) * groups + g];
+            l[r] = l[r] * f + gsum[(r0 + r) * groups + g];
+            o[r] = fmaf(o[r], f, 0.0f);
+#pragma unroll
+            for (int c = 0; c < KC; ++c) o[r] = fmaf(e[c], x[c], o[r]);
         }
     }
+#pragma unroll
+    for (int r = 0; r < RT; ++r)
+        if (i0 + r0 + r < T) out[(long long)(i0 + r0 + r) * C + blockIdx.y * HS + d] = o[r] * ((l[r] > 0.0f) ? 1.0f / l[r] : 0.0f);
 }
 
 }  // namespace
@@ -455,16 +449,29 @@ int decode_attention(float *y, const float *qkv, int pos, int C, int NH, cudaStr
     return launch_in_chain(decode_attention_k<128>, dim3(NH), DA_NT, smem, st, y, qkv, pos, C, scale, stage_v);
 }
 
-int window_attention(float *out, const float *qkv, int T, int C, int NH, cudaStream_t st) {
-    const int hs = C / NH;
-    const float scale = 1.0f / sqrtf((float)hs);
-    const dim3 grid(ceil_div(T, WA_NT / (hs / 16) * RQ), NH);
-    if (hs == 32) window_attention_k<32><<<grid, WA_NT, 0, st>>>(out, qkv, T, C, scale);
-    else if (hs == 64) window_attention_k<64><<<grid, WA_NT, 0, st>>>(out, qkv, T, C, scale);
-    else window_attention_k<128><<<grid, WA_NT, 0, st>>>(out, qkv, T, C, scale);
+template <int HS>
+static int run_window(float *out, const float *qkv, int T, int C, int NH, cudaStream_t st) {
+    static_assert(WA_NT / 32 == WR && WA_NT % HS == 0, "a warp a row, whole rows of columns");
+    const size_t keys = (size_t)ceil_div(T, KC) * KC, v_bytes = keys * HS * sizeof(float);
+    const int stage_v = v_bytes <= WA_MAX_V;
+    const size_t smem = (WR * HS + WR * keys + 2 * WR * (keys / KC)) * sizeof(float) + (stage_v ? v_bytes : 0);
+    static std::mutex mu;
+    static bool set[64];
+    const int d = current_device();
+    if (d < 0 || d >= 64) return fail(BMB_E_ARG, "device index %d out of range", d);
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        if (!set[d]) BMB_CUDA(cudaFuncSetAttribute(window_attention_k<HS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        set[d] = true;
+    }
+    window_attention_k<HS><<<dim3(ceil_div(T, WR), NH), WA_NT, smem, st>>>(out, qkv, T, C, 1.0f / sqrtf((float)HS), stage_v);
     count_launch();
     BMB_LAUNCH_CHECK();
     return BMB_OK;
+}
+int window_attention(float *out, const float *qkv, int T, int C, int NH, cudaStream_t st) {
+    const int hs = C / NH;
+    return hs == 32 ? run_window<32>(out, qkv, T, C, NH, st) : hs == 64 ? run_window<64>(out, qkv, T, C, NH, st) : run_window<128>(out, qkv, T, C, NH, st);
 }
 
 }  // namespace bmb
