@@ -147,6 +147,19 @@ int flash_forward(int cfg, int flags, float *out, float *lse, const float *qkv, 
 int flash_backward(int cfg, int flags, float *dqkv, float *dsum, const float *dout, const float *qkv, const float *out, const float *lse,
                    int B, int T, int C, int NH, bool in_trainer);
 
+// A model as decode_position reads it: its tensors (layer-stacked, as the trainer keeps them), the keys and values so far (rows
+// of 3C, T a layer), the pairs that activations are handed on in, and the logits.
+struct DecodeModel {
+    const float *wte, *wpe, *ln1w, *ln1b, *qkvw, *qkvb, *apw, *apb, *ln2w, *ln2b, *fcw, *fcb, *fpw, *fpb, *lnfw, *lnfb;
+    float *qkv, *logits;
+    uint2 *exchange;
+    int T, C, NH, L, Vp;
+    float scale;
+};
+size_t decode_exchange(int C);
+// `launch` counts the launches with one exchange: another one each time.
+int decode_position(const DecodeModel &m, int token, int pos, unsigned launch, cudaStream_t st);
+
 }  // namespace bmb
 
 // ---- device helpers ---------------------------------------------------------

@@ -20,10 +20,7 @@ bool flash_tc_supported(int T, int C, int NH, const float *qkv, const float *out
 int flash_forward_tc(float *out, float *lse, const float *qkv, int B, int T, int C, int NH, bool qkv_rounded,
                      cudaStream_t st);
 bool decode_accepts(int T, int C, int NH);
-int decode_embed(float *x, const float *wte, const float *wpe, int token, int pos, int C, cudaStream_t st);
-int decode_gemv(float *y, const float *x, const float *W, const float *bias, const float *ln_w, const float *ln_b, const float *add,
-                int in, int out, bool gelu, cudaStream_t st);
-int decode_attention(float *y, const float *qkv, int pos, int C, int NH, cudaStream_t st);
+int decode_gemv(float *y, const float *x, const float *W, int in, int out, cudaStream_t st);
 int window_attention(float *out, const float *qkv, int T, int C, int NH, cudaStream_t st);
 int flash_backward_tc(float *dqkv, float *dsum, const float *dout, const float *qkv, const float *out,
                       const float *lse, int B, int T, int C, int NH, bool rounded, cudaStream_t st, float *dbias_qkv = nullptr);
@@ -109,6 +106,8 @@ struct bmb_trainer {
     std::vector<std::pair<std::string, cudaEvent_t>> tl;
     bool keeps_split = false;     // counted among those whose captured steps hold the split products' block
     float *gen_probs = nullptr;   // one row of next-token probabilities, allocated by the first sampling call
+    uint2 *gen_exchange = nullptr;         // decode_position's, and how often that was launched
+    unsigned gen_launches = 0;
     // The two products of a linear layer's backward (dX = dY W and dW = dY^T X: the same FLOP count, both waiting only
     // for dY) run side by side, each on half of the SMs: dX on the main stream, dW on this one, forked and joined
     // by events -- one launch gap, one ramp and one tail per pair instead of two.
@@ -829,6 +828,7 @@ int bmb_trainer_destroy(bmb_trainer *t) {
     cudaFree(t->acts); cudaFree(t->bacts); cudaFree(t->d_tokens); cudaFree(t->d_targets);
     cudaFree(t->d_loss); cudaFree(t->d_sumsq); cudaFree(t->d_token);
     if (t->gen_probs) cudaFree(t->gen_probs);
+    if (t->gen_exchange) cudaFree(t->gen_exchange);
     if (t->col.arena) cudaFree(t->col.arena);
     if (t->col_jobs_dev) cudaFree(t->col_jobs_dev);
     dp_fused_destroy(t->dp);
@@ -1268,30 +1268,21 @@ static int next_token_logits(bmb_trainer *t, int pos, const float **row) {
     BMB_TRY(fwd_embed(t, d));
     for (int l = 0; l < d.L; ++l) BMB_TRY(fwd_layer(t, d, l));
     *row = t->logits;
-    return decode_gemv(t->logits, t->lnf + (size_t)(d.N - 1) * C, d.P + t->poff[P_WTE], nullptr, nullptr, nullptr, nullptr, C, d.Vp, false, t->st);
+    return decode_gemv(t->logits, t->lnf + (size_t)(d.N - 1) * C, d.P + t->poff[P_WTE], C, d.Vp, t->st);
 }
 
 // The same for the newest position of a growing text: `token` at `pos`, positions before it computed by earlier calls.
 // Their keys and values are the rows of t->qkv, T rows a layer.
 static int decode_logits(bmb_trainer *t, int token, int pos, const float **row) {
     const Dims d = dims_of(t);
-    const int C = d.C;
-    const float *P = d.P;
-    float *x = t->encoded, *x2 = t->residual2, *y = t->atty, *h = t->fch;      // one row each
-    BMB_TRY(decode_embed(x, P + t->poff[P_WTE], P + t->poff[P_WPE], token, pos, C, t->st));
-    for (int l = 0; l < d.L; ++l) {
-        const size_t lC = (size_t)l * C;
-        float *qkv = t->qkv + (size_t)l * d.T * 3 * C;
-        BMB_TRY(decode_gemv(qkv + (size_t)pos * 3 * C, x, P + t->poff[P_QKVW] + 3 * lC * C, P + t->poff[P_QKVB] + 3 * lC,
-                            P + t->poff[P_LN1W] + lC, P + t->poff[P_LN1B] + lC, nullptr, C, 3 * C, false, t->st));
-        BMB_TRY(decode_attention(y, qkv, pos, C, d.NH, t->st));
-        BMB_TRY(decode_gemv(x2, y, P + t->poff[P_APW] + lC * C, P + t->poff[P_APB] + lC, nullptr, nullptr, x, C, C, false, t->st));
-        BMB_TRY(decode_gemv(h, x2, P + t->poff[P_FCW] + 4 * lC * C, P + t->poff[P_FCB] + 4 * lC, P + t->poff[P_LN2W] + lC,
-                            P + t->poff[P_LN2B] + lC, nullptr, C, 4 * C, true, t->st));
-        BMB_TRY(decode_gemv(x, h, P + t->poff[P_FPW] + 4 * lC * C, P + t->poff[P_FPB] + lC, nullptr, nullptr, x2, 4 * C, C, false, t->st));
-    }
+    const auto P = [&](int tensor) { return d.P + t->poff[tensor]; };
+    const DecodeModel m{P(P_WTE), P(P_WPE), P(P_LN1W), P(P_LN1B), P(P_QKVW), P(P_QKVB), P(P_APW), P(P_APB), P(P_LN2W), P(P_LN2B), P(P_FCW), P(P_FCB),
+                        P(P_FPW), P(P_FPB), P(P_LNFW), P(P_LNFB), t->qkv, t->logits, t->gen_exchange,
+                        d.T, d.C, d.NH, d.L, d.Vp, 1.0f / sqrtf((float)(d.C / d.NH))};
     *row = t->logits;
-    return decode_gemv(t->logits, x, P + t->poff[P_WTE], nullptr, P + t->poff[P_LNFW], P + t->poff[P_LNFB], nullptr, C, d.Vp, false, t->st);
+    BMB_TRY(decode_position(m, token, pos, t->gen_launches, t->st));
+    ++t->gen_launches;
+    return BMB_OK;
 }
 
 // Softmax of one row of logits to the host: that of the reference's loss kernel (src/nn.cu:197-237); its target only
@@ -1306,6 +1297,11 @@ static int probs_to_host(bmb_trainer *t, const float *row, float *host_probs) {
 
 static int sampling_buffers(bmb_trainer *t) {
     if (!t->gen_probs) BMB_CUDA(cudaMalloc(&t->gen_probs, ((size_t)t->c.padded_vocab + 1) * sizeof(float)));
+    if (!t->gen_exchange) {
+        const size_t bytes = decode_exchange(t->c.n_embd) * sizeof(uint2);
+        BMB_CUDA(cudaMalloc(&t->gen_exchange, bytes));
+        BMB_CUDA(cudaMemsetAsync(t->gen_exchange, 0, bytes, t->st));
+    }
     return BMB_OK;
 }
 

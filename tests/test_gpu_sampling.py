@@ -111,3 +111,12 @@ def test_long_texts_position_by_position(bmb, cuda, heads, hs, T, layers):
         if s % 49 == 0 or s == T - 2:
             assert np.abs(p / m.probs(tokens[0, :s + 1]) - 1).max() < 1e-4, s
     t.close()
+
+
+@pytest.mark.parametrize("heads,hs,T,layers", [
+    (25, 32, 24, 2),        # 800 channels: 225 tiles of 32 outputs a layer, up to two a block, slices of 128 and of 32 inputs
+    (8, 128, 20, 2),        # the widest: 288 tiles, up to three a block, 4096 inputs
+    (1, 32, 20, 3),         # the narrowest: 9 tiles, one slice of 32 inputs
+])
+def test_several_tiles_a_block(bmb, cuda, heads, hs, T, layers):
+    test_long_texts_position_by_position(bmb, cuda, heads, hs, T, layers)
