@@ -567,7 +567,7 @@ gemm_tc_k(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
 }
 
 // ---- the same GEMM on CTA pairs ----------------------------------------------------------------
-// TF32 only.  Two CTAs (a cluster of 2, on neighbouring SMs) share one 256 x BN output tile: each loads
+// Two CTAs (a cluster of 2, on neighbouring SMs) share one 256 x BN output tile: each loads
 // its own 128 rows of A and HALF of the B slice, one thread of the leader CTA issues
 // tcgen05.mma.cta_group::2 (M = 256) for both, and each CTA ends up with its 128 x BN block of the
 // accumulator in its own tensor memory.  Against one CTA per 128 x 256 tile this halves the B bytes every
@@ -583,10 +583,13 @@ gemm_tc_k(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
 //   epilogue (warps 2..9, both)    as in gemm_tc_k, on the CTA's own 128 rows; the accumulator is handed
 //                                  back by arriving on the leader's barrier.
 // Work items are per pair.  Waits are bounded as everywhere; a pair leaves together (cluster barrier).
-constexpr int PAIR_STAGES = 5;
+// Which products come here: prefer_pair, with both sides measured.  Bound by shared memory at 256 columns (per 512 cycles of
+// products 32 KB read by them and 32 KB landing) and, with a short K, by the stores of the epilogue; six slices deep, which is what
+// fits (five: 4096^3 183.3 us, six 181.3).  TF32 4096^3: 173 us with the operands rounded (795 TFLOP/s), 189 on single CTAs.
+constexpr int PAIR_STAGES = 6;
 constexpr int pair_smem_bytes(int bn) { return PAIR_STAGES * (A_BYTES + (bn / 2) * KBYTES) + 1024 + 256 + EPI_BYTES; }
 
-template <int BN>
+template <int KIND, int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
 gemm_tc_pair_k(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                const __grid_constant__ CUtensorMap mapC, int c_mode, int M, int N, int kblocks, int kelems_per_block,
@@ -679,7 +682,7 @@ gemm_tc_pair_k(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     } else if (warp == 1) {
         // -------------------------------------------------------------- issuer (leader only)
         if (rank == 0 && elect_one()) {
-            const uint32_t idesc = make_idesc(2u, a_mn ? 1u : 0u, b_mn ? 1u : 0u, BN, BMT);
+            const uint32_t idesc = make_idesc(KIND == 0 ? 2u : 1u, a_mn ? 1u : 0u, b_mn ? 1u : 0u, BN, BMT);
             const uint32_t a_step = a_mn ? 1024u : 32u, b_step = b_mn ? 1024u : 32u;
             const uint32_t peer_empty0 = map_to_cta(empty0, 1), peer_tfull0 = map_to_cta(tfull0, 1);
             int s = 0, acc = 0;
@@ -699,7 +702,8 @@ gemm_tc_pair_k(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                     for (int k = 0; k < KBYTES / 32; ++k) {
                         const uint64_t db = b_mn ? smem_desc_mnmajor32(sb + k * b_step, CHUNK_BYTES) : smem_desc_kmajor(sb + k * b_step);
                         const uint64_t da = a_mn ? smem_desc_mnmajor32(sa + k * a_step, CHUNK_BYTES) : smem_desc_kmajor(sa + k * a_step);
-                        mma_tf32_pair(d, da, db, idesc, ((kb - kb0) | k) ? 1u : 0u);
+                        if (KIND == 0) mma_tf32_pair(d, da, db, idesc, ((kb - kb0) | k) ? 1u : 0u);
+                        else mma_f16_pair(d, da, db, idesc, ((kb - kb0) | k) ? 1u : 0u);
                     }
                     commit_pair(empty0 + 8 * s);                 // the slot is reusable, here ...
                     commit_pair(peer_empty0 + 8 * s);            // ... and in the peer CTA
@@ -734,16 +738,14 @@ gemm_tc_pair_k(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
             float *stg = reinterpret_cast<float *>(gen + STAGES * STAGE_BYTES) + (warp - 2) * (32 * 32);
             const int sub_r = lane >> 3, sub_u = lane & 7, sub_c = sub_u * 4;
             const float *part_bias = (kb0 == 0) ? bias : nullptr;
-#pragma unroll 1
-            for (int c = wgroup; c < BN / 32; c += 2) {
-                const int n0 = tn * BN + c * 32;
-                if (n0 >= N) break;
-                if (whole && c_mode == 3) {
-                    float lo[16], hi[16];
+            if (whole && c_mode == 3) {
+                const int r0 = row_base + (lane >> 2), cq = 2 * (lane & 3);
+                auto fetch = [&](int c, float (&lo)[16], float (&hi)[16]) {
                     tmem_ld_16x256b_x4_nowait(trow + (uint32_t)(c * 32), lo);
                     tmem_ld_16x256b_x4_nowait(trow + (uint32_t)(c * 32) + (16u << 16), hi);
-                    tmem_wait_ld();
-                    const int r0 = row_base + (lane >> 2), cq = 2 * (lane & 3);
+                };
+                auto put = [&](int c, const float (&lo)[16], const float (&hi)[16]) {
+                    const int n0 = tn * BN + c * 32;
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const int n = n0 + 8 * j + cq;
@@ -760,8 +762,28 @@ gemm_tc_pair_k(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                             if (m < M) *reinterpret_cast<float2 *>(C + (size_t)m * N + n) = x;
                         }
                     }
-                    continue;
+                };
+                auto live = [&](int c) { return c < BN / 32 && tn * BN + c * 32 < N; };     // warp-uniform
+                float la[16], ha[16], lb[16], hb[16];
+                int c = wgroup;
+                if (live(c)) fetch(c, la, ha);
+#pragma unroll 1
+                while (live(c)) {
+                    tmem_wait_ld();
+                    const int c2 = c + 2;
+                    if (live(c2)) fetch(c2, lb, hb);
+                    put(c, la, ha);
+                    if (!live(c2)) break;
+                    tmem_wait_ld();
+                    c = c2 + 2;
+                    if (live(c)) fetch(c, la, ha);
+                    put(c2, lb, hb);
                 }
+            } else
+#pragma unroll 1
+            for (int c = wgroup; c < BN / 32; c += 2) {
+                const int n0 = tn * BN + c * 32;
+                if (n0 >= N) break;
                 float v[32];
                 tmem_ld32(trow + (uint32_t)(c * 32), v);
                 if (c_mode) {
@@ -1053,7 +1075,7 @@ double slice_cost(int bn) { return bn == 256 ? 256.0 : (bn == 192 ? 200.0 : (bn 
 // measurements: 1.72 for twice the work) and, its epilogue no longer hidden, `tall_epi` slices more per
 // tile; sharing such tiles between CTAs costs more than sharing the small ones.
 void choose_schedule(int M, int N, int kblocks, int ctas, bool allow_split, int force_bn, int force_mh, bool tall_ok,
-                     int *bn_out, int *mh_out, int *dp_tiles_out) {
+                     int *bn_out, int *mh_out, int *dp_tiles_out, double *cost_out) {
     static const double tall_slice = [] { const char *e = getenv("BMB_GEMM_TALL_SLICE"); return e ? atof(e) : 1.72; }();
     static const double tall_epi = [] { const char *e = getenv("BMB_GEMM_TALL_EPI"); return e ? atof(e) : 8.0; }();
     const int widths[5] = {256, 256, 192, 128, 64};
@@ -1083,46 +1105,56 @@ void choose_schedule(int M, int N, int kblocks, int ctas, bool allow_split, int 
         }
         if (best < 0.0 || cost < best) { best = cost; *bn_out = w; *mh_out = mh; *dp_tiles_out = dp; }
     }
+    *cost_out = best;
 }
 
 // Everything the launch decides about how the tiles are handed out.
-struct Plan { int bn, mh, kblocks, tiles_m, tiles_n, tiles, dp_tiles, sk_tiles, g_sk, grid; bool pair; };
+struct Plan { int bn, mh, kblocks, tiles_m, tiles_n, tiles, dp_tiles, sk_tiles, g_sk, grid; bool pair; double cost; };
 
 // CTA pairs this device can keep resident at once for the pair kernel (one CTA per SM, clusters of 2).
 int pair_clusters();
 
-// Whether a problem goes to the pair kernel: TF32, one problem, at least one 256 x 256 tile, and operands
-// the pair kernel's loads take (an M- or N-contiguous operand needs its extent to be a multiple of 32).
-// BMB_GEMM_PAIR / BMB_GEMM_NO_PAIR in the flags decide for a call; the environment variable
-// BMB_GEMM_PAIR=1 makes pairs the default where the shape allows.
-bool wants_pair(bool bf16, int flags, int transA, int transB, int batch, int M, int N) {
-    // Measured on the step's shapes the pair form runs within +-6 % of single CTAs (both sit at the same
-    // shared-memory bandwidth bound: a CTA of a pair still feeds its half of B to both tensor cores), so it
-    // is opt-in.
+// What the pair kernel takes: one problem of at least one 256 x 256 tile, and operands its loads take (an M- or
+// N-contiguous TF32 operand needs its extent to be a multiple of 32).
+bool pair_takes(bool bf16, int transA, int transB, int batch, int M, int N) {
+    if (batch != 1 || M < 2 * BM || N < 256) return false;
+    return bf16 || !((transA && M % 32) || (!transB && N % 32));
+}
+
+// Whether a call asks for pairs: by BMB_GEMM_PAIR in the flags, or by the environment variable BMB_GEMM_PAIR=1 for all.
+bool asks_for_pair(int flags) {
     static const bool env_on = [] { const char *e = getenv("BMB_GEMM_PAIR"); return e && atoi(e) != 0; }();
-    if (bf16 || batch != 1 || M < 2 * BM || N < 256) return false;
-    if ((transA && M % 32) || (!transB && N % 32)) return false;
     if (flags & BMB_GEMM_NO_PAIR) return false;
     if (flags & (BMB_GEMM_TILE_M128 | BMB_GEMM_TILE_M256)) return (flags & BMB_GEMM_PAIR) != 0;
     return (flags & BMB_GEMM_PAIR) ? true : env_on;
 }
 
-// The pair kernel's plan: 256 x 256 tiles handed to `clusters` CTA pairs; what does not fill a wave of
-// pairs is shared along K like in the one-CTA kernel.
-void plan_pair(Plan *p, int flags, int M, int N, int clusters) {
+// Whether a call leaves it to the cost model (prefer_pair): nothing about tiles is forced.
+bool leaves_pair_open(int flags) {
+    static const bool env_forced = getenv("BMB_GEMM_PAIR") || getenv("BMB_GEMM_TILE_N") || getenv("BMB_GEMM_TILE_M");
+    return !env_forced && !(flags & (BMB_GEMM_NO_PAIR | BMB_GEMM_PAIR | BMB_GEMM_TILE_M128 | BMB_GEMM_TILE_M256));
+}
+
+// The pair kernel's plan: 256 x bn tiles handed to `clusters` CTA pairs; what does not fill a wave of
+// pairs is shared along K like in the one-CTA kernel.  Costs in the units of choose_schedule, fitted to the measurements at
+// prefer_pair; a tile of few slices is bound by its epilogue (BF16 4096x4096x512 36.6 us on single CTAs, 41.0 on pairs).
+void plan_pair(Plan *p, int flags, int M, int N, int clusters, int bn) {
+    const double unit = bn == 256 ? 0.89 : 0.70, own = p->kblocks + (bn == 256 ? 3.0 : 4.0), tile = own > 17.4 ? own : 17.4, start = 4.0;
     p->pair = true;
-    p->bn = 256;
+    p->bn = bn;
     p->mh = 2;
     p->tiles_m = (M + 2 * BM - 1) / (2 * BM);
-    p->tiles_n = (N + 255) / 256;
+    p->tiles_n = (N + bn - 1) / bn;
     p->tiles = p->tiles_m * p->tiles_n;
     const bool allow_split = !(flags & (BMB_GEMM_NO_SPLIT | BMB_GEMM_C_ROUNDED));
     const int full = p->tiles / clusters, rem = p->tiles % clusters;
     p->dp_tiles = p->tiles;
+    p->cost = start + (double)(full + (rem ? 1 : 0)) * tile * unit;
     if (allow_split && rem && p->kblocks >= 8) {
-        const double whole = (double)(full + 1) * (p->kblocks + 4.0);
-        const double shared = (double)full * (p->kblocks + 4.0) + (double)(((long long)rem * p->kblocks + clusters - 1) / clusters) + 10.0;
-        if (shared < whole) p->dp_tiles = p->tiles - rem;
+        const double run = (double)(((long long)rem * p->kblocks + clusters - 1) / clusters);
+        const double shared = start + ((double)full * tile + run + 22.0) * unit;
+        const bool short_k_big_run = p->kblocks <= 32 && run > 0.10 * ((double)full * tile + run);
+        if (shared < p->cost && !short_k_big_run) { p->cost = shared; p->dp_tiles = p->tiles - rem; }
     }
     p->sk_tiles = p->tiles - p->dp_tiles;
     p->g_sk = 1;
@@ -1152,7 +1184,7 @@ int plan_gemm(Plan *p, bool bf16, int flags, int batch, int M, int N, int K, int
     // A call may force the height itself (BMB_GEMM_TILE_M128 / _M256), which wins over the environment.
     const int call_mh = (flags & BMB_GEMM_TILE_M256) ? 2 : ((flags & BMB_GEMM_TILE_M128) ? 1 : force_mh);
     choose_schedule(M, N, p->kblocks, ctas, allow_split, (force_bn && N >= force_bn) ? force_bn : 0, call_mh, batch == 1 && !bf16, &p->bn, &p->mh,
-                    &p->dp_tiles);
+                    &p->dp_tiles, &p->cost);
     p->tiles_m = (M + p->mh * BM - 1) / (p->mh * BM);
     p->tiles_n = (N + p->bn - 1) / p->bn;
     const long long tiles_ll = (long long)p->tiles_m * p->tiles_n * batch;
@@ -1192,6 +1224,19 @@ int plan_gemm(Plan *p, bool bf16, int flags, int batch, int M, int N, int K, int
     return BMB_OK;
 }
 
+// The pair kernel's plan in place of *p where it costs less.  The sides of the line, single CTAs / pairs (us, operands from
+// DRAM): TF32 4096^3 199.5 / 181.3, 8192x2304x768 57.2 / 50.0, 8192x3072x768 72.5 / 66.3 (192 columns), 8192x768x768 30.8 / 26.7
+// (192), 768x2304x8192 87.0 / 68.6 (192), 8192x50304x768 1044 / 927; but 1024^3 19.5 / 27.6, 512x512x6144 27.7 / 29.7,
+// 50304x768x8192 799 / 843 and 8192x768x50304 918 / 980.  On half of the SMs 8192x2304x768 96.3 / 76.7, 3072x768x8192 121.9 / 92.2.
+// BF16 (passes over the operands included) 6144^3 425 / 386, 8192x50304x768 701 / 669; 1024^3 23.5 / 33.8.
+void prefer_pair(Plan *p, int flags, int M, int N, int clusters) {
+    for (int bn : {256, 192}) {
+        Plan q = *p;
+        plan_pair(&q, flags, M, N, clusters, bn);
+        if (q.cost < p->cost) *p = q;
+    }
+}
+
 template <int KIND, int BN, int MH, int AUX = 0, int RND = 0>
 int launch_tc(int grid, cudaStream_t st, const CUtensorMap &mapA, const CUtensorMap &mapB, const CUtensorMap &mapC, int c_mode,
               int batch, int M, int N, int kblocks, int kper,
@@ -1211,7 +1256,7 @@ int launch_tc(int grid, cudaStream_t st, const CUtensorMap &mapA, const CUtensor
     return BMB_OK;
 }
 
-template <int BN>
+template <int KIND, int BN>
 int launch_pair(int pairs, cudaStream_t st, const CUtensorMap &mapA, const CUtensorMap &mapB, const CUtensorMap &mapC, int c_mode,
                 int M, int N, int kblocks, int kper, int amn, int bmn, float alpha, float beta, float *C, int vec_ok, int dp_tiles,
                 int g_sk, const float *bias, int round_c, int *status_dev) {
@@ -1220,11 +1265,11 @@ int launch_pair(int pairs, cudaStream_t st, const CUtensorMap &mapA, const CUten
         std::lock_guard<std::mutex> lk(g_attr_mu);
         const int d = current_device();
         if (d >= 0 && d < 64 && !attr_set[d]) {
-            BMB_CUDA(cudaFuncSetAttribute(gemm_tc_pair_k<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, pair_smem_bytes(BN)));
+            BMB_CUDA(cudaFuncSetAttribute(gemm_tc_pair_k<KIND, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, pair_smem_bytes(BN)));
             attr_set[d] = true;
         }
     }
-    gemm_tc_pair_k<BN><<<2 * pairs, NTHREADS, pair_smem_bytes(BN), st>>>(mapA, mapB, mapC, c_mode, M, N, kblocks, kper, amn, bmn, alpha, beta,
+    gemm_tc_pair_k<KIND, BN><<<2 * pairs, NTHREADS, pair_smem_bytes(BN), st>>>(mapA, mapB, mapC, c_mode, M, N, kblocks, kper, amn, bmn, alpha, beta,
                                                                        C, vec_ok, dp_tiles, g_sk, bias, round_c, status_dev);
     return BMB_OK;
 }
@@ -1245,8 +1290,8 @@ int pair_clusters() {
         at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        cudaFuncSetAttribute(gemm_tc_pair_k<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, pair_smem_bytes(256));
-        if (cudaOccupancyMaxActiveClusters(&n, gemm_tc_pair_k<256>, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); n = sm_count() / 2; }
+        cudaFuncSetAttribute(gemm_tc_pair_k<0, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, pair_smem_bytes(256));
+        if (cudaOccupancyMaxActiveClusters(&n, gemm_tc_pair_k<0, 256>, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); n = sm_count() / 2; }
         if (n > sm_count() / 2) n = sm_count() / 2;
         cache[d] = n;
     }
@@ -1260,7 +1305,7 @@ int pair_clusters() {
 // what a slice moves through shared memory, by which the main loop is bound (so large square products keep the pass).
 static bool rounds_on_arrival(Plan *plan, int flags, int transA, int transB, int batch, int M, int N, int K, const float *A, const float *B,
                               bool a_rounded, bool b_rounded, int ctas) {
-    if ((a_rounded && b_rounded) || plan->pair || (flags & (BMB_GEMM_TILE_M256 | BMB_GEMM_PAIR))) return false;
+    if ((a_rounded && b_rounded) || asks_for_pair(flags) || (flags & BMB_GEMM_TILE_M256)) return false;
     // read where they lie: what the tensor maps take
     if ((((uintptr_t)A | (uintptr_t)B) & 15) || (transA ? M : K) % 4 || (transB ? K : N) % 4) return false;
     Plan p = *plan;
@@ -1273,6 +1318,7 @@ static bool rounds_on_arrival(Plan *plan, int flags, int transA, int transB, int
     // 8 of 256x256x32 20 / 9; but 2048^3 55 / 67, 4096^3 234 / 376, 2560x2560x640 33 / 43, 6144x6144x64 48 / 50
     // (and 1024^3, 25.8 / 24.6, which the rule leaves to the pass).
     auto cycles = [&](const Plan &q, bool in_place) {
+        if (q.pair) return 800.0 * q.cost;
         const double slice = q.mh == 2 ? 1.72 * 800.0 : in_place ? (q.bn == 256 ? 1570.0 : q.bn == 192 ? 1250.0 : q.bn == 128 ? 1100.0 : 1000.0)
                                                                  : (q.bn == 256 ? 800.0 : q.bn == 192 ? 650.0 : q.bn == 128 ? 520.0 : 400.0);
         const double store = q.bn <= 128 && !q.sk_tiles ? BM * q.bn * 4 / 20.0 : 0.0;
@@ -1309,8 +1355,11 @@ int gemm_tc(int math, int flags, int transA, int transB, int batch, int M, int N
     const int ctas = (flags & BMB_GEMM_HALF_SMS) ? (sm_count() + 1) / 2 : sm_count();
     Plan plan;
     BMB_TRY(plan_gemm(&plan, bf16, flags, batch, M, N, K, ctas));
-    if (wants_pair(bf16, flags, transA, transB, batch, M, N))
-        plan_pair(&plan, flags, M, N, (flags & BMB_GEMM_HALF_SMS) ? (pair_clusters() + 1) / 2 : pair_clusters());
+    if (pair_takes(bf16, transA, transB, batch, M, N) && (asks_for_pair(flags) || leaves_pair_open(flags))) {
+        const int clusters = (flags & BMB_GEMM_HALF_SMS) ? (pair_clusters() + 1) / 2 : pair_clusters();
+        if (leaves_pair_open(flags)) prefer_pair(&plan, flags, M, N, clusters);
+        else plan_pair(&plan, flags, M, N, clusters, 256);
+    }
     const bool a_rounded = (flags & BMB_GEMM_A_ROUNDED) != 0, b_rounded = (flags & BMB_GEMM_B_ROUNDED) != 0;
     const bool rnd = !bf16 && !aux_gelu && rounds_on_arrival(&plan, flags, transA, transB, batch, M, N, K, A, B, a_rounded, b_rounded, ctas);
     const int kblocks = plan.kblocks, bn = plan.bn, dp_tiles = plan.dp_tiles;
@@ -1348,10 +1397,17 @@ int gemm_tc(int math, int flags, int transA, int transB, int batch, int M, int N
         return fail(BMB_E_UNSUPPORTED, "gemm_tc: the fused activation needs beta 0, an aligned C and whole tiles");
     if (c_mode) BMB_TRY(make_map_2d(&mapC, C, 4, M, N, (long long)N * 4, 32, false));
     if (plan.pair) {
-        // (a K-major operand may have gone the padded-copy route; an MN-major one is 3-d by wants_pair's rule)
+        // (a K-major operand may have gone the padded-copy route; an MN-major one is 3-d by pair_takes' rule)
         if ((a.mn_major && !a.map3d) || (b.mn_major && !b.map3d)) return fail(BMB_E_UNSUPPORTED, "gemm_tc: operand layout not served by the pair kernel");
-        BMB_TRY((launch_pair<256>(grid, st, mapA, mapB, mapC, c_mode, M, N, kblocks, kper, amn, bmn, alpha, beta, C, vec_ok, dp_tiles, g_sk, bias,
-                                  round_c, status_dev)));
+#define BMB_PAIR_ARGS grid, st, mapA, mapB, mapC, c_mode, M, N, kblocks, kper, amn, bmn, alpha, beta, C, vec_ok, dp_tiles, g_sk, bias, round_c, status_dev
+        if (bf16) {
+            if (bn == 256) BMB_TRY((launch_pair<1, 256>(BMB_PAIR_ARGS)));
+            else BMB_TRY((launch_pair<1, 192>(BMB_PAIR_ARGS)));
+        } else {
+            if (bn == 256) BMB_TRY((launch_pair<0, 256>(BMB_PAIR_ARGS)));
+            else BMB_TRY((launch_pair<0, 192>(BMB_PAIR_ARGS)));
+        }
+#undef BMB_PAIR_ARGS
         count_launch();
         BMB_LAUNCH_CHECK();
         return BMB_OK;
@@ -1405,7 +1461,7 @@ extern "C" int bmb_gemm_schedule_check(int math, int flags, int batch, int M, in
     BMB_TRY(plan_gemm(&p, math == BMB_MATH_BF16, flags, batch, M, N, K, ctas));
     // the pair kernel's plan is replayed only when the call asks for it by flag (no device is consulted here):
     // `ctas` then counts CTA pairs
-    if ((flags & BMB_GEMM_PAIR) && wants_pair(math == BMB_MATH_BF16, flags, 0, 1, batch, M, N)) plan_pair(&p, flags, M, N, ctas);
+    if ((flags & BMB_GEMM_PAIR) && asks_for_pair(flags) && pair_takes(math == BMB_MATH_BF16, 0, 1, batch, M, N)) plan_pair(&p, flags, M, N, ctas, 256);
     if (bm_out) *bm_out = p.mh * BM;
     if (bn_out) *bn_out = p.bn;
     if (dp_tiles_out) *dp_tiles_out = p.dp_tiles;

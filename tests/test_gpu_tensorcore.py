@@ -504,3 +504,31 @@ def test_qkv_bias_gradient_from_the_attention_backward(bmb, cuda, monkeypatch):
         assert normwise(qb[0], qb[other]) < 1e-5, (other, normwise(qb[0], qb[other]))
         assert normwise(grads[0], grads[other]) < 1e-5
 
+
+
+@pytest.mark.parametrize("math", ["tf32", "bf16"])
+@pytest.mark.parametrize("ta,tb,M,N,K,beta", [
+    (0, 1, 8192, 768, 768, 0.0),       # pairs of 256 x 192, whole tiles
+    (0, 1, 4000, 3000, 1300, 0.0),     # 256 x 256, ragged, the last wave shared along K
+    (0, 0, 2048, 2112, 2080, 1.0),     # added into C
+    (1, 0, 768, 2304, 4096, 0.5),      # fewer tiles than pairs, both operands M- or N-contiguous
+])
+def test_pairs_taken_by_the_cost_model(bmb, cuda, math, ta, tb, M, N, K, beta):
+    """Products left to the cost model (some go to CTA pairs, 256 or 192 columns wide, TF32 and BF16) against single CTAs by flag and
+    a product in 64 bits of the rounded operands: 2e-5 normwise, as for the other tensor-core forms."""
+    g = cuda.Generator(device="cuda").manual_seed(9)
+    A, B = (cuda.rand(n, device="cuda", generator=g) * 2 - 1 for n in (M * K, K * N))
+    C0 = cuda.rand(M * N, device="cuda", generator=g)
+    for X in (A, B):
+        if math == "tf32":
+            bmb.call("bmb_round_tf32", X, X, X.numel(), None)
+        else:
+            X.copy_(X.bfloat16().float())
+    a = A.view(K, M).t() if ta else A.view(M, K)
+    b = B.view(N, K).t() if tb else B.view(K, N)
+    want = a.double() @ b.double() + beta * C0.view(M, N).double()
+    for flags in (0, bmb.GEMM_NO_SPLIT, bmb.GEMM_HALF_SMS, bmb.GEMM_NO_PAIR):
+        C = C0.clone() if beta else cuda.full((M * N,), float("nan"), device="cuda")
+        bmb.call("bmb_gemm_ex", bmb.MATH_TF32 if math == "tf32" else bmb.MATH_BF16, flags, ta, tb, M, N, K, 1.0, A, B, beta, C, None)
+        cuda.cuda.synchronize()
+        assert ((C.view(M, N).double() - want).norm() / want.norm()).item() < 2e-5, flags
