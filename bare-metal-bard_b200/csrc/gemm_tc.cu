@@ -220,6 +220,44 @@ __device__ __forceinline__ void add_result(float4 o, float *__restrict__ C, int 
     }
 }
 
+// A 32 x 32 block of a whole tile (beta 0, aligned C) from the registers of a 16x256b load to global memory: rows r0 + 8 k
+// of this lane's quarter (lo: k = 0, 1; hi: 2, 3).  Four neighbouring lanes hold 8 columns of a row, two each; one exchange
+// between neighbours makes that four columns each of 16, so that a store covers 64 bytes of a row and not 32.
+// Products with a short K wait for these stores (96 of 1024 x 64 x 1024: the issuer three quarters of the time for an accumulator to
+// be free): with 32 bytes 106 us, with 64 94; filling the result alone takes 57.
+template <int AUX>
+__device__ __forceinline__ void put_block(const float (&lo)[16], const float (&hi)[16], float *__restrict__ C, int M, int N, int r0, int n0, float alpha,
+                                          const float *__restrict__ bias, int round_c, float *__restrict__ aux, int round_aux, int lane) {
+    const bool odd = lane & 1;
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        const int n = n0 + 8 * (2 * p + odd) + 2 * (lane & 2);
+        const bool in = n < N;
+        float4 bb = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (bias && in) bb = *reinterpret_cast<const float4 *>(bias + n);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float *src = k < 2 ? lo : hi;
+            const int at = 8 * p + 2 * (k & 1);
+            const float ax = src[at], ay = src[at + 1], bx = src[at + 4], by = src[at + 5];
+            const float rx = __shfl_xor_sync(0xffffffffu, odd ? ax : bx, 1), ry = __shfl_xor_sync(0xffffffffu, odd ? ay : by, 1);
+            float4 x = odd ? make_float4(rx, ry, bx, by) : make_float4(ax, ay, rx, ry);
+            x = make_float4(fmaf(alpha, x.x, bb.x), fmaf(alpha, x.y, bb.y), fmaf(alpha, x.z, bb.z), fmaf(alpha, x.w, bb.w));
+            if (round_c) x = make_float4(round_tf32(x.x), round_tf32(x.y), round_tf32(x.z), round_tf32(x.w));
+            const int m = r0 + 8 * k;
+            if (in && m < M) {
+                *reinterpret_cast<float4 *>(C + (size_t)m * N + n) = x;
+                if (AUX) {                                       // second output: GELU of the first
+                    float4 g = AUX == 2 ? make_float4(gelu_tanh_fast(x.x), gelu_tanh_fast(x.y), gelu_tanh_fast(x.z), gelu_tanh_fast(x.w))
+                                        : make_float4(gelu_tanh(x.x), gelu_tanh(x.y), gelu_tanh(x.z), gelu_tanh(x.w));
+                    if (round_aux) g = make_float4(round_tf32(g.x), round_tf32(g.y), round_tf32(g.z), round_tf32(g.w));
+                    *reinterpret_cast<float4 *>(aux + (size_t)m * N + n) = g;
+                }
+            }
+        }
+    }
+}
+
 // KIND 0 = tf32 (fp32 operands), 1 = f16 (bf16 operands, always K-major).
 // a_mn / b_mn: the operand's tile is MN-major (TF32 only); 2 = its tensor map is the 3-d one that
 // brings all chunks of a slice in one copy.
@@ -441,35 +479,13 @@ gemm_tc_k(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
                 // memory in whole sectors -- no trip through shared memory, whose bandwidth the main loop needs.
                 // Two register sets: the tensor-memory load of the next 32-column chunk is in flight while this
                 // chunk's stores are issued (the epilogue of a 256-row tile is not hidden behind a main loop).
-                const int r0 = row_base + (lane >> 2), cq = 2 * (lane & 3);
+                const int r0 = row_base + (lane >> 2);
                 auto fetch = [&](int c, float (&lo)[16], float (&hi)[16]) {
                     tmem_ld_16x256b_x4_nowait(trow + (uint32_t)(c * 32), lo);                       // rows 0..15 of this quadrant
                     tmem_ld_16x256b_x4_nowait(trow + (uint32_t)(c * 32) + (16u << 16), hi);         // rows 16..31
                 };
                 auto put = [&](int c, const float (&lo)[16], const float (&hi)[16]) {
-                    const int n0 = tn * BN + c * 32;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int n = n0 + 8 * j + cq;
-                        if (n >= N) continue;
-                        float2 bb = make_float2(0.f, 0.f);
-                        if (bias) bb = *reinterpret_cast<const float2 *>(bias + n);
-                        float2 o[4] = {make_float2(lo[4 * j], lo[4 * j + 1]), make_float2(lo[4 * j + 2], lo[4 * j + 3]),
-                                       make_float2(hi[4 * j], hi[4 * j + 1]), make_float2(hi[4 * j + 2], hi[4 * j + 3])};
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const int m = r0 + 8 * k;
-                            float2 x = make_float2(fmaf(alpha, o[k].x, bb.x), fmaf(alpha, o[k].y, bb.y));
-                            if (round_c) x = make_float2(round_tf32(x.x), round_tf32(x.y));
-                            if (m < M) *reinterpret_cast<float2 *>(C + (size_t)m * N + n) = x;
-                            if (AUX && m < M) {                      // second output: GELU of the first
-                                float2 g = (AUX == 2) ? make_float2(gelu_tanh_fast(x.x), gelu_tanh_fast(x.y))
-                                                      : make_float2(gelu_tanh(x.x), gelu_tanh(x.y));
-                                if (round_aux) g = make_float2(round_tf32(g.x), round_tf32(g.y));
-                                *reinterpret_cast<float2 *>(aux + (size_t)m * N + n) = g;
-                            }
-                        }
-                    }
+                    put_block<AUX>(lo, hi, C, M, N, r0, tn * BN + c * 32, alpha, bias, round_c, aux, round_aux, lane);
                 };
                 auto live = [&](int c) { return c < BN / 32 && tn * BN + c * 32 < N; };     // warp-uniform
                 float la[16], ha[16], lb[16], hb[16];
@@ -739,29 +755,13 @@ gemm_tc_pair_k(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
             const int sub_r = lane >> 3, sub_u = lane & 7, sub_c = sub_u * 4;
             const float *part_bias = (kb0 == 0) ? bias : nullptr;
             if (whole && c_mode == 3) {
-                const int r0 = row_base + (lane >> 2), cq = 2 * (lane & 3);
+                const int r0 = row_base + (lane >> 2);
                 auto fetch = [&](int c, float (&lo)[16], float (&hi)[16]) {
                     tmem_ld_16x256b_x4_nowait(trow + (uint32_t)(c * 32), lo);
                     tmem_ld_16x256b_x4_nowait(trow + (uint32_t)(c * 32) + (16u << 16), hi);
                 };
                 auto put = [&](int c, const float (&lo)[16], const float (&hi)[16]) {
-                    const int n0 = tn * BN + c * 32;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int n = n0 + 8 * j + cq;
-                        if (n >= N) continue;
-                        float2 bb = make_float2(0.f, 0.f);
-                        if (bias) bb = *reinterpret_cast<const float2 *>(bias + n);
-                        float2 o[4] = {make_float2(lo[4 * j], lo[4 * j + 1]), make_float2(lo[4 * j + 2], lo[4 * j + 3]),
-                                       make_float2(hi[4 * j], hi[4 * j + 1]), make_float2(hi[4 * j + 2], hi[4 * j + 3])};
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const int m = r0 + 8 * k;
-                            float2 x = make_float2(fmaf(alpha, o[k].x, bb.x), fmaf(alpha, o[k].y, bb.y));
-                            if (round_c) x = make_float2(round_tf32(x.x), round_tf32(x.y));
-                            if (m < M) *reinterpret_cast<float2 *>(C + (size_t)m * N + n) = x;
-                        }
-                    }
+                    put_block<0>(lo, hi, C, M, N, r0, tn * BN + c * 32, alpha, bias, round_c, nullptr, 0, lane);
                 };
                 auto live = [&](int c) { return c < BN / 32 && tn * BN + c * 32 < N; };     // warp-uniform
                 float la[16], ha[16], lb[16], hb[16];
