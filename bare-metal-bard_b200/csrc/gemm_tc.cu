@@ -316,6 +316,7 @@ gemm_tc_k(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
     __syncthreads();
     fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    wait_for_predecessor();                             // the copies of the operands, or C prepared
     if (threadIdx.x == 0) GTR(1);
 
     if (warp == 0) {
@@ -648,6 +649,7 @@ gemm_tc_pair_k(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     fence_before();
     __syncthreads();
     cluster_sync_all();                                // both CTAs' barriers exist before anyone signals across
+    wait_for_predecessor();
     fence_after();
     const uint32_t tmem_base = *tmem_slot;
     // Each CTA asked its own SM for all the columns it will ever use, so both got the same address; the
@@ -859,6 +861,8 @@ template <> __device__ __forceinline__ __nv_bfloat16 cvt_out<__nv_bfloat16>(floa
 // dst[r][k] (row pitch Kp) = convert(src[r*K + k]), zero for k in [K, Kp).
 template <typename OUT>
 __global__ void prep_rows_k(OUT *__restrict__ dst, const float *__restrict__ src, long long R, int K, int Kp) {
+    wait_for_predecessor();
+    let_successor_start();
     const long long total = R * (long long)Kp;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
          i += (long long)gridDim.x * blockDim.x) {
@@ -869,6 +873,8 @@ __global__ void prep_rows_k(OUT *__restrict__ dst, const float *__restrict__ src
 }
 // Same-layout rounding copy of n4 float4.
 __global__ void prep_round_vec4_k(float *__restrict__ dst, const float *__restrict__ src, long long n4) {
+    wait_for_predecessor();
+    let_successor_start();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4;
          i += (long long)gridDim.x * blockDim.x) {
         const float4 v = reinterpret_cast<const float4 *>(src)[i];
@@ -878,6 +884,8 @@ __global__ void prep_round_vec4_k(float *__restrict__ dst, const float *__restri
 // dst[r][k] (row pitch Kp) = convert(src[k*R + r]): transposing copy through shared memory.
 template <typename OUT>
 __global__ void prep_transpose_k(OUT *__restrict__ dst, const float *__restrict__ src, int R, int K, int Kp) {
+    wait_for_predecessor();
+    let_successor_start();
     __shared__ float t[32][33];
     const int r0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
     for (int j = threadIdx.y; j < 32; j += 8) {
@@ -902,6 +910,8 @@ __device__ __forceinline__ uint4 bf16x8(const float (&v)[8]) {
 }
 // src and dst as one run of n8 groups of 8: needs K % 8 == 0 (then Kp = K).
 __global__ void __launch_bounds__(256) prep_bf16_vec8_k(uint4 *__restrict__ dst, const float4 *__restrict__ src, long long n8) {
+    wait_for_predecessor();
+    let_successor_start();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n8; i += (long long)gridDim.x * blockDim.x) {
         const float4 a = __ldg(src + 2 * i), b = __ldg(src + 2 * i + 1);
         const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
@@ -910,6 +920,8 @@ __global__ void __launch_bounds__(256) prep_bf16_vec8_k(uint4 *__restrict__ dst,
 }
 // 64 x 64 tiles; needs R % 4 == 0 (Kp is a multiple of 8).
 __global__ void __launch_bounds__(256) prep_transpose_bf16_vec_k(__nv_bfloat16 *__restrict__ dst, const float *__restrict__ src, int R, int K, int Kp) {
+    wait_for_predecessor();
+    let_successor_start();
     __shared__ float t[64][65];
     const int r0 = blockIdx.x * 64, k0 = blockIdx.y * 64;
 #pragma unroll
@@ -956,11 +968,36 @@ inline int blocks_for(long long items) {
     return (int)(b > cap ? cap : (b < 1 ? 1 : b));
 }
 
+// The first launch of a call follows what was in the stream before it as ever; the ones behind it are in a chain (common.cuh): each is
+// launched beside the one before and waits for its end first thing, so that only the launches overlap.  Measured with it, without: BF16
+// 512^3 12.6 us, 16.5; 1024^3 16.5, 18.6; TF32 1024^3 19.0, 21.7; 2048^3 42.9, 45.9; 4096^3 216.5, 219.0.
+struct Chain {
+    cudaStream_t st;
+    bool first = true;
+    template <typename... P, typename... A>
+    int launch(void (*kernel)(P...), dim3 grid, dim3 threads, size_t smem, A... args) {
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = grid;
+        cfg.blockDim = threads;
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cfg.attrs = &at;
+        cfg.numAttrs = first ? 0 : 1;
+        BMB_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+        count_launch();
+        first = false;
+        return BMB_OK;
+    }
+};
+
 // Decide how an operand reaches the tensor core.  X = its M or N extent, kcontig =
 // element (x,k) at src[x*K + k], otherwise at src[k*X + x].
 // `batch` dense problems one after the other (batch > 1 only reaches here with geometry the direct route takes).
 int stage_operand(Operand *op, const float *src, bool kcontig, long long X, int K, bool bf16, bool rounded,
-                  ScratchSlot slot, int tile_rows, cudaStream_t st, int batch = 1) {
+                  ScratchSlot slot, int tile_rows, Chain &chain, int batch = 1) {
     const bool aligned = ((uintptr_t)src % 16) == 0;
     if (!bf16) {
         const bool geom_ok = aligned && (kcontig ? (K % 4 == 0) : (X % 4 == 0));
@@ -969,12 +1006,10 @@ int stage_operand(Operand *op, const float *src, bool kcontig, long long X, int 
             if (!rounded) {
                 float *scr = (float *)device_scratch(slot, (size_t)batch * X * K * sizeof(float));
                 if (!scr) return BMB_E_CUDA;
-                BMB_TRY(scratch_acquire(slot, st));
+                BMB_TRY(scratch_acquire(slot, chain.st));
                 op->staged = true;
                 const long long n4 = (long long)batch * X * (long long)K / 4;
-                prep_round_vec4_k<<<blocks_for(n4), 256, 0, st>>>(scr, src, n4);
-                count_launch();
-                BMB_LAUNCH_CHECK();
+                BMB_TRY(chain.launch(prep_round_vec4_k, blocks_for(n4), 256, 0, scr, src, n4));
                 use = scr;
             }
             op->ptr = use;
@@ -991,23 +1026,21 @@ int stage_operand(Operand *op, const float *src, bool kcontig, long long X, int 
     const int Kp = (K + kalign - 1) / kalign * kalign;
     void *scr = device_scratch(slot, (size_t)X * Kp * esize);
     if (!scr) return BMB_E_CUDA;
-    BMB_TRY(scratch_acquire(slot, st));
+    BMB_TRY(scratch_acquire(slot, chain.st));
     op->staged = true;
     if (bf16 && aligned && kcontig && K % 8 == 0) {
         const long long n8 = X * (long long)K / 8;
-        prep_bf16_vec8_k<<<blocks_for(n8), 256, 0, st>>>((uint4 *)scr, (const float4 *)src, n8);
+        BMB_TRY(chain.launch(prep_bf16_vec8_k, blocks_for(n8), 256, 0, (uint4 *)scr, (const float4 *)src, n8));
     } else if (bf16 && aligned && !kcontig && X % 4 == 0 && (Kp + 63) / 64 <= 65535) {
-        prep_transpose_bf16_vec_k<<<dim3((unsigned)((X + 63) / 64), (unsigned)((Kp + 63) / 64)), 256, 0, st>>>((__nv_bfloat16 *)scr, src, (int)X, K, Kp);
+        BMB_TRY(chain.launch(prep_transpose_bf16_vec_k, dim3((unsigned)((X + 63) / 64), (unsigned)((Kp + 63) / 64)), 256, 0, (__nv_bfloat16 *)scr, src, (int)X, K, Kp));
     } else if (kcontig) {
-        if (bf16) prep_rows_k<__nv_bfloat16><<<blocks_for(X * (long long)Kp), 256, 0, st>>>((__nv_bfloat16 *)scr, src, X, K, Kp);
-        else prep_rows_k<float><<<blocks_for(X * (long long)Kp), 256, 0, st>>>((float *)scr, src, X, K, Kp);
+        if (bf16) BMB_TRY(chain.launch(prep_rows_k<__nv_bfloat16>, blocks_for(X * (long long)Kp), 256, 0, (__nv_bfloat16 *)scr, src, X, K, Kp));
+        else BMB_TRY(chain.launch(prep_rows_k<float>, blocks_for(X * (long long)Kp), 256, 0, (float *)scr, src, X, K, Kp));
     } else {
-        dim3 grid((unsigned)((X + 31) / 32), (unsigned)((Kp + 31) / 32));
-        if (bf16) prep_transpose_k<__nv_bfloat16><<<grid, dim3(32, 8), 0, st>>>((__nv_bfloat16 *)scr, src, (int)X, K, Kp);
-        else prep_transpose_k<float><<<grid, dim3(32, 8), 0, st>>>((float *)scr, src, (int)X, K, Kp);
+        const dim3 grid((unsigned)((X + 31) / 32), (unsigned)((Kp + 31) / 32)), threads(32, 8);
+        if (bf16) BMB_TRY(chain.launch(prep_transpose_k<__nv_bfloat16>, grid, threads, 0, (__nv_bfloat16 *)scr, src, (int)X, K, Kp));
+        else BMB_TRY(chain.launch(prep_transpose_k<float>, grid, threads, 0, (float *)scr, src, (int)X, K, Kp));
     }
-    count_launch();
-    BMB_LAUNCH_CHECK();
     op->ptr = scr; op->mn_major = false; op->map3d = false; op->tile_chunks = 0;
     op->rows = X; op->cols = Kp; op->pitch_bytes = (long long)Kp * esize; op->box_rows = tile_rows;
     return BMB_OK;
@@ -1042,6 +1075,8 @@ namespace {
 // C = beta * C over the tiles [dp_tiles, num_tiles) (the stream-K tiles), before their parts are added.
 __global__ void __launch_bounds__(256) sk_prepare_k(float *__restrict__ C, int M, int N, int tiles_m, int tiles_n, int dp_tiles,
                                                     int bm, int bn, float beta, int vec_ok) {
+    wait_for_predecessor();
+    let_successor_start();
     TileSched sch;
     sch.tiles_m = tiles_m; sch.tiles_n = tiles_n; sch.num_tiles = tiles_m * tiles_n;
     int tm, tn;
@@ -1238,7 +1273,7 @@ void prefer_pair(Plan *p, int flags, int M, int N, int clusters) {
 }
 
 template <int KIND, int BN, int MH, int AUX = 0, int RND = 0>
-int launch_tc(int grid, cudaStream_t st, const CUtensorMap &mapA, const CUtensorMap &mapB, const CUtensorMap &mapC, int c_mode,
+int launch_tc(int grid, Chain &chain, const CUtensorMap &mapA, const CUtensorMap &mapB, const CUtensorMap &mapC, int c_mode,
               int batch, int M, int N, int kblocks, int kper,
               int amn, int bmn, float alpha, float beta, float *C, int vec_ok, int dp_tiles, int g_sk, const float *bias,
               int round_c, int *status_dev, float *aux, int round_aux) {
@@ -1251,13 +1286,12 @@ int launch_tc(int grid, cudaStream_t st, const CUtensorMap &mapA, const CUtensor
             attr_set[d] = true;
         }
     }
-    gemm_tc_k<KIND, BN, MH, AUX, RND><<<grid, NTHREADS + RND * RND_THREADS, smem_bytes(BN, MH), st>>>(mapA, mapB, mapC, c_mode, batch, M, N, kblocks, kper, amn, bmn, alpha, beta, C, vec_ok,
-                                                                dp_tiles, g_sk, bias, round_c, status_dev, aux, round_aux);
-    return BMB_OK;
+    return chain.launch(gemm_tc_k<KIND, BN, MH, AUX, RND>, grid, NTHREADS + RND * RND_THREADS, smem_bytes(BN, MH), mapA, mapB, mapC, c_mode, batch, M, N, kblocks, kper, amn, bmn,
+                        alpha, beta, C, vec_ok, dp_tiles, g_sk, bias, round_c, status_dev, aux, round_aux);
 }
 
 template <int KIND, int BN>
-int launch_pair(int pairs, cudaStream_t st, const CUtensorMap &mapA, const CUtensorMap &mapB, const CUtensorMap &mapC, int c_mode,
+int launch_pair(int pairs, Chain &chain, const CUtensorMap &mapA, const CUtensorMap &mapB, const CUtensorMap &mapC, int c_mode,
                 int M, int N, int kblocks, int kper, int amn, int bmn, float alpha, float beta, float *C, int vec_ok, int dp_tiles,
                 int g_sk, const float *bias, int round_c, int *status_dev) {
     static bool attr_set[64];
@@ -1269,9 +1303,8 @@ int launch_pair(int pairs, cudaStream_t st, const CUtensorMap &mapA, const CUten
             attr_set[d] = true;
         }
     }
-    gemm_tc_pair_k<KIND, BN><<<2 * pairs, NTHREADS, pair_smem_bytes(BN), st>>>(mapA, mapB, mapC, c_mode, M, N, kblocks, kper, amn, bmn, alpha, beta,
-                                                                       C, vec_ok, dp_tiles, g_sk, bias, round_c, status_dev);
-    return BMB_OK;
+    return chain.launch(gemm_tc_pair_k<KIND, BN>, 2 * pairs, NTHREADS, pair_smem_bytes(BN), mapA, mapB, mapC, c_mode, M, N, kblocks, kper, amn, bmn, alpha, beta,
+                        C, vec_ok, dp_tiles, g_sk, bias, round_c, status_dev);
 }
 
 int pair_clusters() {
@@ -1366,8 +1399,9 @@ int gemm_tc(int math, int flags, int transA, int transB, int batch, int M, int N
     Operand a, b;
     StagingRelease release_on_return{a, b, st};
     // per CTA: the pair kernel loads 128 rows of A and half of the B tile
-    BMB_TRY(stage_operand(&a, A, !transA, M, K, bf16, a_rounded || rnd, SCR_GEMM_A, plan.pair ? BM : plan.mh * BM, st, batch));
-    BMB_TRY(stage_operand(&b, B, transB != 0, N, K, bf16, b_rounded || rnd, SCR_GEMM_B, plan.pair ? bn / 2 : bn, st, batch));
+    Chain chain{st};
+    BMB_TRY(stage_operand(&a, A, !transA, M, K, bf16, a_rounded || rnd, SCR_GEMM_A, plan.pair ? BM : plan.mh * BM, chain, batch));
+    BMB_TRY(stage_operand(&b, B, transB != 0, N, K, bf16, b_rounded || rnd, SCR_GEMM_B, plan.pair ? bn / 2 : bn, chain, batch));
     CUtensorMap mapA, mapB;
     if (a.map3d) BMB_TRY(make_map_mn3d(&mapA, a.ptr, a.rows, a.cols, a.pitch_bytes, a.tile_chunks));
     else BMB_TRY(make_map_2d(&mapA, a.ptr, esize, a.rows, a.cols, a.pitch_bytes, a.box_rows, a.mn_major));
@@ -1377,8 +1411,8 @@ int gemm_tc(int math, int flags, int transA, int transB, int batch, int M, int N
     const int vec_ok = ((uintptr_t)C % 16 == 0) && (N % 4 == 0);
     const int sk_tiles = plan.sk_tiles, g_sk = plan.g_sk, grid = plan.grid;
     if (sk_tiles > 0 && beta != 1.0f) {
-        sk_prepare_k<<<sk_tiles, 256, 0, st>>>(C, M, N, tiles_m, tiles_n, dp_tiles, plan.mh * BM, bn, beta, vec_ok);
-        count_launch();
+        chain.first = true;        // (launched beside the copies it made 4096^3 16 us slower)
+        BMB_TRY(chain.launch(sk_prepare_k, sk_tiles, 256, 0, C, M, N, tiles_m, tiles_n, dp_tiles, plan.mh * BM, bn, beta, vec_ok));
     }
     const int round_c = (flags & BMB_GEMM_C_ROUNDED) ? 1 : 0;
     const int amn = bf16 ? 0 : (a.mn_major ? (a.map3d ? 2 : 1) : 0), bmn = bf16 ? 0 : (b.mn_major ? (b.map3d ? 2 : 1) : 0);
@@ -1399,7 +1433,7 @@ int gemm_tc(int math, int flags, int transA, int transB, int batch, int M, int N
     if (plan.pair) {
         // (a K-major operand may have gone the padded-copy route; an MN-major one is 3-d by pair_takes' rule)
         if ((a.mn_major && !a.map3d) || (b.mn_major && !b.map3d)) return fail(BMB_E_UNSUPPORTED, "gemm_tc: operand layout not served by the pair kernel");
-#define BMB_PAIR_ARGS grid, st, mapA, mapB, mapC, c_mode, M, N, kblocks, kper, amn, bmn, alpha, beta, C, vec_ok, dp_tiles, g_sk, bias, round_c, status_dev
+#define BMB_PAIR_ARGS grid, chain, mapA, mapB, mapC, c_mode, M, N, kblocks, kper, amn, bmn, alpha, beta, C, vec_ok, dp_tiles, g_sk, bias, round_c, status_dev
         if (bf16) {
             if (bn == 256) BMB_TRY((launch_pair<1, 256>(BMB_PAIR_ARGS)));
             else BMB_TRY((launch_pair<1, 192>(BMB_PAIR_ARGS)));
@@ -1408,11 +1442,10 @@ int gemm_tc(int math, int flags, int transA, int transB, int batch, int M, int N
             else BMB_TRY((launch_pair<0, 192>(BMB_PAIR_ARGS)));
         }
 #undef BMB_PAIR_ARGS
-        count_launch();
         BMB_LAUNCH_CHECK();
         return BMB_OK;
     }
-#define BMB_TC_ARGS grid, st, mapA, mapB, mapC, c_mode, batch, M, N, kblocks, kper, amn, bmn, alpha, beta, C, vec_ok, dp_tiles, g_sk, bias, round_c, status_dev, aux, round_aux
+#define BMB_TC_ARGS grid, chain, mapA, mapB, mapC, c_mode, batch, M, N, kblocks, kper, amn, bmn, alpha, beta, C, vec_ok, dp_tiles, g_sk, bias, round_c, status_dev, aux, round_aux
     if (aux) {
         // the second output is compiled into instances of its own (the plain kernels stay as lean as they were:
         // the activation's code in every epilogue cost all products 13 %), three with the accurate tanh and three
@@ -1443,7 +1476,6 @@ int gemm_tc(int math, int flags, int transA, int transB, int batch, int M, int N
         else BMB_TRY((launch_tc<0, 64, 1>(BMB_TC_ARGS)));
     }
 #undef BMB_TC_ARGS
-    count_launch();
     BMB_LAUNCH_CHECK();
     return BMB_OK;
 }
