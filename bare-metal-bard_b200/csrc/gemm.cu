@@ -8,6 +8,8 @@ int gemm_simt(int transA, int transB, int batch, int M, int N, int K, float alph
               long long sA, const float *B, long long sB, float beta, float *C, long long sC,
               cudaStream_t st);
 // fp32 products on the tensor cores in three bf16 pieces (gemm_x3.cu), bias included.  BMB_E_UNSUPPORTED: the SIMT kernel's.
+int gemm_simt_small(int transA, int transB, int batch, int M, int N, int K, float alpha, const float *A, long long sA,
+                    const float *B, long long sB, float beta, float *C, long long sC, const float *bias, float *gelu, cudaStream_t st);
 int gemm_x3(int transA, int transB, int M, int N, int K, float alpha, const float *A, const float *B, float beta, float *C,
             const float *bias, int flags, cudaStream_t st);
 // Tensor-core path (gemm_tc.cu).  Returns BMB_E_UNSUPPORTED for shapes it does
@@ -42,7 +44,12 @@ int gemm_any_bias(int math, int flags, int ta, int tb, int batch, int M, int N, 
         // (A bias that the pass behind a SIMT product refuses is refused at any size.)
         const bool bias_ok = !bias || (N % 4 == 0 && (((uintptr_t)bias | (uintptr_t)C) & 15) == 0);
         rc = (math == BMB_MATH_FP32 && batch == 1 && A && B && C && bias_ok && !(flags & GEMM_CHAIN)) ? gemm_x3(ta, tb, M, N, K, alpha, A, B, beta, C, bias, flags, st) : BMB_E_UNSUPPORTED;
-        const bool bias_done = rc == BMB_OK;
+        bool bias_done = rc == BMB_OK;
+        // what follows a product of few tiles rides with it
+        if (rc == BMB_E_UNSUPPORTED && (bias || aux_gelu) && bias_ok && !(flags & BMB_GEMM_C_ROUNDED) && batch == 1 && !ta && tb && A && B && C && M > 0 && N > 0 && K > 0) {
+            rc = gemm_simt_small(ta, tb, batch, M, N, K, alpha, A, sA, B, sB, beta, C, sC, bias, aux_gelu, st);
+            bias_done = aux_done = rc == BMB_OK;
+        }
         if (rc == BMB_E_UNSUPPORTED) rc = gemm_simt(ta, tb, batch, M, N, K, alpha, A, sA, B, sB, beta, C, sC, st);
         if (rc != BMB_OK) return rc;
         // the optional rounding is a pass of its own on the same stream, as is the bias behind a SIMT product

@@ -245,7 +245,7 @@ int gemm_simt_tma(int transA, int transB, int batch, int M, int N, int K, float 
                   const float *B, long long sB, float beta, float *C, long long sC, cudaStream_t st);
 
 int gemm_simt_small(int transA, int transB, int batch, int M, int N, int K, float alpha, const float *A, long long sA,
-                    const float *B, long long sB, float beta, float *C, long long sC, cudaStream_t st);
+                    const float *B, long long sB, float beta, float *C, long long sC, const float *bias, float *gelu, cudaStream_t st);
 
 int gemm_simt(int transA, int transB, int batch, int M, int N, int K, float alpha, const float *A,
               long long sA, const float *B, long long sB, float beta, float *C, long long sC,
@@ -264,7 +264,7 @@ int gemm_simt(int transA, int transB, int batch, int M, int N, int K, float alph
     }
     // too few tiles of 128 x 128 for the chip: smaller ones, the same chains (gemm_simt_small.cu)
     {
-        const int rc = gemm_simt_small(transA, transB, batch, M, N, K, alpha, A, sA, B, sB, beta, C, sC, st);
+        const int rc = gemm_simt_small(transA, transB, batch, M, N, K, alpha, A, sA, B, sB, beta, C, sC, nullptr, nullptr, st);
         if (rc != BMB_E_UNSUPPORTED) return rc;
     }
     // NN and TN on aligned shapes: the kernel fed by the copy engine (gemm_simt_tma.cu)

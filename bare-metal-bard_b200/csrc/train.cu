@@ -213,8 +213,8 @@ int mm(bmb_trainer *t, int flags, int ta, int tb, int M, int N, int K, const flo
 
 // X W^T + bias outside the fused mode: in fp32 the product adds the bias as it stores (where it is not a split
 // product, the library does it after it); the other modes keep the pass of its own.
-int mm_bias(bmb_trainer *t, int flags, int M, int N, int K, const float *A, const float *B, float *C, const float *bias) {
-    if (t->c.math == BMB_MATH_FP32) return mm(t, flags, 0, 1, M, N, K, A, B, 0.0f, C, bias);
+int mm_bias(bmb_trainer *t, int flags, int M, int N, int K, const float *A, const float *B, float *C, const float *bias, float *gelu = nullptr) {
+    if (t->c.math == BMB_MATH_FP32) return mm(t, flags, 0, 1, M, N, K, A, B, 0.0f, C, bias, nullptr, gelu);      // (gelu: fp32 only)
     BMB_TRY(mm(t, flags, 0, 1, M, N, K, A, B, 0.0f, C));
     return bmb_bias_forward(C, bias, M, N);
 }
@@ -297,8 +297,9 @@ int fwd_layer(bmb_trainer *t, const Dims &d, int l) {
                    P + t->poff[P_FCB] + (size_t)l * 4 * C, nullptr, t->fuse_gelu ? fchg : nullptr));
         if (!t->fuse_gelu) BMB_TRY(bmb_gelu_forward(fchg, fch, (int)d.BT4C));
     } else {
-        BMB_TRY(mm_bias(t, wflag, N, 4 * C, C, ln2, W + t->poff[P_FCW] + (size_t)l * 4 * C * C, fch, P + t->poff[P_FCB] + (size_t)l * 4 * C));
-        BMB_TRY(bmb_gelu_forward(fchg, fch, (int)d.BT4C));
+        const bool together = (wflag & GEMM_CHAIN) != 0;      // a window's small products take the activation along
+        BMB_TRY(mm_bias(t, wflag, N, 4 * C, C, ln2, W + t->poff[P_FCW] + (size_t)l * 4 * C * C, fch, P + t->poff[P_FCB] + (size_t)l * 4 * C, together ? fchg : nullptr));
+        if (!together) BMB_TRY(bmb_gelu_forward(fchg, fch, (int)d.BT4C));
     }
     if (fz) {
         BMB_TRY(mm(t, wflag, 0, 1, N, C, 4 * C, fchg, W + t->poff[P_FPW] + (size_t)l * C * 4 * C, 0.0f, fcproj,

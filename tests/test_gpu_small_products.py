@@ -26,3 +26,16 @@ def test_small_tiles_follow_the_sequential_chain(bmb, orc, cuda, ta, tb, batch, 
         bmb.lib().bmb_set_math_mode(prev)
         cuda.cuda.synchronize()
         assert np.array_equal(dC.cpu().numpy(), want), offset
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 1152, 384), (70, 132, 33), (33, 64, 97), (1, 4, 1), (257, 700, 130)])
+def test_bias_and_gelu_ride_with_the_product(bmb, cuda, M, N, K):
+    """X W^T + bias and its GELU from one launch have the bits of the three passes (tiles of 64 x 32 and of 32)."""
+    A, W, bias = (cuda.from_numpy(uniform(n, i)).cuda() for i, n in enumerate((M * K, N * K, N)))
+    want, want_gelu, got, gelu = (cuda.full((M * N,), float("nan"), device="cuda") for _ in range(4))
+    bmb.call("bmb_gemm_ex", bmb.MATH_FP32, 0, 0, 1, M, N, K, 1.0, A, W, 0.0, want, None)
+    bmb.call("bmb_bias_forward", want, bias, M, N)
+    bmb.call("bmb_gelu_forward", want_gelu, want, M * N)
+    bmb.call("bmb_gemm_bias_gelu", bmb.MATH_FP32, 0, M, N, K, A, W, bias, got, gelu, None)
+    cuda.cuda.synchronize()
+    assert cuda.equal(got, want) and cuda.equal(gelu, want_gelu)
