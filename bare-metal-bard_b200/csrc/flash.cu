@@ -8,7 +8,8 @@
 // dK/dV (reduced over queries) each stay in registers and are written with
 // plain stores -- dqkv is overwritten, not accumulated.
 //
-// The kernels in use run on warp-level tensor-core instructions, every fp32 product as three TF32 ones
+// Long sequences go to the kernels of flash_x2.cu (wants_x2).  Short ones, captures outside a trainer, and heads with something that
+// two fp16 pieces cannot serve run here, on warp-level tensor-core instructions, every fp32 product as three TF32 ones
 // (flash_mma.cuh).  Behind them stand the row-group kernels (configuration 1): a query row (or, for dK/dV, a key
 // row) belongs to G = HS/32 adjacent lanes, each holding a 32-float slice of the head dimension in registers; key /
 // value (or query / dO) rows are staged in shared memory and read as warp-wide broadcasts; dot products finish with

@@ -17,10 +17,9 @@
 // of 8 bits and six products, so that no bit of x is left out and the products of the first pieces (16 bits) are added
 // up without being cut off.
 //
-// Why these instructions and not tcgen05: the operands stay plain fp32 in shared memory (a split copy of 64 rows of
-// K and V at head size 128 is 128 KB), probabilities go from accumulator to operand without leaving registers, and
-// with the output added up in fp32 registers every 32 keys anyway the accumulators would make the trip from tensor
-// memory each time.  Three TF32 products a multiply-add leave 170 of them per cycle and SM, against 128 on the FMA
+// Why these instructions and not tcgen05 (flash_x2.cu) where sequences are short or a head's elements differ too much: the operands stay
+// plain fp32 in shared memory, of any size, there is no pass over them first, and probabilities go from accumulator to operand
+// without leaving registers.  Three TF32 products a multiply-add leave 170 of them per cycle and SM, against 128 on the FMA
 // pipe, which the kernels these replaced used to 19 %.
 #pragma once
 #include "common.cuh"
