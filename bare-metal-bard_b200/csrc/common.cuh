@@ -148,17 +148,19 @@ int flash_backward(int cfg, int flags, float *dqkv, float *dsum, const float *do
                    int B, int T, int C, int NH, bool in_trainer);
 
 // A model as decode_position reads it: its tensors (layer-stacked, as the trainer keeps them), the keys and values so far (rows
-// of 3C, T a layer), the pairs that activations are handed on in, and the logits.
+// of 3C), the pairs that activations are handed on in, and the logits.
 struct DecodeModel {
-    const float *wte, *wpe, *ln1w, *ln1b, *qkvw, *qkvb, *apw, *apb, *ln2w, *ln2b, *fcw, *fcb, *fpw, *fpb, *lnfw, *lnfb;
+    const float *wte, *ln1w, *ln1b, *qkvw, *qkvb, *apw, *apb, *ln2w, *ln2b, *fcw, *fcb, *fpw, *fpb, *lnfw, *lnfb;
     float *qkv, *logits;
     uint2 *exchange;
-    int T, C, NH, L, Vp;
+    size_t layer;                 // floats from a layer's rows in qkv to the next one's
+    int C, NH, L, Vp;
     float scale;
 };
 size_t decode_exchange(int C);
-// `launch` counts the launches with one exchange: another one each time.
-int decode_position(const DecodeModel &m, int token, int pos, unsigned launch, cudaStream_t st);
+// The position's row before layer `first` (which may be L: the head alone) is x0, or x0 + x1 where that is given. `launch` counts the launches with one
+// exchange: another one each time.
+int decode_position(const DecodeModel &m, const float *x0, const float *x1, int first, int pos, unsigned launch, cudaStream_t st);
 
 }  // namespace bmb
 

@@ -17,10 +17,9 @@
 namespace bmb {
 namespace {
 
-// a warp that follows the chains and four that copy weights ahead of it; rows 4 banks apart
-constexpr int GV_OUT = 32, GV_NT = 160, GV_CP = 128, GV_K = 128, GV_PITCH = GV_K + 4, GV_STAGES = 8;
+// slices of 32 rows of weights and 128 inputs, rows 4 banks apart
+constexpr int GV_OUT = 32, GV_K = 128, GV_PITCH = GV_K + 4, GV_STAGES = 8;
 constexpr int GV_MAX_IN = 4096, GV_MAX_LN = 1024;
-constexpr int GV_SMEM = (GV_STAGES * GV_OUT * GV_PITCH + GV_MAX_IN) * 4;
 
 // s + w[0] a[0] + w[1] a[1] + .. in that order, `left` (a multiple of 4, at most GV_K) steps.
 __device__ __forceinline__ float follow_chain(float s, const float *w, const float *a, int left) {
@@ -35,43 +34,6 @@ __device__ __forceinline__ float follow_chain(float s, const float *w, const flo
         for (int k = 0; k < left; k += 4) step(k);
     }
     return s;
-}
-
-// y[o] = W[o] . x (the head of a window). in % 4 == 0.
-__global__ void __launch_bounds__(GV_NT) decode_gemv_k(float *__restrict__ y, const float *__restrict__ x, const float *__restrict__ W, int in, int out) {
-    extern __shared__ __align__(16) float smem[];
-    float *v = smem + GV_STAGES * GV_OUT * GV_PITCH;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, o0 = blockIdx.x * GV_OUT;
-    const int nk = (in + GV_K - 1) / GV_K;
-    auto fetch = [&](int kt) {
-        if (kt < nk && warp > 0) {
-            float *s = smem + (kt % GV_STAGES) * GV_OUT * GV_PITCH;
-#pragma unroll
-            for (int i = 0; i < GV_OUT * GV_K / 4 / GV_CP; ++i) {
-                const int lin = i * GV_CP + (int)threadIdx.x - 32, r = lin / (GV_K / 4), c = lin % (GV_K / 4) * 4, k = kt * GV_K + c;
-                const bool ok = o0 + r < out && k < in;
-                const float *p = W + (ok ? (size_t)(o0 + r) * in + k : 0);
-                const uint32_t d = (uint32_t)__cvta_generic_to_shared(s + r * GV_PITCH + c);
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(p), "r"(ok ? 16 : 0) : "memory");
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    let_successor_start();
-#pragma unroll
-    for (int i = 0; i < GV_STAGES - 1; ++i) fetch(i);
-    wait_for_predecessor();
-    for (int i = threadIdx.x * 4; i < in; i += GV_NT * 4) *reinterpret_cast<float4 *>(v + i) = *reinterpret_cast<const float4 *>(x + i);
-    float s = 0.0f;
-    for (int kt = 0; kt < nk; ++kt) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(GV_STAGES - 2) : "memory");
-        __syncthreads();
-        fetch(kt + GV_STAGES - 1);
-        if (warp != 0) continue;
-        s = follow_chain(s, smem + (kt % GV_STAGES) * GV_OUT * GV_PITCH + lane * GV_PITCH, v + kt * GV_K, min(GV_K, in - kt * GV_K));
-    }
-    const int o = o0 + lane;
-    if (warp == 0 && o < out) y[o] = s;
 }
 
 // ---- attention, 8 keys at a time -------------------------------------------------------------------------------------
@@ -291,7 +253,7 @@ __device__ __forceinline__ bool look_until(Look look, int *status) {
 }
 
 template <int HS>
-__global__ void __launch_bounds__(DP_NT) decode_position_k(const DecodeModel m, int token, int pos, int stage, unsigned tag0, int *__restrict__ status) {
+__global__ void __launch_bounds__(DP_NT) decode_position_k(const DecodeModel m, const float *__restrict__ x0, const float *__restrict__ x1, int first, int pos, int stage, unsigned tag0, int *__restrict__ status) {
     extern __shared__ __align__(16) float smem[];
     __shared__ uint64_t bars[2 * GV_STAGES + 2];
     __shared__ int giveup;
@@ -300,9 +262,9 @@ __global__ void __launch_bounds__(DP_NT) decode_position_k(const DecodeModel m, 
 
     if ((int)blockIdx.x >= gemv_blocks) {
         const int head = (int)blockIdx.x - gemv_blocks;
-        for (int l = 0; l < m.L; ++l) {
+        for (int l = first; l < m.L; ++l) {
             const unsigned tag = tag0 + l;
-            const bool ok = decode_head<HS>(smem, m.qkv + (size_t)l * m.T * 3 * C, pos, C, head, m.scale, stage, [&](float *last) {
+            const bool ok = decode_head<HS>(smem, m.qkv + l * m.layer, pos, C, head, m.scale, stage, [&](float *last) {
                 bool here = true;
                 if (threadIdx.x < 3 * HS) {
                     const int part = threadIdx.x / HS, d = threadIdx.x % HS;
@@ -331,7 +293,7 @@ __global__ void __launch_bounds__(DP_NT) decode_position_k(const DecodeModel m, 
     // This block's tiles, in the order of their use: those of a layer are counted through, then those of the head.
     const int tc_ = C / GV_OUT, per_layer = 9 * tc_;
     auto jobs = [&](auto use) {
-        for (int l = 0; l < m.L; ++l)
+        for (int l = first; l < m.L; ++l)
             for (int i = blockIdx.x; i < per_layer; i += gemv_blocks) {
                 DecodeJob j{nullptr, C, GV_OUT, DP_QKV, l, 0};
                 const size_t lC = (size_t)l * C;
@@ -368,7 +330,6 @@ __global__ void __launch_bounds__(DP_NT) decode_position_k(const DecodeModel m, 
         return;
     }
     constexpr int RAW = GV_STAGES * GV_OUT * GV_PITCH, NORMED = RAW + GV_MAX_IN;      // a vector as read, and after the layernorm
-    const float *te = m.wte + (size_t)token * C, *pe = m.wpe + (size_t)pos * C;
     int vectors = 0, step = -1, layer = -1;                       // how many so far; of the product and layer that the last one was for
     if (warp >= 2) {
         jobs([&](const DecodeJob &j) {
@@ -380,9 +341,12 @@ __global__ void __launch_bounds__(DP_NT) decode_position_k(const DecodeModel m, 
             ++vectors;
             for (int i = ((int)threadIdx.x - 64) * 4; ok && i < j.in; i += DP_LOAD * 128) {
                 float4 v;
-                if (j.step == DP_QKV && j.layer == 0) {           // the embedding
-                    const float4 a = __ldg(reinterpret_cast<const float4 *>(te + i)), p = __ldg(reinterpret_cast<const float4 *>(pe + i));
-                    v = make_float4(a.x + p.x, a.y + p.y, a.z + p.z, a.w + p.w);
+                if (j.layer == first && (j.step == DP_QKV || j.step == DP_HEAD)) {
+                    v = __ldg(reinterpret_cast<const float4 *>(x0 + i));
+                    if (x1) {
+                        const float4 a = __ldg(reinterpret_cast<const float4 *>(x1 + i));
+                        v = make_float4(v.x + a.x, v.y + a.y, v.z + a.z, v.w + a.w);
+                    }
                 } else {
                     ok = look_until([&]() { return get_pairs4(x + i, want, v); }, status);
                 }
@@ -405,8 +369,8 @@ __global__ void __launch_bounds__(DP_NT) decode_position_k(const DecodeModel m, 
         if (j.step != DP_HEAD)
             bias = __ldg((j.step == DP_QKV ? m.qkvb + (size_t)l * 3 * C : j.step == DP_PROJ ? m.apb + (size_t)l * C : j.step == DP_FC ? m.fcb + (size_t)l * 4 * C
                                                                                                           : m.fpb + (size_t)l * C) + o);
-        if (j.step == DP_PROJ && l == 0) add = te[o] + pe[o];     // (complete before the product's own vector is)
-        if (j.step == DP_PROJ && l > 0) ok = look_until([&]() { return get_pair(m.exchange + ex_x(C) + o, tag - 1, add); }, status);
+        if (j.step == DP_PROJ && l == first) add = x1 ? x0[o] + x1[o] : x0[o];     // (complete before the product's own vector is)
+        if (j.step == DP_PROJ && l > first) ok = look_until([&]() { return get_pair(m.exchange + ex_x(C) + o, tag - 1, add); }, status);
         if (j.step == DP_FCPROJ) ok = look_until([&]() { return get_pair(m.exchange + ex_x2(C) + o, tag, add); }, status);
         const int stages = (j.in + GV_K - 1) / GV_K;
         for (int i = 0, s1 = s, ph1 = ph; i < min(stages, GV_STAGES); ++i) {       // the weights are there long before the vector
@@ -491,7 +455,7 @@ __global__ void __launch_bounds__(DP_NT) decode_position_k(const DecodeModel m, 
         if (lane < j.rows) {
             if (j.step == DP_QKV) {
                 put_pair(m.exchange + ex_qkv(C) + o, sum + bias, tag);
-                m.qkv[((size_t)l * m.T + pos) * 3 * C + o] = sum + bias;       // for the positions to come
+                m.qkv[l * m.layer + (size_t)pos * 3 * C + o] = sum + bias;       // for the positions to come
             } else if (j.step == DP_PROJ) {
                 sum += bias;
                 put_pair(m.exchange + ex_x2(C) + o, add + sum, tag);
@@ -508,7 +472,7 @@ __global__ void __launch_bounds__(DP_NT) decode_position_k(const DecodeModel m, 
     });
 }
 
-// All rows of one sequence's window: as decode_attention_k, WR neighbouring rows of a head a block, so that what is read of a key
+// All rows of one sequence's window: as decode_head, WR neighbouring rows of a head a block, so that what is read of a key
 // or value serves all of them.  Scores and exponentials are computed side by side and only a row's sum and its output follow the
 // keys one after the other, a thread a column: at 256 positions of 6 heads x 64 10 us, against 38 for a walk over the keys in which
 // every 8 of them waited for the 8 before.
@@ -623,30 +587,17 @@ __global__ void __launch_bounds__(WA_NT) window_attention_k(float *__restrict__ 
 }  // namespace
 
 // Sizes these kernels take: the attention's head sizes, a layernorm of one warp, and a context of at most 512 groups of
-// 8 keys (one a thread in decode_attention_k).
+// 8 keys (one a thread in decode_head).
 bool decode_accepts(int T, int C, int NH) {
     const int hs = (NH > 0 && C % NH == 0) ? C / NH : 0;
     return (hs == 32 || hs == 64 || hs == 128) && C <= GV_MAX_LN && T <= DA_NT * KC;
-}
-
-int decode_gemv(float *y, const float *x, const float *W, int in, int out, cudaStream_t st) {
-    static std::mutex mu;
-    static bool set[64];
-    const int d = current_device();
-    if (d < 0 || d >= 64 || in > GV_MAX_IN || in % 4) return fail(BMB_E_UNSUPPORTED, "decode_gemv: %d inputs", in);
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        if (!set[d]) BMB_CUDA(cudaFuncSetAttribute(decode_gemv_k, cudaFuncAttributeMaxDynamicSharedMemorySize, GV_SMEM));
-        set[d] = true;
-    }
-    return launch_in_chain(decode_gemv_k, dim3(ceil_div(out, GV_OUT)), GV_NT, GV_SMEM, st, y, x, W, in, out);
 }
 
 // Pairs of 8 bytes that the launches of decode_position hand vectors on in; zero before the first.
 size_t decode_exchange(int C) { return (size_t)ex_size(C); }
 
 template <int HS>
-static int run_position(const DecodeModel &m, int token, int pos, unsigned launch, cudaStream_t st) {
+static int run_position(const DecodeModel &m, const float *x0, const float *x1, int first, int pos, unsigned launch, cudaStream_t st) {
     const size_t groups = ceil_div(pos + 1, KC), v_bytes = groups * KC * HS * sizeof(float);
     int stage = 2 * v_bytes <= DA_MAX_V ? 2 : v_bytes <= DA_MAX_V ? 1 : 0;
     const size_t att = stage * v_bytes + groups * (KC + 2) * sizeof(float), smem = att > DP_SMEM ? att : DP_SMEM;
@@ -667,15 +618,15 @@ static int run_position(const DecodeModel &m, int token, int pos, unsigned launc
     const int tiles = 9 * m.C / GV_OUT, room = sm_count() - m.NH, blocks = (tiles < room ? tiles : room) + m.NH;
     unsigned tag0 = launch * (unsigned)m.L + 1;
     DecodeModel model = m;
-    void *args[] = {&model, &token, &pos, &stage, &tag0, &status_dev};
+    void *args[] = {&model, &x0, &x1, &first, &pos, &stage, &tag0, &status_dev};
     BMB_CUDA(cudaLaunchCooperativeKernel((const void *)decode_position_k<HS>, dim3(blocks), dim3(DP_NT), args, smem, st));
     count_launch();
     return BMB_OK;
 }
-int decode_position(const DecodeModel &m, int token, int pos, unsigned launch, cudaStream_t st) {
+int decode_position(const DecodeModel &m, const float *x0, const float *x1, int first, int pos, unsigned launch, cudaStream_t st) {
     const int hs = m.C / m.NH;
-    return hs == 32 ? run_position<32>(m, token, pos, launch, st)
-                    : hs == 64 ? run_position<64>(m, token, pos, launch, st) : run_position<128>(m, token, pos, launch, st);
+    return hs == 32 ? run_position<32>(m, x0, x1, first, pos, launch, st)
+                    : hs == 64 ? run_position<64>(m, x0, x1, first, pos, launch, st) : run_position<128>(m, x0, x1, first, pos, launch, st);
 }
 
 template <int HS>

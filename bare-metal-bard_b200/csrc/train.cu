@@ -20,7 +20,6 @@ bool flash_tc_supported(int T, int C, int NH, const float *qkv, const float *out
 int flash_forward_tc(float *out, float *lse, const float *qkv, int B, int T, int C, int NH, bool qkv_rounded,
                      cudaStream_t st);
 bool decode_accepts(int T, int C, int NH);
-int decode_gemv(float *y, const float *x, const float *W, int in, int out, cudaStream_t st);
 int window_attention(float *out, const float *qkv, int T, int C, int NH, cudaStream_t st);
 int flash_backward_tc(float *dqkv, float *dsum, const float *dout, const float *qkv, const float *out,
                       const float *lse, int B, int T, int C, int NH, bool rounded, cudaStream_t st, float *dbias_qkv = nullptr);
@@ -1250,6 +1249,20 @@ int bmb_trainer_load(bmb_trainer *t, const char *path, int load_optimizer_state,
 }
 
 // ---- sampling (src/train_gpt.cu:46-102) ------------------------------------------------------------
+// The logits of row x0 (+ x1) at `pos` from layer `first` on; a layer's queries, keys and values lie `stride` floats after those
+// of the one before.
+static int position_logits(bmb_trainer *t, const float *x0, const float *x1, int first, int pos, size_t stride, const float **row) {
+    const Dims d = dims_of(t);
+    const auto P = [&](int tensor) { return d.P + t->poff[tensor]; };
+    const DecodeModel m{P(P_WTE), P(P_LN1W), P(P_LN1B), P(P_QKVW), P(P_QKVB), P(P_APW), P(P_APB), P(P_LN2W), P(P_LN2B), P(P_FCW), P(P_FCB),
+                        P(P_FPW), P(P_FPB), P(P_LNFW), P(P_LNFB), t->qkv, t->logits, t->gen_exchange,
+                        stride, d.C, d.NH, d.L, d.Vp, 1.0f / sqrtf((float)(d.C / d.NH))};
+    *row = t->logits;
+    BMB_TRY(decode_position(m, x0, x1, first, pos, t->gen_launches, t->st));
+    ++t->gen_launches;
+    return BMB_OK;
+}
+
 // The logits of one position in t->logits, from tokens already on the device.  They depend on that position's sequence
 // up to it and on nothing else, so in fp32 only those rows go through the layers (one sequence of `pos % T + 1`
 // positions instead of the whole batch), and only the last of them through the head.  The tensor-core modes run the
@@ -1267,23 +1280,23 @@ static int next_token_logits(bmb_trainer *t, int pos, const float **row) {
     d.wflag |= GEMM_CHAIN;               // the order of sums that sampling keeps (decode.cu)
     d.tokens = t->d_tokens + pos / T * T;
     BMB_TRY(fwd_embed(t, d));
-    for (int l = 0; l < d.L; ++l) BMB_TRY(fwd_layer(t, d, l));
-    *row = t->logits;
-    return decode_gemv(t->logits, t->lnf + (size_t)(d.N - 1) * C, d.P + t->poff[P_WTE], C, d.Vp, t->st);
+    // Of the last layer only the keys and values of all rows are wanted, and what follows from them for the last row (6 layers,
+    // 6 heads x 64, 256 rows: 0.09 ms of 0.75 less).  Attention over separate heads computes all rows of all layers.
+    const int whole = t->c.use_flash ? d.L - 1 : d.L;
+    for (int l = 0; l < whole; ++l) BMB_TRY(fwd_layer(t, d, l));
+    if (whole < d.L)
+        BMB_TRY(mm_bias(t, d.wflag, d.N, 3 * C, C, t->ln1 + whole * d.BTC, d.W + t->poff[P_QKVW] + (size_t)whole * 3 * C * C, t->qkv + whole * d.BT3C,
+                        d.P + t->poff[P_QKVB] + (size_t)whole * 3 * C));
+    const float *x = (whole == 0 ? t->encoded : t->residual3 + (size_t)(whole - 1) * d.BTC) + (size_t)(d.N - 1) * C;
+    return position_logits(t, x, nullptr, whole, d.N - 1, d.BT3C, row);
 }
 
 // The same for the newest position of a growing text: `token` at `pos`, positions before it computed by earlier calls.
 // Their keys and values are the rows of t->qkv, T rows a layer.
 static int decode_logits(bmb_trainer *t, int token, int pos, const float **row) {
-    const Dims d = dims_of(t);
-    const auto P = [&](int tensor) { return d.P + t->poff[tensor]; };
-    const DecodeModel m{P(P_WTE), P(P_WPE), P(P_LN1W), P(P_LN1B), P(P_QKVW), P(P_QKVB), P(P_APW), P(P_APB), P(P_LN2W), P(P_LN2B), P(P_FCW), P(P_FCB),
-                        P(P_FPW), P(P_FPB), P(P_LNFW), P(P_LNFB), t->qkv, t->logits, t->gen_exchange,
-                        d.T, d.C, d.NH, d.L, d.Vp, 1.0f / sqrtf((float)(d.C / d.NH))};
-    *row = t->logits;
-    BMB_TRY(decode_position(m, token, pos, t->gen_launches, t->st));
-    ++t->gen_launches;
-    return BMB_OK;
+    const int C = t->c.n_embd;
+    const float *P = dims_of(t).P;
+    return position_logits(t, P + t->poff[P_WTE] + (size_t)token * C, P + t->poff[P_WPE] + (size_t)pos * C, 0, pos, (size_t)t->c.T * 3 * C, row);
 }
 
 // Softmax of one row of logits to the host: that of the reference's loss kernel (src/nn.cu:197-237); its target only
