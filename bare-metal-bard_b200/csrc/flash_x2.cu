@@ -183,7 +183,8 @@ __global__ void __launch_bounds__(256) split_x2_k(const Images im, float *__rest
         *reinterpret_cast<uint4 *>(d + G::PIECE) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
     }
     if (threadIdx.x == 0) {
-        im.unscale[((long long)which * BH + bh) * nblk + blk] = pow2(e - 14);
+        // A block of zeros in V or dO has no size of its own: what dS is scaled by (bwd_x2's bound) is then D's.
+        im.unscale[((long long)which * BH + bh) * nblk + blk] = which >= 2 && most == 0.0f ? 0.0f : pow2(e - 14);
         im.flags[((long long)bh * nw + which) * nblk + blk] = bad;
         if (which == 3) im.dtop[(long long)bh * nblk + blk] = pow2(min(max(exponent(__int_as_float(dred)) + 1, -120), 100));
     }

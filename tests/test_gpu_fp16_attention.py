@@ -97,3 +97,51 @@ def test_captured_calls(bmb, cuda):
     graph.replay()
     cuda.cuda.synchronize()
     assert relative(out, eager[0]) <= BOUND and relative(lse, eager[1]) <= BOUND
+
+
+def in_64_bits(cuda, qkv, dout, NH):
+    """out, lse, and dq, dk, dv as (B, NH, T, hs)."""
+    B, T, C = dout.shape
+    hs = C // NH
+    heads = lambda x: x.double().reshape(B, T, NH, hs).transpose(1, 2)      # noqa: E731
+    (q, k, v), do = (heads(x) for x in qkv.chunk(3, dim=-1)), heads(dout)
+    s = (q @ k.transpose(2, 3) / hs ** 0.5).masked_fill(cuda.ones(T, T, dtype=cuda.bool, device="cuda").triu(1), float("-inf"))
+    lse = cuda.logsumexp(s, -1)
+    p = cuda.exp(s - lse[..., None])
+    out = p @ v
+    ds = p * (do @ v.transpose(2, 3) - (do * out).sum(-1, keepdim=True)) / hs ** 0.5
+    return out, lse, ds @ k, ds.transpose(2, 3) @ q, p.transpose(2, 3) @ do
+
+
+def by_heads(cuda, got, NH):
+    out, lse, _, dqkv = got
+    heads = lambda x: x.unflatten(-1, (NH, -1)).transpose(1, 2)      # noqa: E731
+    return heads(out), lse, *(heads(x) for x in dqkv.chunk(3, dim=-1))
+
+
+def no_worse(cuda, bmb, qkv, dout, NH, parts):
+    """Errors against 64 bits of parts of the five results are at most twice the row groups' (or within BOUND: theirs are sums of 32 terms
+    in a row, so their errors vary by less than that with the order).  parts: (result, index of its head and rows)."""
+    want = in_64_bits(cuda, qkv, dout, NH)
+    got, groups = (by_heads(cuda, attention(bmb, cuda, cfg, qkv, dout, NH), NH) for cfg in (0, 1))
+    for r, at in parts:
+        mine, theirs = relative(got[r][at], want[r][at]), relative(groups[r][at], want[r][at])
+        assert mine <= max(BOUND, 2 * theirs), (r, at, mine, theirs)
+
+
+OUT, LSE, DQ, DK, DV = range(5)
+
+
+@pytest.mark.parametrize("hs", [32, 64, 128])
+@pytest.mark.parametrize("which,e", [(2, 0), (2, -7), (2, -14), (2, -20), (3, 0), (3, -14)])
+def test_a_block_of_zeros(bmb, cuda, hs, which, e):
+    """64 positions whose V (or dO) is zero, where the other blocks are small: dS there is - P D, whatever the size of V."""
+    B, T, NH = 1, 640, 2
+    C = NH * hs
+    qkv, dout = inputs(cuda, B, T, NH, hs, hs)
+    x = dout if which == 3 else qkv[..., 2 * C:]
+    x *= 2.0 ** e
+    x[0, 128:192, hs:2 * hs] = 0
+    rows, all_ = slice(128, 192), slice(None)
+    parts = [(r, (0, h, all_)) for r in (OUT, LSE, DQ, DK, DV) for h in (0, 1)] + [(r, (0, 1, rows)) for r in (OUT, DK, DV)]
+    no_worse(cuda, bmb, qkv, dout, NH, parts + ([(DQ, (0, 1, rows))] if which == 2 else []))
