@@ -17,8 +17,8 @@
 //
 // What two pieces cannot serve is left to the kernels of flash.cu, which run behind these and skip every head that has none of
 // it: 64 rows whose largest element is not in 2^-45 .. 2^30 (nor zero) or not finite, a row whose largest element is below
-// 2^-20 of that (and not zero), D beyond 2^70, lse beyond 2^19, a probability beyond 3 (of an lse
-// that is not the scores').  Inside these limits no sum can overflow.
+// 2^-20 of that (and not zero), D beyond 2^70, lse beyond 2^19, a row's largest score beyond 2^22 (MOST_SCORE), a probability beyond 3
+// (of an lse that is not the scores').  Inside these limits no sum can overflow.
 //
 // Bound by what a step of 64 columns waits for in turn (products, exponentials and splits, sums) and by the FMA pipe, on which
 // the splits and exponentials of 128 x 64 elements are 1000 to 1400 cycles; products 2600 (64 columns, keys' side).  Four
@@ -48,6 +48,9 @@ constexpr int COMPUTE = 512, THREADS = COMPUTE + 128, W_COPY = COMPUTE / 32, W_I
 constexpr int REGS_COMPUTE = 104, REGS_OTHER = 64; // 512 x 104 + 128 x 64 = 640 x 96, the launch's registers
 constexpr float LEAST = 2.8421709430404007e-14f, MOST = 1073741824.0f;       // 2^-45, 2^30: the largest element of a block
 constexpr double CUT = 2.17e-8;                    // of a sum, cut off by an instruction, on average
+// Of a row's largest score, times log2(e): the reference of its exponentials is that score rounded to fp32, and what the rounding
+// leaves (at most 1/4 here; 8 at 2^27) is part of the exponents, which have room for 1/2.
+constexpr float MOST_SCORE = 4194304.0f - 8.0f;     // (of the reference, which the score may pass by 6)
 constexpr float WINDOW = 113.0f;                   // exponents of probabilities are followed to 2^-113
 // What scores and lse are both multiplied with: a row whose weight lies on one key has lse = its score, bit for bit, and that
 // key the probability 1, although neither may be rounded little at its size.
@@ -639,8 +642,10 @@ flash_fwd_x2_k(float *__restrict__ out, float *__restrict__ lse, const Images im
             // are small and rounded little), follows it in jumps of more than 2^4, so most steps rescale nothing.  Weights are
             // 2^9 times their exponentials: at most 2^15.
             float alpha = 1.0f;
-            if (e == 0) m = ceilf(top) - 2.0f;
-            else if (top > m + 6.0f) { const float to = ceilf(top) - 2.0f; alpha = exp2f(m - to); m = to; }
+            if (e == 0) {
+                m = ceilf(top) - 2.0f;
+                if (m < -MOST_SCORE) l = NAN;                // (told at the end)
+            } else if (top > m + 6.0f) { const float to = ceilf(top) - 2.0f; alpha = exp2f(m - to); m = to; }
             f2 sum = 0ull;
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
@@ -679,6 +684,7 @@ flash_fwd_x2_k(float *__restrict__ out, float *__restrict__ lse, const Images im
                 o[i] = add2(y, o[i]);
             }
             store_tile<H>(smem + warp * (32 * H * 4), out + ((long long)b * T + first + quad * 32) * C + h * HS + half * H, C, T - first - quad * 32, o, 1.0f);
+            if ((m > MOST_SCORE || l != l) && qi < T) im.flags[(long long)bh * 3 * nblk] = 1;          // (m never falls)
             if (half == 0 && qi < T) lse[(long long)bh * T + qi] = fmaf(m, INV_LOG2E, fmaf(m, INV_LOG2E_REST, logf(l * 1.953125e-3f)));
         }
     }

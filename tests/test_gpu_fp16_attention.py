@@ -145,3 +145,27 @@ def test_a_block_of_zeros(bmb, cuda, hs, which, e):
     rows, all_ = slice(128, 192), slice(None)
     parts = [(r, (0, h, all_)) for r in (OUT, LSE, DQ, DK, DV) for h in (0, 1)] + [(r, (0, 1, rows)) for r in (OUT, DK, DV)]
     no_worse(cuda, bmb, qkv, dout, NH, parts + ([(DQ, (0, 1, rows))] if which == 2 else []))
+
+
+@pytest.mark.parametrize("hs", [32, 64, 128])
+@pytest.mark.parametrize("size", [1e2, 1e3, 3e3, 1e4, 3e4, 1e5])
+@pytest.mark.parametrize("sign", [1, -1])
+def test_large_scores(bmb, cuda, hs, size, sign):
+    """Scores of 10^4 to 10^10, of mixed and (every query a negative multiple of its key and more) of one sign: a row's weight is on one key."""
+    B, T, NH = 1, 640, 2
+    C = NH * hs
+    qkv, dout = inputs(cuda, B, T, NH, hs, hs)
+    if sign < 0:
+        qkv[..., :C] = -qkv[..., :C].abs()
+        qkv[..., C:2 * C] = qkv[..., C:2 * C].abs()
+    qkv[..., :2 * C] *= size
+    got, want = (by_heads(cuda, attention(bmb, cuda, cfg, qkv, dout, NH), NH) for cfg in (0, 1))
+    assert all(bool(cuda.isfinite(x).all()) for x in got)
+    # Scores that are rounded at their size decide between keys that lie that close: such rows differ between any two implementations.
+    (q, k) = (x.unflatten(-1, (NH, hs)).transpose(1, 2).double() for x in qkv.chunk(3, dim=-1)[:2])
+    s = (q @ k.transpose(2, 3) / hs ** 0.5).masked_fill(cuda.ones(T, T, dtype=cuda.bool, device="cuda").triu(1), float("-inf"))
+    two = s.topk(2, dim=-1).values
+    clear = (two[..., 0] - two[..., 1]) > 20 + 2.0 ** -18 * s.masked_fill(s.isinf(), 0).abs().amax(-1)
+    clear[..., 0] = True
+    assert clear.double().mean() > 0.5
+    assert relative(got[OUT][clear], want[OUT][clear]) <= BOUND and relative(got[LSE], want[LSE]) <= BOUND
