@@ -17,8 +17,8 @@
 //
 // What two pieces cannot serve is left to the kernels of flash.cu, which run behind these and skip every head that has none of
 // it: 64 rows whose largest element is not in 2^-45 .. 2^30 (nor zero) or not finite, a row whose largest element is below
-// 2^-20 of that (and not zero), D beyond 2^70, lse beyond 2^19, a row's largest score beyond 2^22 (MOST_SCORE), a probability beyond 3
-// (of an lse that is not the scores').  Inside these limits no sum can overflow.
+// 2^-20 of that (and not zero), D beyond 2^70, lse beyond 2^19, a row's largest score beyond 2^22 (MOST_SCORE), a probability beyond
+// sqrt(2) (of an lse that is not the scores').  Inside these limits no sum can overflow.
 //
 // Bound by what a step of 64 columns waits for in turn (products, exponentials and splits, sums) and by the FMA pipe, on which
 // the splits and exponentials of 128 x 64 elements are 1000 to 1400 cycles; products 2600 (64 columns, keys' side).  Four
@@ -865,8 +865,10 @@ __device__ __forceinline__ void bwd_x2(uint8_t *smem, float *__restrict__ dqkv, 
         const float ca1 = im.unscale[WA1 * side + head + rb] * LOG2E;
         const float ca2 = im.unscale[WA2 * side + head + rb];
         const float *mine = im.rows + (head + rb) * (3 * XB) + (row & 63);
-        const float lr = KV ? 0.0f : mine[0], lb = KV ? 0.0f : mine[XB], drow = KV ? 0.0f : mine[2 * XB];
-        bool ok = true, late = false;                        // (late: a probability of 3, of an lse that is not these scores')
+        const float lr = KV ? 0.0f : mine[0], lb = KV ? 0.0f : mine[XB], drow = KV ? 0.0f : mine[2 * XB], vmost = lb + (WINDOW + 0.5f);
+        // late: a probability beyond sqrt(2), of an lse that is not these scores'.  The queries' side looks, before exponents so far above 0
+        // run over; the keys' side has the same pairs, and the head is computed again for both.
+        bool ok = true, late = false;
         // dS of a step is scaled so that it is at most 2^15 whatever the data: by 1 / (the largest that dP and D can be).
         const float *top = im.dtop + head + (KV ? c0 : rb);
         auto bound = [&](int e) { return fmaxf(__ldg(u2 + e) * ca2 * (1073741824.0f * HS), __ldg(top + (KV ? e : 0))); };
@@ -905,27 +907,31 @@ __device__ __forceinline__ void bwd_x2(uint8_t *smem, float *__restrict__ dqkv, 
             const uint32_t sa = tmem + lanes + (uint32_t)(e % F::BUFS * 64 + 32 * half), da = sa + COL_DP;
             const float4 *cols = reinterpret_cast<const float4 *>(smem + F::OFF_ROWS + e % F::N2 * ROWS_BYTES) + 8 * half;
             const bool edge = KV ? col0 < r0 + 127 : col0 + 31 > r0;
-            float pmost = 0.0f;
+            auto mask = [&](int j, f2 (&p)[8], float with) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int k = col0 + j + 2 * i;
+                    p[i] = pack((KV ? k < ri : k > ri) ? with : low(p[i]), (KV ? k + 1 < ri : k + 1 > ri) ? with : high(p[i]));
+                }
+            };
             // 16 columns at a time, so that the loop stays in the instruction cache and its registers are few
             auto weights = [&](int j, f2 (&p)[8], const f2 (&d)[8]) {
                 // p = 2^14 2^(S - lse): lse's whole part goes to the exponent (exp2_from), so nothing is rounded at its size.
+                float vtop = -INFINITY;
+                if (!KV && edge) mask(j, p, -INFINITY);
 #pragma unroll
                 for (int i = 0; i < 8; i += 2) {
                     float4 r = make_float4(lr, lr, lr, lr), b = make_float4(lb, lb, lb, lb);
                     if (KV) { r = cols[(j + 2 * i) / 4]; b = cols[16 + (j + 2 * i) / 4]; }
                     const f2 b0 = pack(b.x, b.y), b1 = pack(b.z, b.w);
-                    p[i] = exp2_unit(max2(fma2(p[i], both(cs), pack(r.x, r.y)), b0), fma2(b0, both(-1.0f), both(MAGIC - 99.0f)));
-                    p[i + 1] = exp2_unit(max2(fma2(p[i + 1], both(cs), pack(r.z, r.w)), b1), fma2(b1, both(-1.0f), both(MAGIC - 99.0f)));
+                    p[i] = max2(fma2(p[i], both(cs), pack(r.x, r.y)), b0);
+                    p[i + 1] = max2(fma2(p[i + 1], both(cs), pack(r.z, r.w)), b1);
+                    if (!KV) vtop = fmax3(fmax3(vtop, low(p[i]), high(p[i])), low(p[i + 1]), high(p[i + 1]));
+                    p[i] = exp2_unit(p[i], fma2(b0, both(-1.0f), both(MAGIC - 99.0f)));
+                    p[i + 1] = exp2_unit(p[i + 1], fma2(b1, both(-1.0f), both(MAGIC - 99.0f)));
                 }
-                if (edge) {
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const int k = col0 + j + 2 * i;
-                        p[i] = pack((KV ? k < ri : k > ri) ? 0.0f : low(p[i]), (KV ? k + 1 < ri : k + 1 > ri) ? 0.0f : high(p[i]));
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < 8; ++i) asm("max.abs.f32 %0, %0, %1, %2;" : "+f"(pmost) : "f"(low(p[i])), "f"(high(p[i])));
+                if (!KV) late = late || vtop > vmost;
+                if (KV && edge) mask(j, p, 0.0f);
                 if (KV) put_weights(sa + j, p);
 #pragma unroll
                 for (int i = 0; i < 8; i += 2) {
@@ -943,7 +949,6 @@ __device__ __forceinline__ void bwd_x2(uint8_t *smem, float *__restrict__ dqkv, 
                 ld_scores<F::HALVES>(da + j, d);
                 weights(j, p, d);
             }
-            late = late || !(pmost <= 49152.0f);
             tmem_wait_st();
             fence_before();
             __syncwarp();
@@ -956,7 +961,7 @@ __device__ __forceinline__ void bwd_x2(uint8_t *smem, float *__restrict__ dqkv, 
         if (!last) { take2(n - 2); take1(n - 2); }
         take2(n - 1);
         take1(n - 1);
-        if (late && ri < T) im.flags[(long long)bh * 4 * nblk] = 1;
+        if (!KV && late && ri < T) im.flags[(long long)bh * 4 * nblk] = 1;
         if (ok) {
             // every product has retired: the tiles' memory is free
             const int b = bh / NH, h = bh % NH, C = NH * HS, valid = T - r0 - quad * 32;

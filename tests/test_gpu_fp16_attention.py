@@ -169,3 +169,17 @@ def test_large_scores(bmb, cuda, hs, size, sign):
     clear[..., 0] = True
     assert clear.double().mean() > 0.5
     assert relative(got[OUT][clear], want[OUT][clear]) <= BOUND and relative(got[LSE], want[LSE]) <= BOUND
+
+
+@pytest.mark.parametrize("hs", [32, 64, 128])
+@pytest.mark.parametrize("shift", [-0.5, -1.0, -30.0, -60.0, -84.0, -100.0, -150.0, -200.0, -300.0])
+def test_lse_far_below_the_scores(bmb, cuda, hs, shift):
+    """Weights of 1.6 to e^90 come out as from the row groups, and what overflows there is not finite here either.  (An exponential's
+    argument, up to |shift| + 12 in natural units, is rounded to 24 bits on either side, and so is its product with log2 e.)"""
+    qkv, dout = inputs(cuda, 1, 512, 2, hs, hs)
+    got, want = (by_heads(cuda, attention(bmb, cuda, cfg, qkv, dout, 2, shift), 2) for cfg in (0, 1))
+    for r in (DQ, DK, DV):
+        assert cuda.equal(cuda.isfinite(got[r]), cuda.isfinite(want[r])), r
+        fin = cuda.isfinite(want[r])
+        if bool(fin.any()):
+            assert relative(got[r][fin], want[r][fin]) <= BOUND + 4 * 2.0 ** -24 * (abs(shift) + 12), r
