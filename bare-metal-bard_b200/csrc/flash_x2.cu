@@ -666,7 +666,7 @@ flash_fwd_x2_k(float *__restrict__ out, float *__restrict__ lse, const Images im
                 for (int i = 0; i < H / 2; ++i) o[i] = mul2(o[i], both(alpha));
             }
         }
-        if (ok && mine > 0) {
+        if (mine > 0) {                                      // (also who has given up: the barrier is the whole tile's)
             take(mine - 1);
             float *at = tops + mine % F::BUFS * 512;
             at[half * 128] = l;
