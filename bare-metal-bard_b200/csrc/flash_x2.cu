@@ -6,7 +6,8 @@
 // hi and lo hold 22 to 23 bits of x; a b is hi hi + 2^-11 (hi lo + lo hi) up to 2^-22 of |a b|.  The products of the small
 // pieces come first and are scaled by 2^-11 by the first instruction that adds products of the large ones (scale-input-d), so
 // one accumulator serves all.  Elements down to 2^-28 of the largest of their 64 rows keep all bits that hi and lo have, smaller
-// ones are held to 2^-51 of it.  Probabilities and dS are split in registers, scaled by the most that they can be.
+// ones are held to 2^-51 of it, which is 2^-31 of the largest in their row or column (see below).  Probabilities and dS are split in registers, scaled by the
+// most that they can be.
 // Why fp16 and not bf16 or TF32: at the same accuracy bf16 takes six products, TF32 three at half the rate and twice the
 // bytes in shared memory, which is what bounds the 64-column products below (69 cycles with both operands there, 40 with
 // one in tensor memory, 32 by the pipe's rate).
@@ -16,7 +17,7 @@
 // fp32 registers.
 //
 // What two pieces cannot serve is left to the kernels of flash.cu, which run behind these and skip every head that has none of
-// it: 64 rows whose largest element is not in 2^-45 .. 2^30 (nor zero) or not finite, a row whose largest element is below
+// it: 64 rows whose largest element is not in 2^-45 .. 2^30 (nor zero) or not finite, a row or column whose largest element is below
 // 2^-20 of that (and not zero), D beyond 2^70, lse beyond 2^19, a row's largest score beyond 2^22 (MOST_SCORE), a probability beyond
 // sqrt(2) (of an lse that is not the scores').  Inside these limits no sum can overflow.
 //
@@ -90,16 +91,22 @@ __device__ __forceinline__ void split2(float x, float xe, float y, float ye, uin
 }
 __device__ __forceinline__ float pow2(int e) { return __int_as_float((e + 127) << 23); }      // -126 <= e <= 127
 __device__ __forceinline__ int exponent(float x) { return (int)(__float_as_uint(x) >> 23 & 255) - 127; }
+__device__ __forceinline__ uint32_t max_u16x2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("max.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
 
 // One block: 64 positions of one head of q, k, v or dO; bound by memory (4 bytes read and 4 written an element).  With dO also
 // D = rowsum(dO O).
 template <int HS>
-__global__ void __launch_bounds__(256) split_x2_k(const Images im, float *__restrict__ dsum, const float *__restrict__ qkv,
+__global__ void __launch_bounds__(256, HS == 32 ? 5 : HS == 64 ? 4 : 2) split_x2_k(const Images im, float *__restrict__ dsum, const float *__restrict__ qkv,
                                                   const float *__restrict__ dout, const float *__restrict__ out,
                                                   const float *__restrict__ lse, int T, int NH, int BH, int nblk, int nw, Factors fac) {
     using G = Geo<HS>;
     constexpr int UPR = HS / 8, ITEMS = XB * UPR / 256;
     __shared__ float red[8];
+    __shared__ __align__(16) uint32_t columns[8][4 * UPR];
     __shared__ int dred;
     if (threadIdx.x == 0) dred = 0;
     const int blk = (int)(blockIdx.x % (unsigned)nblk), which = (int)(blockIdx.x / (unsigned)nblk % (unsigned)nw);
@@ -107,6 +114,7 @@ __global__ void __launch_bounds__(256) split_x2_k(const Images im, float *__rest
     const long long ld = which < 3 ? 3LL * C : C;
     const float *src = (which < 3 ? qkv + which * C : dout) + ((long long)b * T + blk * XB) * ld + h * HS;
     float v[ITEMS][8], rest[ITEMS][8], rowmax[ITEMS], most = 0.0f, dmax = 0.0f;      // rest: of q only
+    uint32_t colmax[4] = {0u, 0u, 0u, 0u};
     bool bad = false;
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
@@ -125,6 +133,10 @@ __global__ void __launch_bounds__(256) split_x2_k(const Images im, float *__rest
                 rest[i][j] = fmaf(q, fac.q, -v[i][j]) + q * fac.q_rest;
             }
         }
+        // the upper 16 bits of a column's largest element
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            colmax[j] = max_u16x2(colmax[j], __byte_perm(__float_as_uint(v[i][2 * j]), __float_as_uint(v[i][2 * j + 1]), 0x7632) & 0x7fff7fffu);
         float m = 0.0f;
 #pragma unroll
         for (int j = 0; j < 8; j += 2) asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(v[i][j]), "f"(v[i][j + 1]));
@@ -158,13 +170,28 @@ __global__ void __launch_bounds__(256) split_x2_k(const Images im, float *__rest
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) asm("max.NaN.f32 %0, %0, %1;" : "+f"(most) : "f"(__shfl_xor_sync(0xffffffffu, most, o)));
+#pragma unroll
+    for (int o = 16; o >= UPR; o >>= 1)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) colmax[j] = max_u16x2(colmax[j], __shfl_xor_sync(0xffffffffu, colmax[j], o));
+    if ((threadIdx.x & 31) < UPR) *reinterpret_cast<uint4 *>(&columns[threadIdx.x >> 5][4 * (threadIdx.x & 31)]) = make_uint4(colmax[0], colmax[1], colmax[2], colmax[3]);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = most;
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < 8; ++i) asm("max.NaN.f32 %0, %0, %1;" : "+f"(most) : "f"(red[i]));
     bad = bad || (most != 0.0f && !(most >= LEAST && most < MOST));
+    // Rows and columns of the block against its largest element: products sum along both, and hold 2^-31 of a row's or column's largest
+    // element where that is 2^-20 of the block's.
+    const float low_end = 9.5367432e-7f * most;
 #pragma unroll
-    for (int i = 0; i < ITEMS; ++i) bad = bad || (rowmax[i] != 0.0f && rowmax[i] < 9.5367432e-7f * most);
+    for (int i = 0; i < ITEMS; ++i) bad = bad || (rowmax[i] != 0.0f && rowmax[i] < low_end);
+    if (threadIdx.x < 4 * UPR) {
+        uint32_t m = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) m = max_u16x2(m, columns[i][threadIdx.x]);
+        const uint32_t least = __float_as_uint(low_end) >> 16, x = m & 0xffffu, y = m >> 16;
+        bad = bad || (x && x < least) || (y && y < least);
+    }
     if (dmax > 0.0f) atomicMax(&dred, __float_as_int(dmax));             // (not negative: ordered as whole numbers are)
     bad = __syncthreads_or(bad);
     const bool usable = most >= LEAST && most < MOST;

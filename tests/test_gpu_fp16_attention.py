@@ -183,3 +183,17 @@ def test_lse_far_below_the_scores(bmb, cuda, hs, shift):
         fin = cuda.isfinite(want[r])
         if bool(fin.any()):
             assert relative(got[r][fin], want[r][fin]) <= BOUND + 4 * 2.0 ** -24 * (abs(shift) + 12), r
+
+
+@pytest.mark.parametrize("hs", [32, 64, 128])
+@pytest.mark.parametrize("which,e", [(w, e) for w in range(4) for e in (-16, -28, -40)])
+def test_a_small_column(bmb, cuda, hs, which, e):
+    """One column of a head's q, k, v or dO is 2^e of the others: out, dv, dk and dq are sums per column."""
+    B, T, NH = 1, 640, 2
+    C = NH * hs
+    qkv, dout = inputs(cuda, B, T, NH, hs, hs)
+    x = dout if which == 3 else qkv[..., which * C:(which + 1) * C]
+    x[..., hs + 5] *= 2.0 ** e
+    col = (0, 1, slice(None), 5)
+    parts = {0: [(DK, col)], 1: [(DQ, col)], 2: [(OUT, col)], 3: [(DV, col)]}[which]
+    no_worse(cuda, bmb, qkv, dout, NH, parts + [(r, (0, h, slice(None))) for r in range(5) for h in (0, 1)])
