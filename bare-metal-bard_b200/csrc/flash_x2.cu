@@ -18,7 +18,7 @@
 //
 // What two pieces cannot serve is left to the kernels of flash.cu, which run behind these and skip every head that has none of
 // it: 64 rows whose largest element is not in 2^-45 .. 2^30 (nor zero) or not finite, a row or column whose largest element is below
-// 2^-20 of that (and not zero), D beyond 2^70, lse beyond 2^19, a row's largest score beyond 2^22 (MOST_SCORE), a probability beyond
+// 2^-20 of that (and not zero; of V and dO in the backward, a row below 2^-12), D beyond 2^70, lse beyond 2^19, a row's largest score beyond 2^22 (MOST_SCORE), a probability beyond
 // sqrt(2) (of an lse that is not the scores').  Inside these limits no sum can overflow.
 //
 // Bound by what a step of 64 columns waits for in turn (products, exponentials and splits, sums) and by the FMA pipe, on which
@@ -52,6 +52,7 @@ constexpr double CUT = 2.17e-8;                    // of a sum, cut off by an in
 // Of a row's largest score, times log2(e): the reference of its exponentials is that score rounded to fp32, and what the rounding
 // leaves (at most 1/4 here; 8 at 2^27) is part of the exponents, which have room for 1/2.
 constexpr float MOST_SCORE = 4194304.0f - 8.0f;     // (of the reference, which the score may pass by 6)
+constexpr float TINY = 7.5231638e-37f;             // 2^-120: dS is scaled by no more than its inverse
 constexpr float WINDOW = 113.0f;                   // exponents of probabilities are followed to 2^-113
 // What scores and lse are both multiplied with: a row whose weight lies on one key has lse = its score, bit for bit, and that
 // key the probability 1, although neither may be rounded little at its size.
@@ -79,7 +80,9 @@ struct Images {
     uint8_t *flags;                // [BH][which][nblk]: a block that two pieces cannot serve
     // Backward, [BH][nblk][3][64]: of every query minus the rest of lse log2(e) (past the end: - infinity), its whole part - WINDOW, and D
     float *rows;
-    float *dtop;                   // [BH][nblk]: a power of two, no less than any |D| of the block
+    // Backward, powers of two (or zero), no less than any element of what they stand for:
+    float4 *tops;                  // [BH][nblk]: V, dO, and D of the block
+    uint8_t *ptops;                // [BH][nblk][3][64], as codes: of a row of V, of a row of dO, of its D
 };
 
 // x + xe, y + ye (xe, ye: what fp32 does not hold of them)
@@ -96,6 +99,9 @@ __device__ __forceinline__ uint32_t max_u16x2(uint32_t a, uint32_t b) {
     asm("max.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
     return r;
 }
+// The least power of two above |x| (at most 2^127), or zero, and its code: the exponent's bits.
+__device__ __forceinline__ uint32_t top_code(float x) { return x == 0.0f ? 0u : min((__float_as_uint(x) >> 23 & 255) + 1, 254u); }
+__device__ __forceinline__ float top_of(uint32_t code) { return __uint_as_float(code << 23); }
 
 // One block: 64 positions of one head of q, k, v or dO; bound by memory (4 bytes read and 4 written an element).  With dO also
 // D = rowsum(dO O).
@@ -114,6 +120,7 @@ __global__ void __launch_bounds__(256, HS == 32 ? 5 : HS == 64 ? 4 : 2) split_x2
     const long long ld = which < 3 ? 3LL * C : C;
     const float *src = (which < 3 ? qkv + which * C : dout) + ((long long)b * T + blk * XB) * ld + h * HS;
     float v[ITEMS][8], rest[ITEMS][8], rowmax[ITEMS], most = 0.0f, dmax = 0.0f;      // rest: of q only
+    uint8_t *ptops = im.ptops + ((long long)bh * nblk + blk) * (3 * XB);
     uint32_t colmax[4] = {0u, 0u, 0u, 0u};
     bool bad = false;
 #pragma unroll
@@ -157,6 +164,7 @@ __global__ void __launch_bounds__(256, HS == 32 ? 5 : HS == 64 ? 4 : 2) split_x2
                     bad = bad || !(fabsf(a) <= 1.1805916e21f) || !(fabsf(L) <= 524288.0f);
                 }
                 dmax = fmaxf(dmax, fabsf(a));
+                ptops[2 * XB + r] = (uint8_t)top_code(a);
                 im.rows[to + 2 * XB] = fmaf(a, -fac.dp, a);
                 const float w = rintf(L * LOG2E);
                 im.rows[to + XB] = (pos < T ? w : 0.0f) - WINDOW;
@@ -166,6 +174,7 @@ __global__ void __launch_bounds__(256, HS == 32 ? 5 : HS == 64 ? 4 : 2) split_x2
 #pragma unroll
         for (int o = UPR / 2; o > 0; o >>= 1) asm("max.NaN.f32 %0, %0, %1;" : "+f"(m) : "f"(__shfl_xor_sync(0xffffffffu, m, o)));
         rowmax[i] = m;
+        if (nw == 4 && which >= 2 && c == 0) ptops[(which - 2) * XB + r] = (uint8_t)top_code(m);
         asm("max.NaN.f32 %0, %0, %1;" : "+f"(most) : "f"(m));
     }
 #pragma unroll
@@ -182,9 +191,11 @@ __global__ void __launch_bounds__(256, HS == 32 ? 5 : HS == 64 ? 4 : 2) split_x2
     bad = bad || (most != 0.0f && !(most >= LEAST && most < MOST));
     // Rows and columns of the block against its largest element: products sum along both, and hold 2^-31 of a row's or column's largest
     // element where that is 2^-20 of the block's.
-    const float low_end = 9.5367432e-7f * most;
+    // (In V and dO of a backward rows from 2^-12 on: dS of a block's 64 columns has one scale, so what belongs to a column's small
+    // row loses bits where the columns of large ones have hardly any weight.)
+    const float low_end = 9.5367432e-7f * most, low_row = nw == 4 && which >= 2 ? 2.44140625e-4f * most : low_end;
 #pragma unroll
-    for (int i = 0; i < ITEMS; ++i) bad = bad || (rowmax[i] != 0.0f && rowmax[i] < low_end);
+    for (int i = 0; i < ITEMS; ++i) bad = bad || (rowmax[i] != 0.0f && rowmax[i] < low_row);
     if (threadIdx.x < 4 * UPR) {
         uint32_t m = 0;
 #pragma unroll
@@ -216,7 +227,8 @@ __global__ void __launch_bounds__(256, HS == 32 ? 5 : HS == 64 ? 4 : 2) split_x2
         // A block of zeros in V or dO has no size of its own: what dS is scaled by (bwd_x2's bound) is then D's.
         im.unscale[((long long)which * BH + bh) * nblk + blk] = which >= 2 && most == 0.0f ? 0.0f : pow2(e - 14);
         im.flags[((long long)bh * nw + which) * nblk + blk] = bad;
-        if (which == 3) im.dtop[(long long)bh * nblk + blk] = pow2(min(max(exponent(__int_as_float(dred)) + 1, -120), 100));
+        if (nw == 4 && which >= 2) reinterpret_cast<float *>(im.tops + (long long)bh * nblk + blk)[which - 2] = top_of(top_code(most));
+        if (which == 3) im.tops[(long long)bh * nblk + blk].z = fmaxf(top_of(top_code(__int_as_float(dred))), TINY);
     }
     let_successor_start();
 }
@@ -410,7 +422,7 @@ __device__ __forceinline__ void st8(uint32_t addr, const uint32_t (&v)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
                  ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
 }
-// 16 weights of this thread's row, at most 2^15, as pieces over the 16 columns at `addr`.  (Complete after tmem_wait_st().)
+// 16 weights of this thread's row, below 2^16, as pieces over the 16 columns at `addr`.  (Complete after tmem_wait_st().)
 __device__ __forceinline__ void put_weights(uint32_t addr, const f2 *p) {
     uint32_t hi[8], lo[8];
 #pragma unroll
@@ -738,7 +750,8 @@ template <int HS> struct Bwd {
     // Tensor memory: S and dP, two buffers of 64 columns each or, at 128 columns, one with the two halves of the head apart.
     static constexpr bool HALVES = HS == 128;
     static constexpr int BUFS = HALVES ? 1 : 2;
-    static constexpr int OFF_B1 = 2 * G::TILE, OFF_B2 = OFF_B1 + N1 * G::BLK, OFF_ROWS = OFF_B2 + N2 * G::BLK, OFF_BAR = OFF_ROWS + N2 * ROWS_BYTES;
+    static constexpr int OFF_B1 = 2 * G::TILE, OFF_B2 = OFF_B1 + N1 * G::BLK, OFF_ROWS = OFF_B2 + N2 * G::BLK, OFF_OWN = OFF_ROWS + N2 * ROWS_BYTES;
+    static constexpr int OFF_BAR = OFF_OWN + 128 * 4;      // (OFF_OWN: what a row's dS is scaled by in its own block)
     static constexpr int SMEM = OFF_BAR + 256;
     static_assert(N1 >= BUFS && N2 >= BUFS, "a step's blocks stay until its sums are done");
 };
@@ -896,13 +909,39 @@ __device__ __forceinline__ void bwd_x2(uint8_t *smem, float *__restrict__ dqkv, 
         // late: a probability beyond sqrt(2), of an lse that is not these scores'.  The queries' side looks, before exponents so far above 0
         // run over; the keys' side has the same pairs, and the head is computed again for both.
         bool ok = true, late = false;
-        // dS of a step is scaled so that it is at most 2^15 whatever the data: by 1 / (the largest that dP and D can be).
-        const float *top = im.dtop + head + (KV ? c0 : rb);
-        auto bound = [&](int e) { return fmaxf(__ldg(u2 + e) * ca2 * (1073741824.0f * HS), __ldg(top + (KV ? e : 0))); };
+        // dS of a row and a step is scaled so that it is at most 2^15.5 whatever the data: by 1 / (the largest that dP and D can be there, of
+        // the row itself and of the columns that it sees; not below 2^-60 of all columns', so that the others stay finite).
+        const float4 *tops = im.tops + head + c0;
+        const float dtop = KV ? 0.0f : fmaxf(top_of(top_code(drow)), TINY);
+        float own, *own_block = reinterpret_cast<float *>(smem + F::OFF_OWN) + row;
+        {
+            // largest of what a row sees in its own block: a queries' row V up to it, a keys' row dO and D from it on
+            const uint8_t *pt = im.ptops + (head + rb) * (3 * XB) + (KV ? XB : 0);
+            auto code = [&](int r) { return KV ? pt[r] | (uint32_t)pt[XB + r] << 16 : (uint32_t)pt[r]; };
+            const int hb = quad & 1;                         // the row's half of the block
+            uint32_t sees = code(hb * 32 + lane), other = hb != KV ? code((hb ^ 1) * 32 + lane) : 0u;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t next = KV ? __shfl_down_sync(0xffffffffu, sees, o) : __shfl_up_sync(0xffffffffu, sees, o);
+                if (KV ? lane + o < 32 : lane >= o) sees = max_u16x2(sees, next);
+                other = max_u16x2(other, __shfl_xor_sync(0xffffffffu, other, o));
+            }
+            sees = max_u16x2(sees, other);
+            const float4 b = im.tops[head + rb];
+            own = top_of(KV ? pt[(row & 63) - XB] : pt[(row & 63) + XB]) * HS;
+            const float of_row = KV ? TINY : dtop, all = KV ? fmaxf(own * b.y, b.z) : own * b.x;
+            // (four threads write what each of them reads)
+            *own_block = fmaxf(fmaxf(own * top_of(sees & 255u), KV ? top_of(sees >> 16) : 0.0f), fmaxf(of_row, all * 8.6736174e-19f));
+        }
+        auto bound = [&](int e) {
+            const float4 b = __ldg(tops + e);
+            return e == rb - c0 ? *own_block : KV ? fmaxf(own * b.y, b.z) : fmaxf(own * b.x, dtop);
+        };
         constexpr float DOWN = 6.103515625e-5f;              // 2^-14
-        auto take1 = [&](int e) {
+        float carried = 0.0f;
+        auto take1 = [&](int e, float bnd) {
             if (!ok || e < 0) return;
-            const float g = __ldg(u1 + e) * DOWN * bound(e);
+            const float g = __ldg(u1 + e) * (DOWN * bnd);
             if (!warp_wait(bar(DONE1 + (e & 1)), (uint32_t)(e >> 1 & 1), giveup)) { ok = false; return; }
             fence_after();
             drain<H>(tmem + COL_1 + lanes + (uint32_t)((warp >> 2) * H), acc1, g);
@@ -925,9 +964,10 @@ __device__ __forceinline__ void bwd_x2(uint8_t *smem, float *__restrict__ dqkv, 
         for (int e = w; e < n; e += 2) {
             // the sums of this warpgroup's last step, in order
             take2(e - 2);
-            take1(e - 2);
+            take1(e - 2, carried);
             if (!ok) break;
-            const float g = 1.0f / bound(e), cs = __ldg(u1 + e) * ca1, cp = __ldg(u2 + e) * ca2 * g;
+            carried = bound(e);
+            const float g = __uint_as_float(0x7f000000u - __float_as_uint(carried)), cs = __ldg(u1 + e) * ca1, cp = __ldg(u2 + e) * ca2 * g;
             const int col0 = (c0 + e) * XB + 32 * half;
             if (!warp_wait(bar(S_FULL + w), (uint32_t)(e >> 1 & 1), giveup) || !warp_wait(bar(DP_FULL + w), (uint32_t)(e >> 1 & 1), giveup)) { ok = false; break; }
             fence_after();
@@ -981,13 +1021,13 @@ __device__ __forceinline__ void bwd_x2(uint8_t *smem, float *__restrict__ dqkv, 
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(W_FULL + w));
             take2(e - 1);
-            take1(e - 1);
+            take1(e - 1, e > 0 ? bound(e - 1) : 0.0f);
         }
         // steps n - 2 and n - 1, as far as this warpgroup has not taken their sums
         const bool last = ((n - 1) & 1) == w;                // this warpgroup's own last step is n - 1 (and took n - 2)
-        if (!last) { take2(n - 2); take1(n - 2); }
+        if (!last) { take2(n - 2); if (n > 1) take1(n - 2, bound(n - 2)); }
         take2(n - 1);
-        take1(n - 1);
+        take1(n - 1, bound(n - 1));
         if (!KV && late && ri < T) im.flags[(long long)bh * 4 * nblk] = 1;
         if (ok) {
             // every product has retired: the tiles' memory is free
@@ -1036,7 +1076,7 @@ int prepare(const void *kernel, int bytes) {
     return done[key] = at.numRegs * THREADS >= REGS_COMPUTE * COMPUTE + REGS_OTHER * 128 ? BMB_OK : BMB_E_UNSUPPORTED;
 }
 
-struct Layout { size_t images, unscale, flags, rows, dtop, total; };
+struct Layout { size_t images, unscale, flags, rows, tops, ptops, total; };
 Layout layout(long long BH, int nblk, int HS, int nw) {
     auto up = [](size_t n) { return (n + 255) / 256 * 256; };
     const size_t blocks = (size_t)BH * nblk;
@@ -1045,8 +1085,9 @@ Layout layout(long long BH, int nblk, int HS, int nw) {
     L.unscale = up(blocks * nw * 4);
     L.flags = up(blocks * nw);
     L.rows = nw == 4 ? up(blocks * ROWS_BYTES) : 0;
-    L.dtop = nw == 4 ? up(blocks * 4) : 0;
-    L.total = L.images + L.unscale + L.flags + L.rows + L.dtop;
+    L.tops = nw == 4 ? up(blocks * sizeof(float4)) : 0;
+    L.ptops = nw == 4 ? up(blocks * 3 * XB) : 0;
+    L.total = L.images + L.unscale + L.flags + L.rows + L.tops + L.ptops;
     return L;
 }
 constexpr size_t KEPT = 1ull << 30;                 // a larger block is given back by the call that took it (unless a trainer keeps it)
@@ -1089,7 +1130,8 @@ int run_x2(const Call &a, bool in_trainer, cudaStream_t st) {
     im.unscale = (float *)(scr + L.images);
     im.flags = scr + L.images + L.unscale;
     im.rows = (float *)(im.flags + L.flags);
-    im.dtop = (float *)(im.flags + L.flags + L.rows);
+    im.tops = (float4 *)(im.flags + L.flags + L.rows);
+    im.ptops = im.flags + L.flags + L.rows + L.tops;
     const double cut = (HS == 32 ? 2 : 4) * CUT, sums = 4 * CUT, q = a.scale * (1.0 + cut);      // products in a row
     Factors fac;
     fac.q = (float)q;

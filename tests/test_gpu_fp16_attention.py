@@ -197,3 +197,34 @@ def test_a_small_column(bmb, cuda, hs, which, e):
     col = (0, 1, slice(None), 5)
     parts = {0: [(DK, col)], 1: [(DQ, col)], 2: [(OUT, col)], 3: [(DV, col)]}[which]
     no_worse(cuda, bmb, qkv, dout, NH, parts + [(r, (0, h, slice(None))) for r in range(5) for h in (0, 1)])
+
+
+@pytest.mark.parametrize("hs", [32, 64, 128])
+@pytest.mark.parametrize("e", [11, 13, 19])
+def test_rows_beside_large_ones(bmb, cuda, hs, e):
+    """A row of V or dO 2^e times the others, which the queries before it or the keys behind it do not see, and one 2^-e of the others."""
+    B, T, NH, all_ = 1, 640, 2, slice(None)
+    C = NH * hs
+    for which, at, size, rows in ((2, 150, e, [(DQ, slice(128, 150)), (OUT, slice(128, 150))]), (3, 600, e, [(DK, slice(601, T)), (DV, slice(601, T))]),
+                                  (2, 150, -e, [(DK, slice(150, 151))]), (3, 600, -e, [(DQ, slice(600, 601))]),
+                                  (3, T - 1, -e, [(DK, slice(T - 1, T)), (DV, slice(T - 1, T))])):
+        qkv, dout = inputs(cuda, B, T, NH, hs, hs)
+        (dout if which == 3 else qkv[..., 2 * C:])[0, at, hs:2 * hs] *= 2.0 ** size
+        no_worse(cuda, bmb, qkv, dout, NH, [(r, (0, 1, x)) for r, x in rows] + [(r, (0, h, all_)) for r in range(5) for h in (0, 1)])
+
+
+@pytest.mark.parametrize("hs", [32, 64, 128])
+def test_rows_of_zeros(bmb, cuda, hs):
+    """Keys whose V and queries whose dO is zero, to the left and right of a block's edge, and all that a row of the block sees."""
+    B, T, NH, all_ = 1, 640, 2, slice(None)
+    C = NH * hs
+    qkv, dout = inputs(cuda, B, T, NH, hs, hs)
+    qkv[0, :70, 2 * C + hs:2 * C + 2 * hs] = 0
+    qkv[0, 300, 2 * C:2 * C + hs] = 0
+    dout[0, 600:, hs:2 * hs] = 0
+    dout[0, 300, :hs] = 0
+    no_worse(cuda, bmb, qkv, dout, NH, [(r, (0, h, all_)) for r in range(5) for h in (0, 1)])
+    got = by_heads(cuda, attention(bmb, cuda, 0, qkv, dout, NH), NH)
+    assert all(bool(cuda.isfinite(x).all()) for x in got)
+    assert not got[OUT][0, 1, :70].any() and not got[DQ][0, 1, :70].any() and not got[DQ][0, 1, 600:].any()
+    assert not got[DK][0, 1, 600:].any() and not got[DV][0, 1, 600:].any() and not got[DQ][0, 0, 300].any()
