@@ -219,21 +219,22 @@ __host__ __device__ constexpr int ex_qkv(int C) { return 3 * C; }
 __host__ __device__ constexpr int ex_h(int C) { return 6 * C; }
 __host__ __device__ constexpr int ex_size(int C) { return 10 * C; }
 
+// (One 64-bit access a pair: the halves of a vector access are accesses of their own, in no order.)
 __device__ __forceinline__ void put_pair(uint2 *p, float v, unsigned tag) {
-    asm volatile("st.volatile.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(__float_as_uint(v)), "r"(tag) : "memory");
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"((unsigned long long)tag << 32 | __float_as_uint(v)) : "memory");
 }
 __device__ __forceinline__ bool get_pair(const uint2 *p, unsigned tag, float &v) {
-    uint32_t a, b;
-    asm volatile("ld.volatile.global.v2.u32 {%0, %1}, [%2];" : "=r"(a), "=r"(b) : "l"(p) : "memory");
-    v = __uint_as_float(a);
-    return b == tag;
+    unsigned long long a;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(a) : "l"(p) : "memory");
+    v = __uint_as_float((uint32_t)a);
+    return (uint32_t)(a >> 32) == tag;
 }
 __device__ __forceinline__ bool get_pairs4(const uint2 *p, unsigned tag, float4 &v) {
-    uint32_t a[8];
-    asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "l"(p) : "memory");
-    asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(a[4]), "=r"(a[5]), "=r"(a[6]), "=r"(a[7]) : "l"(p + 2) : "memory");
-    v = make_float4(__uint_as_float(a[0]), __uint_as_float(a[2]), __uint_as_float(a[4]), __uint_as_float(a[6]));
-    return a[1] == tag && a[3] == tag && a[5] == tag && a[7] == tag;
+    unsigned long long a[4];
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a[0]), "=l"(a[1]) : "l"(p) : "memory");
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a[2]), "=l"(a[3]) : "l"(p + 2) : "memory");
+    v = make_float4(__uint_as_float((uint32_t)a[0]), __uint_as_float((uint32_t)a[1]), __uint_as_float((uint32_t)a[2]), __uint_as_float((uint32_t)a[3]));
+    return (uint32_t)(a[0] >> 32) == tag && (uint32_t)(a[1] >> 32) == tag && (uint32_t)(a[2] >> 32) == tag && (uint32_t)(a[3] >> 32) == tag;
 }
 // Calls `look` until it is true for this thread; false when the limit ran out.
 template <typename Look>
