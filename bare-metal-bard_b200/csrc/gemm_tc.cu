@@ -1408,7 +1408,8 @@ int gemm_tc(int math, int flags, int transA, int transB, int batch, int M, int N
     if (b.map3d) BMB_TRY(make_map_mn3d(&mapB, b.ptr, b.rows, b.cols, b.pitch_bytes, b.tile_chunks));
     else BMB_TRY(make_map_2d(&mapB, b.ptr, esize, b.rows, b.cols, b.pitch_bytes, b.box_rows, b.mn_major));
     const int tiles_m = plan.tiles_m, tiles_n = plan.tiles_n;
-    const int vec_ok = ((uintptr_t)C % 16 == 0) && (N % 4 == 0);
+    // (the bias is read four at a time wherever C is written so)
+    const int vec_ok = (((uintptr_t)C | (uintptr_t)bias) % 16 == 0) && (N % 4 == 0);
     const int sk_tiles = plan.sk_tiles, g_sk = plan.g_sk, grid = plan.grid;
     if (sk_tiles > 0 && beta != 1.0f) {
         chain.first = true;        // (launched beside the copies it made 4096^3 16 us slower)

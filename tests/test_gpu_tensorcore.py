@@ -532,3 +532,23 @@ def test_pairs_taken_by_the_cost_model(bmb, cuda, math, ta, tb, M, N, K, beta):
         bmb.call("bmb_gemm_ex", bmb.MATH_TF32 if math == "tf32" else bmb.MATH_BF16, flags, ta, tb, M, N, K, 1.0, A, B, beta, C, None)
         cuda.cuda.synchronize()
         assert ((C.view(M, N).double() - want).norm() / want.norm()).item() < 2e-5, flags
+
+
+@pytest.mark.parametrize("math", ["tf32", "bf16"])
+@pytest.mark.parametrize("M,N,K", [(256, 256, 64), (512, 768, 2048), (8192, 768, 768), (300, 520, 96)])
+@pytest.mark.parametrize("offset", [1, 2])
+def test_bias_at_any_address(bmb, cuda, math, M, N, K, offset):
+    """A bias that is not 16-byte aligned (whole tiles, tiles shared along K, pairs): 2e-5 normwise from one that is, as for the other
+    tensor-core forms (the two may be cut along K differently)."""
+    g = cuda.Generator(device="cuda").manual_seed(3)
+    A, W = (cuda.rand(n, device="cuda", generator=g) * 2 - 1 for n in (M * K, N * K))
+    bias = cuda.rand(N, device="cuda", generator=g)
+    moved = cuda.empty(N + 4, device="cuda")[offset:offset + N]
+    moved.copy_(bias)
+    m = bmb.MATH_TF32 if math == "tf32" else bmb.MATH_BF16
+    (C, G), (C2, G2) = (tuple(cuda.full((M * N,), float("nan"), device="cuda") for _ in range(2)) for _ in range(2))
+    bmb.call("bmb_gemm_bias_gelu", m, 0, M, N, K, A, W, bias, C, G, None)
+    bmb.call("bmb_gemm_bias_gelu", m, 0, M, N, K, A, W, moved, C2, G2, None)
+    cuda.cuda.synchronize()
+    for x, y in ((C, C2), (G, G2)):
+        assert ((x - y).norm() / x.norm()).item() < 2e-5
