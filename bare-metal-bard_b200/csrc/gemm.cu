@@ -45,8 +45,8 @@ int gemm_any_bias(int math, int flags, int ta, int tb, int batch, int M, int N, 
         const bool bias_ok = !bias || (N % 4 == 0 && (((uintptr_t)bias | (uintptr_t)C) & 15) == 0);
         rc = (math == BMB_MATH_FP32 && batch == 1 && A && B && C && bias_ok && !(flags & GEMM_CHAIN)) ? gemm_x3(ta, tb, M, N, K, alpha, A, B, beta, C, bias, flags, st) : BMB_E_UNSUPPORTED;
         bool bias_done = rc == BMB_OK;
-        // what follows a product of few tiles rides with it
-        if (rc == BMB_E_UNSUPPORTED && (bias || aux_gelu) && bias_ok && !(flags & BMB_GEMM_C_ROUNDED) && batch == 1 && !ta && tb && A && B && C && M > 0 && N > 0 && K > 0) {
+        // what follows a product of few tiles rides with it (but for rounding passes, and a GELU in place)
+        if (rc == BMB_E_UNSUPPORTED && (bias || aux_gelu) && aux_gelu != C && !emit_rounded() && bias_ok && !(flags & BMB_GEMM_C_ROUNDED) && batch == 1 && !ta && tb && A && B && C && M > 0 && N > 0 && K > 0) {
             rc = gemm_simt_small(ta, tb, batch, M, N, K, alpha, A, sA, B, sB, beta, C, sC, bias, aux_gelu, st);
             bias_done = aux_done = rc == BMB_OK;
         }

@@ -73,7 +73,7 @@ template <int T, int N, bool KC>
 __device__ __forceinline__ int place(int t, int i) { return KC ? t + N * i : T % 4 == 0 ? (t + N * (i / 4)) * 4 + i % 4 : t * T + i; }
 
 // Behind the product, where FUSED: + bias (a row), and GELU of the result as a second output.
-struct Behind { const float *bias; float *gelu; int round_gelu; };
+struct Behind { const float *bias; float *gelu; };
 
 template <int BM, int BN, int TM, int TN, bool TA, bool TB, bool VEC, bool FUSED>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
@@ -162,10 +162,7 @@ gemm_simt_small_k(int M, int N, int K, float alpha, const float *__restrict__ A,
             if (beta != 0.0f) o = fmaf(beta, *c, o);
             if (FUSED && behind.bias) o = __fadd_rn(o, __ldg(behind.bias + n));
             *c = o;
-            if (FUSED && behind.gelu) {
-                const float g = gelu_tanh(o);
-                behind.gelu[(size_t)m * N + n] = behind.round_gelu ? round_tf32(g) : g;
-            }
+            if (FUSED && behind.gelu) behind.gelu[(size_t)m * N + n] = gelu_tanh(o);
         }
     }
 }
@@ -203,7 +200,7 @@ int pick_small(int bm, int bn, int batch, int M, int N, int K, float alpha, cons
 }  // namespace
 
 // BMB_E_UNSUPPORTED: the product has tiles enough for the 128 x 128 kernels. bias, gelu (may be null; op(A) = A, op(B) = B^T only):
-// as bmb_bias_forward and bmb_gelu_forward behind it, to the bit.
+// as bmb_bias_forward and bmb_gelu_forward behind it, to the bit, where those do not round (emit_rounded).
 int gemm_simt_small(int transA, int transB, int batch, int M, int N, int K, float alpha, const float *A, long long sA, const float *B,
                     long long sB, float beta, float *C, long long sC, const float *bias, float *gelu, cudaStream_t st) {
     // Cycles per k of the SM with the most tiles: what one tile takes by itself, and each where there are several (measured, B with
@@ -221,7 +218,7 @@ int gemm_simt_small(int transA, int transB, int batch, int M, int N, int K, floa
     if (ceil_div(M, bm) > 65535 || batch > 65535) return BMB_E_UNSUPPORTED;
     const bool vec = (((uintptr_t)A | (uintptr_t)B) & 15) == 0 && (transA ? M : K) % 4 == 0 && (transB ? K : N) % 4 == 0 &&
                      sA % 4 == 0 && sB % 4 == 0;
-    const Behind behind{bias, gelu, emit_rounded() ? 1 : 0};
+    const Behind behind{bias, gelu};
     if (bias || gelu) {
         if (transA || !transB || batch != 1) return BMB_E_UNSUPPORTED;
         return vec ? pick_small<false, true, true, true>(bm, bn, batch, M, N, K, alpha, A, sA, B, sB, beta, C, sC, behind, st)

@@ -39,3 +39,23 @@ def test_bias_and_gelu_ride_with_the_product(bmb, cuda, M, N, K):
     bmb.call("bmb_gemm_bias_gelu", bmb.MATH_FP32, 0, M, N, K, A, W, bias, got, gelu, None)
     cuda.cuda.synchronize()
     assert cuda.equal(got, want) and cuda.equal(gelu, want_gelu)
+
+
+@pytest.mark.parametrize("M,N,K", [(70, 132, 33), (33, 64, 97), (1, 4, 1), (130, 68, 40)])
+@pytest.mark.parametrize("rounded,in_place", [(True, False), (False, True), (True, True)])
+def test_rounded_and_in_place(bmb, cuda, M, N, K, rounded, in_place):
+    """The passes behind a product round what they store where the activation is asked for rounded, the sum with the bias included, and
+    the activation may take the product's place."""
+    A, W, bias = (cuda.from_numpy(uniform(n, i)).cuda() for i, n in enumerate((M * K, N * K, N)))
+    want, want_gelu, got = (cuda.full((M * N,), float("nan"), device="cuda") for _ in range(3))
+    gelu = got if in_place else cuda.full((M * N,), float("nan"), device="cuda")
+    bmb.call("bmb_gemm_ex", bmb.MATH_FP32, 0, 0, 1, M, N, K, 1.0, A, W, 0.0, want, None)
+    bmb.call("bmb_bias_forward", want, bias, M, N)
+    if rounded:
+        bmb.call("bmb_round_tf32", want, want, M * N, None)
+    bmb.call("bmb_gelu_forward", want_gelu, want, M * N)
+    if rounded:
+        bmb.call("bmb_round_tf32", want_gelu, want_gelu, M * N, None)
+    bmb.call("bmb_gemm_bias_gelu", bmb.MATH_FP32, bmb.GEMM_AUX_ROUNDED if rounded else 0, M, N, K, A, W, bias, got, gelu, None)
+    cuda.cuda.synchronize()
+    assert cuda.equal(gelu, want_gelu) and (in_place or cuda.equal(got, want))
