@@ -147,6 +147,10 @@ int flash_forward(int cfg, int flags, float *out, float *lse, const float *qkv, 
 int flash_backward(int cfg, int flags, float *dqkv, float *dsum, const float *dout, const float *qkv, const float *out, const float *lse,
                    int B, int T, int C, int NH, bool in_trainer);
 
+// Heads that the attention of flash_x2.cu leaves to the kernels behind it: a byte each of `heads`, and how many pieces of their work are taken
+// (zero before the launch).
+struct LeftOut { uint8_t *flagged; int *taken, heads; };
+
 // A model as decode_position reads it: its tensors (layer-stacked, as the trainer keeps them), the keys and values so far (rows
 // of 3C), the pairs that activations are handed on in, and the logits.
 struct DecodeModel {

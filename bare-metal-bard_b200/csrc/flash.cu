@@ -175,11 +175,36 @@ __device__ __noinline__ void fwd_rows_again(float *smem, float *out, float *lse,
     for (int r = 0; r < nrows; r += R) fwd_rows<HS, 16, NT>(smem, out, lse, qkv, T, NH, scale, bh, i0 + r, min(R, nrows - r));
 }
 
-// Whether head blockIdx.x has one of its nflags bytes set (flash_x2.cu leaves such heads to these kernels).
-__device__ __forceinline__ bool head_flagged(const uint8_t *flags, int nflags) {
-    bool f = false;
-    for (int i = threadIdx.x; i < nflags; i += blockDim.x) f = f || flags[(long long)blockIdx.x * nflags + i];
-    return __syncthreads_or(f);
+// The items (`each` a head) of the heads that flash_x2.cu leaves to these kernels (none as a rule, or one, or all): body(head, item), its
+// shared memory free.  Blocks take them as they come free, the first item of every head before any second one (1024 heads at a time).
+template <typename Body>
+__device__ __forceinline__ void for_left_out(const LeftOut &left, int each, Body body) {
+    __shared__ uint16_t list[1024];
+    __shared__ int count;
+    __shared__ long long next;
+    long long item = blockIdx.x, first = 0;                        // this block's; the first of these heads
+    for (int h0 = 0; h0 < left.heads; h0 += 1024) {
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            int n = 0;
+            for (int i = threadIdx.x; i < 1024 && h0 + i - (int)threadIdx.x < left.heads; i += 32) {
+                const bool f = h0 + i < left.heads && left.flagged[h0 + i];
+                const uint32_t word = __ballot_sync(0xffffffffu, f);
+                if (f) list[n + __popc(word & ((1u << threadIdx.x) - 1u))] = (uint16_t)i;
+                n += __popc(word);
+            }
+            if (threadIdx.x == 0) count = n;
+        }
+        __syncthreads();
+        const int heads = count;
+        for (; item < first + (long long)heads * each; item = next) {
+            const int i = (int)(item - first);                     // (at most 1024 heads of 65535 items)
+            body(h0 + list[i % heads], i / heads);
+            if (threadIdx.x == 0) next = (long long)gridDim.x + atomicAdd(left.taken, 1);
+            __syncthreads();
+        }
+        first += (long long)heads * each;
+    }
 }
 
 // How the products are split (flash_mma.cuh): scores and output, and sums of gradients.
@@ -197,10 +222,10 @@ __host__ __device__ constexpr fm::Form gradient_form(bool fine) { return fine ? 
 // 2.7e-7 -> 1.7e-7, 3.5e-7 -> 1.8e-7, 2.5e-7 -> 1.6e-7, 1.2e-7 -> 0.9e-7.
 template <int HS, bool FINE>
 __device__ __forceinline__ void fwd_mma(float *__restrict__ smem, float *__restrict__ out, float *__restrict__ lse, const float *__restrict__ qkv,
-                                        int T, int NH, float scale, int i0) {
+                                        int T, int NH, float scale, int bh, int i0) {
     float *Qs = smem, *Ks = Qs + 64 * HS, *Vs = Ks + 2 * 32 * HS;      // Ks, Vs: two buffers each
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int bh = blockIdx.x, b = bh / NH, h = bh % NH;
+    const int b = bh / NH, h = bh % NH;
     const int C = NH * HS;
     const long long ld = 3LL * C;
     const float *base = qkv + (long long)b * T * ld + h * HS;
@@ -281,18 +306,21 @@ __device__ __forceinline__ void fwd_mma(float *__restrict__ smem, float *__restr
     bad = fm::store_rows<HS>(out + ((long long)b * T + row0) * C + h * HS, C, g, T - row0, o, inv[0], inv[1]) || bad;
     if (__syncthreads_or(bad)) fwd_rows_again<HS, 128>(smem, out, lse, qkv, T, NH, scale, bh, i0, 64);
 }
-// `blocks` blocks of rows a head, the longest first; a grid that is lower walks them.
+// Blocks of 64 rows, a head's longest first: of every head (grid: heads x blocks) ...
 template <int HS, bool FINE>
 __global__ void __launch_bounds__(128, HS == 32 ? 3 : 2)
-flash_fwd_mma_k(float *__restrict__ out, float *__restrict__ lse, const float *__restrict__ qkv, int T, int NH, float scale,
-                const uint8_t *__restrict__ flags, int nflags, int blocks) {
+flash_fwd_mma_k(float *__restrict__ out, float *__restrict__ lse, const float *__restrict__ qkv, int T, int NH, float scale) {
     extern __shared__ __align__(16) float smem[];
-    if (flags) wait_for_predecessor();
-    if (flags && !head_flagged(flags, nflags)) return;
-    for (int y = blockIdx.y; y < blocks; y += gridDim.y) {
-        if (y != (int)blockIdx.y) __syncthreads();             // the rows before have been read
-        fwd_mma<HS, FINE>(smem, out, lse, qkv, T, NH, scale, (blocks - 1 - y) * 64);
-    }
+    fwd_mma<HS, FINE>(smem, out, lse, qkv, T, NH, scale, blockIdx.x, ((int)gridDim.y - 1 - (int)blockIdx.y) * 64);
+}
+// ... or of those left out.
+template <int HS>
+__global__ void __launch_bounds__(128, HS == 32 ? 3 : 2)
+flash_fwd_left_k(float *__restrict__ out, float *__restrict__ lse, const float *__restrict__ qkv, int T, int NH, float scale, LeftOut left) {
+    extern __shared__ __align__(16) float smem[];
+    wait_for_predecessor();
+    const int blocks = (T + 63) / 64;
+    for_left_out(left, blocks, [&](int bh, int y) { fwd_mma<HS, false>(smem, out, lse, qkv, T, NH, scale, bh, (blocks - 1 - y) * 64); });
 }
 
 // ----------------------------------------------------------------- backward
@@ -548,6 +576,7 @@ __device__ __noinline__ void bwd_kv_rows_again(float *smem, float *dqkv, const f
 // Backward on warp-level tensor-core instructions: blocks of 16 rows a warp (4 warps; 8 at head size 128, where two
 // tiles of 64 rows would leave one block of 4 warps to an SM), 32 rows of the other side at a time in two buffers.
 template <int HS> struct bwd_warps { static constexpr int value = HS == 128 ? 8 : 4; };
+template <int HS> constexpr int fwd_smem() { return (64 + 4 * 32) * HS * 4; }
 template <int HS> constexpr int bwd_smem() { return (2 * bwd_warps<HS>::value * 16 * HS + 4 * 32 * HS + 4 * 32) * 4; }
 
 // dQ = scale * sum over keys of dS K, dS = P (dO V^T - D), P = exp(scale Q K^T - lse).
@@ -685,19 +714,28 @@ __device__ __forceinline__ void bwd_kv_mma(float *__restrict__ smem, float *__re
 // Measured with D, row-group kernels -> this: B8 T1024 12 heads of 64 2436 -> 960 us, B4 T2048 8 x 128 18754 -> 2501,
 // B2 T777 12 x 32 445 -> 105.  2-norm errors of dq / dk / dv against 64 bits at 8 x 128: 4.9 / 10.8 / 10.8e-7 -> 3.2 / 3.7 / 3.3e-7.
 template <int HS, bool FINE>
+__device__ __forceinline__ void bwd_mma(float *__restrict__ smem, float *__restrict__ dqkv, const float *__restrict__ qkv, const float *__restrict__ dout,
+                                        const float *__restrict__ lse, const float *__restrict__ dsum, int T, int NH, float scale, int bh, int y, int blocks) {
+    constexpr int ROWS = bwd_warps<HS>::value * 16;
+    if (y & 1) bwd_q_mma<HS, FINE>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, bh, (blocks - 1 - (y >> 1)) * ROWS);
+    else bwd_kv_mma<HS, FINE>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, bh, (y >> 1) * ROWS);
+}
+template <int HS, bool FINE>
 __global__ void __launch_bounds__(bwd_warps<HS>::value * 32, HS == 128 ? 1 : HS == 64 ? 2 : 3)
 flash_bwd_mma_k(float *__restrict__ dqkv, const float *__restrict__ qkv, const float *__restrict__ dout,
-                const float *__restrict__ lse, const float *__restrict__ dsum, int T, int NH, float scale,
-                const uint8_t *__restrict__ flags, int nflags, int blocks) {
+                const float *__restrict__ lse, const float *__restrict__ dsum, int T, int NH, float scale) {
     extern __shared__ __align__(16) float smem[];
-    if (flags) wait_for_predecessor();
-    if (flags && !head_flagged(flags, nflags)) return;
+    bwd_mma<HS, FINE>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, blockIdx.x, blockIdx.y, gridDim.y >> 1);
+}
+template <int HS>
+__global__ void __launch_bounds__(bwd_warps<HS>::value * 32, HS == 128 ? 1 : HS == 64 ? 2 : 3)
+flash_bwd_left_k(float *__restrict__ dqkv, const float *__restrict__ qkv, const float *__restrict__ dout,
+                 const float *__restrict__ lse, const float *__restrict__ dsum, int T, int NH, float scale, LeftOut left) {
+    extern __shared__ __align__(16) float smem[];
+    wait_for_predecessor();
     constexpr int ROWS = bwd_warps<HS>::value * 16;
-    for (int y = blockIdx.y; y < 2 * blocks; y += gridDim.y) {
-        if (y != (int)blockIdx.y) __syncthreads();             // the rows before have been read
-        if (y & 1) bwd_q_mma<HS, FINE>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, blockIdx.x, (blocks - 1 - (y >> 1)) * ROWS);
-        else bwd_kv_mma<HS, FINE>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, blockIdx.x, (y >> 1) * ROWS);
-    }
+    const int blocks = (T + ROWS - 1) / ROWS;
+    for_left_out(left, 2 * blocks, [&](int bh, int y) { bwd_mma<HS, false>(smem, dqkv, qkv, dout, lse, dsum, T, NH, scale, bh, y, blocks); });
 }
 
 struct FwdCfg { int kc; const char *name; };
@@ -743,36 +781,41 @@ int allow_smem(const void *kernel, int bytes) {
     return BMB_OK;
 }
 
-// With flags hardly a head has work: about two blocks an SM look at them.
-int grid_height(int blocks, int heads, const uint8_t *flags) {
-    return flags ? std::min(blocks, std::max(1, ceil_div(2 * sm_count(), heads))) : blocks;
-}
 template <int HS>
-int launch_fwd_mma(float *out, float *lse, const float *qkv, int B, int T, int NH, float scale, const uint8_t *flags, int nflags, cudaStream_t st) {
-    constexpr int SMEM = (64 + 4 * 32) * HS * 4;
+int launch_fwd_mma(float *out, float *lse, const float *qkv, int B, int T, int NH, float scale, cudaStream_t st) {
     const auto kernel = T <= FINE_T ? flash_fwd_mma_k<HS, true> : flash_fwd_mma_k<HS, false>;
-    BMB_TRY(allow_smem((const void *)kernel, SMEM));
-    const int blocks = ceil_div(T, 64);
-    const dim3 grid(B * NH, grid_height(blocks, B * NH, flags));
-    if (flags) return launch_in_chain(kernel, grid, 128, SMEM, st, out, lse, qkv, T, NH, scale, flags, nflags, blocks);
-    kernel<<<grid, 128, SMEM, st>>>(out, lse, qkv, T, NH, scale, flags, nflags, blocks);
+    BMB_TRY(allow_smem((const void *)kernel, fwd_smem<HS>()));
+    kernel<<<dim3(B * NH, ceil_div(T, 64)), 128, fwd_smem<HS>(), st>>>(out, lse, qkv, T, NH, scale);
     count_launch();
     BMB_LAUNCH_CHECK();
     return BMB_OK;
 }
 template <int HS>
 int launch_bwd_mma(float *dqkv, const float *dsum, const float *dout, const float *qkv, const float *lse, int B, int T, int NH, float scale,
-                   const uint8_t *flags, int nflags, cudaStream_t st) {
+                   cudaStream_t st) {
     constexpr int ROWS = bwd_warps<HS>::value * 16;
     const auto kernel = T <= FINE_T ? flash_bwd_mma_k<HS, true> : flash_bwd_mma_k<HS, false>;
     BMB_TRY(allow_smem((const void *)kernel, bwd_smem<HS>()));
-    const int blocks = ceil_div(T, ROWS), threads = bwd_warps<HS>::value * 32;
-    const dim3 grid(B * NH, grid_height(2 * blocks, B * NH, flags));
-    if (flags) return launch_in_chain(kernel, grid, threads, bwd_smem<HS>(), st, dqkv, qkv, dout, lse, dsum, T, NH, scale, flags, nflags, blocks);
-    kernel<<<grid, threads, bwd_smem<HS>(), st>>>(dqkv, qkv, dout, lse, dsum, T, NH, scale, flags, nflags, blocks);
+    kernel<<<dim3(B * NH, 2 * ceil_div(T, ROWS)), bwd_warps<HS>::value * 32, bwd_smem<HS>(), st>>>(dqkv, qkv, dout, lse, dsum, T, NH, scale);
     count_launch();
     BMB_LAUNCH_CHECK();
     return BMB_OK;
+}
+// Two blocks an SM, which is what runs side by side of most of these kernels.
+int left_grid(long long items) { return (int)std::min<long long>(items, 2 * sm_count()); }
+template <int HS>
+int launch_fwd_left(float *out, float *lse, const float *qkv, int T, int NH, float scale, LeftOut left, cudaStream_t st) {
+    BMB_TRY(allow_smem((const void *)flash_fwd_left_k<HS>, fwd_smem<HS>()));
+    return launch_in_chain(flash_fwd_left_k<HS>, left_grid((long long)left.heads * ceil_div(T, 64)), 128, fwd_smem<HS>(), st, out, lse, qkv, T, NH, scale,
+                           left);
+}
+template <int HS>
+int launch_bwd_left(float *dqkv, const float *dsum, const float *dout, const float *qkv, const float *lse, int T, int NH, float scale,
+                    LeftOut left, cudaStream_t st) {
+    constexpr int ROWS = bwd_warps<HS>::value * 16;
+    BMB_TRY(allow_smem((const void *)flash_bwd_left_k<HS>, bwd_smem<HS>()));
+    return launch_in_chain(flash_bwd_left_k<HS>, left_grid(2LL * left.heads * ceil_div(T, ROWS)), bwd_warps<HS>::value * 32, bwd_smem<HS>(), st,
+                           dqkv, qkv, dout, lse, dsum, T, NH, scale, left);
 }
 
 template <int HS>
@@ -784,7 +827,7 @@ int run_fwd(int cfg, float *out, float *lse, const float *qkv, int B, int T, int
             const int rc = flash_forward_x2(out, lse, qkv, B, T, NH, HS, scale, in_trainer, st);
             if (rc != BMB_E_UNSUPPORTED) return rc;
         }
-        return launch_fwd_mma<HS>(out, lse, qkv, B, T, NH, scale, nullptr, 0, st);
+        return launch_fwd_mma<HS>(out, lse, qkv, B, T, NH, scale, st);
     } else {
         constexpr int R = FT / (HS / 32);
         dim3 grid(ceil_div(T, R), B * NH);
@@ -810,7 +853,7 @@ int run_bwd(int cfg, float *dqkv, float *dsum, const float *dout, const float *q
             if (rc != BMB_E_UNSUPPORTED) return rc;
         }
         BMB_TRY(launch_flash_dsum(dsum, dout, out, B, T, NH, HS, st));
-        return launch_bwd_mma<HS>(dqkv, dsum, dout, qkv, lse, B, T, NH, scale, nullptr, 0, st);
+        return launch_bwd_mma<HS>(dqkv, dsum, dout, qkv, lse, B, T, NH, scale, st);
     }
     constexpr int R = FT / (HS / 32);
     const long long rows = (long long)B * NH * T;
@@ -825,14 +868,15 @@ int run_bwd(int cfg, float *dqkv, float *dsum, const float *dout, const float *q
 
 }  // namespace
 
-int flash_fwd_mma(int hs, float *out, float *lse, const float *qkv, int B, int T, int NH, float scale, const uint8_t *flags, int nflags, cudaStream_t st) {
-    const auto run = hs == 32 ? launch_fwd_mma<32> : hs == 64 ? launch_fwd_mma<64> : launch_fwd_mma<128>;
-    return run(out, lse, qkv, B, T, NH, scale, flags, nflags, st);
+// Behind flash_x2.cu (T > FINE_T), for the heads that it leaves out.
+int flash_fwd_left(int hs, float *out, float *lse, const float *qkv, int T, int NH, float scale, LeftOut left, cudaStream_t st) {
+    const auto run = hs == 32 ? launch_fwd_left<32> : hs == 64 ? launch_fwd_left<64> : launch_fwd_left<128>;
+    return run(out, lse, qkv, T, NH, scale, left, st);
 }
-int flash_bwd_mma(int hs, float *dqkv, const float *dsum, const float *dout, const float *qkv, const float *lse, int B, int T, int NH, float scale,
-                  const uint8_t *flags, int nflags, cudaStream_t st) {
-    const auto run = hs == 32 ? launch_bwd_mma<32> : hs == 64 ? launch_bwd_mma<64> : launch_bwd_mma<128>;
-    return run(dqkv, dsum, dout, qkv, lse, B, T, NH, scale, flags, nflags, st);
+int flash_bwd_left(int hs, float *dqkv, const float *dsum, const float *dout, const float *qkv, const float *lse, int T, int NH, float scale,
+                   LeftOut left, cudaStream_t st) {
+    const auto run = hs == 32 ? launch_bwd_left<32> : hs == 64 ? launch_bwd_left<64> : launch_bwd_left<128>;
+    return run(dqkv, dsum, dout, qkv, lse, T, NH, scale, left, st);
 }
 
 int launch_flash_dsum(float *dsum, const float *dout, const float *out, int B, int T, int NH, int HS, cudaStream_t st) {

@@ -34,10 +34,10 @@
 #include <mutex>
 
 namespace bmb {
-// flash.cu: the kernels on warp-level instructions; with `flags` (nflags bytes a head) only for the heads that have one set.
-int flash_fwd_mma(int hs, float *out, float *lse, const float *qkv, int B, int T, int NH, float scale, const uint8_t *flags, int nflags, cudaStream_t st);
-int flash_bwd_mma(int hs, float *dqkv, const float *dsum, const float *dout, const float *qkv, const float *lse, int B, int T, int NH, float scale,
-                  const uint8_t *flags, int nflags, cudaStream_t st);
+// flash.cu: the kernels on warp-level instructions, for the heads left out here.
+int flash_fwd_left(int hs, float *out, float *lse, const float *qkv, int T, int NH, float scale, LeftOut left, cudaStream_t st);
+int flash_bwd_left(int hs, float *dqkv, const float *dsum, const float *dout, const float *qkv, const float *lse, int T, int NH, float scale,
+                      LeftOut left, cudaStream_t st);
 namespace {
 
 using namespace tc;
@@ -78,6 +78,7 @@ struct Images {
     uint8_t *img;                  // [which: q, k, v, dO][BH][nblk][BLK]
     float *unscale;                // [which][BH][nblk]: what an image's values are multiplied with
     uint8_t *flags;                // [BH][which][nblk]: a block that two pieces cannot serve
+    LeftOut left;                  // heads that these kernels leave to those of flash.cu
     // Backward, [BH][nblk][3][64]: of every query minus the rest of lse log2(e) (past the end: - infinity), its whole part - WINDOW, and D
     float *rows;
     // Backward, powers of two (or zero), no less than any element of what they stand for:
@@ -227,6 +228,8 @@ __global__ void __launch_bounds__(256, HS == 32 ? 5 : HS == 64 ? 4 : 2) split_x2
         // A block of zeros in V or dO has no size of its own: what dS is scaled by (bwd_x2's bound) is then D's.
         im.unscale[((long long)which * BH + bh) * nblk + blk] = which >= 2 && most == 0.0f ? 0.0f : pow2(e - 14);
         im.flags[((long long)bh * nw + which) * nblk + blk] = bad;
+        if (which == 0 && blk == 0) im.left.flagged[bh] = 0;
+        if (blockIdx.x == 0) *im.left.taken = 0;
         if (nw == 4 && which >= 2) reinterpret_cast<float *>(im.tops + (long long)bh * nblk + blk)[which - 2] = top_of(top_code(most));
         if (which == 3) im.tops[(long long)bh * nblk + blk].z = fmaxf(top_of(top_code(__int_as_float(dred))), TINY);
     }
@@ -308,7 +311,7 @@ __device__ __forceinline__ bool pair_all(int t, bool ok) {
 }
 __device__ __forceinline__ bool any_flag(const uint8_t *flags, int n) {
     bool f = false;
-    for (int i = threadIdx.x; i < n; i += THREADS) f = f || *reinterpret_cast<const volatile uint8_t *>(flags + i);
+    for (int i = threadIdx.x; i < n; i += THREADS) f = f || flags[i];
     return __syncthreads_or(f);
 }
 // Two floats in one register pair (FFMA2 and its like do two in one issue slot).
@@ -522,6 +525,7 @@ flash_fwd_x2_k(float *__restrict__ out, float *__restrict__ lse, const Images im
     const int nsteps = max(steps[0], steps[1]);
 
     if (left) {
+        if (threadIdx.x == 0) im.left.flagged[bh] = 1;
     } else if (warp >= W_COPY) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_OTHER));
         if (warp == W_COPY && elect_one()) {
@@ -723,7 +727,7 @@ flash_fwd_x2_k(float *__restrict__ out, float *__restrict__ lse, const Images im
                 o[i] = add2(y, o[i]);
             }
             store_tile<H>(smem + warp * (32 * H * 4), out + ((long long)b * T + first + quad * 32) * C + h * HS + half * H, C, T - first - quad * 32, o, 1.0f);
-            if ((m > MOST_SCORE || l != l) && qi < T) im.flags[(long long)bh * 3 * nblk] = 1;          // (m never falls)
+            if ((m > MOST_SCORE || l != l) && qi < T) im.left.flagged[bh] = 1;          // (m never falls)
             if (half == 0 && qi < T) lse[(long long)bh * T + qi] = fmaf(m, INV_LOG2E, fmaf(m, INV_LOG2E_REST, logf(l * 1.953125e-3f)));
         }
     }
@@ -800,6 +804,7 @@ __device__ __forceinline__ void bwd_x2(uint8_t *smem, float *__restrict__ dqkv, 
     constexpr int WA1 = KV ? 1 : 0, WA2 = KV ? 2 : 3, WB1 = KV ? 0 : 1, WB2 = KV ? 3 : 2;
 
     if (left) {
+        if (threadIdx.x == 0) im.left.flagged[bh] = 1;
     } else if (warp >= W_COPY) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_OTHER));
         if (warp == W_COPY && elect_one()) {
@@ -1028,7 +1033,7 @@ __device__ __forceinline__ void bwd_x2(uint8_t *smem, float *__restrict__ dqkv, 
         if (!last) { take2(n - 2); if (n > 1) take1(n - 2, bound(n - 2)); }
         take2(n - 1);
         take1(n - 1, bound(n - 1));
-        if (!KV && late && ri < T) im.flags[(long long)bh * 4 * nblk] = 1;
+        if (!KV && late && ri < T) im.left.flagged[bh] = 1;
         if (ok) {
             // every product has retired: the tiles' memory is free
             const int b = bh / NH, h = bh % NH, C = NH * HS, valid = T - r0 - quad * 32;
@@ -1076,7 +1081,7 @@ int prepare(const void *kernel, int bytes) {
     return done[key] = at.numRegs * THREADS >= REGS_COMPUTE * COMPUTE + REGS_OTHER * 128 ? BMB_OK : BMB_E_UNSUPPORTED;
 }
 
-struct Layout { size_t images, unscale, flags, rows, tops, ptops, total; };
+struct Layout { size_t images, unscale, flags, left_out, rows, tops, ptops, total; };
 Layout layout(long long BH, int nblk, int HS, int nw) {
     auto up = [](size_t n) { return (n + 255) / 256 * 256; };
     const size_t blocks = (size_t)BH * nblk;
@@ -1084,10 +1089,11 @@ Layout layout(long long BH, int nblk, int HS, int nw) {
     L.images = up(blocks * nw * XB * HS * 4);
     L.unscale = up(blocks * nw * 4);
     L.flags = up(blocks * nw);
+    L.left_out = up((size_t)BH + 4);
     L.rows = nw == 4 ? up(blocks * ROWS_BYTES) : 0;
     L.tops = nw == 4 ? up(blocks * sizeof(float4)) : 0;
     L.ptops = nw == 4 ? up(blocks * 3 * XB) : 0;
-    L.total = L.images + L.unscale + L.flags + L.rows + L.tops + L.ptops;
+    L.total = L.images + L.unscale + L.flags + L.left_out + L.rows + L.tops + L.ptops;
     return L;
 }
 constexpr size_t KEPT = 1ull << 30;                 // a larger block is given back by the call that took it (unless a trainer keeps it)
@@ -1129,9 +1135,10 @@ int run_x2(const Call &a, bool in_trainer, cudaStream_t st) {
     im.img = scr;
     im.unscale = (float *)(scr + L.images);
     im.flags = scr + L.images + L.unscale;
-    im.rows = (float *)(im.flags + L.flags);
-    im.tops = (float4 *)(im.flags + L.flags + L.rows);
-    im.ptops = im.flags + L.flags + L.rows + L.tops;
+    im.left = LeftOut{im.flags + L.flags + 4, (int *)(im.flags + L.flags), (int)BH};
+    im.rows = (float *)(im.flags + L.flags + L.left_out);
+    im.tops = (float4 *)(im.flags + L.flags + L.left_out + L.rows);
+    im.ptops = im.flags + L.flags + L.left_out + L.rows + L.tops;
     const double cut = (HS == 32 ? 2 : 4) * CUT, sums = 4 * CUT, q = a.scale * (1.0 + cut);      // products in a row
     Factors fac;
     fac.q = (float)q;
@@ -1149,8 +1156,8 @@ int run_x2(const Call &a, bool in_trainer, cudaStream_t st) {
     const dim3 grid((unsigned)BH, rows);
     if (BACKWARD) BMB_TRY(launch_in_chain(flash_bwd_x2_k<HS>, grid, THREADS, smem, st, a.dqkv, im, a.T, a.NH, (int)BH, nblk, fac, status_dev));
     else BMB_TRY(launch_in_chain(flash_fwd_x2_k<HS>, grid, THREADS, smem, st, a.out, a.lse, im, a.T, a.NH, (int)BH, nblk, span, fac, status_dev));
-    if (BACKWARD) BMB_TRY(flash_bwd_mma(HS, a.dqkv, a.dsum, a.dout, a.qkv, a.lse, a.B, a.T, a.NH, a.scale, im.flags, nw * nblk, st));
-    else BMB_TRY(flash_fwd_mma(HS, a.out, a.lse, a.qkv, a.B, a.T, a.NH, a.scale, im.flags, nw * nblk, st));
+    if (BACKWARD) BMB_TRY(flash_bwd_left(HS, a.dqkv, a.dsum, a.dout, a.qkv, a.lse, a.T, a.NH, a.scale, im.left, st));
+    else BMB_TRY(flash_fwd_left(HS, a.out, a.lse, a.qkv, a.T, a.NH, a.scale, im.left, st));
     release.on = false;
     BMB_TRY(scratch_release(SCR_SPLIT, st));
     if (!in_trainer) split_scratch_give_back(KEPT);

@@ -228,3 +228,18 @@ def test_rows_of_zeros(bmb, cuda, hs):
     assert all(bool(cuda.isfinite(x).all()) for x in got)
     assert not got[OUT][0, 1, :70].any() and not got[DQ][0, 1, :70].any() and not got[DQ][0, 1, 600:].any()
     assert not got[DK][0, 1, 600:].any() and not got[DV][0, 1, 600:].any() and not got[DQ][0, 0, 300].any()
+
+
+@pytest.mark.parametrize("hs", [32, 64, 128])
+@pytest.mark.parametrize("heads", [[0], [299], [127, 128], [0, 31, 32, 255, 256, 299], range(300)])
+def test_some_of_many_heads(bmb, cuda, hs, heads):
+    """Heads with a row out of range, among more heads than a block of the kernels behind has threads."""
+    B, T, NH = 100, 384, 3
+    C = NH * hs
+    qkv, dout = inputs(cuda, B, T, NH, hs, hs)
+    for i in heads:
+        qkv[i // NH, 70, 2 * C + i % NH * hs:2 * C + (i % NH + 1) * hs] *= 2.0 ** -30
+    got, want = (by_heads(cuda, attention(bmb, cuda, cfg, qkv, dout, NH), NH) for cfg in (0, 1))
+    for x, y in zip(got, want):
+        x, y = (z.flatten(0, 1).flatten(1).double() for z in (x, y))
+        assert bool(((x - y).norm(dim=1) <= BOUND * y.norm(dim=1)).all())
