@@ -29,6 +29,7 @@
 // 2-norm errors against 64 bits there: 8 x 160 x 4 heads of 64 and up, output 0.95 to 1.0 of those kernels', lse 0.7, dqkv 0.82 to 1.0.
 #include "tc_common.cuh"
 #include <cuda_fp16.h>
+#include <algorithm>
 #include <cmath>
 #include <map>
 #include <mutex>
@@ -1096,7 +1097,7 @@ Layout layout(long long BH, int nblk, int HS, int nw) {
     L.total = L.images + L.unscale + L.flags + L.left_out + L.rows + L.tops + L.ptops;
     return L;
 }
-constexpr size_t KEPT = 1ull << 30;                 // a larger block is given back by the call that took it (unless a trainer keeps it)
+constexpr size_t KEPT = 1ull << 30;                 // a larger block (of one head) is given back by the call that took it, unless a trainer keeps it
 
 struct Call {
     float *out, *lse, *dqkv, *dsum;
@@ -1105,37 +1106,16 @@ struct Call {
     float scale;
 };
 
+// Heads whose images lie in `scr`: the head `a` points at and those behind it.
 template <int HS, bool BACKWARD>
-int run_x2(const Call &a, bool in_trainer, cudaStream_t st) {
-    const long long BH = (long long)a.B * a.NH;
-    const int nblk = ceil_div(a.T, XB), nw = BACKWARD ? 4 : 3;
-    // A CTA's two tiles of queries share its keys and hide each other's latency, but one is faster alone where SMs are free.
-    const int span = BH * ceil_div(a.T, 256) <= sm_count() * 9 / 10 ? 128 : 256;
-    const int rows = BACKWARD ? 2 * ceil_div(a.T, 128) : ceil_div(a.T, span);
-    if (rows > 65535 || BH * nblk * nw >= (1LL << 31)) return BMB_E_UNSUPPORTED;
-    // A captured launch would carry the scratch's address.
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (!in_trainer && (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)) {
-        cudaGetLastError();
-        return BMB_E_UNSUPPORTED;
-    }
-    const void *kernel = BACKWARD ? (const void *)flash_bwd_x2_k<HS> : (const void *)flash_fwd_x2_k<HS>;
-    const int smem = BACKWARD ? Bwd<HS>::SMEM : Fwd<HS>::SMEM;
-    BMB_TRY(prepare(kernel, smem));
+int launch_x2(const Call &a, int BH, int span, uint8_t *scr, int *status_dev, cudaStream_t st) {
+    const int nblk = ceil_div(a.T, XB), nw = BACKWARD ? 4 : 3, smem = BACKWARD ? Bwd<HS>::SMEM : Fwd<HS>::SMEM;
     const Layout L = layout(BH, nblk, HS, nw);
-    if (L.total > (16ull << 30)) return BMB_E_UNSUPPORTED;
-    int *status_dev = nullptr;
-    volatile int *status_host = nullptr;
-    BMB_TRY(status_word(&status_dev, &status_host));
-    if (*status_host != 0) return fail(BMB_E_TIMEOUT, "an earlier kernel on this device gave up waiting on a barrier");
-    std::lock_guard<std::mutex> turn(split_mutex());
-    uint8_t *scr = (uint8_t *)split_scratch(L.total, st);
-    if (!scr) return BMB_E_UNSUPPORTED;
     Images im;
     im.img = scr;
     im.unscale = (float *)(scr + L.images);
     im.flags = scr + L.images + L.unscale;
-    im.left = LeftOut{im.flags + L.flags + 4, (int *)(im.flags + L.flags), (int)BH};
+    im.left = LeftOut{im.flags + L.flags + 4, (int *)(im.flags + L.flags), BH};
     im.rows = (float *)(im.flags + L.flags + L.left_out);
     im.tops = (float4 *)(im.flags + L.flags + L.left_out + L.rows);
     im.ptops = im.flags + L.flags + L.left_out + L.rows + L.tops;
@@ -1148,16 +1128,56 @@ int run_x2(const Call &a, bool in_trainer, cudaStream_t st) {
     fac.dk = (float)(a.scale / q * (1.0 + cut) * (1.0 + sums));
     fac.dq = (float)(a.scale * (1.0 + cut) * (1.0 + sums));
     fac.dv = (float)(1.0 + sums);
-    BMB_TRY(scratch_acquire(SCR_SPLIT, st));
-    ScratchRelease release{SCR_SPLIT, st, true};
-    split_x2_k<HS><<<(unsigned)(BH * nblk * nw), 256, 0, st>>>(im, a.dsum, a.qkv, a.dout, a.out, a.lse, a.T, a.NH, (int)BH, nblk, nw, fac);
+    split_x2_k<HS><<<(unsigned)((long long)BH * nblk * nw), 256, 0, st>>>(im, a.dsum, a.qkv, a.dout, a.out, a.lse, a.T, a.NH, BH, nblk, nw, fac);
     count_launch();
     BMB_LAUNCH_CHECK();
-    const dim3 grid((unsigned)BH, rows);
-    if (BACKWARD) BMB_TRY(launch_in_chain(flash_bwd_x2_k<HS>, grid, THREADS, smem, st, a.dqkv, im, a.T, a.NH, (int)BH, nblk, fac, status_dev));
-    else BMB_TRY(launch_in_chain(flash_fwd_x2_k<HS>, grid, THREADS, smem, st, a.out, a.lse, im, a.T, a.NH, (int)BH, nblk, span, fac, status_dev));
-    if (BACKWARD) BMB_TRY(flash_bwd_left(HS, a.dqkv, a.dsum, a.dout, a.qkv, a.lse, a.T, a.NH, a.scale, im.left, st));
-    else BMB_TRY(flash_fwd_left(HS, a.out, a.lse, a.qkv, a.T, a.NH, a.scale, im.left, st));
+    const dim3 grid((unsigned)BH, BACKWARD ? 2 * ceil_div(a.T, 128) : ceil_div(a.T, span));
+    if (BACKWARD) {
+        BMB_TRY(launch_in_chain(flash_bwd_x2_k<HS>, grid, THREADS, smem, st, a.dqkv, im, a.T, a.NH, BH, nblk, fac, status_dev));
+        return flash_bwd_left(HS, a.dqkv, a.dsum, a.dout, a.qkv, a.lse, a.T, a.NH, a.scale, im.left, st);
+    }
+    BMB_TRY(launch_in_chain(flash_fwd_x2_k<HS>, grid, THREADS, smem, st, a.out, a.lse, im, a.T, a.NH, BH, nblk, span, fac, status_dev));
+    return flash_fwd_left(HS, a.out, a.lse, a.qkv, a.T, a.NH, a.scale, im.left, st);
+}
+
+template <int HS, bool BACKWARD>
+int run_x2(const Call &a, bool in_trainer, cudaStream_t st) {
+    const int nblk = ceil_div(a.T, XB), nw = BACKWARD ? 4 : 3;
+    // Images of more than KEPT bytes are made and used one after the other: of some of the sequences, or of some of a sequence's heads.
+    const size_t head = layout(1, nblk, HS, nw).total, fit = std::max<size_t>(1, KEPT / head);
+    int nb = (int)std::min<size_t>(a.B, fit / a.NH), nh = a.NH;
+    if (nb) nb = ceil_div(a.B, ceil_div(a.B, nb));           // (parts of one size)
+    else { nb = 1; nh = ceil_div(a.NH, ceil_div(a.NH, (long long)fit)); }
+    // A CTA's two tiles of queries share its keys and hide each other's latency, but one is faster alone where SMs are free.
+    const long long BH = (long long)nb * nh;
+    const int span = BH * ceil_div(a.T, 256) <= sm_count() * 9 / 10 ? 128 : 256;
+    if ((BACKWARD ? 2 * ceil_div(a.T, 128) : ceil_div(a.T, span)) > 65535 || BH * nblk * nw >= (1LL << 31)) return BMB_E_UNSUPPORTED;
+    // A captured launch would carry the scratch's address.
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (!in_trainer && (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)) {
+        cudaGetLastError();
+        return BMB_E_UNSUPPORTED;
+    }
+    BMB_TRY(prepare(BACKWARD ? (const void *)flash_bwd_x2_k<HS> : (const void *)flash_fwd_x2_k<HS>, BACKWARD ? Bwd<HS>::SMEM : Fwd<HS>::SMEM));
+    const size_t bytes = layout(BH, nblk, HS, nw).total;
+    if (bytes > (16ull << 30)) return BMB_E_UNSUPPORTED;
+    int *status_dev = nullptr;
+    volatile int *status_host = nullptr;
+    BMB_TRY(status_word(&status_dev, &status_host));
+    if (*status_host != 0) return fail(BMB_E_TIMEOUT, "an earlier kernel on this device gave up waiting on a barrier");
+    std::lock_guard<std::mutex> turn(split_mutex());
+    uint8_t *scr = (uint8_t *)split_scratch(bytes, st);
+    if (!scr) return BMB_E_UNSUPPORTED;
+    BMB_TRY(scratch_acquire(SCR_SPLIT, st));
+    ScratchRelease release{SCR_SPLIT, st, true};
+    for (int b = 0; b < a.B; b += nb)
+        for (int h = 0; h < a.NH; h += nh) {
+            const long long C = (long long)a.NH * HS, x = b * (C * a.T) + (long long)h * HS, x3 = b * (3 * C * a.T) + (long long)h * HS;
+            const long long row = ((long long)b * a.NH + h) * a.T;
+            const Call part{a.out + x, a.lse + row, BACKWARD ? a.dqkv + x3 : nullptr, BACKWARD ? a.dsum + row : nullptr, a.qkv + x3,
+                            BACKWARD ? a.dout + x : nullptr, a.B, a.T, a.NH, a.scale};
+            BMB_TRY((launch_x2<HS, BACKWARD>(part, std::min(nb, a.B - b) * std::min(nh, a.NH - h), span, scr, status_dev, st)));
+        }
     release.on = false;
     BMB_TRY(scratch_release(SCR_SPLIT, st));
     if (!in_trainer) split_scratch_give_back(KEPT);

@@ -243,3 +243,15 @@ def test_some_of_many_heads(bmb, cuda, hs, heads):
     for x, y in zip(got, want):
         x, y = (z.flatten(0, 1).flatten(1).double() for z in (x, y))
         assert bool(((x - y).norm(dim=1) <= BOUND * y.norm(dim=1)).all())
+
+
+@pytest.mark.parametrize("B,T,NH,hs", [(9, 8192, 8, 128), (11, 8192, 26, 32), (1, 65600, 9, 128)])
+def test_images_in_parts(bmb, cuda, B, T, NH, hs):
+    """More heads than images of 1 GiB hold (some sequences at a time, or some heads of one): the first and the last, bit for bit as by themselves."""
+    qkv, dout = inputs(cuda, B, T, NH, hs, 1)
+    out, lse, dsum, dqkv = attention(bmb, cuda, 0, qkv, dout, NH)
+    for b, h in ((0, 0), (B - 1, NH - 1)):
+        pick = lambda x: x[b:b + 1].unflatten(-1, (-1, NH, hs))[:, :, :, h].flatten(2).contiguous()      # noqa: E731
+        alone = attention(bmb, cuda, 0, pick(qkv), pick(dout), 1)
+        for x, y in zip((pick(out), lse[b:b + 1, h:h + 1], dsum[b:b + 1, h:h + 1], pick(dqkv)), alone):
+            assert cuda.equal(x, y)
