@@ -182,6 +182,9 @@ __device__ __forceinline__ void for_left_out(const LeftOut &left, int each, Body
     __shared__ uint16_t list[1024];
     __shared__ int count;
     __shared__ long long next;
+    bool any = false;
+    for (int i = threadIdx.x; i < left.heads; i += blockDim.x) any = any || left.flagged[i];
+    if (!__syncthreads_or(any)) return;
     long long item = blockIdx.x, first = 0;                        // this block's; the first of these heads
     for (int h0 = 0; h0 < left.heads; h0 += 1024) {
         __syncthreads();

@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(256, HS == 32 ? 5 : HS == 64 ? 4 : 2) split_x2
     using G = Geo<HS>;
     constexpr int UPR = HS / 8, ITEMS = XB * UPR / 256;
     __shared__ float red[8];
-    __shared__ __align__(16) uint32_t columns[8][4 * UPR];
+    __shared__ __align__(16) __half2 columns[8][4 * UPR];
     __shared__ int dred;
     if (threadIdx.x == 0) dred = 0;
     const int blk = (int)(blockIdx.x % (unsigned)nblk), which = (int)(blockIdx.x / (unsigned)nblk % (unsigned)nw);
@@ -123,8 +123,7 @@ __global__ void __launch_bounds__(256, HS == 32 ? 5 : HS == 64 ? 4 : 2) split_x2
     const float *src = (which < 3 ? qkv + which * C : dout) + ((long long)b * T + blk * XB) * ld + h * HS;
     float v[ITEMS][8], rest[ITEMS][8], rowmax[ITEMS], most = 0.0f, dmax = 0.0f;      // rest: of q only
     uint8_t *ptops = im.ptops + ((long long)bh * nblk + blk) * (3 * XB);
-    uint32_t colmax[4] = {0u, 0u, 0u, 0u};
-    bool bad = false;
+    bool lost = false;                                       // D or lse out of range
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
         const int u = i * 256 + (int)threadIdx.x, r = u / UPR, c = u % UPR * 8, pos = blk * XB + r;
@@ -142,10 +141,6 @@ __global__ void __launch_bounds__(256, HS == 32 ? 5 : HS == 64 ? 4 : 2) split_x2
                 rest[i][j] = fmaf(q, fac.q, -v[i][j]) + q * fac.q_rest;
             }
         }
-        // the upper 16 bits of a column's largest element
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            colmax[j] = max_u16x2(colmax[j], __byte_perm(__float_as_uint(v[i][2 * j]), __float_as_uint(v[i][2 * j + 1]), 0x7632) & 0x7fff7fffu);
         float m = 0.0f;
 #pragma unroll
         for (int j = 0; j < 8; j += 2) asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(v[i][j]), "f"(v[i][j + 1]));
@@ -163,7 +158,7 @@ __global__ void __launch_bounds__(256, HS == 32 ? 5 : HS == 64 ? 4 : 2) split_x2
                 const float L = pos < T ? lse[at] : INFINITY;
                 if (pos < T) {
                     dsum[at] = a;
-                    bad = bad || !(fabsf(a) <= 1.1805916e21f) || !(fabsf(L) <= 524288.0f);
+                    lost = lost || !(fabsf(a) <= 1.1805916e21f) || !(fabsf(L) <= 524288.0f);
                 }
                 dmax = fmaxf(dmax, fabsf(a));
                 ptops[2 * XB + r] = (uint8_t)top_code(a);
@@ -181,16 +176,13 @@ __global__ void __launch_bounds__(256, HS == 32 ? 5 : HS == 64 ? 4 : 2) split_x2
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) asm("max.NaN.f32 %0, %0, %1;" : "+f"(most) : "f"(__shfl_xor_sync(0xffffffffu, most, o)));
-#pragma unroll
-    for (int o = 16; o >= UPR; o >>= 1)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) colmax[j] = max_u16x2(colmax[j], __shfl_xor_sync(0xffffffffu, colmax[j], o));
-    if ((threadIdx.x & 31) < UPR) *reinterpret_cast<uint4 *>(&columns[threadIdx.x >> 5][4 * (threadIdx.x & 31)]) = make_uint4(colmax[0], colmax[1], colmax[2], colmax[3]);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = most;
     __syncthreads();
+    if (dmax > 0.0f) atomicMax(&dred, __float_as_int(dmax));             // (not negative: ordered as whole numbers are)
 #pragma unroll
     for (int i = 0; i < 8; ++i) asm("max.NaN.f32 %0, %0, %1;" : "+f"(most) : "f"(red[i]));
-    bad = bad || (most != 0.0f && !(most >= LEAST && most < MOST));
+    const bool usable = most >= LEAST && most < MOST;
+    bool bad = lost || (most != 0.0f && !usable);
     // Rows and columns of the block against its largest element: products sum along both, and hold 2^-31 of a row's or column's largest
     // element where that is 2^-20 of the block's.
     // (In V and dO of a backward rows from 2^-12 on: dS of a block's 64 columns has one scale, so what belongs to a column's small
@@ -198,32 +190,56 @@ __global__ void __launch_bounds__(256, HS == 32 ? 5 : HS == 64 ? 4 : 2) split_x2
     const float low_end = 9.5367432e-7f * most, low_row = nw == 4 && which >= 2 ? 2.44140625e-4f * most : low_end;
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) bad = bad || (rowmax[i] != 0.0f && rowmax[i] < low_row);
-    if (threadIdx.x < 4 * UPR) {
-        uint32_t m = 0;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) m = max_u16x2(m, columns[i][threadIdx.x]);
-        const uint32_t least = __float_as_uint(low_end) >> 16, x = m & 0xffffu, y = m >> 16;
-        bad = bad || (x && x < least) || (y && y < least);
-    }
-    if (dmax > 0.0f) atomicMax(&dred, __float_as_int(dmax));             // (not negative: ordered as whole numbers are)
-    bad = __syncthreads_or(bad);
-    const bool usable = most >= LEAST && most < MOST;
     const int e = usable ? exponent(most) : 14;
     const float f = usable ? pow2(14 - e) : 0.0f;
     uint8_t *img = im.img + (((long long)which * BH + bh) * nblk + blk) * G::BLK;
+    __half2 colmax[4];                                       // the largest elements of this thread's columns, by their large pieces
 #pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-        const int u = i * 256 + (int)threadIdx.x, r = u / UPR, c = u % UPR;
-        uint32_t hi[4], lo[4];
+    for (int j = 0; j < 4; ++j) colmax[j] = __half2(0.0f, 0.0f);
+    auto put = [&](bool q) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const bool q = which == 0 && usable;
-            split2(usable ? v[i][2 * j] * f : 0.0f, q ? rest[i][2 * j] * f : 0.0f, usable ? v[i][2 * j + 1] * f : 0.0f, q ? rest[i][2 * j + 1] * f : 0.0f, hi[j], lo[j]);
+        for (int i = 0; i < ITEMS; ++i) {
+            const int u = i * 256 + (int)threadIdx.x, r = u / UPR, c = u % UPR;
+            uint32_t hi[4], lo[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                split2(v[i][2 * j] * f, q ? rest[i][2 * j] * f : 0.0f, v[i][2 * j + 1] * f, q ? rest[i][2 * j + 1] * f : 0.0f, hi[j], lo[j]);
+                colmax[j] = __hmax2(colmax[j], __habs2(*reinterpret_cast<const __half2 *>(&hi[j])));
+            }
+            const int ch = c / (G::CE / 8), uc = c % (G::CE / 8), x = G::ROWB == 128 ? (r & 7) : (r >> 1 & 3);
+            uint8_t *d = img + ch * (XB * G::ROWB) + r * G::ROWB + ((uc ^ x) << 4);
+            *reinterpret_cast<uint4 *>(d) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            *reinterpret_cast<uint4 *>(d + G::PIECE) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
         }
-        const int ch = c / (G::CE / 8), uc = c % (G::CE / 8), x = G::ROWB == 128 ? (r & 7) : (r >> 1 & 3);
-        uint8_t *d = img + ch * (XB * G::ROWB) + r * G::ROWB + ((uc ^ x) << 4);
-        *reinterpret_cast<uint4 *>(d) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-        *reinterpret_cast<uint4 *>(d + G::PIECE) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    };
+    if (which == 0) put(true);
+    else put(false);
+#pragma unroll
+    for (int o = 16; o >= UPR; o >>= 1)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) colmax[j] = __hmax2(colmax[j], __shfl_xor_sync(0xffffffffu, colmax[j], o));
+    if ((threadIdx.x & 31) < UPR) *reinterpret_cast<uint4 *>(&columns[threadIdx.x >> 5][4 * (threadIdx.x & 31)]) = *reinterpret_cast<const uint4 *>(colmax);
+    __syncthreads();
+    if (threadIdx.x < 4 * UPR) {
+        __half2 m = columns[0][threadIdx.x];
+#pragma unroll
+        for (int i = 1; i < 8; ++i) m = __hmax2(m, columns[i][threadIdx.x]);
+        columns[0][threadIdx.x] = m;
+        bad = bad || fminf(__low2float(m), __high2float(m)) < low_end * f;
+    }
+    bad = __syncthreads_or(bad);
+    if (bad && usable) {                                     // something is small, or a column is zero, which is no harm
+        bool small = false;
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            small = small || (rowmax[i] != 0.0f && rowmax[i] < low_row);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const __half2 m = columns[0][4 * ((int)threadIdx.x % UPR) + j / 2];
+                small = small || (v[i][j] != 0.0f && (j & 1 ? __high2float(m) : __low2float(m)) < low_end * f);
+            }
+        }
+        bad = __syncthreads_or(small || lost);
     }
     if (threadIdx.x == 0) {
         // A block of zeros in V or dO has no size of its own: what dS is scaled by (bwd_x2's bound) is then D's.
