@@ -129,6 +129,12 @@ void *split_scratch(size_t bytes, cudaStream_t st);
 void split_scratch_give_back(size_t above);
 void split_scratch_keep(int change);
 unsigned long long split_scratch_generation();      // counts the block's moves, as scratch_generation() those of the others
+// A block for one call's launches on `st` (not captured), until call_scratch_done: calls on several streams have blocks of their own, up to
+// CALL_SCRATCH_KEPT bytes of a device in all (a larger one is given back by the call that took it); beyond that they take turns.
+// nullptr: there is no memory.
+constexpr size_t CALL_SCRATCH_KEPT = 1ull << 30;
+void *call_scratch(size_t bytes, cudaStream_t st);
+int call_scratch_done(void *p, cudaStream_t st);
 // Internal GEMM dispatch shared by attention and the trainer: math is a
 // BMB_MATH_* value, flags the BMB_GEMM_* bits, strides in elements.
 int gemm_any(int math, int flags, int ta, int tb, int batch, int M, int N, int K, float alpha,

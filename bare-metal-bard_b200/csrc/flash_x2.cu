@@ -1113,7 +1113,7 @@ Layout layout(long long BH, int nblk, int HS, int nw) {
     L.total = L.images + L.unscale + L.flags + L.left_out + L.rows + L.tops + L.ptops;
     return L;
 }
-constexpr size_t KEPT = 1ull << 30;                 // a larger block (of one head) is given back by the call that took it, unless a trainer keeps it
+constexpr size_t KEPT = CALL_SCRATCH_KEPT;          // bytes of images at a time (or one head's)
 
 struct Call {
     float *out, *lse, *dqkv, *dsum;
@@ -1181,11 +1181,19 @@ int run_x2(const Call &a, bool in_trainer, cudaStream_t st) {
     volatile int *status_host = nullptr;
     BMB_TRY(status_word(&status_dev, &status_host));
     if (*status_host != 0) return fail(BMB_E_TIMEOUT, "an earlier kernel on this device gave up waiting on a barrier");
-    std::lock_guard<std::mutex> turn(split_mutex());
-    uint8_t *scr = (uint8_t *)split_scratch(bytes, st);
+    // A trainer's launches use the block that its captured steps hold, other calls one of their own.
+    std::unique_lock<std::mutex> turn(split_mutex(), std::defer_lock);
+    if (in_trainer) turn.lock();
+    uint8_t *scr = (uint8_t *)(in_trainer ? split_scratch(bytes, st) : call_scratch(bytes, st));
     if (!scr) return BMB_E_UNSUPPORTED;
-    BMB_TRY(scratch_acquire(SCR_SPLIT, st));
-    ScratchRelease release{SCR_SPLIT, st, true};
+    struct Done {
+        uint8_t *scr;
+        cudaStream_t st;
+        bool in_trainer;
+        ~Done() { if (in_trainer) scratch_release(SCR_SPLIT, st); else call_scratch_done(scr, st); }
+    };
+    const Done done{scr, st, in_trainer};
+    if (in_trainer) BMB_TRY(scratch_acquire(SCR_SPLIT, st));
     for (int b = 0; b < a.B; b += nb)
         for (int h = 0; h < a.NH; h += nh) {
             const long long C = (long long)a.NH * HS, x = b * (C * a.T) + (long long)h * HS, x3 = b * (3 * C * a.T) + (long long)h * HS;
@@ -1194,9 +1202,6 @@ int run_x2(const Call &a, bool in_trainer, cudaStream_t st) {
                             BACKWARD ? a.dout + x : nullptr, a.B, a.T, a.NH, a.scale};
             BMB_TRY((launch_x2<HS, BACKWARD>(part, std::min(nb, a.B - b) * std::min(nh, a.NH - h), span, scr, status_dev, st)));
         }
-    release.on = false;
-    BMB_TRY(scratch_release(SCR_SPLIT, st));
-    if (!in_trainer) split_scratch_give_back(KEPT);
     return BMB_OK;
 }
 

@@ -171,6 +171,91 @@ unsigned long long split_scratch_generation() {
     return (d < 0 || d >= 64) ? 0ULL : g_split_gen[d];
 }
 
+// ---- blocks for the length of a call ----
+namespace {
+struct CallBlock {
+    void *p = nullptr;
+    size_t cap = 0;
+    cudaEvent_t done = nullptr;      // behind its last use, on `last`
+    cudaStream_t last = nullptr;
+    bool taken = false;              // a call is making its launches
+    unsigned long long when = 0;
+};
+struct CallBlocks {
+    CallBlock of[8];
+    size_t total = 0;
+    unsigned long long uses = 0;
+};
+std::mutex g_call_mu;
+CallBlocks g_call_blocks[64];
+
+bool drop_block(CallBlocks &all, CallBlock &b) {
+    if (b.p && (cudaEventSynchronize(b.done) != cudaSuccess || cudaFree(b.p) != cudaSuccess)) { cudaGetLastError(); return false; }
+    all.total -= b.cap;
+    b.p = nullptr;
+    b.cap = 0;
+    return true;
+}
+}  // namespace
+
+void *call_scratch(size_t bytes, cudaStream_t st) {
+    const int d = current_device();
+    if (d < 0 || d >= 64) return nullptr;
+    RelaxedCapture relaxed;
+    std::lock_guard<std::mutex> lk(g_call_mu);
+    CallBlocks &all = g_call_blocks[d];
+    // this stream's last block, or one that nobody uses any more, or a new one, or the one that has been in use for longest
+    CallBlock *mine = nullptr, *idle = nullptr, *oldest = nullptr, *empty = nullptr;
+    for (CallBlock &b : all.of) {
+        if (b.taken) continue;
+        if (!b.p) { empty = &b; continue; }
+        if (b.cap < bytes) continue;
+        if (b.last == st) { if (!mine || b.cap < mine->cap) mine = &b; }
+        else if (!oldest || b.when < oldest->when) oldest = &b;
+    }
+    if (!mine && oldest) {
+        if (cudaEventQuery(oldest->done) == cudaSuccess) idle = oldest;
+        else cudaGetLastError();
+    }
+    CallBlock *use = mine ? mine : idle;
+    if (!use && !(oldest && (!empty || all.total + bytes > CALL_SCRATCH_KEPT))) {
+        for (CallBlock &b : all.of) {                        // (none is large enough: smaller ones make room)
+            if (empty && all.total + bytes <= CALL_SCRATCH_KEPT) break;
+            if (b.p && !b.taken && drop_block(all, b)) empty = &b;
+        }
+        if (!empty) return nullptr;
+        if (!empty->done && cudaEventCreateWithFlags(&empty->done, cudaEventDisableTiming) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        const size_t want = bytes < (1u << 20) ? (1u << 20) : bytes;
+        if (cudaMalloc(&empty->p, want) != cudaSuccess) { cudaGetLastError(); empty->p = nullptr; return nullptr; }
+        empty->cap = want;
+        all.total += want;
+        use = empty;
+    } else {
+        if (!use) use = oldest;
+        // (also behind the same stream's work: a handle may have come back for another stream)
+        if (cudaStreamWaitEvent(st, use->done, 0) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    }
+    use->taken = true;
+    use->last = st;
+    use->when = ++all.uses;
+    return use->p;
+}
+
+int call_scratch_done(void *p, cudaStream_t st) {
+    const int d = current_device();
+    RelaxedCapture relaxed;
+    std::lock_guard<std::mutex> lk(g_call_mu);
+    CallBlocks &all = g_call_blocks[d];
+    for (CallBlock &b : all.of)
+        if (b.p == p) {
+            BMB_CUDA(cudaEventRecord(b.done, st));
+            b.taken = false;
+            if (all.total > CALL_SCRATCH_KEPT) drop_block(all, b);
+            break;
+        }
+    return BMB_OK;
+}
+
 void split_scratch_keep(int change) {
     const int d = current_device();
     if (d >= 0 && d < 64) g_split_keepers[d] += change;

@@ -255,3 +255,23 @@ def test_images_in_parts(bmb, cuda, B, T, NH, hs):
         alone = attention(bmb, cuda, 0, pick(qkv), pick(dout), 1)
         for x, y in zip((pick(out), lse[b:b + 1, h:h + 1], dsum[b:b + 1, h:h + 1], pick(dqkv)), alone):
             assert cuda.equal(x, y)
+
+
+def test_calls_on_several_streams(bmb, cuda):
+    """Calls on four streams, of several sizes, without a wait between them: what each gives by itself."""
+    shapes = [(1, 512, 4, 64), (2, 777, 12, 32), (1, 1024, 8, 128), (4, 1024, 12, 64)]
+    data = [inputs(cuda, *shape, i) for i, shape in enumerate(shapes)]
+    want = [attention(bmb, cuda, 0, qkv, dout, shape[2]) for shape, (qkv, dout) in zip(shapes, data)]
+    streams = [cuda.cuda.Stream() for _ in shapes]
+    got = [[cuda.full_like(x, float("nan")) for x in w] for w in want]
+    cuda.cuda.synchronize()
+    try:
+        for _ in range(20):
+            for st, (B, T, NH, hs), (qkv, dout), (out, lse, dsum, dqkv) in zip(streams, shapes, data, got):
+                bmb.lib().bmb_set_stream(st.cuda_stream)
+                bmb.call("bmb_flash_attention_forward_cfg", 0, out, lse, qkv, B, T, NH * hs, NH)
+                bmb.call("bmb_flash_attention_backward_cfg", 0, dqkv, dsum, dout, qkv, out, lse, B, T, NH * hs, NH)
+    finally:
+        bmb.lib().bmb_set_stream(None)
+    cuda.cuda.synchronize()
+    assert all(cuda.equal(x, y) for g, w in zip(got, want) for x, y in zip(g, w))
