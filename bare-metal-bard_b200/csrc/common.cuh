@@ -183,20 +183,24 @@ namespace bmb {
 __device__ __forceinline__ void let_successor_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <typename... P, typename... A>
-int launch_in_chain(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+int launch(bool in_chain, void (*kernel)(P...), dim3 grid, dim3 threads, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
+    cfg.blockDim = threads;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = in_chain ? 1 : 0;
     BMB_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
     count_launch();
     return BMB_OK;
+}
+template <typename... P, typename... A>
+int launch_in_chain(void (*kernel)(P...), dim3 grid, dim3 threads, size_t smem, cudaStream_t st, A... args) {
+    return launch(true, kernel, grid, threads, smem, st, args...);
 }
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll

@@ -7,9 +7,10 @@ namespace bmb {
 int gemm_simt(int transA, int transB, int batch, int M, int N, int K, float alpha, const float *A,
               long long sA, const float *B, long long sB, float beta, float *C, long long sC,
               cudaStream_t st);
-// fp32 products on the tensor cores in three bf16 pieces (gemm_x3.cu), bias included.  BMB_E_UNSUPPORTED: the SIMT kernel's.
+// Products of few tiles, bias and GELU included.  BMB_E_UNSUPPORTED: the other SIMT kernels'.
 int gemm_simt_small(int transA, int transB, int batch, int M, int N, int K, float alpha, const float *A, long long sA,
                     const float *B, long long sB, float beta, float *C, long long sC, const float *bias, float *gelu, cudaStream_t st);
+// fp32 products on the tensor cores in three bf16 pieces (gemm_x3.cu), bias included.  BMB_E_UNSUPPORTED: the SIMT kernel's.
 int gemm_x3(int transA, int transB, int M, int N, int K, float alpha, const float *A, const float *B, float beta, float *C,
             const float *bias, int flags, cudaStream_t st);
 // Tensor-core path (gemm_tc.cu).  Returns BMB_E_UNSUPPORTED for shapes it does

@@ -976,18 +976,7 @@ struct Chain {
     bool first = true;
     template <typename... P, typename... A>
     int launch(void (*kernel)(P...), dim3 grid, dim3 threads, size_t smem, A... args) {
-        cudaLaunchAttribute at{};
-        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at.val.programmaticStreamSerializationAllowed = 1;
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = grid;
-        cfg.blockDim = threads;
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = st;
-        cfg.attrs = &at;
-        cfg.numAttrs = first ? 0 : 1;
-        BMB_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
-        count_launch();
+        BMB_TRY(bmb::launch(!first, kernel, grid, threads, smem, st, args...));
         first = false;
         return BMB_OK;
     }
