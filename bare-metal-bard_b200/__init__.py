@@ -51,6 +51,7 @@ SIGNATURES = {
     "bmb_version": (C.c_char_p, []),
     "bmb_launch_count": (_ll, []),
     "bmb_gemm_schedule_check": (_i, [_i, _i, _i, _i, _i, _i, _i, C.POINTER(_i), C.POINTER(_i), C.POINTER(_i), C.POINTER(_i)]),
+    "bmb_gemm_plan_check": (_i, [_i] * 10 + [C.POINTER(_i)] * 5),
     "bmb_kernel_status": (_i, [C.POINTER(_i)]),
     "bmb_kernel_status_clear": (_i, []),
     "bmb_selftest_wait_expiry": (_i, [_ll, C.POINTER(_ll)]),

@@ -1177,6 +1177,9 @@ void plan_pair(Plan *p, int flags, int M, int N, int clusters, int bn) {
     if (allow_split && rem && p->kblocks >= 8) {
         const double run = (double)(((long long)rem * p->kblocks + clusters - 1) / clusters);
         const double shared = start + ((double)full * tile + run + 22.0) * unit;
+        // A short K is not shared unless the run is small beside the whole tiles: the preparing launch and the parts' additions cost more than the
+        // part of a wave that they save, whole / shared us, 256 columns: TF32 4096x4096x512 38.9 / 48.1, x1024 57.4 / 62.5, 8192x2304x768 49.2 / 60.4,
+        // 6144x6144x1024 104.4 / 111.6; BF16 4096x4096x2048 78.6 / 85.1, 6144x6144x2048 132.1 / 142.3.
         const bool short_k_big_run = p->kblocks <= 32 && run > 0.10 * ((double)full * tile + run);
         if (shared < p->cost && !short_k_big_run) { p->cost = shared; p->dp_tiles = p->tiles - rem; }
     }
@@ -1250,8 +1253,9 @@ int plan_gemm(Plan *p, bool bf16, int flags, int batch, int M, int N, int K, int
 
 // The pair kernel's plan in place of *p where it costs less.  The sides of the line, single CTAs / pairs (us, operands from
 // DRAM): TF32 4096^3 199.5 / 181.3, 8192x2304x768 57.2 / 50.0, 8192x3072x768 72.5 / 66.3 (192 columns), 8192x768x768 30.8 / 26.7
-// (192), 768x2304x8192 87.0 / 68.6 (192), 8192x50304x768 1044 / 927; but 1024^3 19.5 / 27.6, 512x512x6144 27.7 / 29.7,
-// 50304x768x8192 799 / 843 and 8192x768x50304 918 / 980.  On half of the SMs 8192x2304x768 96.3 / 76.7, 3072x768x8192 121.9 / 92.2.
+// (192), 8192x50304x768 1044 / 927; but 1024^3 19.5 / 27.6, 512x512x6144 27.7 / 29.7, 50304x768x8192 799 / 843 and 8192x768x50304
+// 918 / 980.  (768x2304x8192 stays with single CTAs, 82.7 us, although pairs of 192 columns that share their tiles take 62.5: the costs of
+// a long run are not that well known to this model.)  On half of the SMs 8192x2304x768 96.3 / 76.7, 3072x768x8192 121.9 / 92.2.
 // BF16 (passes over the operands included) 6144^3 425 / 386, 8192x50304x768 701 / 669; 1024^3 23.5 / 33.8.
 void prefer_pair(Plan *p, int flags, int M, int N, int clusters) {
     for (int bn : {256, 192}) {
@@ -1259,6 +1263,16 @@ void prefer_pair(Plan *p, int flags, int M, int N, int clusters) {
         plan_pair(&q, flags, M, N, clusters, bn);
         if (q.cost < p->cost) *p = q;
     }
+}
+
+// The plan that a call takes (rounds_on_arrival may still put one of 128-row tiles in its place): single CTAs, `ctas` of them, or, where it
+// asks for them or they cost less, CTA pairs, `clusters` of them.
+int choose_plan(Plan *p, bool bf16, int flags, int transA, int transB, int batch, int M, int N, int K, int ctas, int clusters) {
+    BMB_TRY(plan_gemm(p, bf16, flags, batch, M, N, K, ctas));
+    if (clusters < 1 || !pair_takes(bf16, transA, transB, batch, M, N)) return BMB_OK;
+    if (leaves_pair_open(flags)) prefer_pair(p, flags, M, N, clusters);
+    else if (asks_for_pair(flags)) plan_pair(p, flags, M, N, clusters, 256);
+    return BMB_OK;
 }
 
 template <int KIND, int BN, int MH, int AUX = 0, int RND = 0>
@@ -1376,12 +1390,9 @@ int gemm_tc(int math, int flags, int transA, int transB, int batch, int M, int N
     // BMB_GEMM_HALF_SMS: plan for half of the SMs, so that two such launches on two streams run side by side
     const int ctas = (flags & BMB_GEMM_HALF_SMS) ? (sm_count() + 1) / 2 : sm_count();
     Plan plan;
-    BMB_TRY(plan_gemm(&plan, bf16, flags, batch, M, N, K, ctas));
-    if (pair_takes(bf16, transA, transB, batch, M, N) && (asks_for_pair(flags) || leaves_pair_open(flags))) {
-        const int clusters = (flags & BMB_GEMM_HALF_SMS) ? (pair_clusters() + 1) / 2 : pair_clusters();
-        if (leaves_pair_open(flags)) prefer_pair(&plan, flags, M, N, clusters);
-        else plan_pair(&plan, flags, M, N, clusters, 256);
-    }
+    const bool maybe_pair = pair_takes(bf16, transA, transB, batch, M, N) && (asks_for_pair(flags) || leaves_pair_open(flags));
+    const int clusters = !maybe_pair ? 0 : (flags & BMB_GEMM_HALF_SMS) ? (pair_clusters() + 1) / 2 : pair_clusters();
+    BMB_TRY(choose_plan(&plan, bf16, flags, transA, transB, batch, M, N, K, ctas, clusters));
     const bool a_rounded = (flags & BMB_GEMM_A_ROUNDED) != 0, b_rounded = (flags & BMB_GEMM_B_ROUNDED) != 0;
     const bool rnd = !bf16 && !aux_gelu && rounds_on_arrival(&plan, flags, transA, transB, batch, M, N, K, A, B, a_rounded, b_rounded, ctas);
     const int kblocks = plan.kblocks, bn = plan.bn, dp_tiles = plan.dp_tiles;
@@ -1472,23 +1483,12 @@ int gemm_tc(int math, int flags, int transA, int transB, int batch, int M, int N
 
 }  // namespace bmb
 
-// Host-side replay of the tile schedule a tensor-core GEMM of this shape would use on `ctas` SMs:
-// returns BMB_OK when the work items of all CTAs cover every (tile, K slice) exactly once, whole
-// tiles only where no tile is shared.  Runs no kernel; the CPU tests sweep shapes through it.
-extern "C" int bmb_gemm_schedule_check(int math, int flags, int batch, int M, int N, int K, int ctas, int *bm_out, int *bn_out,
-                                       int *dp_tiles_out, int *grid_out) {
-    using namespace bmb;
-    if (M < 1 || N < 1 || K < 1 || batch < 1 || ctas < 1) return fail(BMB_E_ARG, "schedule_check: bad argument");
-    Plan p;
-    BMB_TRY(plan_gemm(&p, math == BMB_MATH_BF16, flags, batch, M, N, K, ctas));
-    // the pair kernel's plan is replayed only when the call asks for it by flag (no device is consulted here):
-    // `ctas` then counts CTA pairs
-    if ((flags & BMB_GEMM_PAIR) && asks_for_pair(flags) && pair_takes(math == BMB_MATH_BF16, 0, 1, batch, M, N)) plan_pair(&p, flags, M, N, ctas, 256);
-    if (bm_out) *bm_out = p.mh * BM;
-    if (bn_out) *bn_out = p.bn;
-    if (dp_tiles_out) *dp_tiles_out = p.dp_tiles;
-    if (grid_out) *grid_out = p.grid;
-    if (p.grid < 1 || p.grid > ctas) return fail(BMB_E_LIMIT, "schedule_check: grid %d", p.grid);
+namespace {
+using namespace bmb;
+// BMB_OK when the work items of all `units` (CTAs, or CTA pairs) cover every (tile, K slice) exactly once, whole tiles only where no
+// tile is shared.
+int replay(const Plan &p, int units) {
+    if (p.grid < 1 || p.grid > units) return fail(BMB_E_LIMIT, "schedule_check: grid %d", p.grid);
     if ((long long)p.tiles * p.kblocks > (1LL << 28)) return fail(BMB_E_LIMIT, "schedule_check: problem too large to replay");
     std::vector<unsigned char> seen((size_t)p.tiles * p.kblocks, 0);
     for (int c = 0; c < p.grid; ++c) {
@@ -1507,6 +1507,33 @@ extern "C" int bmb_gemm_schedule_check(int math, int flags, int batch, int M, in
     for (size_t i = 0; i < seen.size(); ++i)
         if (!seen[i]) return fail(BMB_E_LIMIT, "schedule_check: tile %zu slice %zu never computed", i / p.kblocks, i % p.kblocks);
     return BMB_OK;
+}
+void tell(const Plan &p, int *bm_out, int *bn_out, int *dp_tiles_out, int *grid_out) {
+    if (bm_out) *bm_out = p.mh * BM;
+    if (bn_out) *bn_out = p.bn;
+    if (dp_tiles_out) *dp_tiles_out = p.dp_tiles;
+    if (grid_out) *grid_out = p.grid;
+}
+}  // namespace
+
+// Host-side replays of tile schedules.  They run no kernel; the CPU tests sweep shapes through them.
+extern "C" int bmb_gemm_schedule_check(int math, int flags, int batch, int M, int N, int K, int ctas, int *bm_out, int *bn_out,
+                                       int *dp_tiles_out, int *grid_out) {
+    if (M < 1 || N < 1 || K < 1 || batch < 1 || ctas < 1) return fail(BMB_E_ARG, "schedule_check: bad argument");
+    Plan p;
+    BMB_TRY(plan_gemm(&p, math == BMB_MATH_BF16, flags, batch, M, N, K, ctas));
+    if ((flags & BMB_GEMM_PAIR) && asks_for_pair(flags) && pair_takes(math == BMB_MATH_BF16, 0, 1, batch, M, N)) plan_pair(&p, flags, M, N, ctas, 256);
+    tell(p, bm_out, bn_out, dp_tiles_out, grid_out);
+    return replay(p, ctas);
+}
+extern "C" int bmb_gemm_plan_check(int math, int flags, int transA, int transB, int batch, int M, int N, int K, int ctas, int pairs, int *pair_out,
+                                   int *bm_out, int *bn_out, int *dp_tiles_out, int *grid_out) {
+    if (M < 1 || N < 1 || K < 1 || batch < 1 || ctas < 1 || pairs < 0) return fail(BMB_E_ARG, "plan_check: bad argument");
+    Plan p;
+    BMB_TRY(choose_plan(&p, math == BMB_MATH_BF16, flags, transA, transB, batch, M, N, K, ctas, pairs));
+    if (pair_out) *pair_out = p.pair ? 1 : 0;
+    tell(p, bm_out, bn_out, dp_tiles_out, grid_out);
+    return replay(p, p.pair ? pairs : ctas);
 }
 
 #ifdef BMB_GEMM_TRACE

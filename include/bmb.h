@@ -33,11 +33,18 @@ extern "C" {
 
 const char *bmb_last_error(void);
 const char *bmb_version(void);
-/* No counterpart in the reference.  Replays on the host the tile schedule a tensor-core GEMM of
- * this shape would use on `ctas` SMs (tile height and width, whole tiles, tiles shared along K) and returns 0
- * when every (tile, K slice) is computed exactly once.  Launches nothing; usable without a GPU. */
+/* No counterparts in the reference.  Both replay on the host a tile schedule of the tensor-core GEMM (tile height and
+ * width, whole tiles, tiles shared along K) and return 0 when every (tile, K slice) is computed exactly once.  They
+ * launch nothing and are usable without a GPU.
+ * bmb_gemm_plan_check: the schedule that a call with these flags takes on `ctas` SMs that hold `pairs` CTA pairs (74 on a
+ * B200; half of either with BMB_GEMM_HALF_SMS), *pair_out: whether it goes to pairs, which *grid_out then counts.  (A TF32
+ * product whose operands are rounded as they arrive may take 128-row tiles in its place.)
+ * bmb_gemm_schedule_check: the schedule on single CTAs, whatever a call of this shape takes; with BMB_GEMM_PAIR the one of
+ * 256 x 256 tiles on pairs, and `ctas` counts pairs. */
 int bmb_gemm_schedule_check(int math, int flags, int batch, int M, int N, int K, int ctas,
                             int *tile_m_out, int *tile_n_out, int *whole_tiles_out, int *grid_out);
+int bmb_gemm_plan_check(int math, int flags, int transA, int transB, int batch, int M, int N, int K, int ctas, int pairs, int *pair_out,
+                        int *tile_m_out, int *tile_n_out, int *whole_tiles_out, int *grid_out);
 /* Kernels this library has launched in this process so far (launches replayed from a CUDA
  * graph included).  No counterpart in the reference; bench.py reports it. */
 long long bmb_launch_count(void);
@@ -45,8 +52,9 @@ long long bmb_launch_count(void);
 /* ---- device-side waits that ran out ------------------------------------ */
 /* No counterparts in the reference.  Every wait inside the tensor-core kernels (on a copy, on the
  * tensor core, on another role of the CTA) is bounded; when one runs out the kernel drains what it
- * has in flight, returns, and leaves a nonzero word per device that makes every later tensor-core
- * call on that device return BMB_E_TIMEOUT.  bmb_kernel_status reads the word of the current device
+ * has in flight, returns, and leaves a nonzero word per device that makes every later call on that device
+ * which goes to such kernels return BMB_E_TIMEOUT: TF32 and BF16 products, large fp32 products, fused attention
+ * (fp32 of longer sequences included) and sampling in fp32.  bmb_kernel_status reads the word of the current device
  * (0 = nothing happened).  bmb_kernel_status_clear waits for the device to go idle and resets it,
  * so that a process can carry on after it has dealt with the failed step.
  * bmb_selftest_wait_expiry exercises that path without any fault: one CTA waits at most

@@ -131,8 +131,8 @@ def test_tensorcore_gemm_schedule_covers_every_slice_once(bmb):
                 st = lib.bmb_gemm_schedule_check(bmb.MATH_TF32, flags, 1, M, N, K, units, C.byref(bm), C.byref(bn), C.byref(dp), C.byref(grid))
                 assert st == 0, (M, N, K, units, flags, lib.bmb_last_error())
                 assert (bm.value, bn.value) == (256, 256) and 1 <= grid.value <= units
-    # a short K whose shared run would be a sizeable part of a CTA's work keeps its tiles whole (dX of the attention
-    # projection on half of the SMs: 192 tiles on 74 CTAs end in a partly filled wave instead); a long K is shared
+    # on single CTAs a short K whose shared run would be a sizeable part of a CTA's work keeps its tiles whole (192 tiles on
+    # 74 CTAs end in a partly filled wave instead); a long K is shared
     bm, bn, dp = C.c_int(), C.c_int(), C.c_int()
     assert lib.bmb_gemm_schedule_check(bmb.MATH_TF32, 0, 1, 8192, 768, 768, 74, C.byref(bm), C.byref(bn), C.byref(dp), None) == 0
     assert dp.value == -(-8192 // bm.value) * -(-768 // bn.value)
@@ -143,6 +143,47 @@ def test_tensorcore_gemm_schedule_covers_every_slice_once(bmb):
             bm = C.c_int()
             assert lib.bmb_gemm_schedule_check(bmb.MATH_TF32, flags, 1, M, N, K, 148, C.byref(bm), None, None, None) == 0
             assert bm.value == want
+
+
+def gemm_plan(bmb, math, M, N, K, ctas=148, pairs=74, flags=0, ta=0, tb=1):
+    import ctypes as C
+    out = [C.c_int() for _ in range(5)]
+    lib = bmb.lib()
+    assert lib.bmb_gemm_plan_check(math, flags, ta, tb, 1, M, N, K, ctas, pairs, *[C.byref(x) for x in out]) == 0, (M, N, K, lib.bmb_last_error())
+    return tuple(x.value for x in out)                # on pairs, tile height, width, whole tiles, CTAs or pairs
+
+
+def test_tensorcore_plans_taken_by_default(bmb):
+    """The plans that calls take with nothing forced: which products go to CTA pairs, how wide, and that every (tile, K slice) of any of
+    them is computed once, on whole and half GPUs and with fewer pairs than SMs would hold."""
+    import random
+    T, B = bmb.MATH_TF32, bmb.MATH_BF16
+    pairs = {(T, 4096, 4096, 4096): 256, (T, 8192, 2304, 768): 256, (T, 8192, 3072, 768): 192, (T, 8192, 768, 768): 192, (T, 8192, 50304, 768): 256,
+             (B, 6144, 6144, 6144): 256, (B, 8192, 50304, 768): 256, (T, 4000, 3000, 1300): 256, (B, 4000, 3000, 1300): 256, (T, 2048, 2112, 2080): 256}
+    for shape, width in pairs.items():
+        assert gemm_plan(bmb, *shape)[:3] == (1, 256, width), shape
+        assert gemm_plan(bmb, *shape, flags=bmb.GEMM_NO_PAIR)[0] == 0 and gemm_plan(bmb, *shape, pairs=0)[0] == 0
+    for shape in ((T, 1024, 1024, 1024), (B, 1024, 1024, 1024), (T, 512, 512, 6144), (T, 50304, 768, 8192), (T, 8192, 768, 50304), (B, 4096, 4096, 512)):
+        assert gemm_plan(bmb, *shape)[0] == 0, shape
+    # half of the SMs: the two gradients of a linear layer side by side
+    for M, N, K, width in ((8192, 768, 768, 256), (2304, 768, 8192, 192), (3072, 768, 8192, 256)):
+        assert gemm_plan(bmb, T, M, N, K, 74, 37, bmb.GEMM_HALF_SMS)[:3] == (1, 256, width), (M, N, K)
+    # an M- or N-contiguous TF32 operand whose extent is no multiple of 32 is not for pairs; BF16 operands are copied anyway
+    assert gemm_plan(bmb, T, 4100, 4096, 4096, ta=1)[0] == 0 and gemm_plan(bmb, T, 4096, 4100, 4096, tb=0)[0] == 0
+    assert gemm_plan(bmb, B, 4100, 4096, 4096, ta=1)[0] == 1
+    # a short K keeps its tiles whole, a long one shares the last wave's
+    assert gemm_plan(bmb, T, 4096, 4096, 512)[3] == 256 and gemm_plan(bmb, T, 4096, 4096, 4096)[3] == 222
+    rng = random.Random(5)
+    seen = set()
+    for _ in range(150):
+        M, N, K = (rng.randrange(256, 6000) for _ in range(3))
+        for math in (T, B):
+            for ctas, npairs, flags in ((148, 74, 0), (148, 74, bmb.GEMM_NO_SPLIT), (74, 37, bmb.GEMM_HALF_SMS), (148, 66, 0), (7, 3, 0)):
+                pair, bm, bn, whole, grid = gemm_plan(bmb, math, M, N, K, ctas, npairs, flags)
+                tiles = -(-M // bm) * -(-N // bn)
+                assert whole <= tiles and (not flags & bmb.GEMM_NO_SPLIT or whole == tiles) and 1 <= grid <= (npairs if pair else ctas)
+                seen.add((pair, bn, whole < tiles))
+    assert {(1, 256, False), (1, 256, True), (1, 192, False), (1, 192, True)} <= seen
 
 
 def test_checkpoint_header_reads_the_gpt1_layout(bmb, tmp_path):
