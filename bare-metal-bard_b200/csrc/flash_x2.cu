@@ -16,10 +16,10 @@
 // back with the factor that unscales the sums (CUT), and sums over positions leave tensor memory every 64 positions for
 // fp32 registers.
 //
-// What two pieces cannot serve is left to the kernels of flash.cu, which run behind these and skip every head that has none of
-// it: 64 rows whose largest element is not in 2^-45 .. 2^30 (nor zero) or not finite, a row or column whose largest element is below
-// 2^-20 of that (and not zero; of V and dO in the backward, a row below 2^-12), D beyond 2^70, lse beyond 2^19, a row's largest score beyond 2^22 (MOST_SCORE), a probability beyond
-// sqrt(2) (of an lse that is not the scores').  Inside these limits no sum can overflow.
+// What two pieces cannot serve is left to the kernels of flash.cu, which run behind these for the heads that have any of it: 64 rows
+// whose largest element is not in 2^-45 .. 2^30 (nor zero) or not finite, a row or column whose largest element is below 2^-20 of that
+// (and not zero; of V in the backward, a row below 2^-12), D beyond 2^70, lse beyond 2^19, a row's largest score beyond 2^22
+// (MOST_SCORE), a probability beyond sqrt(2) (of an lse that is not the scores').  Inside these limits no sum can overflow.
 //
 // Bound by what a step of 64 columns waits for in turn (products, exponentials and splits, sums) and by the FMA pipe, on which
 // the splits and exponentials of 128 x 64 elements are 1000 to 1400 cycles; products 2600 (64 columns, keys' side).  Four
@@ -185,9 +185,11 @@ __global__ void __launch_bounds__(256, HS == 32 ? 5 : HS == 64 ? 4 : 2) split_x2
     bool bad = lost || (most != 0.0f && !usable);
     // Rows and columns of the block against its largest element: products sum along both, and hold 2^-31 of a row's or column's largest
     // element where that is 2^-20 of the block's.
-    // (In V and dO of a backward rows from 2^-12 on: dS of a block's 64 columns has one scale, so what belongs to a column's small
-    // row loses bits where the columns of large ones have hardly any weight.)
-    const float low_end = 9.5367432e-7f * most, low_row = nw == 4 && which >= 2 ? 2.44140625e-4f * most : low_end;
+    // (In V of a backward rows from 2^-12 on: dS of a row has one scale for a block's 64 keys, so what belongs to small rows of V loses bits
+    // where the large ones have hardly any weight.  The same of dO would be a rule for its time alone: gradients of single positions fall
+    // below 2^-12 of their neighbours' as soon as a model is sure of some of them, and with that rule 10 % and more of a character model's
+    // step went to the kernels behind; a key that only such positions look at has its dK to 2^-42 of what a large one could give.)
+    const float low_end = 9.5367432e-7f * most, low_row = nw == 4 && which == 2 ? 2.44140625e-4f * most : low_end;
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) bad = bad || (rowmax[i] != 0.0f && rowmax[i] < low_row);
     const int e = usable ? exponent(most) : 14;
