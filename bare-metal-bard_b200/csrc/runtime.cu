@@ -176,8 +176,8 @@ namespace {
 struct CallBlock {
     void *p = nullptr;
     size_t cap = 0;
-    cudaEvent_t done = nullptr;      // behind its last use, on `last`
-    cudaStream_t last = nullptr;
+    cudaEvent_t done = nullptr;      // behind its last use, which `user`'s stream had
+    const void *user = nullptr;
     bool taken = false;              // a call is making its launches
     unsigned long long when = 0;
 };
@@ -201,6 +201,8 @@ bool drop_block(CallBlocks &all, CallBlock &b) {
 void *call_scratch(size_t bytes, cudaStream_t st) {
     const int d = current_device();
     if (d < 0 || d >= 64) return nullptr;
+    static thread_local char thread;         // (cudaStreamPerThread is one handle for a stream of each thread)
+    const void *user = st == cudaStreamPerThread ? (const void *)&thread : (const void *)st;
     RelaxedCapture relaxed;
     std::lock_guard<std::mutex> lk(g_call_mu);
     CallBlocks &all = g_call_blocks[d];
@@ -210,7 +212,7 @@ void *call_scratch(size_t bytes, cudaStream_t st) {
         if (b.taken) continue;
         if (!b.p) { empty = &b; continue; }
         if (b.cap < bytes) continue;
-        if (b.last == st) { if (!mine || b.cap < mine->cap) mine = &b; }
+        if (b.user == user) { if (!mine || b.cap < mine->cap) mine = &b; }
         else if (!oldest || b.when < oldest->when) oldest = &b;
     }
     if (!mine && oldest) {
@@ -236,7 +238,7 @@ void *call_scratch(size_t bytes, cudaStream_t st) {
         if (cudaStreamWaitEvent(st, use->done, 0) != cudaSuccess) { cudaGetLastError(); return nullptr; }
     }
     use->taken = true;
-    use->last = st;
+    use->user = user;
     use->when = ++all.uses;
     return use->p;
 }

@@ -275,3 +275,35 @@ def test_calls_on_several_streams(bmb, cuda):
         bmb.lib().bmb_set_stream(None)
     cuda.cuda.synchronize()
     assert all(cuda.equal(x, y) for g, w in zip(got, want) for x, y in zip(g, w))
+
+
+def test_calls_of_several_threads(bmb, cuda):
+    """Four threads, each with its stream of the one handle cudaStreamPerThread, on blocks of several sizes: what each gives by itself."""
+    import threading
+    shapes = [(1, 512, 4, 64), (2, 777, 12, 32), (1, 1024, 8, 128), (4, 1024, 12, 64)]
+    data = [inputs(cuda, *shape, i) for i, shape in enumerate(shapes)]
+    want = [attention(bmb, cuda, 0, qkv, dout, shape[2]) for shape, (qkv, dout) in zip(shapes, data)]
+    got = [[cuda.full_like(x, float("nan")) for x in w] for w in want]
+    cuda.cuda.synchronize()
+    failed = []
+
+    def work(i):
+        (B, T, NH, hs), (qkv, dout), (out, lse, dsum, dqkv) = shapes[i], data[i], got[i]
+        try:
+            bmb.lib().bmb_set_stream(2)                # cudaStreamPerThread
+            for _ in range(20):
+                bmb.call("bmb_flash_attention_forward_cfg", 0, out, lse, qkv, B, T, NH * hs, NH)
+                bmb.call("bmb_flash_attention_backward_cfg", 0, dqkv, dsum, dout, qkv, out, lse, B, T, NH * hs, NH)
+        except Exception as e:
+            failed.append(e)
+        finally:
+            bmb.lib().bmb_set_stream(None)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    cuda.cuda.synchronize()
+    assert not failed
+    assert all(cuda.equal(x, y) for g, w in zip(got, want) for x, y in zip(g, w))
