@@ -6,8 +6,8 @@
 // hi and lo hold 22 to 23 bits of x; a b is hi hi + 2^-11 (hi lo + lo hi) up to 2^-22 of |a b|.  The products of the small
 // pieces come first and are scaled by 2^-11 by the first instruction that adds products of the large ones (scale-input-d), so
 // one accumulator serves all.  Elements down to 2^-28 of the largest of their 64 rows keep all bits that hi and lo have, smaller
-// ones are held to 2^-51 of it, which is 2^-31 of the largest in their row or column (see below).  Probabilities and dS are split in registers, scaled by the
-// most that they can be.
+// ones are held to 2^-51 of it, which is 2^-31 of the largest in their row or column (see below).  Probabilities and dS are split in
+// registers, scaled by the most that they can be, and so are held to 2^-45 (forward) or 2^-50 (backward) of a weight of 1.
 // Why fp16 and not bf16 or TF32: at the same accuracy bf16 takes six products, TF32 three at half the rate and twice the
 // bytes in shared memory, which is what bounds the 64-column products below (69 cycles with both operands there, 40 with
 // one in tensor memory, 32 by the pipe's rate).
@@ -25,7 +25,7 @@
 // the splits and exponentials of 128 x 64 elements are 1000 to 1400 cycles; products 2600 (64 columns, keys' side).  Four
 // warpgroups compute: with two, as with longer pieces of a row in registers, the step was no faster (12.5 KB of code a loop instead
 // of 35 and 16 columns at a time count for more).  us, the kernels of flash.cu -> these, split pass included: B8 T1024 12 heads of
-// 64 forward 253 -> 123, backward 958 -> 264; B4 T2048 8 x 128 664 -> 211, 2490 -> 627; B2 T777 12 x 32 41 -> 36, 105 -> 50.
+// 64 forward 253 -> 123, backward 958 -> 283; B4 T2048 8 x 128 664 -> 211, 2490 -> 649; B2 T777 12 x 32 41 -> 31, 105 -> 47.
 // 2-norm errors against 64 bits there: 8 x 160 x 4 heads of 64 and up, output 0.95 to 1.0 of those kernels', lse 0.7, dqkv 0.82 to 1.0.
 #include "tc_common.cuh"
 #include <cuda_fp16.h>
@@ -38,7 +38,7 @@ namespace bmb {
 // flash.cu: the kernels on warp-level instructions, for the heads left out here.
 int flash_fwd_left(int hs, float *out, float *lse, const float *qkv, int T, int NH, float scale, LeftOut left, cudaStream_t st);
 int flash_bwd_left(int hs, float *dqkv, const float *dsum, const float *dout, const float *qkv, const float *lse, int T, int NH, float scale,
-                      LeftOut left, cudaStream_t st);
+                   LeftOut left, cudaStream_t st);
 namespace {
 
 using namespace tc;
@@ -702,7 +702,7 @@ flash_fwd_x2_k(float *__restrict__ out, float *__restrict__ lse, const Images im
             top = fmaxf(top, at[(half ^ 1) * 128]) * c;      // key 0 is visible to every row: finite in step 0
             // The reference of the exponentials, a whole number two below the maximum (where most of a row's weight is, exponents
             // are small and rounded little), follows it in jumps of more than 2^4, so most steps rescale nothing.  Weights are
-            // 2^9 times their exponentials: at most 2^15.
+            // 2^9 times their exponentials: at most 2^15, and a quarter more where scores are large (MOST_SCORE).
             float alpha = 1.0f;
             if (e == 0) {
                 m = ceilf(top) - 2.0f;
